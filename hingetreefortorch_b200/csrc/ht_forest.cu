@@ -7,6 +7,7 @@
 #include <atomic>
 
 #include "ht_common.cuh"
+#include "ht_forest_multi.cuh"
 #include "ht_forest_tiled.cuh"
 
 namespace ht {
@@ -436,13 +437,18 @@ const char *ht_status_string(int status) {
 }
 
 int ht_forest_forward_saves(const ht_forest_problem *p) {
-  return check_forest_problem(p) == HT_OK && forward_saves(p) ? 1 : 0;
+  return check_forest_problem(p) == HT_OK && (forward_saves(p) || multi_area_bytes(p, sizeof(float)) > 0) ? 1 : 0;
+}
+
+// What a backward keeps per evaluation: the records of the tile kernels (one output per leaf) or the paths (several).
+static size_t records_bytes(const ht_forest_problem *p) {
+  return p->M > 1 ? multi_area_bytes(p, sizeof(float)) : backward_records_bytes(p);
 }
 
 size_t ht_forest_workspace_bytes(const ht_forest_problem *p) {
   if (check_forest_problem(p) != HT_OK) return 0;
   const size_t base = ordinals_bytes(p) + forward_tiled_workspace_bytes(p) + 256;
-  return (p->flags & HT_WORKSPACE_FOR_BACKWARD) != 0 ? base + backward_records_bytes(p) : base;
+  return (p->flags & HT_WORKSPACE_FOR_BACKWARD) != 0 ? base + records_bytes(p) : base;
 }
 
 int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const float *thr, const int64_t *ord,
@@ -456,12 +462,16 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
   // HT_SAVE_FOR_BACKWARD: the traversal goes to the evaluation-record area of the workspace, when it is there
   unsigned char *ws = static_cast<unsigned char *>(workspace);
   void *eval_records = nullptr;
-  if ((p->flags & HT_SAVE_FOR_BACKWARD) != 0 && forward_saves(p)) {
+  if ((p->flags & HT_SAVE_FOR_BACKWARD) != 0 && ht_forest_forward_saves(p)) {
     const size_t records_at = ordinals_bytes(p) + forward_tiled_workspace_bytes(p);
-    if (workspace_bytes >= records_at + backward_records_bytes(p)) eval_records = ws + records_at;
+    if (workspace_bytes >= records_at + records_bytes(p)) eval_records = ws + records_at;
   }
   const int trc = forward_tiled(p, x, thr, pr.args.ord, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
   if (trc != HT_ERR_UNSUPPORTED) return trc;
+  if (p->M > 1) {
+    const int mrc = multi_forward(p, x, thr, pr.args.ord, w, out, eval_records, pr.stream);
+    if (mrc != HT_ERR_UNSUPPORTED) return mrc;
+  }
   return launch_any<MODE_FORWARD>(p, pr, out, nullptr);
 }
 
@@ -517,9 +527,9 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
     // they serve both modes (that path is fixed-order), without it only the default mode.
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     const size_t records_at = ordinals_bytes(p) + forward_tiled_workspace_bytes(p);
-    const size_t eval_bytes = backward_records_bytes(p);
+    const size_t eval_bytes = records_bytes(p);
     void *eval_records = eval_bytes > 0 && workspace_bytes >= records_at + eval_bytes ? ws + records_at : nullptr;
-    if ((p->flags & HT_SAVED_FORWARD) != 0 && eval_records != nullptr) {
+    if ((p->flags & HT_SAVED_FORWARD) != 0 && eval_records != nullptr && p->M == 1) {
       // the records of the forward that ran on these inputs are still there: no tree is walked again
       const int src = backward_saved(p, a.ord, w, g, gx, gthr, gw, eval_records, pr.stream);
       if (src != HT_ERR_UNSUPPORTED) return src;
@@ -529,9 +539,16 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
     const int trc = backward_tiled(p, x, thr, a.ord, w, g, gx, gthr, gw, ws + ordinals_bytes(p), eval_records,
                                    status_word, pr.stream);
     if (trc != HT_ERR_UNSUPPORTED) return trc;
-    const int mrc = backward_tiled_multi(p, x, thr, a.ord, w, g, gx, gthr, gw, ws + ordinals_bytes(p),
-                                         forward_tiled_workspace_bytes(p), status_word, pr.stream);
-    if (mrc != HT_ERR_UNSUPPORTED) return mrc;
+    if (p->M > 1 && eval_records != nullptr && (p->flags & HT_DETERMINISTIC) == 0) {
+      if ((p->flags & HT_SAVED_FORWARD) == 0) {  // nothing was kept: the paths first
+        float *none = nullptr;
+        int prc = forward_tiled(p, x, thr, a.ord, w, none, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
+        if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, eval_records, pr.stream);
+        if (prc != HT_OK) return prc;
+      }
+      const int mrc = backward_multi(p, a.ord, w, g, gx, gthr, gw, eval_records, pr.stream);
+      if (mrc != HT_ERR_UNSUPPORTED) return mrc;
+    }
   }
   return backward_any(p, pr, g, gx, gthr, gw);
 }

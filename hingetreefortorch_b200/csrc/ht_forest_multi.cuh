@@ -1,0 +1,38 @@
+// Several outputs per leaf: forward that leaves its paths, and the backward that sorts them (ht_forest_multi.cu).
+#pragma once
+
+#include "ht_common.cuh"
+#include "ht_eval_records.cuh"
+
+namespace ht {
+
+// Whether the kernels of ht_forest_multi.cu take the backward of this problem (any number of inner positions, several
+// outputs per leaf), given a scratch area of multi_area_bytes() bytes for the paths.
+bool multi_takes(const ht_forest_problem *p, size_t real_bytes);
+size_t multi_area_bytes(const ht_forest_problem *p, size_t real_bytes);
+
+// The paths of all evaluations inside that area: threshold - feature at the deciding vertex, and the deciding vertex
+// with the leaf key, in the layout of the evaluation records.
+template <typename Real>
+struct PathRecordsOf {
+  Real *margin;
+  void *where;  // 8 + 8 bits up to depth 8, 16 + 16 beyond
+};
+template <typename Real>
+PathRecordsOf<Real> multi_paths(const ht_forest_problem *p, void *area) {
+  unsigned char *base = static_cast<unsigned char *>(area);
+  return PathRecordsOf<Real>{reinterpret_cast<Real *>(base), base + record_array_bytes(p, sizeof(Real))};
+}
+
+// Forward of any shape with the results of a warp written together; with `area` it also leaves the paths there, and
+// with out == nullptr it leaves nothing else.  HT_ERR_UNSUPPORTED: nothing was launched.
+template <typename Real>
+int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, const int32_t *ord, const Real *w, Real *out,
+                  void *area, cudaStream_t stream);
+
+// Gradients from the paths in `area`.  The gradients that are asked for (the others are null) must have been cleared.
+template <typename Real>
+int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w, const Real *g, Real *gx, Real *gthr,
+                   Real *gw, void *area, cudaStream_t stream);
+
+}  // namespace ht

@@ -36,6 +36,7 @@
 // go left, as `margin > 0` does in the reference).  |threshold - feature| equals
 // |feature - threshold| bit for bit.
 #include "ht_eval_records.cuh"
+#include "ht_forest_multi.cuh"
 #include "ht_forest_tiled.cuh"
 #include "ht_tile_common.cuh"
 #include "ht_tma.cuh"
@@ -386,33 +387,56 @@ __global__ void __launch_bounds__(kThreads, 1) forest_forward_tiled_kernel(const
     const int t_first = slot * per_warp;  // this warp's consecutive trees inside the group
     float result[4] = {0.f, 0.f, 0.f, 0.f};
     uint32_t path[4] = {kL, kL, kL, kL};
+    // SAVE with several outputs per leaf; after a lost copy the paths are those of a zero margin at the root
+    [[maybe_unused]] Walked wk[4] = {{0.f, 1u, kL}, {0.f, 1u, kL}, {0.f, 1u, kL}, {0.f, 1u, kL}};
     if (t_first < in_group && !poisoned) {  // after a lost copy the buffer is not read: zeros leave instead
       // trees beyond the end of a short last group repeat the last valid one (results unused)
-      if (per_warp == 4) {
-        uint32_t rec[4];
+      auto walk_trees = [&](auto trees) {
+        constexpr int n = decltype(trees)::value;
+        uint32_t rec[n], p[n];
+        float r[n];
 #pragma unroll
-        for (int u = 0; u < 4; ++u)
+        for (int u = 0; u < n; ++u)
           rec[u] = base_addr + (uint32_t)(in_group == G ? t_first + u : min(t_first + u, in_group - 1)) * lay.bytes;
-        walk<KIND, DEPTH, OrdT, 4, WREC>(rec, xl_addr, x_stride, result, path);
-      } else if (per_warp == 2) {
-        uint32_t rec[2], p2[2];
+        if constexpr (SAVE && !WREC) {
+          Walked found[n];
+          walk_full<KIND, DEPTH, OrdT, n, lay.paired>(rec, xl_addr, x_stride, found);
 #pragma unroll
-        for (int u = 0; u < 2; ++u) rec[u] = base_addr + (uint32_t)min(t_first + u, in_group - 1) * lay.bytes;
-        float r2[2];
-        walk<KIND, DEPTH, OrdT, 2, WREC>(rec, xl_addr, x_stride, r2, p2);
-        result[0] = r2[0];
-        result[1] = r2[1];
-        path[0] = p2[0];
-        path[1] = p2[1];
-      } else {
-        uint32_t rec[1] = {base_addr + (uint32_t)t_first * lay.bytes}, p1[1];
-        float r1[1];
-        walk<KIND, DEPTH, OrdT, 1, WREC>(rec, xl_addr, x_stride, r1, p1);
-        result[0] = r1[0];
-        path[0] = p1[0];
-      }
+          for (int u = 0; u < n; ++u) {
+            wk[u] = found[u];
+            r[u] = fabsf(found[u].nm);
+            p[u] = found[u].path;
+          }
+        } else {
+          walk<KIND, DEPTH, OrdT, n, WREC>(rec, xl_addr, x_stride, r, p);
+        }
+#pragma unroll
+        for (int u = 0; u < n; ++u) {
+          result[u] = r[u];
+          path[u] = p[u];
+        }
+      };
+      if (per_warp == 4)
+        walk_trees(std::integral_constant<int, 4>{});
+      else if (per_warp == 2)
+        walk_trees(std::integral_constant<int, 2>{});
+      else
+        walk_trees(std::integral_constant<int, 1>{});
     }
     done_with_buffer(it);
+    if constexpr (SAVE && !WREC) {
+      using WhereT = typename std::conditional<(DEPTH <= 8), unsigned short, uint32_t>::type;
+      const int64_t sample = row0 + sample_group * 32 + lane;
+      const int64_t at = record_index(sample, (int64_t)group * G + t_first, a.T);
+      if (sample < a.B) {
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (u < per_warp && t_first + u < in_group) {
+            a.save_margin[at + u * kRecordBlock] = wk[u].nm;
+            store_where<WhereT>(a.save_where, at + u * kRecordBlock, wk[u].v, __brev(wk[u].path - kL) >> (32 - DEPTH));
+          }
+      }
+    }
 
     const int64_t col0 = (int64_t)group * G;
     if (!WREC) {
@@ -428,7 +452,7 @@ __global__ void __launch_bounds__(kThreads, 1) forest_forward_tiled_kernel(const
       for (int u = 0; u < 4; ++u)
         pairs[lane * 4 + u] = make_float2(result[u], __uint_as_float(__brev(path[u] - kL) >> (32 - DEPTH)));
       __syncwarp();
-      if (trees_here > 0) {
+      if (trees_here > 0 && (!SAVE || a.out != nullptr)) {
         const int run = trees_here * M;  // outputs of one sample that this warp owns, contiguous
         const int64_t first_row = row0 + sample_group * 32;
         const int rows_here = (int)min((int64_t)32, a.B - first_row);
@@ -621,8 +645,10 @@ int launch_depth(const TilePlan &plan, const TiledArgs &a, dim3 grid, cudaStream
   const bool wrec = a.M == 1;
   if (a.save_margin != nullptr) {
     if (plan.ord_bytes == 1)
-      return launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint8_t, true, true>, plan, a, grid, stream);
-    return launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint16_t, true, true>, plan, a, grid, stream);
+      return wrec ? launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint8_t, true, true>, plan, a, grid, stream)
+                  : launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint8_t, false, true>, plan, a, grid, stream);
+    return wrec ? launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint16_t, true, true>, plan, a, grid, stream)
+                : launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint16_t, false, true>, plan, a, grid, stream);
   }
   if (plan.ord_bytes == 1)
     return wrec ? launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint8_t, true>, plan, a, grid, stream)
@@ -705,7 +731,11 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
   a.per_warp = plan.per_warp;
   a.save_margin = nullptr;
   a.save_where = nullptr;
-  if (eval_records != nullptr && forward_saves(p)) {
+  if (eval_records != nullptr && p->M > 1) {
+    const PathRecordsOf<float> paths = multi_paths<float>(p, eval_records);
+    a.save_margin = paths.margin;
+    a.save_where = paths.where;
+  } else if (eval_records != nullptr && forward_saves(p)) {
     const EvalRecords saved = eval_record_arrays(p, eval_records);
     a.save_margin = saved.dx;
     a.save_where = saved.where;

@@ -14,7 +14,8 @@ size_t forward_tiled_workspace_bytes(const ht_forest_problem *p);
 // scratch of forward_tiled_workspace_bytes() bytes.
 // With `eval_records` (backward_records_bytes() bytes) and a problem for which forward_saves() holds, the forward
 // also leaves its traversal there: the signed margin and the deciding vertex / leaf of every evaluation, from which
-// backward_saved() computes the gradients without walking the trees again.
+// backward_saved() computes the gradients without walking the trees again.  Several outputs per leaf: `eval_records` is
+// the paths' area of ht_forest_multi.cuh (every shape), and with out == nullptr nothing but the paths is written.
 bool forward_saves(const ht_forest_problem *p);
 int saved_samples_per_cta(const ht_forest_problem *p);  // 0: the backward from saved records does not take the shape
 int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w,
@@ -36,12 +37,5 @@ size_t backward_records_bytes(const ht_forest_problem *p);
 int backward_tiled(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w,
                    const float *g, float *gx, float *gthr, float *gw, void *records, void *eval_records,
                    uint32_t *status_word, cudaStream_t stream);
-
-// Backward for several outputs per leaf (default mode, tabular input) with the tile kernel of
-// ht_forest_tiled_bwd_multi.cu; same contract as backward_tiled without evaluation records.
-// `records` is scratch of `records_bytes` bytes (the forward's record area is large enough).
-int backward_tiled_multi(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w,
-                         const float *g, float *gx, float *gthr, float *gw, void *records, size_t records_bytes,
-                         uint32_t *status_word, cudaStream_t stream);
 
 }  // namespace ht

@@ -1,0 +1,53 @@
+"""Several outputs per leaf: rows of every width the kernels distinguish, tiles of evaluations that end anywhere, inner
+positions, both ways to the paths (kept by the forward, or walked again)."""
+import numpy as np
+import pytest
+
+import hingetreefortorch_b200._cabi as _cabi
+from conftest import grad_close
+from oracle import hinge_oracle as ho
+from test_forest_gpu import dev, random_forest_inputs
+
+pytestmark = pytest.mark.gpu
+
+# B, C, inner, T, depth, M: evaluations per tree around multiples of 1024; pieces of one, two and four numbers per row, up
+# to one lane, half a warp and a whole warp of them; one level and twelve
+SHAPES = [
+    (1025, 9, (), 40, 3, 2),
+    (1024, 300, (), 33, 4, 3),
+    (2047, 20, (), 17, 12, 4),
+    (1500, 8, (), 30, 1, 5),
+    (300, 31, (7,), 21, 6, 6),
+    (999, 16, (), 37, 9, 7),
+    (3, 50, (41, 25), 12, 5, 8),
+    (1100, 40, (), 31, 10, 10),
+    (1, 12, (1023,), 35, 7, 17),
+    (2100, 64, (), 16, 8, 26),
+    (513, 11, (2,), 33, 4, 33),
+    (5, 16, (900,), 9, 11, 63),
+    (2, 100, (24, 24), 30, 7, 64),
+]
+
+
+@pytest.mark.parametrize("kind", ["tree", "fern"])
+@pytest.mark.parametrize("shape", SHAPES, ids=[str(s) for s in SHAPES])
+def test_forward_and_backward(kind, shape):
+    B, C, inner, T, depth, M = shape
+    x, thr, ord_, w = random_forest_inputs(300 + SHAPES.index(shape), kind, B, C, inner, T, depth, (M,), quantise=True)
+    want = ho.forward(kind, x, thr, ord_, w)
+    g = np.random.default_rng(5).standard_normal(want.shape).astype(np.float32)
+    ref = ho.backward(kind, x, thr, ord_, w, g)
+    sizes = ho.backward_magnitudes(kind, x, thr, ord_, w, g)
+    dx, dthr, dord, dw, dg = dev(x, thr, ord_, w, g)
+    f = _cabi.Forest(kind, dx, dw)
+    for got, r, s in zip(f.backward(dx, dthr, dord, dw, dg), ref, sizes):
+        assert grad_close(got, r, s)
+    only_thr = f.backward(dx, dthr, dord, dw, dg, need=(False, True, False))
+    assert only_thr[0] is None and grad_close(only_thr[1], ref[1], sizes[1]) and only_thr[2] is None
+    assert np.array_equal(f.forward(dx, dthr, dord, dw, save=True).cpu().numpy(), want)
+    for got, r, s in zip(f.backward(dx, dthr, dord, dw, dg, saved=True), ref, sizes):
+        assert grad_close(got, r, s)
+    x.reshape(-1)[:3] = [np.inf, -np.inf, np.nan]
+    got = f.forward(dev(x)[0], dthr, dord, dw).cpu().numpy()
+    assert np.array_equal(got, ho.forward(kind, x, thr, ord_, w), equal_nan=True)
+    assert f.ordinal_flags() == 0
