@@ -361,6 +361,7 @@ std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torc
     return {forest_forward(kind, x, thr, ord, w), torch::empty({0}, x.options().dtype(torch::kUInt8))};
   ForestCall call(kind, x, thr, ord, w, nullptr);
   c10::DeviceGuard guard(x.device());
+  if (at::globalContext().deterministicAlgorithms()) call.problem.flags |= HT_DETERMINISTIC;  // the scratch its backward needs
   const bool saves = g_save_forward && ht_forest_forward_saves(&call.problem) != 0;
   if (saves) call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD | HT_SAVE_FOR_BACKWARD;
   if (saves && (int64_t)ht_forest_workspace_bytes(&call.problem) > g_backward_scratch_limit)
@@ -394,6 +395,9 @@ std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, t
   if (!need_x && !need_thr && !need_w) return grads;
   if (deterministic) call.problem.flags |= HT_DETERMINISTIC;
   call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD | HT_SAVED_FORWARD;
+  if (saved.defined() && deterministic && (size_t)saved.numel() < ht_forest_workspace_bytes(&call.problem))
+    // the mode was switched on after the forward, which kept less than the fixed order needs
+    return forest_backward(kind, deterministic, x, need_x, thr, need_thr, ord, need_ord, w, need_w, g);
   if (!saved.defined() || saved.device() != x.device() || saved.scalar_type() != torch::kUInt8 ||
       (size_t)saved.numel() < ht_forest_workspace_bytes(&call.problem) || ht_forest_forward_saves(&call.problem) == 0)
     bad_argument("Error: `saved` is not the scratch a saving forward returned for these tensors.");

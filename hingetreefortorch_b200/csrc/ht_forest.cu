@@ -436,13 +436,34 @@ const char *ht_status_string(int status) {
   }
 }
 
-int ht_forest_forward_saves(const ht_forest_problem *p) {
-  return check_forest_problem(p) == HT_OK && (forward_saves(p) || multi_area_bytes(p, sizeof(float)) > 0) ? 1 : 0;
+// The paths that a forward leaves for the backward: arrays of the tile kernels' records (one output per leaf, where those
+// kernels take the problem), or arrays of their own.
+static size_t saved_bytes(const ht_forest_problem *p) {
+  const size_t records = p->M == 1 ? backward_records_bytes(p) : 0;
+  return records > 0 ? records : path_bytes(p, sizeof(float));
+}
+static PathRecordsOf<float> saved_paths(const ht_forest_problem *p, void *area) {
+  if (p->M > 1 || backward_records_bytes(p) == 0) return multi_paths<float>(p, area);
+  const EvalRecords records = eval_record_arrays(p, area);
+  return {records.dx, records.where};
 }
 
-// What a backward keeps per evaluation: the records of the tile kernels (one output per leaf) or the paths (several).
+// Whether the fixed-order parameter gradients come from sorted paths.  The lists take 16 bytes per evaluation, which
+// stops being worth its memory with one output per leaf and so many evaluations that the trees alone fill the machine.
+static bool ordered_from_paths(const ht_forest_problem *p) {
+  return (p->flags & HT_DETERMINISTIC) != 0 && (p->M > 1 || p->B * p->T * p->K <= (1 << 26)) && ordered_list_bytes(p, sizeof(float)) > 0;
+}
+
+// What a backward keeps per evaluation: the records of the tile kernels (one output per leaf), or the paths (several) and,
+// in fixed-order mode, their lists.
 static size_t records_bytes(const ht_forest_problem *p) {
+  if (ordered_from_paths(p)) return saved_bytes(p) + ordered_list_bytes(p, sizeof(float));
   return p->M > 1 ? multi_area_bytes(p, sizeof(float)) : backward_records_bytes(p);
+}
+
+int ht_forest_forward_saves(const ht_forest_problem *p) {
+  if (check_forest_problem(p) != HT_OK) return 0;
+  return p->M == 1 ? forward_saves(p) : records_bytes(p) > 0;
 }
 
 size_t ht_forest_workspace_bytes(const ht_forest_problem *p) {
@@ -468,9 +489,10 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
   }
   const int trc = forward_tiled(p, x, thr, pr.args.ord, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
   if (trc != HT_ERR_UNSUPPORTED) return trc;
-  if (p->M > 1) {
-    const int mrc = multi_forward(p, x, thr, pr.args.ord, w, out, eval_records, pr.stream);
-    if (mrc != HT_ERR_UNSUPPORTED) return mrc;
+  if (p->M > 1 || eval_records != nullptr) {
+    const PathRecordsOf<float> paths = eval_records != nullptr ? saved_paths(p, eval_records) : PathRecordsOf<float>{nullptr, nullptr};
+    const int mrc = multi_forward(p, x, thr, pr.args.ord, w, out, paths, pr.stream);
+    if (mrc != HT_ERR_UNSUPPORTED || eval_records != nullptr) return mrc;
   }
   return launch_any<MODE_FORWARD>(p, pr, out, nullptr);
 }
@@ -529,22 +551,41 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
     const size_t records_at = ordinals_bytes(p) + forward_tiled_workspace_bytes(p);
     const size_t eval_bytes = records_bytes(p);
     void *eval_records = eval_bytes > 0 && workspace_bytes >= records_at + eval_bytes ? ws + records_at : nullptr;
-    if ((p->flags & HT_SAVED_FORWARD) != 0 && eval_records != nullptr && p->M == 1) {
+    const bool ordered = ordered_from_paths(p);
+    if ((p->flags & HT_SAVED_FORWARD) != 0 && eval_records != nullptr && p->M == 1 && !ordered) {
       // the records of the forward that ran on these inputs are still there: no tree is walked again
       const int src = backward_saved(p, a.ord, w, g, gx, gthr, gw, eval_records, pr.stream);
       if (src != HT_ERR_UNSUPPORTED) return src;
     }
     crc = clear_gradients(pr, gx, static_cast<float *>(nullptr), static_cast<float *>(nullptr));
     if (crc != HT_OK) return crc;
-    const int trc = backward_tiled(p, x, thr, a.ord, w, g, gx, gthr, gw, ws + ordinals_bytes(p), eval_records,
-                                   status_word, pr.stream);
-    if (trc != HT_ERR_UNSUPPORTED) return trc;
-    if (p->M > 1 && eval_records != nullptr && (p->flags & HT_DETERMINISTIC) == 0) {
-      if ((p->flags & HT_SAVED_FORWARD) == 0) {  // nothing was kept: the paths first
+    if (!ordered || eval_records == nullptr) {
+      const int trc = backward_tiled(p, x, thr, a.ord, w, g, gx, gthr, gw, ws + ordinals_bytes(p), eval_records,
+                                     status_word, pr.stream);
+      if (trc != HT_ERR_UNSUPPORTED) return trc;
+    }
+    if ((p->M > 1 || ordered) && eval_records != nullptr) {
+      const bool kept = (p->flags & HT_SAVED_FORWARD) != 0 && ht_forest_forward_saves(p);
+      if (!kept && (!ordered || gthr != nullptr || gw != nullptr)) {  // the paths first
         float *none = nullptr;
-        int prc = forward_tiled(p, x, thr, a.ord, w, none, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
-        if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, eval_records, pr.stream);
+        int prc = p->M == 1 ? HT_ERR_UNSUPPORTED
+                            : forward_tiled(p, x, thr, a.ord, w, none, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
+        if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, saved_paths(p, eval_records), pr.stream);
         if (prc != HT_OK) return prc;
+      }
+      if (ordered) {
+        const int orc = ordered_parameters(p, w, g, gthr, gw, saved_paths(p, eval_records),
+                                           static_cast<unsigned char *>(eval_records) + saved_bytes(p), pr.stream);
+        if (orc != HT_OK || gx == nullptr) return orc;
+        float *none = nullptr;
+        // the tile kernels' x gradient has the reference's order too; tabular samples too few for their tiles take a warp each
+        if (p->M == 1) {
+          int xrc = kept ? backward_saved(p, a.ord, w, g, gx, none, none, eval_records, pr.stream) : HT_ERR_UNSUPPORTED;
+          if (xrc == HT_ERR_UNSUPPORTED && (p->B * p->K >= 32768 || p->K > 1) && backward_records_bytes(p) > 0)
+            xrc = backward_tiled(p, x, thr, a.ord, w, g, gx, none, none, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
+          if (xrc != HT_ERR_UNSUPPORTED) return xrc;
+        }
+        return backward_any(p, pr, g, gx, none, none);
       }
       const int mrc = backward_multi(p, a.ord, w, g, gx, gthr, gw, eval_records, pr.stream);
       if (mrc != HT_ERR_UNSUPPORTED) return mrc;

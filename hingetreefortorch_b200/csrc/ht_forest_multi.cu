@@ -17,7 +17,7 @@ constexpr int kForwardThreads = 256;
 constexpr int kSortThreads = 256;
 constexpr uint32_t kSlice = 1024;  // evaluations per CTA
 constexpr int kMaxSortDepth = 12;
-constexpr int64_t kMaxForwardOutputs = 4096;
+constexpr int64_t kMaxDivisor = 4096;
 
 // V adjacent numbers as one load or store.
 template <typename Real, int V>
@@ -69,7 +69,7 @@ struct MultiForwardArgs {
   void *where;
   int64_t evals, T, C, K, N, L;
   int M, depth, narrow;
-  uint32_t divide_M;  // ceil(2^32 / M): quotients of numbers below 32 M
+  uint32_t divide_M;  // ceil(2^32 / M): quotients of numbers below 32 M (0: M is too large for it)
 };
 
 // Bound by the traversal's gathers for few outputs per leaf and by writing them for many.  A thread that writes the M
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kForwardThreads) multi_forward_kernel(const __
 #pragma unroll 4
   for (int t = lane; t - lane < pieces; t += 32) {
     const uint32_t element = (uint32_t)t * V;
-    const uint32_t owner = min(__umulhi(element, a.divide_M), 31u);
+    const uint32_t owner = min(a.divide_M != 0 ? __umulhi(element, a.divide_M) : element / (uint32_t)a.M, 31u);
     const Real scale = __shfl_sync(0xffffffffu, am, (int)owner);
     const uint32_t row = __shfl_sync(0xffffffffu, leaf, (int)owner);
     if (t < pieces) {
@@ -480,13 +480,13 @@ bool multi_takes(const ht_forest_problem *p, size_t real_bytes) {
 
 size_t multi_area_bytes(const ht_forest_problem *p, size_t real_bytes) {
   if (!multi_takes(p, real_bytes)) return 0;
-  const size_t bytes = record_array_bytes(p, real_bytes) + record_array_bytes(p, where_bytes(p->depth));
+  const size_t bytes = path_bytes(p, real_bytes);
   return bytes <= ((size_t)32 << 30) ? bytes : 0;
 }
 
 template <typename Real>
 int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, const int32_t *ord, const Real *w, Real *out,
-                  void *area, cudaStream_t stream) {
+                  PathRecordsOf<Real> paths, cudaStream_t stream) {
   MultiForwardArgs<Real> a = {};
   a.evals = p->B * p->T * p->K;
   a.T = p->T;
@@ -494,7 +494,7 @@ int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, co
   a.K = p->K;
   a.N = threshold_count(p->kind, p->depth);
   a.L = ((int64_t)1) << p->depth;
-  if (p->M > kMaxForwardOutputs || a.T * a.L > 0xffffffffll || a.evals > ((int64_t)kForwardThreads << 31) - kForwardThreads)
+  if (p->M < 1 || p->M > (1 << 26) || a.T * a.L > 0xffffffffll || a.evals > ((int64_t)kForwardThreads << 31) - kForwardThreads)
     return HT_ERR_UNSUPPORTED;
   a.x = x;
   a.thr = thr;
@@ -504,12 +504,9 @@ int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, co
   a.M = (int)p->M;
   a.depth = p->depth;
   a.narrow = where_bytes(p->depth) == 2;
-  a.divide_M = (uint32_t)(((1ull << 32) + p->M - 1) / (uint64_t)p->M);
-  if (area != nullptr) {
-    const PathRecordsOf<Real> paths = multi_paths<Real>(p, area);
-    a.margin = paths.margin;
-    a.where = paths.where;
-  }
+  a.divide_M = p->M > kMaxDivisor ? 0 : (uint32_t)(((1ull << 32) + p->M - 1) / (uint64_t)p->M);
+  a.margin = paths.margin;
+  a.where = paths.where;
   const int width = vector_width(p->M, sizeof(Real), {w, out});
   return p->kind == TREE ? launch_forward<TREE>(a, width, stream) : launch_forward<FERN>(a, width, stream);
 }
@@ -552,9 +549,9 @@ int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w
 }
 
 template int multi_forward<float>(const ht_forest_problem *, const float *, const float *, const int32_t *, const float *,
-                                  float *, void *, cudaStream_t);
+                                  float *, PathRecordsOf<float>, cudaStream_t);
 template int multi_forward<double>(const ht_forest_problem *, const double *, const double *, const int32_t *, const double *,
-                                   double *, void *, cudaStream_t);
+                                   double *, PathRecordsOf<double>, cudaStream_t);
 template int backward_multi<float>(const ht_forest_problem *, const int32_t *, const float *, const float *, float *, float *,
                                    float *, void *, cudaStream_t);
 template int backward_multi<double>(const ht_forest_problem *, const int32_t *, const double *, const double *, double *,

@@ -11,6 +11,11 @@ namespace ht {
 bool multi_takes(const ht_forest_problem *p, size_t real_bytes);
 size_t multi_area_bytes(const ht_forest_problem *p, size_t real_bytes);
 
+// Bytes of the paths of all evaluations.
+inline size_t path_bytes(const ht_forest_problem *p, size_t real_bytes) {
+  return record_array_bytes(p, real_bytes) + record_array_bytes(p, where_bytes(p->depth));
+}
+
 // The paths of all evaluations inside that area: threshold - feature at the deciding vertex, and the deciding vertex
 // with the leaf key, in the layout of the evaluation records.
 template <typename Real>
@@ -24,15 +29,22 @@ PathRecordsOf<Real> multi_paths(const ht_forest_problem *p, void *area) {
   return PathRecordsOf<Real>{reinterpret_cast<Real *>(base), base + record_array_bytes(p, sizeof(Real))};
 }
 
-// Forward of any shape with the results of a warp written together; with `area` it also leaves the paths there, and
-// with out == nullptr it leaves nothing else.  HT_ERR_UNSUPPORTED: nothing was launched.
+// Forward of any shape with the results of a warp written together; where `paths` has a place for them it also leaves the
+// paths, and with out == nullptr nothing else.  HT_ERR_UNSUPPORTED: nothing was launched.
 template <typename Real>
 int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, const int32_t *ord, const Real *w, Real *out,
-                  void *area, cudaStream_t stream);
+                  PathRecordsOf<Real> paths, cudaStream_t stream);
 
 // Gradients from the paths in `area`.  The gradients that are asked for (the others are null) must have been cleared.
 template <typename Real>
 int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w, const Real *g, Real *gx, Real *gthr,
                    Real *gw, void *area, cudaStream_t stream);
+
+// Fixed-order mode (ht_forest_ordered.cu), any number of outputs per leaf: bytes of the lists that the paths are sorted
+// into (0: not for this problem), and the threshold and leaf-weight gradients from the paths.
+size_t ordered_list_bytes(const ht_forest_problem *p, size_t real_bytes);
+template <typename Real>
+int ordered_parameters(const ht_forest_problem *p, const Real *w, const Real *g, Real *gthr, Real *gw, PathRecordsOf<Real> paths,
+                       void *lists, cudaStream_t stream);
 
 }  // namespace ht

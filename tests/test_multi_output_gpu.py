@@ -26,6 +26,11 @@ SHAPES = [
     (513, 11, (2,), 33, 4, 33),
     (5, 16, (900,), 9, 11, 63),
     (2, 100, (24, 24), 30, 7, 64),
+    # too few evaluations for the sorted backward, but not for the fixed order; one output, more than a buffer of terms holds
+    (31, 5, (), 3, 2, 2),
+    (700, 20, (), 6, 7, 1),
+    (130, 9, (5,), 2, 3, 70),
+    (3, 4, (), 2, 1, 4500),
 ]
 
 
@@ -47,6 +52,12 @@ def test_forward_and_backward(kind, shape):
     assert np.array_equal(f.forward(dx, dthr, dord, dw, save=True).cpu().numpy(), want)
     for got, r, s in zip(f.backward(dx, dthr, dord, dw, dg, saved=True), ref, sizes):
         assert grad_close(got, r, s)
+    ordered = _cabi.Forest(kind, dx, dw, deterministic=True)
+    for got, r in zip(ordered.backward(dx, dthr, dord, dw, dg), ref):
+        assert np.array_equal(got.cpu().numpy(), r)
+    assert np.array_equal(ordered.forward(dx, dthr, dord, dw, save=True).cpu().numpy(), want)
+    for got, r in zip(ordered.backward(dx, dthr, dord, dw, dg, saved=True), ref):
+        assert np.array_equal(got.cpu().numpy(), r)
     x.reshape(-1)[:3] = [np.inf, -np.inf, np.nan]
     got = f.forward(dev(x)[0], dthr, dord, dw).cpu().numpy()
     assert np.array_equal(got, ho.forward(kind, x, thr, ord_, w), equal_nan=True)
