@@ -2,7 +2,8 @@
 
 Class names, argument order and behaviour follow the reference's HingeTree/_HingeTree.py so
 that model code written against it keeps working; the classes themselves are generated from a
-few templates instead of being spelled out one by one.
+few templates instead of being spelled out one by one.  Those that training steps are made of (plain, fused linear,
+convolution) are nodes of the extension (hingetree_cpp_autograd.cpp): their `apply` does not go through Python.
 
 Every Function saves its raw inputs and lets the backward operator redo the traversal, as the
 reference does (_HingeTree.py:92-108); the plain tree and fern additionally keep the forward's
@@ -133,57 +134,19 @@ def _utilities(kind):
     return members
 
 
-class _HingeFunction(torch.autograd.Function):
-    """A Function with a way around autograd for calls that will not be differentiated (`ctx.needs_input_grad` does not
-    tell them apart: it repeats the inputs' requires_grad, also under torch.no_grad()).  Such a call keeps no traversal,
-    which costs 6 to 8 bytes written per evaluation (1048576 samples x 1024 trees: 5.0 ms with it, 3.8 ms without), and
-    builds no node."""
-    _predict = None
-
-    @classmethod
-    def apply(cls, *tensors):
-        if torch.is_grad_enabled() and any(t.requires_grad for t in tensors):
-            return super().apply(*tensors)
-        return cls._predict(*tensors)
+# `apply` of the classes that have forward and backward in Python below one that has not.
+_python_apply = classmethod(torch.autograd.Function.apply.__func__)
 
 
 def _plain_function(name, kind):
-    fwd, bwd, bwd_det = _op(kind + "_forward"), _op(kind + "_backward"), _op(kind + "_backward_deterministic")
-    fwd_saving, bwd_saved = _op(kind + "_forward_saving"), _op(kind + "_backward_saved")
-
-    def forward(ctx, inData, inThresholds, inOrdinals, inWeights):
-        # When a gradient will be asked for, the forward keeps its traversal (signed margin, deciding vertex and
-        # leaf of every evaluation) so that the backward does not walk the trees again; the operator returns an
-        # empty `kept` for problems it does not do this for, and the backward then re-walks, as the reference does.
-        kept = None
-        if inData.is_cuda and any(ctx.needs_input_grad):
-            out, kept = fwd_saving(inData, inThresholds, inOrdinals, inWeights)
-            if kept.numel() == 0:
-                kept = None
-        else:
-            out = fwd(inData, inThresholds, inOrdinals, inWeights)
-        ctx.kept = kept
-        ctx.save_for_backward(inData, inThresholds, inOrdinals, inWeights)
-        return out
-
-    def backward(ctx, outDataGrad):
-        kept, ctx.kept = ctx.kept, None  # one backward per forward: the scratch is rewritten by it
-        if kept is not None:
-            return tuple(bwd_saved(*_interleave(ctx.saved_tensors, ctx.needs_input_grad), outDataGrad.contiguous(), kept,
-                                   _is_deterministic()))
-        op = bwd_det if _is_deterministic() else bwd
-        return tuple(op(*_interleave(ctx.saved_tensors, ctx.needs_input_grad), outDataGrad.contiguous()))
-
-    members = {"forward": staticmethod(forward), "backward": staticmethod(backward), "_predict": staticmethod(fwd)}
+    members = {"apply": staticmethod(_op(kind + "_apply"))}
     members.update(_utilities(kind))
-    return type(name, (_HingeFunction,), members)
+    return type(name, (torch.autograd.Function,), members)
 
 
 def _sparse_function(name, base, kind, label):
     """Backward returns sparse COO gradients; only the data gradient is densified (as in the reference)."""
-    bwd = _op("sparse_%s_backward" % kind)
-
-    fwd = _op(kind + "_forward")
+    fwd, bwd = _op(kind + "_forward"), _op("sparse_%s_backward" % kind)
 
     def forward(ctx, inData, inThresholds, inOrdinals, inWeights):  # the sparse backward has no use for a kept traversal
         ctx.save_for_backward(inData, inThresholds, inOrdinals, inWeights)
@@ -196,12 +159,15 @@ def _sparse_function(name, base, kind, label):
             grads[0] = grads[0].to_dense()
         return tuple(grads)
 
-    return type(name, (base,), {"forward": staticmethod(forward), "backward": staticmethod(backward)})
+    return type(name, (base,), {"forward": staticmethod(forward), "backward": staticmethod(backward), "apply": _python_apply})
 
 
-def _fused_linear_function(name, base, kind, label, sparse):
-    fwd = _op(kind + "_fused_linear_forward")
-    bwd = _op(("sparse_" if sparse else "") + kind + "_fused_linear_backward")
+def _fused_linear_function(name, base, kind):
+    return type(name, (base,), {"apply": staticmethod(_op(kind + "_fused_linear_apply"))})
+
+
+def _sparse_fused_linear_function(name, base, kind, label):
+    fwd, bwd = _op(kind + "_fused_linear_forward"), _op("sparse_%s_fused_linear_backward" % kind)
 
     def forward(ctx, inData, inThresholds, inOrdinals, inWeights, inLinearWeights, inLinearBias):
         _refuse_deterministic(inData, "forward for hinge %s + linear" % label)
@@ -211,19 +177,11 @@ def _fused_linear_function(name, base, kind, label, sparse):
     def backward(ctx, outDataGrad):
         _refuse_deterministic(outDataGrad, "backpropagation for hinge %s + linear" % label)
         grads = list(bwd(*_interleave(ctx.saved_tensors, ctx.needs_input_grad), outDataGrad.contiguous()))
-        if sparse and grads[0] is not None:
+        if grads[0] is not None:
             grads[0] = grads[0].to_dense()
         return tuple(grads)
 
-    def predict(inData, *params):
-        _refuse_deterministic(inData, "forward for hinge %s + linear" % label)
-        return fwd(inData, *params)
-
-    members = {"backward": staticmethod(backward)}
-    if not sparse:
-        members["forward"] = staticmethod(forward)
-        members["_predict"] = staticmethod(predict)
-    return type(name, (base,), members)
+    return type(name, (base,), {"forward": staticmethod(forward), "backward": staticmethod(backward), "apply": _python_apply})
 
 
 def _fusion_function(name, kind, label):
@@ -257,20 +215,8 @@ def _fusion_fused_linear_function(name, base, kind, label):
     return type(name, (base,), {"forward": staticmethod(forward), "backward": staticmethod(backward)})
 
 
-def _conv_function(name, kind, dims, label):
-    fwd, bwd = _op("%s_conv%dd_forward" % (kind, dims)), _op("%s_conv%dd_backward" % (kind, dims))
-
-    def forward(ctx, inData, inThresholds, inOrdinals, inWeights, kernelSize, stride, padding, dilation):
-        ctx.save_for_backward(inData, inThresholds, inOrdinals, inWeights)
-        ctx.geometry = (kernelSize, stride, padding, dilation)
-        return fwd(inData, inThresholds, inOrdinals, inWeights, kernelSize, stride, padding, dilation)
-
-    def backward(ctx, outDataGrad):
-        _refuse_deterministic(outDataGrad, "backpropagation for hinge %s convolution" % label)
-        grads = bwd(*_interleave(ctx.saved_tensors, ctx.needs_input_grad[:4]), outDataGrad.contiguous(), *ctx.geometry)
-        return tuple(grads) + (None, None, None, None)
-
-    return type(name, (torch.autograd.Function,), {"forward": staticmethod(forward), "backward": staticmethod(backward)})
+def _conv_function(name, kind, dims):
+    return type(name, (torch.autograd.Function,), {"apply": staticmethod(_op("%s_conv%dd_apply" % (kind, dims)))})
 
 
 HingeTree = _plain_function("HingeTree", "tree")
@@ -279,24 +225,22 @@ HingeFern = _plain_function("HingeFern", "fern")
 SparseHingeTree = _sparse_function("SparseHingeTree", HingeTree, "tree", "tree")
 SparseHingeFern = _sparse_function("SparseHingeFern", HingeFern, "fern", "fern")
 
-HingeTreeFusedLinear = _fused_linear_function("HingeTreeFusedLinear", HingeTree, "tree", "tree", sparse=False)
-HingeFernFusedLinear = _fused_linear_function("HingeFernFusedLinear", HingeFern, "fern", "fern", sparse=False)
-SparseHingeTreeFusedLinear = _fused_linear_function("SparseHingeTreeFusedLinear", HingeTreeFusedLinear, "tree", "tree",
-                                                    sparse=True)
-SparseHingeFernFusedLinear = _fused_linear_function("SparseHingeFernFusedLinear", HingeFernFusedLinear, "fern", "fern",
-                                                    sparse=True)
+HingeTreeFusedLinear = _fused_linear_function("HingeTreeFusedLinear", HingeTree, "tree")
+HingeFernFusedLinear = _fused_linear_function("HingeFernFusedLinear", HingeFern, "fern")
+SparseHingeTreeFusedLinear = _sparse_fused_linear_function("SparseHingeTreeFusedLinear", HingeTreeFusedLinear, "tree", "tree")
+SparseHingeFernFusedLinear = _sparse_fused_linear_function("SparseHingeFernFusedLinear", HingeFernFusedLinear, "fern", "fern")
 
 HingeTreeFusion = _fusion_function("HingeTreeFusion", "tree", "tree")
 HingeFernFusion = _fusion_function("HingeFernFusion", "fern", "fern")
 HingeTreeFusionFusedLinear = _fusion_fused_linear_function("HingeTreeFusionFusedLinear", HingeTreeFusion, "tree", "tree")
 HingeFernFusionFusedLinear = _fusion_fused_linear_function("HingeFernFusionFusedLinear", HingeFernFusion, "fern", "fern")
 
-HingeTreeConv1d = _conv_function("HingeTreeConv1d", "tree", 1, "tree")
-HingeTreeConv2d = _conv_function("HingeTreeConv2d", "tree", 2, "tree")
-HingeTreeConv3d = _conv_function("HingeTreeConv3d", "tree", 3, "tree")
-HingeFernConv1d = _conv_function("HingeFernConv1d", "fern", 1, "fern")
-HingeFernConv2d = _conv_function("HingeFernConv2d", "fern", 2, "fern")
-HingeFernConv3d = _conv_function("HingeFernConv3d", "fern", 3, "fern")
+HingeTreeConv1d = _conv_function("HingeTreeConv1d", "tree", 1)
+HingeTreeConv2d = _conv_function("HingeTreeConv2d", "tree", 2)
+HingeTreeConv3d = _conv_function("HingeTreeConv3d", "tree", 3)
+HingeFernConv1d = _conv_function("HingeFernConv1d", "fern", 1)
+HingeFernConv2d = _conv_function("HingeFernConv2d", "fern", 2)
+HingeFernConv3d = _conv_function("HingeFernConv3d", "fern", 3)
 
 
 class HingeTrie(torch.autograd.Function):

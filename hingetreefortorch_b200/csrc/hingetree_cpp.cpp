@@ -275,8 +275,6 @@ ForestCall::ForestCall(int kind, const torch::Tensor &x, const torch::Tensor &th
   }
 }
 
-namespace {
-
 torch::Tensor forest_forward(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w) {
   ForestCall call(kind, x, thr, ord, w, nullptr, true);
   c10::DeviceGuard guard(x.device());
@@ -469,6 +467,23 @@ std::vector<torch::Tensor> batchnorm_statistics(torch::Tensor sum, torch::Tensor
   return {out[0], out[1], out[2]};
 }
 
+void batchnorm_running(torch::Tensor mean, torch::Tensor var, int64_t rows, double momentum, torch::Tensor running_mean,
+                       torch::Tensor running_var, torch::Tensor batches) {
+  for (const torch::Tensor *t : {&mean, &var, &running_mean, &running_var})
+    if (t->scalar_type() != torch::kFloat32 || t->dim() != 1 || t->size(0) != mean.size(0) || t->device() != mean.device() ||
+        !t->is_contiguous())
+      bad_argument("Error: the statistics are expected to be contiguous torch.float32 vectors of the same length on one device.");
+  if (batches.scalar_type() != torch::kInt64 || batches.numel() != 1 || batches.device() != mean.device())
+    bad_argument("Error: the batch count is expected to be one torch.int64 number on the same device.");
+  require_cuda(mean);
+  c10::DeviceGuard guard(mean.device());
+  raise_status(ht_batchnorm_running_f32(mean.data_ptr<float>(), var.data_ptr<float>(), rows, mean.size(0), (float)momentum,
+                                        running_mean.data_ptr<float>(), running_var.data_ptr<float>(), batches.data_ptr<int64_t>(),
+                                        current_stream(mean)),
+               "running statistics");
+  for (torch::Tensor *t : {&running_mean, &running_var, &batches}) t->unsafeGetTensorImpl()->bump_version();
+}
+
 // Returns {out, margin, where}: with `keep` the forward leaves its traversal (signed margin; deciding vertex and leaf
 // key) for forest_normalised_backward, else the two are empty tensors.
 std::vector<torch::Tensor> forest_normalised_forward(int kind, torch::Tensor z, torch::Tensor mean, torch::Tensor invstd,
@@ -530,6 +545,8 @@ std::vector<torch::Tensor> forest_normalised_backward(int kind, torch::Tensor z,
   og.finish();
   return {dz, gthr, gw};
 }
+
+namespace {
 
 torch::Tensor forest_leafmap(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w) {
   ForestCall call(kind, x, thr, ord, w, nullptr, true);
@@ -856,4 +873,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "version), 'always' (every call, like the reference) or 'never'.");
   m.def("abi_version", []() { return ht_version(); });
   htx::bind_more_ops(m);
+  htx::bind_autograd(m);
 }

@@ -212,6 +212,8 @@ std::vector<torch::Tensor> fusion_backward(int kind, torch::Tensor img, bool nee
 
 // ---- fused linear (plain and fusion) -------------------------------------------------------
 
+}  // namespace
+
 torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *vec, torch::Tensor thr, torch::Tensor ord,
                              torch::Tensor w, torch::Tensor lin, torch::Tensor bias) {
   FamilyCall call(kind, data, vec, thr, ord, w, &lin, &bias, nullptr);
@@ -276,6 +278,8 @@ std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool ne
   if (fusion) return {gdata, gvec, gthr, torch::Tensor(), gw, glin, gbias};
   return {gdata, gthr, torch::Tensor(), gw, glin, gbias};
 }
+
+namespace {
 
 // ---- sparse gradients ----------------------------------------------------------------------------
 // The dense backward gives the values, ht_forest_touched_f32 the elements that were contributed
@@ -342,10 +346,6 @@ std::vector<torch::Tensor> sparse_backward(int kind, torch::Tensor x, bool need_
   return grads;
 }
 
-std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool need_data, const torch::Tensor *vec,
-                                           bool need_vec, torch::Tensor thr, bool need_thr, torch::Tensor ord,
-                                           bool need_ord, torch::Tensor w, bool need_w, torch::Tensor lin, bool need_lin,
-                                           torch::Tensor bias, bool need_bias, torch::Tensor g);
 
 // Sparse data / threshold / leaf-weight gradients; the linear layer's gradients stay dense
 // (hingetree_sparse_gpu.cu:743-761).
@@ -531,6 +531,8 @@ struct ConvCall {
   }
 };
 
+}  // namespace
+
 torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w,
                            std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
                            std::vector<int64_t> dilation) {
@@ -575,6 +577,8 @@ std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bo
   og.finish();
   return grads;
 }
+
+namespace {
 
 // ---- contract / expand (expand.cpp:353-457, 475-577) ---------------------------------------
 

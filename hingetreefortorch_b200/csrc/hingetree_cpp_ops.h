@@ -50,6 +50,40 @@ struct ForestCall {
   std::vector<int64_t> map_sizes;  // [B, T, inner data dims...]
 };
 
+// The operators that the autograd nodes are made of (hingetree_cpp.cpp, hingetree_cpp_more.cpp).
+torch::Tensor forest_forward(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w);
+std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w);
+std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::Tensor x, bool need_x, torch::Tensor thr, bool need_thr,
+                                           torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w, torch::Tensor g);
+std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, torch::Tensor x, bool need_x, torch::Tensor thr,
+                                                 bool need_thr, torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w,
+                                                 torch::Tensor g, torch::Tensor saved);
+torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *vec, torch::Tensor thr, torch::Tensor ord,
+                             torch::Tensor w, torch::Tensor lin, torch::Tensor bias);
+std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool need_data, const torch::Tensor *vec, bool need_vec,
+                                           torch::Tensor thr, bool need_thr, torch::Tensor ord, bool need_ord, torch::Tensor w,
+                                           bool need_w, torch::Tensor lin, bool need_lin, torch::Tensor bias, bool need_bias,
+                                           torch::Tensor g);
+torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w,
+                           std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
+                           std::vector<int64_t> dilation);
+std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bool need_x, torch::Tensor thr, bool need_thr,
+                                         torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w, torch::Tensor g,
+                                         std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
+                                         std::vector<int64_t> dilation);
+std::vector<torch::Tensor> linear_tf32_stats(torch::Tensor x, torch::Tensor w);
+std::vector<torch::Tensor> batchnorm_statistics(torch::Tensor sum, torch::Tensor sumsq, int64_t rows, double eps);
+void batchnorm_running(torch::Tensor mean, torch::Tensor var, int64_t rows, double momentum, torch::Tensor running_mean,
+                       torch::Tensor running_var, torch::Tensor batches);
+std::vector<torch::Tensor> forest_normalised_forward(int kind, torch::Tensor z, torch::Tensor mean, torch::Tensor invstd,
+                                                     torch::Tensor thr, torch::Tensor ord, torch::Tensor w, bool keep);
+std::vector<torch::Tensor> forest_normalised_backward(int kind, torch::Tensor z, torch::Tensor mean, torch::Tensor invstd,
+                                                      torch::Tensor thr, bool need_thr, torch::Tensor ord, torch::Tensor w,
+                                                      bool need_w, torch::Tensor g, torch::Tensor margin, torch::Tensor where);
+
+// Registers the autograd nodes (hingetree_cpp_autograd.cpp).
+void bind_autograd(pybind11::module_ &m);
+
 // Registers the convolution, fused-linear, fusion, sparse, trie and contract/expand operators.
 void bind_more_ops(pybind11::module_ &m);
 

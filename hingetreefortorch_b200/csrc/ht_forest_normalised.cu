@@ -180,6 +180,17 @@ __global__ void __launch_bounds__(kNormBlock) statistics_kernel(const float *__r
   invstd[c] = rsqrtf(__fadd_rn(v, eps));
 }
 
+// One step of the running statistics (nn.BatchNorm1d: unbiased variance) and of the batch count.
+__global__ void __launch_bounds__(kNormBlock) running_kernel(const float *__restrict__ mean, const float *__restrict__ var, int64_t C,
+                                                            float unbiased, float momentum, float *running_mean, float *running_var,
+                                                            int64_t *batches) {
+  const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (c == 0) *batches += 1;
+  if (c >= C) return;
+  running_mean[c] += momentum * (mean[c] - running_mean[c]);
+  running_var[c] += momentum * (var[c] * unbiased - running_var[c]);
+}
+
 int check(const ht_forest_problem *p, NormalisedArgs &a) {
   if (p == nullptr) return HT_ERR_INVALID_ARGUMENT;
   if (p->kind != TREE && p->kind != FERN) return HT_ERR_INVALID_ARGUMENT;
@@ -309,6 +320,18 @@ extern "C" int ht_batchnorm_statistics_f32(const float *sum, const float *sumsq,
   if (sum == nullptr || sumsq == nullptr || mean == nullptr || var == nullptr || invstd == nullptr) return HT_ERR_INVALID_ARGUMENT;
   statistics_kernel<<<norm_blocks(C), kNormBlock, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(sum, sumsq, C, 1.0f / (float)rows, eps,
                                                                                               mean, var, invstd);
+  HT_CHECK_LAUNCH();
+  return HT_OK;
+}
+
+extern "C" int ht_batchnorm_running_f32(const float *mean, const float *var, int64_t rows, int64_t C, float momentum,
+                                        float *running_mean, float *running_var, int64_t *batches, ht_stream_t stream_) {
+  if (rows < 1 || C < 1) return HT_ERR_INVALID_ARGUMENT;
+  if (mean == nullptr || var == nullptr || running_mean == nullptr || running_var == nullptr || batches == nullptr)
+    return HT_ERR_INVALID_ARGUMENT;
+  const float unbiased = rows > 1 ? (float)((double)rows / (double)(rows - 1)) : 1.0f;
+  running_kernel<<<norm_blocks(C), kNormBlock, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(mean, var, C, unbiased, momentum,
+                                                                                           running_mean, running_var, batches);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }

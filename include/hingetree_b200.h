@@ -356,6 +356,10 @@ int ht_forest_normalised_backward_f32(const ht_forest_problem *p, const float *z
  * as one launch. */
 int ht_batchnorm_statistics_f32(const float *sum, const float *sumsq, int64_t rows, int64_t C, float eps, float *mean,
                                 float *var, float *invstd, ht_stream_t stream);
+/* running_mean += momentum * (mean - running_mean), the same for running_var with the unbiased variance of `rows` rows, and
+ * batches += 1: what nn.BatchNorm1d does with a training batch, as one launch. */
+int ht_batchnorm_running_f32(const float *mean, const float *var, int64_t rows, int64_t C, float momentum, float *running_mean,
+                             float *running_var, int64_t *batches, ht_stream_t stream);
 /* Gradient with respect to z of y = (z - mean) * invstd with batch statistics (training mode, no affine part):
  * dz[i, c] = invstd[c] * (gy[i, c] - sum_g[c] / B - y[i, c] * sum_gy[c] / B), gy given by the records above: one pass
  * over z for the dense part, one over the records (the formula of torch's batch-norm backward,
