@@ -6,6 +6,7 @@
 // itself only runs on CPU tensors (module constructors call them before .to(device)).
 #include <torch/extension.h>
 
+#include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/DeviceGuard.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAStream.h>
@@ -214,8 +215,12 @@ void set_ordinal_check(const std::string &mode) {
     bad_argument("Error: ordinal check mode must be 'cached', 'always' or 'never'.");
 }
 
+torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like, c10::ScalarType type) {
+  return at::detail::empty_cuda(sizes, type, like.device(), c10::nullopt);
+}
+
 torch::Tensor make_workspace(size_t bytes, const torch::Tensor &like) {
-  return torch::empty({(int64_t)std::max<size_t>(bytes, 256)}, torch::TensorOptions().dtype(torch::kUInt8).device(like.device()));
+  return fresh({(int64_t)std::max<size_t>(bytes, 256)}, like, torch::kUInt8);
 }
 
 // ---- plain forest ------------------------------------------------------------------------
@@ -278,7 +283,7 @@ ForestCall::ForestCall(int kind, const torch::Tensor &x, const torch::Tensor &th
 torch::Tensor forest_forward(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w) {
   ForestCall call(kind, x, thr, ord, w, nullptr, true);
   c10::DeviceGuard guard(x.device());
-  torch::Tensor out = torch::empty(call.out_sizes, x.options());
+  torch::Tensor out = fresh(call.out_sizes, x);
   torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.problem.C);
   if (call.is_double) {
@@ -306,9 +311,9 @@ std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::
   std::vector<torch::Tensor> grads(4);
   if (!need_x && !need_thr && !need_w) return grads;
   if (deterministic) call.problem.flags |= HT_DETERMINISTIC;
-  if (need_x) grads[0] = torch::empty_like(x);
-  if (need_thr) grads[1] = torch::empty_like(thr);
-  if (need_w) grads[3] = torch::empty_like(w);
+  if (need_x) grads[0] = fresh_like(x);
+  if (need_thr) grads[1] = fresh_like(thr);
+  if (need_w) grads[3] = fresh_like(w);
   if (call.is_double) {
     torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
     OrdinalGuard og(ord, call.problem.C);
@@ -356,7 +361,7 @@ static bool g_save_forward = true;
 std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord,
                                                  torch::Tensor w) {
   if (x.scalar_type() == torch::kFloat64)  // no kept traversal in double precision: the plain forward
-    return {forest_forward(kind, x, thr, ord, w), torch::empty({0}, x.options().dtype(torch::kUInt8))};
+    return {forest_forward(kind, x, thr, ord, w), fresh({0}, x, torch::kUInt8)};
   ForestCall call(kind, x, thr, ord, w, nullptr);
   c10::DeviceGuard guard(x.device());
   if (at::globalContext().deterministicAlgorithms()) call.problem.flags |= HT_DETERMINISTIC;  // the scratch its backward needs
@@ -364,7 +369,7 @@ std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torc
   if (saves) call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD | HT_SAVE_FOR_BACKWARD;
   if (saves && (int64_t)ht_forest_workspace_bytes(&call.problem) > g_backward_scratch_limit)
     call.problem.flags &= ~(HT_WORKSPACE_FOR_BACKWARD | HT_SAVE_FOR_BACKWARD);
-  torch::Tensor out = torch::empty(call.out_sizes, x.options());
+  torch::Tensor out = fresh(call.out_sizes, x);
   torch::Tensor ws;
   try {
     ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
@@ -380,7 +385,7 @@ std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torc
                "forest forward");
   og.finish();
   const bool saved = (call.problem.flags & HT_SAVE_FOR_BACKWARD) != 0;
-  return {out, saved ? ws : torch::empty({0}, ws.options())};
+  return {out, saved ? ws : fresh({0}, ws)};
 }
 
 std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, torch::Tensor x, bool need_x,
@@ -399,9 +404,9 @@ std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, t
   if (!saved.defined() || saved.device() != x.device() || saved.scalar_type() != torch::kUInt8 ||
       (size_t)saved.numel() < ht_forest_workspace_bytes(&call.problem) || ht_forest_forward_saves(&call.problem) == 0)
     bad_argument("Error: `saved` is not the scratch a saving forward returned for these tensors.");
-  if (need_x) grads[0] = torch::empty_like(x);
-  if (need_thr) grads[1] = torch::empty_like(thr);
-  if (need_w) grads[3] = torch::empty_like(w);
+  if (need_x) grads[0] = fresh_like(x);
+  if (need_thr) grads[1] = fresh_like(thr);
+  if (need_w) grads[3] = fresh_like(w);
   OrdinalGuard og(ord, call.problem.C);
   raise_status(
       ht_forest_backward_f32(&call.problem, x.data_ptr<float>(), thr.data_ptr<float>(), ord.data_ptr<int64_t>(),
@@ -427,8 +432,8 @@ std::vector<torch::Tensor> linear_tf32_stats(torch::Tensor x, torch::Tensor w) {
   if (!x.is_contiguous() || !w.is_contiguous()) bad_argument("Error: All tensors are expected to be contiguous.");
   c10::DeviceGuard guard(x.device());
   const int64_t M = x.size(0), K = x.size(1), N = w.size(0);
-  torch::Tensor z = torch::empty({M, N}, x.options());
-  torch::Tensor sum = torch::empty({N}, x.options()), sumsq = torch::empty({N}, x.options());
+  torch::Tensor z = fresh({M, N}, x);
+  torch::Tensor sum = fresh({N}, x), sumsq = fresh({N}, x);
   torch::Tensor status = sticky_word(x.device(), true);
   raise_status(ht_linear_tf32_stats_f32(x.data_ptr<float>(), w.data_ptr<float>(), z.data_ptr<float>(), sum.data_ptr<float>(),
                                         sumsq.data_ptr<float>(), M, N, K,
@@ -458,7 +463,7 @@ std::vector<torch::Tensor> batchnorm_statistics(torch::Tensor sum, torch::Tensor
   require_cuda(sum);
   if (rows < 1) bad_argument("Error: rows must be positive.");
   c10::DeviceGuard guard(sum.device());
-  torch::Tensor out = torch::empty({3, sum.size(0)}, sum.options());
+  torch::Tensor out = fresh({3, sum.size(0)}, sum);
   const int64_t C = sum.size(0);
   raise_status(ht_batchnorm_statistics_f32(sum.data_ptr<float>(), sumsq.data_ptr<float>(), rows, C, (float)eps,
                                            out.data_ptr<float>(), out.data_ptr<float>() + C, out.data_ptr<float>() + 2 * C,
@@ -492,9 +497,9 @@ std::vector<torch::Tensor> forest_normalised_forward(int kind, torch::Tensor z, 
   check_statistics(z, mean, invstd);
   c10::DeviceGuard guard(z.device());
   const int64_t B = call.problem.B, T = call.problem.T;
-  torch::Tensor out = torch::empty(call.out_sizes, z.options());
-  torch::Tensor margin = torch::empty({keep ? B : 0, T}, z.options());
-  torch::Tensor where = torch::empty({keep ? B : 0, T, 2}, z.options().dtype(torch::kInt32));
+  torch::Tensor out = fresh(call.out_sizes, z);
+  torch::Tensor margin = fresh({keep ? B : 0, T}, z);
+  torch::Tensor where = fresh({keep ? B : 0, T, 2}, z, torch::kInt32);
   torch::Tensor ws = make_workspace(ht_forest_normalised_workspace_bytes(&call.problem), z);
   OrdinalGuard og(ord, call.problem.C);
   raise_status(ht_forest_normalised_forward_f32(&call.problem, z.data_ptr<float>(), mean.data_ptr<float>(),
@@ -523,12 +528,12 @@ std::vector<torch::Tensor> forest_normalised_backward(int kind, torch::Tensor z,
                where.numel() != 2 * B * T || margin.device() != z.device() || where.device() != z.device() ||
                !margin.is_contiguous() || !where.is_contiguous()))
     bad_argument("Error: margin / where are not what the forward of this call kept.");
-  torch::Tensor gthr = need_thr ? torch::empty_like(thr) : torch::Tensor();
-  torch::Tensor gw = need_w ? torch::empty_like(w) : torch::Tensor();
-  torch::Tensor column = torch::empty({B, T}, z.options().dtype(torch::kInt32));
-  torch::Tensor value = torch::empty({B, T}, z.options());
-  torch::Tensor sums = torch::empty({2, C}, z.options());
-  torch::Tensor dz = torch::empty_like(z);
+  torch::Tensor gthr = need_thr ? fresh_like(thr) : torch::Tensor();
+  torch::Tensor gw = need_w ? fresh_like(w) : torch::Tensor();
+  torch::Tensor column = fresh({B, T}, z, torch::kInt32);
+  torch::Tensor value = fresh({B, T}, z);
+  torch::Tensor sums = fresh({2, C}, z);
+  torch::Tensor dz = fresh_like(z);
   torch::Tensor ws = make_workspace(ht_forest_normalised_workspace_bytes(&call.problem), z);
   OrdinalGuard og(ord, C);
   raise_status(ht_forest_normalised_backward_f32(
@@ -551,7 +556,7 @@ namespace {
 torch::Tensor forest_leafmap(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w) {
   ForestCall call(kind, x, thr, ord, w, nullptr, true);
   c10::DeviceGuard guard(x.device());
-  torch::Tensor leaf = torch::empty(call.map_sizes, x.options().dtype(torch::kInt64));
+  torch::Tensor leaf = fresh(call.map_sizes, x, torch::kInt64);
   torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.problem.C);
   if (call.is_double) {
@@ -572,8 +577,8 @@ std::vector<torch::Tensor> forest_marginmap(int kind, torch::Tensor x, torch::Te
                                             torch::Tensor w) {
   ForestCall call(kind, x, thr, ord, w, nullptr, true);
   c10::DeviceGuard guard(x.device());
-  torch::Tensor margins = torch::empty(call.map_sizes, x.options());
-  torch::Tensor ords = torch::empty(call.map_sizes, x.options().dtype(torch::kInt64));
+  torch::Tensor margins = fresh(call.map_sizes, x);
+  torch::Tensor ords = fresh(call.map_sizes, x, torch::kInt64);
   torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.problem.C);
   if (call.is_double) {
@@ -597,7 +602,7 @@ std::vector<torch::Tensor> forest_marginmap(int kind, torch::Tensor x, torch::Te
 torch::Tensor forest_reachability(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w) {
   ForestCall call(kind, x, thr, ord, w, nullptr, true);
   c10::DeviceGuard guard(x.device());
-  torch::Tensor counts = torch::empty({w.size(0), w.size(1)}, x.options().dtype(torch::kInt64));
+  torch::Tensor counts = fresh({w.size(0), w.size(1)}, x, torch::kInt64);
   torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.problem.C);
   if (call.is_double) {

@@ -166,7 +166,7 @@ torch::Tensor fusion_forward(int kind, torch::Tensor img, torch::Tensor vec, tor
                              torch::Tensor w) {
   FamilyCall call(kind, img, &vec, thr, ord, w, nullptr, nullptr, nullptr);
   c10::DeviceGuard guard(img.device());
-  torch::Tensor out = torch::empty(call.out_sizes, img.options());
+  torch::Tensor out = fresh(call.out_sizes, img);
   torch::Tensor ws = make_workspace(ht_forest_fusion_workspace_bytes(&call.problem), img);
   OrdinalGuard og(ord, call.problem.C + call.vec_channels);
   dispatch_real(img, [&](auto real) {
@@ -190,11 +190,11 @@ std::vector<torch::Tensor> fusion_backward(int kind, torch::Tensor img, bool nee
   std::vector<torch::Tensor> grads(5);
   if (!need_img && !need_vec && !need_thr && !need_w) return grads;
   if (need_img || need_vec) {  // the reference returns both when either is requested
-    grads[0] = torch::empty_like(img);
-    grads[1] = torch::empty_like(vec);
+    grads[0] = fresh_like(img);
+    grads[1] = fresh_like(vec);
   }
-  if (need_thr) grads[2] = torch::empty_like(thr);
-  if (need_w) grads[4] = torch::empty_like(w);
+  if (need_thr) grads[2] = fresh_like(thr);
+  if (need_w) grads[4] = fresh_like(w);
   torch::Tensor ws = make_workspace(ht_forest_fusion_workspace_bytes(&call.problem), img);
   OrdinalGuard og(ord, call.problem.C + call.vec_channels);
   dispatch_real(img, [&](auto real) {
@@ -218,7 +218,7 @@ torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *
                              torch::Tensor w, torch::Tensor lin, torch::Tensor bias) {
   FamilyCall call(kind, data, vec, thr, ord, w, &lin, &bias, nullptr);
   c10::DeviceGuard guard(data.device());
-  torch::Tensor out = torch::empty(call.out_sizes, data.options());
+  torch::Tensor out = fresh(call.out_sizes, data);
   torch::Tensor ws = make_workspace(data.scalar_type() == torch::kFloat64 ? ht_forest_linear_workspace_bytes_f64(&call.problem)
                                                                                   : ht_forest_linear_workspace_bytes(&call.problem),
                                      data);
@@ -247,12 +247,12 @@ std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool ne
   const bool fusion = vec != nullptr;
   torch::Tensor gdata, gvec, gthr, gw, glin, gbias;
   if (fusion ? (need_data || need_vec) : need_data) {
-    gdata = torch::empty_like(data);
-    if (fusion) gvec = torch::empty_like(*vec);
+    gdata = fresh_like(data);
+    if (fusion) gvec = fresh_like(*vec);
   }
-  if (need_thr) gthr = torch::empty_like(thr);
-  if (need_w) gw = torch::empty_like(w);
-  if (need_lin) glin = torch::empty_like(lin);
+  if (need_thr) gthr = fresh_like(thr);
+  if (need_w) gw = fresh_like(w);
+  if (need_lin) glin = fresh_like(lin);
   if (gdata.defined() || gthr.defined() || gw.defined() || glin.defined()) {
     torch::Tensor ws = make_workspace(data.scalar_type() == torch::kFloat64 ? ht_forest_linear_workspace_bytes_f64(&call.problem)
                                                                                   : ht_forest_linear_workspace_bytes(&call.problem),
@@ -326,9 +326,9 @@ std::vector<torch::Tensor> sparse_backward(int kind, torch::Tensor x, bool need_
   std::vector<torch::Tensor> grads(4);
   if (!need_x && !need_thr && !need_w) return grads;
   torch::Tensor gx, gthr, gw;
-  if (need_x) gx = torch::empty_like(x);
-  if (need_thr) gthr = torch::empty_like(thr);
-  if (need_w) gw = torch::empty_like(w);
+  if (need_x) gx = fresh_like(x);
+  if (need_thr) gthr = fresh_like(thr);
+  if (need_w) gw = fresh_like(w);
   torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.problem.C);
   dispatch_real(x, [&](auto real) {
@@ -411,7 +411,7 @@ struct TrieCall {
 torch::Tensor trie_forward(torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w) {
   TrieCall call(x, thr, ord, w, nullptr);
   c10::DeviceGuard guard(x.device());
-  torch::Tensor out = torch::empty(call.out_sizes, x.options());
+  torch::Tensor out = fresh(call.out_sizes, x);
   torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.problem.C);
   dispatch_real(x, [&](auto real) {
@@ -432,9 +432,9 @@ std::vector<torch::Tensor> trie_backward(torch::Tensor x, bool need_x, torch::Te
   c10::DeviceGuard guard(x.device());
   std::vector<torch::Tensor> grads(4);
   if (!need_x && !need_thr && !need_w) return grads;
-  if (need_x) grads[0] = torch::empty_like(x);
-  if (need_thr) grads[1] = torch::empty_like(thr);
-  if (need_w) grads[3] = torch::empty_like(w);
+  if (need_x) grads[0] = fresh_like(x);
+  if (need_thr) grads[1] = fresh_like(thr);
+  if (need_w) grads[3] = fresh_like(w);
   torch::Tensor ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.problem.C);
   dispatch_real(x, [&](auto real) {
@@ -538,7 +538,7 @@ torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor th
                            std::vector<int64_t> dilation) {
   ConvCall call(kind, dims, x, thr, ord, w, nullptr, kernel, stride, padding, dilation);
   c10::DeviceGuard guard(x.device());
-  torch::Tensor out = torch::empty(call.out_sizes, x.options());
+  torch::Tensor out = fresh(call.out_sizes, x);
   torch::Tensor ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.window_cells);
   dispatch_real(x, [&](auto real) {
@@ -561,9 +561,9 @@ std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bo
   c10::DeviceGuard guard(x.device());
   std::vector<torch::Tensor> grads(4);
   if (!need_x && !need_thr && !need_w) return grads;
-  if (need_x) grads[0] = torch::empty_like(x);
-  if (need_thr) grads[1] = torch::empty_like(thr);
-  if (need_w) grads[3] = torch::empty_like(w);
+  if (need_x) grads[0] = fresh_like(x);
+  if (need_thr) grads[1] = fresh_like(thr);
+  if (need_w) grads[3] = fresh_like(w);
   torch::Tensor ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.window_cells);
   dispatch_real(x, [&](auto real) {

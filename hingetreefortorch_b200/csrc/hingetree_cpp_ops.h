@@ -21,6 +21,11 @@ int64_t threshold_count(int kind, int depth);
 void require_cuda(const torch::Tensor &t);
 void require_float32(const torch::Tensor &t);
 torch::Tensor make_workspace(size_t bytes, const torch::Tensor &like);
+// Uninitialised contiguous memory on `like`'s device.  Straight from the allocator: torch.empty costs 2.5 us of dispatch, and
+// in deterministic mode a launch that fills it (with what every operator here overwrites).
+torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like, c10::ScalarType type);
+inline torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like) { return fresh(sizes, like, like.scalar_type()); }
+inline torch::Tensor fresh_like(const torch::Tensor &like) { return fresh(like.sizes(), like); }
 void set_ordinal_check(const std::string &mode);
 int64_t pipeline_status();
 

@@ -109,10 +109,11 @@ using FusionFeature = FusionFeatureOf<float>;
 // The traversal.  One plain fp32 subtract per level; `m > 0` sends NaN and 0 to the left;
 // strict `<` keeps the shallowest minimum.  Level 0 seeds the minimum, which is what the
 // reference's initialisation from vertex 0 amounts to (also for NaN margins).
-template <int KIND, typename OrdT, typename Feature>
+// `ord`: the tree's feature indices, a pointer or anything with [].
+template <int KIND, typename Ordinals, typename Feature>
 __device__ __forceinline__ PathOf<typename Feature::value_type> traverse(const Feature &feat,
                                                                         const typename Feature::value_type *__restrict__ thr,
-                                                                        const OrdT *__restrict__ ord, int depth) {
+                                                                        const Ordinals &ord, int depth) {
   typedef typename Feature::value_type Real;
   PathOf<Real> p;
   p.key = 0;
@@ -146,8 +147,37 @@ inline int check_forest_problem(const ht_forest_problem *p) {
   return HT_OK;
 }
 
-// Converts int64 ordinals to int32, clamping out-of-range values to 0 and flagging them.
-int pack_ordinals(const int64_t *ord, int64_t n, int64_t C, int32_t *packed, uint32_t *status_word,
-                  cudaStream_t stream);
+// The int64 feature indices of a call, read in place: out-of-range ones count as 0.
+struct WideOrdinals {
+  const int64_t *__restrict__ at;
+  int64_t channels;
+  __device__ __forceinline__ int operator[](int64_t e) const {
+    const int64_t o = __ldg(at + e);
+    return (uint64_t)o < (uint64_t)channels ? (int)o : 0;
+  }
+  __device__ __forceinline__ bool valid(int64_t e) const { return (uint64_t)__ldg(at + e) < (uint64_t)channels; }
+};
+
+// Memory to be zeroed before the kernels of a call add into it.
+struct ClearList {
+  static constexpr int kMost = 5;
+  void *at[kMost];
+  size_t bytes[kMost];
+  int count = 0;
+  // `p` may be null (nothing to clear); addresses and sizes are multiples of 4 bytes
+  void add(void *p, size_t size) {
+    if (p == nullptr || size == 0) return;
+    at[count] = p;
+    bytes[count++] = size;
+  }
+};
+
+// What comes before the kernels of most calls, as one launch: int64 ordinals to int32 (n of them, none with ord == nullptr),
+// out-of-range ones to 0 and flagged, and the memory in `clear` to zero.  Launches nothing when there is nothing to do.
+int pack_and_clear(const int64_t *ord, int64_t n, int64_t C, int32_t *packed, uint32_t *status_word, const ClearList &clear,
+                   cudaStream_t stream);
+inline int pack_ordinals(const int64_t *ord, int64_t n, int64_t C, int32_t *packed, uint32_t *status_word, cudaStream_t stream) {
+  return pack_and_clear(ord, n, C, packed, status_word, ClearList(), stream);
+}
 
 }  // namespace ht

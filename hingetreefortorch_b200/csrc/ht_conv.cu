@@ -399,7 +399,8 @@ size_t conv_records_bytes(const ht_conv_problem *p, const ConvShape &a) {
 
 template <typename Real>
 int prepare_conv(const ht_conv_problem *p, const Real *x, const Real *thr, const int64_t *ord, const Real *w,
-                 void *workspace, size_t workspace_bytes, uint32_t *status_word, cudaStream_t stream, ConvArgsOf<Real> &a) {
+                 void *workspace, size_t workspace_bytes, uint32_t *status_word, cudaStream_t stream, ConvArgsOf<Real> &a,
+                 Real *gx = nullptr, Real *gthr = nullptr, Real *gw = nullptr) {
   const int rc = check_conv(p, a);
   if (rc != HT_OK) return rc;
   const int64_t decisions = a.Co * a.Ci * a.N;
@@ -413,7 +414,11 @@ int prepare_conv(const ht_conv_problem *p, const Real *x, const Real *thr, const
   a.thr = thr;
   a.w = w;
   a.ord = static_cast<const int32_t *>(workspace);
-  return pack_ordinals(ord, decisions, a.cells, static_cast<int32_t *>(workspace), status_word, stream);
+  ClearList clear;
+  clear.add(gx, sizeof(Real) * (size_t)(a.B * a.Ci * a.in_count));
+  clear.add(gthr, sizeof(Real) * (size_t)decisions);
+  clear.add(gw, sizeof(Real) * (size_t)(a.Co * a.Ci * a.L * a.M));
+  return pack_and_clear(ord, decisions, a.cells, static_cast<int32_t *>(workspace), status_word, clear, stream);
 }
 
 template <typename Word>
@@ -521,14 +526,8 @@ int conv_backward(const ht_conv_problem *p, const Real *x, const Real *thr, cons
                   ht_stream_t stream) {
   ConvArgsOf<Real> a;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const int rc = prepare_conv<Real>(p, x, thr, ord, w, workspace, workspace_bytes, status_word, s, a);
+  const int rc = prepare_conv<Real>(p, x, thr, ord, w, workspace, workspace_bytes, status_word, s, a, gx, gthr, gw);
   if (rc != HT_OK) return rc;
-  if (gx != nullptr && a.B * a.Ci * a.in_count > 0)
-    HT_CUDA_TRY(cudaMemsetAsync(gx, 0, sizeof(Real) * (size_t)(a.B * a.Ci * a.in_count), s));
-  if (gthr != nullptr && a.Co * a.Ci * a.N > 0)
-    HT_CUDA_TRY(cudaMemsetAsync(gthr, 0, sizeof(Real) * (size_t)(a.Co * a.Ci * a.N), s));
-  if (gw != nullptr && a.Co * a.Ci * a.L * a.M > 0)
-    HT_CUDA_TRY(cudaMemsetAsync(gw, 0, sizeof(Real) * (size_t)(a.Co * a.Ci * a.L * a.M), s));
   const int64_t threads = a.B * a.Co * a.out_count;
   if (threads * a.M == 0 || (gx == nullptr && gthr == nullptr && gw == nullptr)) return HT_OK;
   if (g == nullptr) return HT_ERR_INVALID_ARGUMENT;

@@ -4,6 +4,7 @@
 // parameters and the input through L1/L2.  They accept every shape the reference accepts
 // (any C, K, M, depth up to 31).  Shapes the shared-memory tile kernel (ht_forest_tiled.cu)
 // can take are routed there by ht_forest_forward_f32.
+#include <algorithm>
 #include <atomic>
 
 #include "ht_common.cuh"
@@ -21,16 +22,27 @@ namespace {
 
 constexpr int kBlock = 256;
 
-__global__ void pack_ordinals_kernel(const int64_t *__restrict__ ord, int64_t n, int64_t C,
-                                     int32_t *__restrict__ packed, uint32_t *status_word) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  int64_t o = ord[e];
-  if (o < 0 || o >= C) {
-    o = 0;
-    if (status_word != nullptr) atomicOr(status_word, HT_FLAG_ORDINAL_RANGE);
+// Bound by launch latency for small calls (three memsets and a packing kernel took 4 launches, 8 us of host and device
+// time, in a step of 100 x 100 evaluations) and by HBM writes for large gradients.
+__global__ void __launch_bounds__(kBlock) pack_and_clear_kernel(const int64_t *__restrict__ ord, int64_t n, int64_t C,
+                                                                int32_t *__restrict__ packed, uint32_t *status_word,
+                                                                const __grid_constant__ ClearList clear) {
+  const int64_t first = (int64_t)blockIdx.x * kBlock + threadIdx.x, step = (int64_t)gridDim.x * kBlock;
+  for (int64_t e = first; e < n; e += step) {
+    int64_t o = ord[e];
+    if (o < 0 || o >= C) {
+      o = 0;
+      if (status_word != nullptr) atomicOr(status_word, HT_FLAG_ORDINAL_RANGE);
+    }
+    packed[e] = (int32_t)o;
   }
-  packed[e] = (int32_t)o;
+  for (int r = 0; r < clear.count; ++r) {
+    unsigned char *at = static_cast<unsigned char *>(clear.at[r]);
+    const size_t bytes = clear.bytes[r];
+    const int64_t quads = (reinterpret_cast<uintptr_t>(at) & 15u) == 0 ? (int64_t)(bytes / 16) : 0;
+    for (int64_t e = first; e < quads; e += step) reinterpret_cast<uint4 *>(at)[e] = make_uint4(0, 0, 0, 0);
+    for (int64_t e = 4 * quads + first; e < (int64_t)(bytes / 4); e += step) reinterpret_cast<uint32_t *>(at)[e] = 0;
+  }
 }
 
 template <typename Real>
@@ -290,11 +302,10 @@ struct PreparedOf {
 };
 using Prepared = PreparedOf<float>;
 
-// Validates the call, converts the ordinals into the workspace and fills the kernel arguments.
+// Validates the call and fills the kernel arguments; pack_now() then converts the ordinals into the workspace.
 template <typename Real>
 int prepare(const ht_forest_problem *p, const Real *x, const Real *thr, const int64_t *ord, const Real *w,
-            bool need_w, void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream,
-            PreparedOf<Real> &out) {
+            bool need_w, void *workspace, size_t workspace_bytes, ht_stream_t stream, PreparedOf<Real> &out) {
   const int rc = check_forest_problem(p);
   if (rc != HT_OK) return rc;
   // a null pointer is only acceptable for a tensor without elements
@@ -321,11 +332,14 @@ int prepare(const ht_forest_problem *p, const Real *x, const Real *thr, const in
   a.L = ((int64_t)1) << p->depth;
   out.stream = reinterpret_cast<cudaStream_t>(stream);
   out.evals = p->B * p->T * p->K;
-  if (a.T * a.N > 0) {
-    const int prc = pack_ordinals(ord, a.T * a.N, a.C, static_cast<int32_t *>(workspace), status_word, out.stream);
-    if (prc != HT_OK) return prc;
-  }
   return HT_OK;
+}
+
+// Small calls read the int64 ordinals in place: packing them first is a launch of its own (2 us of host time and as much on
+// the device), which pays from a million evaluations on, or where a tree has far more decisions than samples to check them.
+template <typename Real>
+bool small_enough_for_wide(const PreparedOf<Real> &pr) {
+  return pr.evals <= (1 << 20) && pr.args.T * pr.args.N <= 4 * pr.evals;
 }
 
 template <int MODE, typename Real>
@@ -340,17 +354,16 @@ int launch_any(const ht_forest_problem *p, const PreparedOf<Real> &pr, Real *out
   return HT_OK;
 }
 
-// Clears the requested gradients (the entry points' contract).
+// Ordinals into the workspace (not with ord == nullptr) and the given gradients to zero (the entry points' contract).
 template <typename Real>
-int clear_gradients(const PreparedOf<Real> &pr, Real *gx, Real *gthr, Real *gw) {
+int pack_now(const PreparedOf<Real> &pr, const int64_t *ord, uint32_t *status_word, Real *gx = nullptr, Real *gthr = nullptr,
+             Real *gw = nullptr) {
   const ForestArgsOf<Real> &a = pr.args;
-  if (gx != nullptr && a.B * a.C * a.K > 0)
-    HT_CUDA_TRY(cudaMemsetAsync(gx, 0, sizeof(Real) * (size_t)(a.B * a.C * a.K), pr.stream));
-  if (gthr != nullptr && a.T * a.N > 0)
-    HT_CUDA_TRY(cudaMemsetAsync(gthr, 0, sizeof(Real) * (size_t)(a.T * a.N), pr.stream));
-  if (gw != nullptr && a.T * a.L * a.M > 0)
-    HT_CUDA_TRY(cudaMemsetAsync(gw, 0, sizeof(Real) * (size_t)(a.T * a.L * a.M), pr.stream));
-  return HT_OK;
+  ClearList clear;
+  clear.add(gx, sizeof(Real) * (size_t)(a.B * a.C * a.K));
+  clear.add(gthr, sizeof(Real) * (size_t)(a.T * a.N));
+  clear.add(gw, sizeof(Real) * (size_t)(a.T * a.L * a.M));
+  return pack_and_clear(ord, a.T * a.N, a.C, const_cast<int32_t *>(a.ord), status_word, clear, pr.stream);
 }
 
 // The backward with the any-shape kernels: one traversal and atomic scatters in default mode; in fixed-order
@@ -404,10 +417,14 @@ int backward_any(const ht_forest_problem *p, const PreparedOf<Real> &pr, const R
 
 }  // namespace
 
-int pack_ordinals(const int64_t *ord, int64_t n, int64_t C, int32_t *packed, uint32_t *status_word,
-                  cudaStream_t stream) {
-  if (n <= 0) return HT_OK;
-  pack_ordinals_kernel<<<blocks_for(n, kBlock), kBlock, 0, stream>>>(ord, n, C, packed, status_word);
+int pack_and_clear(const int64_t *ord, int64_t n, int64_t C, int32_t *packed, uint32_t *status_word, const ClearList &clear,
+                   cudaStream_t stream) {
+  if (ord == nullptr) n = 0;
+  int64_t work = n;
+  for (int r = 0; r < clear.count; ++r) work = std::max<int64_t>(work, (int64_t)(clear.bytes[r] / 16) + 4);
+  if (work <= 0) return HT_OK;
+  const int64_t blocks = std::min<int64_t>((work + kBlock - 1) / kBlock, 148 * 8);
+  pack_and_clear_kernel<<<(unsigned)blocks, kBlock, 0, stream>>>(ord, n, C, packed, status_word, clear);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }
@@ -476,9 +493,9 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
                           const float *w, float *out, void *workspace, size_t workspace_bytes,
                           uint32_t *status_word, ht_stream_t stream) {
   Prepared pr;
-  const int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, stream, pr);
   if (rc != HT_OK) return rc;
-  if (pr.evals * p->M == 0) return HT_OK;
+  if (pr.evals * p->M == 0) return pack_now(pr, ord, status_word);
   if (out == nullptr) return HT_ERR_INVALID_ARGUMENT;
   // HT_SAVE_FOR_BACKWARD: the traversal goes to the evaluation-record area of the workspace, when it is there
   unsigned char *ws = static_cast<unsigned char *>(workspace);
@@ -487,12 +504,20 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
     const size_t records_at = ordinals_bytes(p) + forward_tiled_workspace_bytes(p);
     if (workspace_bytes >= records_at + records_bytes(p)) eval_records = ws + records_at;
   }
-  const int trc = forward_tiled(p, x, thr, pr.args.ord, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
-  if (trc != HT_ERR_UNSUPPORTED) return trc;
+  const WideOrdinals wide = {ord, p->C};
+  int32_t *packed = static_cast<int32_t *>(workspace);
+  rc = forward_tiled(p, x, thr, packed, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream, &wide);
+  if (rc != HT_ERR_UNSUPPORTED) return rc;
+  if (eval_records == nullptr && small_enough_for_wide(pr)) {
+    rc = multi_forward(p, x, thr, nullptr, w, out, PathRecordsOf<float>{nullptr, nullptr}, pr.stream, &wide, status_word);
+    if (rc != HT_ERR_UNSUPPORTED) return rc;
+  }
+  rc = pack_now(pr, ord, status_word);
+  if (rc != HT_OK) return rc;
   if (p->M > 1 || eval_records != nullptr) {
     const PathRecordsOf<float> paths = eval_records != nullptr ? saved_paths(p, eval_records) : PathRecordsOf<float>{nullptr, nullptr};
-    const int mrc = multi_forward(p, x, thr, pr.args.ord, w, out, paths, pr.stream);
-    if (mrc != HT_ERR_UNSUPPORTED || eval_records != nullptr) return mrc;
+    rc = multi_forward(p, x, thr, packed, w, out, paths, pr.stream);
+    if (rc != HT_ERR_UNSUPPORTED || eval_records != nullptr) return rc;
   }
   return launch_any<MODE_FORWARD>(p, pr, out, nullptr);
 }
@@ -501,7 +526,8 @@ int ht_forest_leafmap_f32(const ht_forest_problem *p, const float *x, const floa
                           int64_t *leaf, void *workspace, size_t workspace_bytes, uint32_t *status_word,
                           ht_stream_t stream) {
   Prepared pr;
-  const int rc = prepare<float>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare<float>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, stream, pr);
+  if (rc == HT_OK) rc = pack_now(pr, ord, status_word);
   if (rc != HT_OK) return rc;
   if (leaf == nullptr && pr.evals > 0) return HT_ERR_INVALID_ARGUMENT;
   return launch_any<MODE_LEAFMAP, float>(p, pr, nullptr, leaf);
@@ -511,7 +537,8 @@ int ht_forest_marginmap_f32(const ht_forest_problem *p, const float *x, const fl
                             float *margin, int64_t *margin_ord, void *workspace, size_t workspace_bytes,
                             uint32_t *status_word, ht_stream_t stream) {
   Prepared pr;
-  const int rc = prepare<float>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare<float>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, stream, pr);
+  if (rc == HT_OK) rc = pack_now(pr, ord, status_word);
   if (rc != HT_OK) return rc;
   if ((margin == nullptr || margin_ord == nullptr) && pr.evals > 0) return HT_ERR_INVALID_ARGUMENT;
   return launch_any<MODE_MARGINMAP>(p, pr, margin, margin_ord);
@@ -521,7 +548,8 @@ int ht_forest_reachability_f32(const ht_forest_problem *p, const float *x, const
                                int64_t *counts, void *workspace, size_t workspace_bytes, uint32_t *status_word,
                                ht_stream_t stream) {
   Prepared pr;
-  const int rc = prepare<float>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare<float>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, stream, pr);
+  if (rc == HT_OK) rc = pack_now(pr, ord, status_word);
   if (rc != HT_OK) return rc;
   if (counts == nullptr && pr.args.T > 0) return HT_ERR_INVALID_ARGUMENT;
   if (pr.args.T * pr.args.L > 0)
@@ -533,16 +561,11 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
                            const float *w, const float *g, float *gx, float *gthr, float *gw, void *workspace,
                            size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {
   Prepared pr;
-  const int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr);
+  const int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, stream, pr);
   if (rc != HT_OK) return rc;
   if (g == nullptr && pr.evals * p->M > 0) return HT_ERR_INVALID_ARGUMENT;
   const ForestArgs &a = pr.args;
-  // The parameter gradients are sums into cleared memory on every path.  The x gradient is cleared only for the
-  // paths that add into it: from a kept traversal it is written tile by tile, every element once.
-  int crc = clear_gradients(pr, static_cast<float *>(nullptr), gthr, gw);
-  if (crc != HT_OK) return crc;
-  if (pr.evals * a.M == 0 || (gx == nullptr && gthr == nullptr && gw == nullptr))
-    return clear_gradients(pr, gx, static_cast<float *>(nullptr), static_cast<float *>(nullptr));
+  if (pr.evals * a.M == 0 || (gx == nullptr && gthr == nullptr && gw == nullptr)) return pack_now(pr, ord, status_word, gx, gthr, gw);
 
   {
     // Tile kernels when the shape qualifies; with room for the evaluation records in the workspace
@@ -552,24 +575,32 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
     const size_t eval_bytes = records_bytes(p);
     void *eval_records = eval_bytes > 0 && workspace_bytes >= records_at + eval_bytes ? ws + records_at : nullptr;
     const bool ordered = ordered_from_paths(p);
-    if ((p->flags & HT_SAVED_FORWARD) != 0 && eval_records != nullptr && p->M == 1 && !ordered) {
+    // what a saving forward left in the workspace: the paths, and the packed ordinals
+    const bool kept = (p->flags & HT_SAVED_FORWARD) != 0 && eval_records != nullptr && ht_forest_forward_saves(p);
+    const int64_t *to_pack = kept ? nullptr : ord;
+    // The parameter gradients are sums into cleared memory on every path.  The x gradient is cleared only for the
+    // paths that add into it: from a kept traversal it is written tile by tile, every element once.
+    float *none = nullptr;
+    bool gx_cleared = !(kept && p->M == 1 && !ordered);
+    int crc = pack_now(pr, to_pack, status_word, gx_cleared ? gx : none, gthr, gw);
+    if (crc != HT_OK) return crc;
+    if (!gx_cleared) {
       // the records of the forward that ran on these inputs are still there: no tree is walked again
       const int src = backward_saved(p, a.ord, w, g, gx, gthr, gw, eval_records, pr.stream);
       if (src != HT_ERR_UNSUPPORTED) return src;
+      crc = pack_now(pr, nullptr, status_word, gx);
+      if (crc != HT_OK) return crc;
     }
-    crc = clear_gradients(pr, gx, static_cast<float *>(nullptr), static_cast<float *>(nullptr));
-    if (crc != HT_OK) return crc;
     if (!ordered || eval_records == nullptr) {
       const int trc = backward_tiled(p, x, thr, a.ord, w, g, gx, gthr, gw, ws + ordinals_bytes(p), eval_records,
                                      status_word, pr.stream);
       if (trc != HT_ERR_UNSUPPORTED) return trc;
     }
     if ((p->M > 1 || ordered) && eval_records != nullptr) {
-      const bool kept = (p->flags & HT_SAVED_FORWARD) != 0 && ht_forest_forward_saves(p);
       if (!kept && (!ordered || gthr != nullptr || gw != nullptr)) {  // the paths first
-        float *none = nullptr;
         int prc = p->M == 1 ? HT_ERR_UNSUPPORTED
-                            : forward_tiled(p, x, thr, a.ord, w, none, ws + ordinals_bytes(p), eval_records, status_word, pr.stream);
+                            : forward_tiled(p, x, thr, static_cast<int32_t *>(workspace), w, none, ws + ordinals_bytes(p), eval_records,
+                                          status_word, pr.stream);
         if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, saved_paths(p, eval_records), pr.stream);
         if (prc != HT_OK) return prc;
       }
@@ -577,7 +608,6 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
         const int orc = ordered_parameters(p, w, g, gthr, gw, saved_paths(p, eval_records),
                                            static_cast<unsigned char *>(eval_records) + saved_bytes(p), pr.stream);
         if (orc != HT_OK || gx == nullptr) return orc;
-        float *none = nullptr;
         // the tile kernels' x gradient has the reference's order too; tabular samples too few for their tiles take a warp each
         if (p->M == 1) {
           int xrc = kept ? backward_saved(p, a.ord, w, g, gx, none, none, eval_records, pr.stream) : HT_ERR_UNSUPPORTED;
@@ -600,17 +630,29 @@ int ht_forest_forward_f64(const ht_forest_problem *p, const double *x, const dou
                           const double *w, double *out, void *workspace, size_t workspace_bytes, uint32_t *status_word,
                           ht_stream_t stream) {
   PreparedOf<double> pr;
-  const int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, stream, pr);
   if (rc != HT_OK) return rc;
-  if (pr.evals * p->M == 0) return HT_OK;
+  if (pr.evals * p->M == 0) return pack_now(pr, ord, status_word);
   if (out == nullptr) return HT_ERR_INVALID_ARGUMENT;
+  if (small_enough_for_wide(pr)) {
+    const WideOrdinals wide = {ord, p->C};
+    rc = multi_forward(p, x, thr, nullptr, w, out, PathRecordsOf<double>{nullptr, nullptr}, pr.stream, &wide, status_word);
+    if (rc != HT_ERR_UNSUPPORTED) return rc;
+  }
+  rc = pack_now(pr, ord, status_word);
+  if (rc != HT_OK) return rc;
+  if (p->M > 1) {
+    rc = multi_forward(p, x, thr, pr.args.ord, w, out, PathRecordsOf<double>{nullptr, nullptr}, pr.stream);
+    if (rc != HT_ERR_UNSUPPORTED) return rc;
+  }
   return launch_any<MODE_FORWARD>(p, pr, out, nullptr);
 }
 
 int ht_forest_leafmap_f64(const ht_forest_problem *p, const double *x, const double *thr, const int64_t *ord, int64_t *leaf,
                           void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {
   PreparedOf<double> pr;
-  const int rc = prepare<double>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare<double>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, stream, pr);
+  if (rc == HT_OK) rc = pack_now(pr, ord, status_word);
   if (rc != HT_OK) return rc;
   if (leaf == nullptr && pr.evals > 0) return HT_ERR_INVALID_ARGUMENT;
   return launch_any<MODE_LEAFMAP, double>(p, pr, nullptr, leaf);
@@ -620,7 +662,8 @@ int ht_forest_marginmap_f64(const ht_forest_problem *p, const double *x, const d
                             double *margin, int64_t *margin_ord, void *workspace, size_t workspace_bytes,
                             uint32_t *status_word, ht_stream_t stream) {
   PreparedOf<double> pr;
-  const int rc = prepare<double>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare<double>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, stream, pr);
+  if (rc == HT_OK) rc = pack_now(pr, ord, status_word);
   if (rc != HT_OK) return rc;
   if ((margin == nullptr || margin_ord == nullptr) && pr.evals > 0) return HT_ERR_INVALID_ARGUMENT;
   return launch_any<MODE_MARGINMAP>(p, pr, margin, margin_ord);
@@ -630,7 +673,8 @@ int ht_forest_reachability_f64(const ht_forest_problem *p, const double *x, cons
                                int64_t *counts, void *workspace, size_t workspace_bytes, uint32_t *status_word,
                                ht_stream_t stream) {
   PreparedOf<double> pr;
-  const int rc = prepare<double>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, status_word, stream, pr);
+  int rc = prepare<double>(p, x, thr, ord, nullptr, false, workspace, workspace_bytes, stream, pr);
+  if (rc == HT_OK) rc = pack_now(pr, ord, status_word);
   if (rc != HT_OK) return rc;
   if (counts == nullptr && pr.args.T > 0) return HT_ERR_INVALID_ARGUMENT;
   if (pr.args.T * pr.args.L > 0)
@@ -642,10 +686,10 @@ int ht_forest_backward_f64(const ht_forest_problem *p, const double *x, const do
                            const double *w, const double *g, double *gx, double *gthr, double *gw, void *workspace,
                            size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {
   PreparedOf<double> pr;
-  const int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr);
+  const int rc = prepare(p, x, thr, ord, w, true, workspace, workspace_bytes, stream, pr);
   if (rc != HT_OK) return rc;
   if (g == nullptr && pr.evals * p->M > 0) return HT_ERR_INVALID_ARGUMENT;
-  const int crc = clear_gradients(pr, gx, gthr, gw);
+  const int crc = pack_now(pr, ord, status_word, gx, gthr, gw);
   if (crc != HT_OK) return crc;
   if (pr.evals * p->M == 0 || (gx == nullptr && gthr == nullptr && gw == nullptr)) return HT_OK;
   return backward_any(p, pr, g, gx, gthr, gw);

@@ -220,7 +220,7 @@ size_t record_bytes(const ht_forest_problem *p, size_t real_bytes) { return alig
 template <typename Real>
 int prepare(const ht_forest_problem *p, const Real *img, const Real *vec, int64_t Cv, const Real *thr,
             const int64_t *ord, const Real *w, bool with_records, void *workspace, size_t workspace_bytes,
-            uint32_t *status_word, ht_stream_t stream, PreparedOf<Real> &out) {
+            uint32_t *status_word, ht_stream_t stream, PreparedOf<Real> &out, const ClearList &clear = ClearList()) {
   const int rc = check_forest_problem(p);
   if (rc != HT_OK) return rc;
   if (Cv < 0 || (vec == nullptr && p->B * Cv > 0)) return HT_ERR_INVALID_ARGUMENT;
@@ -255,7 +255,7 @@ int prepare(const ht_forest_problem *p, const Real *img, const Real *vec, int64_
     out.records.leaf = reinterpret_cast<int32_t *>(ws + ordinal_bytes(p) + record_bytes(p, sizeof(Real)));
     out.records.vertex = reinterpret_cast<int32_t *>(ws + ordinal_bytes(p) + record_bytes(p, sizeof(Real)) + record_bytes(p, 4));
   }
-  return pack_ordinals(ord, decisions, p->C + Cv, reinterpret_cast<int32_t *>(ws), status_word, out.stream);
+  return pack_and_clear(ord, decisions, p->C + Cv, reinterpret_cast<int32_t *>(ws), status_word, clear, out.stream);
 }
 
 template <typename Real>
@@ -269,10 +269,17 @@ int run_paths(const ht_forest_problem *p, const PreparedOf<Real> &pr) {
   return HT_OK;
 }
 
+// The gradients of a backward, all of them sums into cleared memory (those that are not asked for are null).
 template <typename Real>
-int clear(Real *ptr, int64_t count, cudaStream_t stream) {
-  if (ptr != nullptr && count > 0) HT_CUDA_TRY(cudaMemsetAsync(ptr, 0, sizeof(Real) * (size_t)count, stream));
-  return HT_OK;
+ClearList gradients(const ht_forest_problem *p, int64_t Cv, Real *gimg, Real *gvec, Real *gthr, Real *gw, Real *glin, int64_t linear) {
+  ClearList clear;
+  if (check_forest_problem(p) != HT_OK || Cv < 0 || linear < 0) return clear;
+  clear.add(gimg, sizeof(Real) * (size_t)(p->B * p->C * p->K));
+  clear.add(gvec, sizeof(Real) * (size_t)(p->B * Cv));
+  clear.add(gthr, sizeof(Real) * (size_t)(p->T * threshold_count(p->kind, p->depth)));
+  clear.add(gw, sizeof(Real) * ((size_t)(p->T * p->M) << p->depth));
+  clear.add(glin, sizeof(Real) * (size_t)(linear * p->T));
+  return clear;
 }
 
 }  // namespace
@@ -303,14 +310,10 @@ int fusion_backward(const ht_forest_problem *p, const Real *img, const Real *vec
                     const int64_t *ord, const Real *w, const Real *g, Real *gimg, Real *gvec, Real *gthr, Real *gw,
                     void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {
   PreparedOf<Real> pr;
-  const int rc = prepare<Real>(p, img, vec, vec_channels, thr, ord, w, false, workspace, workspace_bytes, status_word, stream, pr);
+  const int rc = prepare<Real>(p, img, vec, vec_channels, thr, ord, w, false, workspace, workspace_bytes, status_word, stream, pr,
+                               gradients<Real>(p, vec_channels, gimg, gvec, gthr, gw, nullptr, 0));
   if (rc != HT_OK) return rc;
   const FusionArgsOf<Real> &a = pr.args;
-  int crc;
-  if ((crc = clear(gimg, a.B * a.C * a.K, pr.stream)) != HT_OK) return crc;
-  if ((crc = clear(gvec, a.B * a.Cv, pr.stream)) != HT_OK) return crc;
-  if ((crc = clear(gthr, a.T * a.N, pr.stream)) != HT_OK) return crc;
-  if ((crc = clear(gw, a.T * a.L * a.M, pr.stream)) != HT_OK) return crc;
   if (pr.evals * a.M == 0) return HT_OK;
   if (g == nullptr) return HT_ERR_INVALID_ARGUMENT;
   if (p->kind == TREE)
@@ -345,16 +348,11 @@ int linear_backward(const ht_forest_problem *p, int64_t out_channels, const Real
                     Real *gthr, Real *gw, Real *glin, void *workspace, size_t workspace_bytes, uint32_t *status_word,
                     ht_stream_t stream) {
   PreparedOf<Real> pr;
-  const int rc = prepare<Real>(p, img, vec, vec_channels, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr);
+  const int rc = prepare<Real>(p, img, vec, vec_channels, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr,
+                               gradients<Real>(p, vec_channels, gimg, gvec, gthr, gw, glin, out_channels));
   if (rc != HT_OK) return rc;
   if (out_channels < 0) return HT_ERR_INVALID_ARGUMENT;
   const FusionArgsOf<Real> &a = pr.args;
-  int crc;
-  if ((crc = clear(gimg, a.B * a.C * a.K, pr.stream)) != HT_OK) return crc;
-  if ((crc = clear(gvec, a.B * a.Cv, pr.stream)) != HT_OK) return crc;
-  if ((crc = clear(gthr, a.T * a.N, pr.stream)) != HT_OK) return crc;
-  if ((crc = clear(gw, a.T * a.L * a.M, pr.stream)) != HT_OK) return crc;
-  if ((crc = clear(glin, out_channels * a.T, pr.stream)) != HT_OK) return crc;
   if (pr.evals * a.M * out_channels == 0) return HT_OK;
   if (g == nullptr || lin == nullptr) return HT_ERR_INVALID_ARGUMENT;
   const int prc = run_paths<Real>(p, pr);

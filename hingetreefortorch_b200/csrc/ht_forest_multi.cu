@@ -64,6 +64,8 @@ template <typename Real>
 struct MultiForwardArgs {
   const Real *x, *thr, *w;
   const int32_t *ord;
+  WideOrdinals wide;  // WIDE kernels
+  uint32_t *status_word;
   Real *out;
   Real *margin;
   void *where;
@@ -76,7 +78,7 @@ struct MultiForwardArgs {
 // outputs of its own evaluation makes every store of the warp touch 32 rows; here the warp's outputs, which are 32 * M
 // consecutive numbers, leave in 16-byte pieces that consecutive lanes own, each lane asking the evaluation's owner for
 // |margin| and the leaf.  x [8, 100, 32, 32], 100 trees of depth 7, 8 x 8 outputs (210 MB): 287 -> 41 us.
-template <int KIND, int V, typename Real>
+template <int KIND, int V, bool WIDE, typename Real>
 __global__ void __launch_bounds__(kForwardThreads) multi_forward_kernel(const __grid_constant__ MultiForwardArgs<Real> a) {
   const int64_t e = (int64_t)blockIdx.x * kForwardThreads + threadIdx.x;
   const int lane = threadIdx.x & 31;
@@ -94,7 +96,15 @@ __global__ void __launch_bounds__(kForwardThreads) multi_forward_kernel(const __
       j = ij - i * a.T;
     }
     const PlainFeatureOf<Real> feat{a.x + i * a.C * a.K + k, a.K};
-    const PathOf<Real> p = traverse<KIND>(feat, a.thr + j * a.N, a.ord + j * a.N, a.depth);
+    PathOf<Real> p;
+    if constexpr (WIDE) {
+      // small calls: this launch checks the ordinals too, which a packing kernel would have done
+      for (int64_t o = e; o < a.T * a.N; o += a.evals)
+        if (!a.wide.valid(o) && a.status_word != nullptr) atomicOr(a.status_word, HT_FLAG_ORDINAL_RANGE);
+      p = traverse<KIND>(feat, a.thr + j * a.N, WideOrdinals{a.wide.at + j * a.N, a.wide.channels}, a.depth);
+    } else {
+      p = traverse<KIND>(feat, a.thr + j * a.N, a.ord + j * a.N, a.depth);
+    }
     am = abs_of(p.margin);
     leaf = (uint32_t)(j * a.L) + p.key;  // T * L < 2^32 (host)
     if (a.margin != nullptr) {
@@ -456,15 +466,15 @@ int launch_sorted_width(const SortedArgs<Real> &a, unsigned grid, size_t smem, c
   return HT_ERR_UNSUPPORTED;
 }
 
-template <int KIND, typename Real>
+template <int KIND, bool WIDE, typename Real>
 int launch_forward(const MultiForwardArgs<Real> &a, int width, cudaStream_t stream) {
   const unsigned grid = (unsigned)((a.evals + kForwardThreads - 1) / kForwardThreads);
   if (width == 1)
-    multi_forward_kernel<KIND, 1, Real><<<grid, kForwardThreads, 0, stream>>>(a);
+    multi_forward_kernel<KIND, 1, WIDE, Real><<<grid, kForwardThreads, 0, stream>>>(a);
   else if (width == 2)
-    multi_forward_kernel<KIND, 2, Real><<<grid, kForwardThreads, 0, stream>>>(a);
+    multi_forward_kernel<KIND, 2, WIDE, Real><<<grid, kForwardThreads, 0, stream>>>(a);
   else if constexpr (sizeof(Real) == 4)
-    multi_forward_kernel<KIND, 4, Real><<<grid, kForwardThreads, 0, stream>>>(a);
+    multi_forward_kernel<KIND, 4, WIDE, Real><<<grid, kForwardThreads, 0, stream>>>(a);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }
@@ -486,7 +496,7 @@ size_t multi_area_bytes(const ht_forest_problem *p, size_t real_bytes) {
 
 template <typename Real>
 int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, const int32_t *ord, const Real *w, Real *out,
-                  PathRecordsOf<Real> paths, cudaStream_t stream) {
+                  PathRecordsOf<Real> paths, cudaStream_t stream, const WideOrdinals *wide, uint32_t *status_word) {
   MultiForwardArgs<Real> a = {};
   a.evals = p->B * p->T * p->K;
   a.T = p->T;
@@ -508,7 +518,12 @@ int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, co
   a.margin = paths.margin;
   a.where = paths.where;
   const int width = vector_width(p->M, sizeof(Real), {w, out});
-  return p->kind == TREE ? launch_forward<TREE>(a, width, stream) : launch_forward<FERN>(a, width, stream);
+  if (wide != nullptr) {
+    a.wide = *wide;
+    a.status_word = status_word;
+    return p->kind == TREE ? launch_forward<TREE, true>(a, width, stream) : launch_forward<FERN, true>(a, width, stream);
+  }
+  return p->kind == TREE ? launch_forward<TREE, false>(a, width, stream) : launch_forward<FERN, false>(a, width, stream);
 }
 
 template <typename Real>
@@ -549,9 +564,9 @@ int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w
 }
 
 template int multi_forward<float>(const ht_forest_problem *, const float *, const float *, const int32_t *, const float *,
-                                  float *, PathRecordsOf<float>, cudaStream_t);
+                                  float *, PathRecordsOf<float>, cudaStream_t, const WideOrdinals *, uint32_t *);
 template int multi_forward<double>(const ht_forest_problem *, const double *, const double *, const int32_t *, const double *,
-                                   double *, PathRecordsOf<double>, cudaStream_t);
+                                   double *, PathRecordsOf<double>, cudaStream_t, const WideOrdinals *, uint32_t *);
 template int backward_multi<float>(const ht_forest_problem *, const int32_t *, const float *, const float *, float *, float *,
                                    float *, void *, cudaStream_t);
 template int backward_multi<double>(const ht_forest_problem *, const int32_t *, const double *, const double *, double *,

@@ -30,10 +30,11 @@ PathRecordsOf<Real> multi_paths(const ht_forest_problem *p, void *area) {
 }
 
 // Forward of any shape with the results of a warp written together; where `paths` has a place for them it also leaves the
-// paths, and with out == nullptr nothing else.  HT_ERR_UNSUPPORTED: nothing was launched.
+// paths, and with out == nullptr nothing else.  With `wide` the ordinals are read from there, not from `ord`, and all of them
+// are checked on the way.  HT_ERR_UNSUPPORTED: nothing was launched.
 template <typename Real>
 int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, const int32_t *ord, const Real *w, Real *out,
-                  PathRecordsOf<Real> paths, cudaStream_t stream);
+                  PathRecordsOf<Real> paths, cudaStream_t stream, const WideOrdinals *wide = nullptr, uint32_t *status_word = nullptr);
 
 // Gradients from the paths in `area`.  The gradients that are asked for (the others are null) must have been cleared.
 template <typename Real>

@@ -39,18 +39,6 @@ struct NormalisedArgs {
   int depth;
 };
 
-__global__ void __launch_bounds__(kNormBlock) compact_ordinals_kernel(const int64_t *__restrict__ ord, int64_t n, int64_t C,
-                                                                     int32_t *__restrict__ packed, uint32_t *status_word) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= n) return;
-  int64_t c = ord[e];
-  if (c < 0 || c >= C) {
-    if (status_word != nullptr) atomicOr(status_word, HT_FLAG_ORDINAL_RANGE);
-    c = 0;
-  }
-  packed[e] = (int32_t)c;
-}
-
 // save_margin / save_where (both or neither): the signed margin and the pair (deciding vertex, leaf key) of every
 // (sample, tree), 12 bytes, so that the backward need not read z and walk again.
 template <int KIND>
@@ -231,8 +219,8 @@ extern "C" int ht_forest_normalised_forward_f32(const ht_forest_problem *p, cons
   if (workspace == nullptr || workspace_bytes < ht_forest_normalised_workspace_bytes(p)) return HT_ERR_WORKSPACE;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   int32_t *packed = static_cast<int32_t *>(workspace);
-  compact_ordinals_kernel<<<norm_blocks(a.T * a.N), kNormBlock, 0, stream>>>(ord, a.T * a.N, a.C, packed, status_word);
-  HT_CHECK_LAUNCH();
+  const int prc = pack_ordinals(ord, a.T * a.N, a.C, packed, status_word, stream);
+  if (prc != HT_OK) return prc;
   a.z = z;
   a.mean = mean;
   a.invstd = invstd;
@@ -258,18 +246,19 @@ extern "C" int ht_forest_normalised_backward_f32(const ht_forest_problem *p, con
   if (rc != HT_OK) return rc;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   if (sum_g == nullptr || sum_gy == nullptr) return HT_ERR_INVALID_ARGUMENT;
-  HT_CUDA_TRY(cudaMemsetAsync(sum_g, 0, sizeof(float) * (size_t)a.C, stream));
-  HT_CUDA_TRY(cudaMemsetAsync(sum_gy, 0, sizeof(float) * (size_t)a.C, stream));
-  if (gthr != nullptr) HT_CUDA_TRY(cudaMemsetAsync(gthr, 0, sizeof(float) * (size_t)(a.T * a.N), stream));
-  if (gw != nullptr) HT_CUDA_TRY(cudaMemsetAsync(gw, 0, sizeof(float) * (size_t)(a.T * a.L * a.M), stream));
-  if (a.B == 0 || a.T == 0) return HT_OK;
+  ClearList clear;
+  clear.add(sum_g, sizeof(float) * (size_t)a.C);
+  clear.add(sum_gy, sizeof(float) * (size_t)a.C);
+  clear.add(gthr, sizeof(float) * (size_t)(a.T * a.N));
+  clear.add(gw, sizeof(float) * (size_t)(a.T * a.L * a.M));
+  if (a.B == 0 || a.T == 0) return pack_and_clear(nullptr, 0, 1, nullptr, nullptr, clear, stream);
   if (z == nullptr || mean == nullptr || invstd == nullptr || thr == nullptr || ord == nullptr || w == nullptr || g == nullptr ||
       column == nullptr || value == nullptr)
     return HT_ERR_INVALID_ARGUMENT;
   if (workspace == nullptr || workspace_bytes < ht_forest_normalised_workspace_bytes(p)) return HT_ERR_WORKSPACE;
   int32_t *packed = static_cast<int32_t *>(workspace);
-  compact_ordinals_kernel<<<norm_blocks(a.T * a.N), kNormBlock, 0, stream>>>(ord, a.T * a.N, a.C, packed, status_word);
-  HT_CHECK_LAUNCH();
+  const int prc = pack_and_clear(ord, a.T * a.N, a.C, packed, status_word, clear, stream);
+  if (prc != HT_OK) return prc;
   a.z = z;
   a.mean = mean;
   a.invstd = invstd;

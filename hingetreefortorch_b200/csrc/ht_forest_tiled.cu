@@ -698,8 +698,8 @@ bool forward_saves(const ht_forest_problem *p) {
          saved_samples_per_cta(p) != 0;
 }
 
-int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w,
-                  float *out, void *records, void *eval_records, uint32_t *status_word, cudaStream_t stream) {
+int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, int32_t *ord, const float *w,
+                  float *out, void *records, void *eval_records, uint32_t *status_word, cudaStream_t stream, const WideOrdinals *wide) {
   TilePlan plan;
   if (!(p->K > 1 ? make_inner_plan(p, plan) : make_plan(p, plan))) return HT_ERR_UNSUPPORTED;
   if ((reinterpret_cast<uintptr_t>(x) & 15u) != 0 || (reinterpret_cast<uintptr_t>(out) & 15u) != 0)
@@ -709,10 +709,12 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
   const int64_t elements = p->T * (N + L);
   const unsigned pack_grid = (unsigned)((elements + 255) / 256);
   unsigned char *rec = static_cast<unsigned char *>(records);
+  PackOnTheWay pack;
+  if (wide != nullptr) pack = PackOnTheWay{wide->at, wide->channels, ord, status_word};
   if (plan.ord_bytes == 1)
-    repack_records_kernel<uint8_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec);
+    repack_records_kernel<uint8_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec, RecordMap(), pack);
   else
-    repack_records_kernel<uint16_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec);
+    repack_records_kernel<uint16_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec, RecordMap(), pack);
   HT_CHECK_LAUNCH();
 
   TiledArgs a = {};

@@ -18,8 +18,10 @@ size_t forward_tiled_workspace_bytes(const ht_forest_problem *p);
 // the paths' area of ht_forest_multi.cuh (every shape), and with out == nullptr nothing but the paths is written.
 bool forward_saves(const ht_forest_problem *p);
 int saved_samples_per_cta(const ht_forest_problem *p);  // 0: the backward from saved records does not take the shape
-int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w,
-                  float *out, void *records, void *eval_records, uint32_t *status_word, cudaStream_t stream);
+// With `wide` the ordinals are packed into `ord` on the way to the records.
+int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, int32_t *ord, const float *w,
+                  float *out, void *records, void *eval_records, uint32_t *status_word, cudaStream_t stream,
+                  const WideOrdinals *wide = nullptr);
 
 // The backward from the records a saving forward left (default mode; forward_saves(p) must hold and the inputs must
 // be the forward's).  `ord` are the compact ordinals.  Any of gx / gthr / gw may be null; the others must have been

@@ -304,8 +304,11 @@ extern "C" int ht_linear_tf32_stats_f32(const float *x, const float *w, float *z
   int device = 0, sms = 0;
   HT_CUDA_TRY(cudaGetDevice(&device));
   HT_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-  HT_CUDA_TRY(cudaMemsetAsync(colsum, 0, sizeof(float) * (size_t)N, stream));
-  HT_CUDA_TRY(cudaMemsetAsync(colsumsq, 0, sizeof(float) * (size_t)N, stream));
+  ClearList clear;
+  clear.add(colsum, sizeof(float) * (size_t)N);
+  clear.add(colsumsq, sizeof(float) * (size_t)N);
+  const int crc = pack_and_clear(nullptr, 0, 1, nullptr, nullptr, clear, stream);
+  if (crc != HT_OK) return crc;
   HT_CUDA_TRY(cudaFuncSetAttribute(linear_tf32_stats_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kGemmSmem));
   const unsigned grid = (unsigned)std::min<int64_t>(tiles, std::max(sms, 1));  // one CTA per SM, each walks its tiles
   linear_tf32_stats_kernel<<<grid, kGemmThreads, kGemmSmem, stream>>>(a);

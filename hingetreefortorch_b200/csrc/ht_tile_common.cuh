@@ -87,12 +87,21 @@ struct RecordMap {
   __host__ __device__ int64_t slot(int64_t t) const { return inner == 0 ? t : (t % inner) * outer_count + t / inner; }
 };
 
+// Ordinals that the repack kernel packs on its way (at == nullptr: they are packed already).
+struct PackOnTheWay {
+  const int64_t *at = nullptr;
+  int64_t channels = 0;
+  int32_t *packed = nullptr;
+  uint32_t *status_word = nullptr;
+};
+
 // One thread per record element.  Leaf weights are permuted so that the path bits in the order
 // the traversal collects them (root first, most significant) address them directly.
 template <typename OrdT>
 __global__ void repack_records_kernel(const float *__restrict__ thr, const int32_t *__restrict__ ord,
                                       const float *__restrict__ w, unsigned char *__restrict__ records, int kind,
-                                      int depth, int64_t T, RecordLayout lay, RecordMap map = RecordMap()) {
+                                      int depth, int64_t T, RecordLayout lay, RecordMap map = RecordMap(),
+                                      PackOnTheWay pack = PackOnTheWay()) {
   const int64_t N = threshold_count(kind, depth);
   const int64_t L = ((int64_t)1) << depth;
   const int64_t per_tree = N + L;
@@ -104,7 +113,17 @@ __global__ void repack_records_kernel(const float *__restrict__ thr, const int32
   if (r < N) {
     float t = thr[j * N + r];
     t = t == 0.0f ? 0.0f : t;  // -0 becomes +0
-    const uint32_t c = map.feature((uint32_t)ord[j * N + r]);
+    int32_t feature;
+    if (pack.at != nullptr) {
+      const int64_t o = pack.at[j * N + r];
+      const bool valid = o >= 0 && o < pack.channels;
+      if (!valid && pack.status_word != nullptr) atomicOr(pack.status_word, HT_FLAG_ORDINAL_RANGE);
+      feature = valid ? (int32_t)o : 0;
+      pack.packed[j * N + r] = feature;
+    } else {
+      feature = ord[j * N + r];
+    }
+    const uint32_t c = map.feature((uint32_t)feature);
     reinterpret_cast<float *>(rec + lay.thr)[r] = t;
     if (!lay.paired) {
       reinterpret_cast<OrdT *>(rec + lay.ord)[r] = (OrdT)c;
