@@ -71,15 +71,25 @@ struct LinearNode : public torch::autograd::Function<LinearNode> {
                                const torch::Tensor &w, const torch::Tensor &lin, const torch::Tensor &bias, int64_t kind) {
     ctx->save_for_backward({x, thr, ord, w, lin, bias});
     ctx->saved_data["kind"] = kind;
-    return linear_forward((int)kind, x, nullptr, thr, ord, w, lin, bias);
+    torch::Tensor scratch;
+    const torch::Tensor out = linear_forward((int)kind, x, nullptr, thr, ord, w, lin, bias, &scratch);
+    ctx->saved_data["kept"] = scratch;
+    return out;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const variable_list s = ctx->get_saved_variables();
     const int64_t kind = ctx->saved_data["kind"].toInt();
     refuse_deterministic(grads[0], "backpropagation for hinge " + name_of(kind) + " + linear");
+    torch::Tensor scratch;  // used once: the backward rewrites it
+    const auto kept = ctx->saved_data.find("kept");
+    if (kept != ctx->saved_data.end()) {
+      scratch = kept->second.toTensor();
+      ctx->saved_data.erase(kept);
+    }
     std::vector<torch::Tensor> r =
         linear_backward((int)kind, s[0], ctx->needs_input_grad(0), nullptr, false, s[1], ctx->needs_input_grad(1), s[2], false, s[3],
-                        ctx->needs_input_grad(3), s[4], ctx->needs_input_grad(4), s[5], ctx->needs_input_grad(5), grads[0].contiguous());
+                        ctx->needs_input_grad(3), s[4], ctx->needs_input_grad(4), s[5], ctx->needs_input_grad(5), grads[0].contiguous(),
+                        scratch.defined() ? &scratch : nullptr);
     r.push_back(torch::Tensor());
     return r;
   }

@@ -215,7 +215,7 @@ std::vector<torch::Tensor> fusion_backward(int kind, torch::Tensor img, bool nee
 }  // namespace
 
 torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *vec, torch::Tensor thr, torch::Tensor ord,
-                             torch::Tensor w, torch::Tensor lin, torch::Tensor bias) {
+                             torch::Tensor w, torch::Tensor lin, torch::Tensor bias, torch::Tensor *scratch) {
   FamilyCall call(kind, data, vec, thr, ord, w, &lin, &bias, nullptr);
   c10::DeviceGuard guard(data.device());
   torch::Tensor out = fresh(call.out_sizes, data);
@@ -233,6 +233,7 @@ torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *
                  "fused linear forward");
   });
   og.finish();
+  if (scratch != nullptr) *scratch = ws;
   return out;
 }
 
@@ -240,9 +241,10 @@ torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *
 std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool need_data, const torch::Tensor *vec,
                                            bool need_vec, torch::Tensor thr, bool need_thr, torch::Tensor ord,
                                            bool need_ord, torch::Tensor w, bool need_w, torch::Tensor lin, bool need_lin,
-                                           torch::Tensor bias, bool need_bias, torch::Tensor g) {
+                                           torch::Tensor bias, bool need_bias, torch::Tensor g, const torch::Tensor *scratch) {
   if (need_ord) bad_runtime("Error: Gradient on inOrdinals is requested, but inOrdinals never has a gradient.");
   FamilyCall call(kind, data, vec, thr, ord, w, &lin, &bias, &g);
+  if (scratch != nullptr) call.problem.flags |= HT_SAVED_FORWARD;
   c10::DeviceGuard guard(data.device());
   const bool fusion = vec != nullptr;
   torch::Tensor gdata, gvec, gthr, gw, glin, gbias;
@@ -254,9 +256,11 @@ std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool ne
   if (need_w) gw = fresh_like(w);
   if (need_lin) glin = fresh_like(lin);
   if (gdata.defined() || gthr.defined() || gw.defined() || glin.defined()) {
-    torch::Tensor ws = make_workspace(data.scalar_type() == torch::kFloat64 ? ht_forest_linear_workspace_bytes_f64(&call.problem)
-                                                                                  : ht_forest_linear_workspace_bytes(&call.problem),
-                                     data);
+    torch::Tensor ws = scratch != nullptr ? *scratch
+                                          : make_workspace(data.scalar_type() == torch::kFloat64
+                                                               ? ht_forest_linear_workspace_bytes_f64(&call.problem)
+                                                               : ht_forest_linear_workspace_bytes(&call.problem),
+                                                           data);
     OrdinalGuard og(ord, call.problem.C + call.vec_channels);
     dispatch_real(data, [&](auto real) {
       using Real = decltype(real);

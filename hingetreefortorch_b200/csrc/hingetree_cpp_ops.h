@@ -63,12 +63,14 @@ std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::
 std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, torch::Tensor x, bool need_x, torch::Tensor thr,
                                                  bool need_thr, torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w,
                                                  torch::Tensor g, torch::Tensor saved);
+// `scratch`: receives the forward's workspace, which holds the paths of all evaluations; given to the backward it saves it
+// another walk.
 torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *vec, torch::Tensor thr, torch::Tensor ord,
-                             torch::Tensor w, torch::Tensor lin, torch::Tensor bias);
+                             torch::Tensor w, torch::Tensor lin, torch::Tensor bias, torch::Tensor *scratch = nullptr);
 std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool need_data, const torch::Tensor *vec, bool need_vec,
                                            torch::Tensor thr, bool need_thr, torch::Tensor ord, bool need_ord, torch::Tensor w,
                                            bool need_w, torch::Tensor lin, bool need_lin, torch::Tensor bias, bool need_bias,
-                                           torch::Tensor g);
+                                           torch::Tensor g, const torch::Tensor *scratch = nullptr);
 torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w,
                            std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
                            std::vector<int64_t> dilation);

@@ -9,6 +9,7 @@
 #include <algorithm>
 
 #include "ht_common.cuh"
+#include "ht_forest_linear_tiled.cuh"
 
 namespace ht {
 
@@ -217,10 +218,22 @@ size_t ordinal_bytes(const ht_forest_problem *p) {
 
 size_t record_bytes(const ht_forest_problem *p, size_t real_bytes) { return align_up((size_t)(p->B * p->T * p->K) * real_bytes, 256); }
 
+// Scratch behind the packed ordinals: paths sample by sample, or what the tabular kernels keep, whichever is more.
+size_t path_scratch_bytes(const ht_forest_problem *p, size_t real_bytes) {
+  const size_t paths = record_bytes(p, real_bytes) + 2 * record_bytes(p, 4);
+  return real_bytes == 4 && p->M == 1 && p->K == 1 ? std::max(paths, linear_tiled_bytes(p)) : paths;
+}
+
+// Whether the kernels of ht_forest_linear_tiled.cu take the call (tabular data without a vector beside it).
+bool tiled_takes(const ht_forest_problem *p, const float *vec, int64_t outputs, const float *x) {
+  return vec == nullptr && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && p->B * p->T > 0 && linear_tiled_takes(p, outputs);
+}
+
 template <typename Real>
 int prepare(const ht_forest_problem *p, const Real *img, const Real *vec, int64_t Cv, const Real *thr,
             const int64_t *ord, const Real *w, bool with_records, void *workspace, size_t workspace_bytes,
-            uint32_t *status_word, ht_stream_t stream, PreparedOf<Real> &out, const ClearList &clear = ClearList()) {
+            uint32_t *status_word, ht_stream_t stream, PreparedOf<Real> &out, const ClearList &clear = ClearList(),
+            bool packed = false) {
   const int rc = check_forest_problem(p);
   if (rc != HT_OK) return rc;
   if (Cv < 0 || (vec == nullptr && p->B * Cv > 0)) return HT_ERR_INVALID_ARGUMENT;
@@ -229,7 +242,7 @@ int prepare(const ht_forest_problem *p, const Real *img, const Real *vec, int64_
   if ((img == nullptr && p->B * p->C * p->K > 0) || ((thr == nullptr || ord == nullptr) && decisions > 0) ||
       (w == nullptr && p->T * p->M > 0))
     return HT_ERR_INVALID_ARGUMENT;
-  const size_t need = ordinal_bytes(p) + (with_records ? record_bytes(p, sizeof(Real)) + 2 * record_bytes(p, 4) : 0) + 256;
+  const size_t need = ordinal_bytes(p) + (with_records ? path_scratch_bytes(p, sizeof(Real)) : 0) + 256;
   if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
     return HT_ERR_WORKSPACE;
   unsigned char *ws = static_cast<unsigned char *>(workspace);
@@ -255,7 +268,7 @@ int prepare(const ht_forest_problem *p, const Real *img, const Real *vec, int64_
     out.records.leaf = reinterpret_cast<int32_t *>(ws + ordinal_bytes(p) + record_bytes(p, sizeof(Real)));
     out.records.vertex = reinterpret_cast<int32_t *>(ws + ordinal_bytes(p) + record_bytes(p, sizeof(Real)) + record_bytes(p, 4));
   }
-  return pack_and_clear(ord, decisions, p->C + Cv, reinterpret_cast<int32_t *>(ws), status_word, clear, out.stream);
+  return pack_and_clear(packed ? nullptr : ord, decisions, p->C + Cv, reinterpret_cast<int32_t *>(ws), status_word, clear, out.stream);
 }
 
 template <typename Real>
@@ -335,6 +348,13 @@ int linear_forward(const ht_forest_problem *p, int64_t out_channels, const Real 
   const int64_t elements = p->B * out_channels * p->K * p->M;
   if (elements == 0) return HT_OK;
   if (out == nullptr || bias == nullptr || (lin == nullptr && p->T > 0)) return HT_ERR_INVALID_ARGUMENT;
+  if constexpr (std::is_same<Real, float>::value) {
+    if (tiled_takes(p, vec, out_channels, img)) {
+      const int trc = linear_tiled_forward(p, out_channels, img, thr, pr.args.ord, w, lin, bias, out,
+                                           static_cast<unsigned char *>(workspace) + ordinal_bytes(p), status_word, pr.stream);
+      if (trc != HT_ERR_UNSUPPORTED) return trc;
+    }
+  }
   const int prc = run_paths<Real>(p, pr);
   if (prc != HT_OK) return prc;
   linear_forward_kernel<Real><<<blocks_for(elements), kBlock, 0, pr.stream>>>(pr.args, pr.records, lin, bias, out_channels, out);
@@ -348,14 +368,23 @@ int linear_backward(const ht_forest_problem *p, int64_t out_channels, const Real
                     Real *gthr, Real *gw, Real *glin, void *workspace, size_t workspace_bytes, uint32_t *status_word,
                     ht_stream_t stream) {
   PreparedOf<Real> pr;
+  // the workspace of the forward on these tensors: packed ordinals and paths are there
+  const bool kept = p != nullptr && (p->flags & HT_SAVED_FORWARD) != 0;
+  bool tiled = false;
+  if constexpr (std::is_same<Real, float>::value) tiled = check_forest_problem(p) == HT_OK && tiled_takes(p, vec, out_channels, img);
   const int rc = prepare<Real>(p, img, vec, vec_channels, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr,
-                               gradients<Real>(p, vec_channels, gimg, gvec, gthr, gw, glin, out_channels));
+                               gradients<Real>(p, vec_channels, tiled ? nullptr : gimg, gvec, gthr, gw, glin, out_channels), kept);
   if (rc != HT_OK) return rc;
   if (out_channels < 0) return HT_ERR_INVALID_ARGUMENT;
   const FusionArgsOf<Real> &a = pr.args;
   if (pr.evals * a.M * out_channels == 0) return HT_OK;
   if (g == nullptr || lin == nullptr) return HT_ERR_INVALID_ARGUMENT;
-  const int prc = run_paths<Real>(p, pr);
+  if constexpr (std::is_same<Real, float>::value) {
+    if (tiled)
+      return linear_tiled_backward(p, out_channels, img, thr, a.ord, w, lin, g, gimg, gthr, gw, glin,
+                                   static_cast<unsigned char *>(workspace) + ordinal_bytes(p), kept, status_word, pr.stream);
+  }
+  const int prc = kept ? HT_OK : run_paths<Real>(p, pr);
   if (prc != HT_OK) return prc;
   if (gimg != nullptr || gvec != nullptr || gthr != nullptr || gw != nullptr) {
     linear_backward_kernel<Real><<<blocks_for(pr.evals), kBlock, 0, pr.stream>>>(a, pr.records, lin, g, out_channels, gimg, gvec,
@@ -375,7 +404,7 @@ int linear_backward(const ht_forest_problem *p, int64_t out_channels, const Real
 
 size_t linear_workspace(const ht_forest_problem *p, size_t real_bytes) {
   if (check_forest_problem(p) != HT_OK) return 0;
-  return ordinal_bytes(p) + record_bytes(p, real_bytes) + 2 * record_bytes(p, 4) + 256;
+  return ordinal_bytes(p) + path_scratch_bytes(p, real_bytes) + 256;
 }
 
 }  // namespace

@@ -29,6 +29,11 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
 int backward_saved(const ht_forest_problem *p, const int32_t *ord, const float *w, const float *g, float *gx, float *gthr,
                    float *gw, void *eval_records, cudaStream_t stream);
 
+// Threshold and leaf-weight gradients (added to; null where not asked for) from records that hold the x-gradient and
+// leaf-weight terms.
+struct EvalRecords;
+int reduce_parameter_terms(const ht_forest_problem *p, const EvalRecords &records, float *gthr, float *gw, cudaStream_t stream);
+
 // Backward with the tile kernels of ht_forest_tiled_bwd.cu; same contract as forward_tiled.  With
 // `eval_records` (backward_records_bytes() bytes of 256-byte aligned scratch; 0 = shape not
 // supported) the traversal kernel writes per-evaluation records and two reduction kernels add

@@ -1072,6 +1072,12 @@ int reduce_parameters(const ht_forest_problem *p, const EvalRecords &evals, int6
 
 }  // namespace
 
+int reduce_parameter_terms(const ht_forest_problem *p, const EvalRecords &records, float *gthr, float *gw, cudaStream_t stream) {
+  const int64_t N = threshold_count(p->kind, p->depth), L = ((int64_t)1) << p->depth;
+  return where_bytes(p->depth) == 2 ? reduce_parameters<unsigned short>(p, records, p->B * p->K, N, L, gthr, gw, stream)
+                                    : reduce_parameters<uint32_t>(p, records, p->B * p->K, N, L, gthr, gw, stream);
+}
+
 size_t backward_records_bytes(const ht_forest_problem *p) {
   BwdPlan plan;
   if (!make_bwd_plan(p, plan) || p->depth > 15) return 0;

@@ -53,7 +53,8 @@ typedef enum ht_status {
 #define HT_DETERMINISTIC 1u /* backward: fixed summation order equal to the reference CPU loops */
 #define HT_WORKSPACE_FOR_BACKWARD 2u /* ht_forest_workspace_bytes: include the backward's evaluation records */
 #define HT_SAVE_FOR_BACKWARD 4u /* ht_forest_forward_f32: also leave the traversal in the workspace (see below) */
-#define HT_SAVED_FORWARD 8u     /* ht_forest_backward_f32: the workspace still holds that traversal */
+#define HT_SAVED_FORWARD 8u     /* ht_forest_backward_f32, ht_forest_linear_backward_*: the workspace still holds the traversal of
+                                 * the forward on the same tensors (the linear forward always leaves it) */
 
 typedef struct ht_forest_problem {
   int32_t kind;   /* HT_KIND_TREE or HT_KIND_FERN */
