@@ -68,8 +68,11 @@ struct RowArgs {
 // lanes on average, as many for the thresholds, which start at an odd pitch per tree): 10 wavefronts per level against 3.4 in
 // the tile kernels, but nothing is transposed and the copies run under the walk.  The paths leave through a staging area in
 // runs of consecutive samples.
-// Bound by shared-memory wavefronts.  262144 x 784, 100 trees of depth 7: MEASURED.
-template <int KIND, typename WhereT>
+// Bound by shared-memory wavefronts.  262144 x 784, 100 trees of depth 7: 358 us (383 without the heads in registers, 608 with
+// a thread per evaluation gathering through L1).
+// HEADS: a lane meets the same (up to four) trees in every row, so their roots' and the roots' children's decisions, two of
+// the levels, stay in registers.
+template <int KIND, typename WhereT, bool HEADS>
 __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid_constant__ RowArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int R = a.rows, G = a.trees, C = a.C, N = a.N;
@@ -110,6 +113,20 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid
   __syncthreads();
 
   const int per_row = kRowWarps / R, my_row = warp / per_row, part = warp % per_row;
+  constexpr int kAtOnce = 4;
+  float head_thr[HEADS ? kAtOnce : 1][3];
+  int head_ord[HEADS ? kAtOnce : 1][3];
+  if constexpr (HEADS) {
+#pragma unroll
+    for (int u = 0; u < kAtOnce; ++u) {
+      const int base = min(part * 32 + lane + u * per_row * 32, trees - 1) * N;
+#pragma unroll
+      for (int h = 0; h < 3; ++h) {
+        head_thr[u][h] = thr[base + min(h, N - 1)];
+        head_ord[u][h] = ord[base + min(h, N - 1)];
+      }
+    }
+  }
   bool poisoned = false;
   for (int64_t s = 0; s < steps; ++s) {
     const int here = rows_of(s);
@@ -125,7 +142,6 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid
     const float *x = rows + my_row * C;
     if (my_row < here) {
       for (int t0 = part * 32 + lane; t0 - lane < trees; t0 += per_row * 128) {
-        constexpr int kAtOnce = 4;
         int base[kAtOnce];
         uint32_t v[kAtOnce], at[kAtOnce];
         float best[kAtOnce];
@@ -137,18 +153,33 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid
           best[u] = 0.0f;
         }
         if (!poisoned) {  // a buffer that never arrived is not read: the paths are those of a zero margin at the root
-          for (int l = 0; l < a.depth; ++l) {
+          auto level = [&](int l) {
 #pragma unroll
             for (int u = 0; u < kAtOnce; ++u) {
               const int vertex = KIND == FERN ? l + 1 : (int)v[u];
-              const float nm = thr[base[u] + vertex] - x[ord[base[u] + vertex]];
+              float t;
+              int feature;
+              if (HEADS && l == 0) {
+                t = head_thr[u][0];
+                feature = head_ord[u][0];
+              } else if (HEADS && l == 1) {
+                t = vertex == 3 ? head_thr[u][2] : head_thr[u][1];
+                feature = vertex == 3 ? head_ord[u][2] : head_ord[u][1];
+              } else {
+                t = thr[base[u] + vertex];
+                feature = ord[base[u] + vertex];
+              }
+              const float nm = t - x[feature];
               if (l == 0 || fabsf(nm) < fabsf(best[u])) {
                 best[u] = nm;
                 at[u] = (uint32_t)vertex;
               }
               v[u] = 2 * v[u] + (nm < 0.0f ? 1u : 0u);
             }
-          }
+          };
+          level(0);
+          if (a.depth > 1) level(1);
+          for (int l = 2; l < a.depth; ++l) level(l);
         }
 #pragma unroll
         for (int u = 0; u < kAtOnce; ++u) {
@@ -182,7 +213,9 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid
 
 template <typename WhereT>
 int launch_rows(const RowArgs &a, int kind, size_t smem, cudaStream_t stream) {
-  auto kernel = kind == TREE ? rows_paths_kernel<TREE, WhereT> : rows_paths_kernel<FERN, WhereT>;
+  const bool heads = a.trees <= 128 * (kRowWarps / a.rows);
+  auto kernel = kind == TREE ? (heads ? rows_paths_kernel<TREE, WhereT, true> : rows_paths_kernel<TREE, WhereT, false>)
+                             : (heads ? rows_paths_kernel<FERN, WhereT, true> : rows_paths_kernel<FERN, WhereT, false>);
   HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   kernel<<<(unsigned)(a.groups * a.slices), kRowThreads, smem, stream>>>(a);
   HT_CHECK_LAUNCH();
@@ -207,7 +240,7 @@ struct RowXArgs {
 // into an element at the same time, hence atomics; on different rows they do not meet.  Every element of gx is written once,
 // where scattering into cleared global memory touches it twice and half of it in 32-byte pieces.
 // Bound by writing gx: two CTAs per SM for rows of up to 880 features, so that one adds while the other writes.
-// 262144 x 784, 100 trees: MEASURED.
+// 262144 x 784, 100 trees: 234 us, 3.5 TB/s (clearing and scattering took over 500).
 template <typename WhereT>
 __global__ void __launch_bounds__(kXThreads) rows_x_gradient_kernel(const __grid_constant__ RowXArgs a) {
   extern __shared__ __align__(16) float tile_rows[];
@@ -241,17 +274,9 @@ __global__ void __launch_bounds__(kXThreads) rows_x_gradient_kernel(const __grid
   }
   __syncthreads();
   float *out = a.gx + row0 * a.C;
-  if ((a.C & 3) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
-    const int quads = a.C / 4;
-    for (int r = warp; r < rows; r += kWarps)
-      for (int q = lane; q < quads; q += 32) {
-        const float *from = tile_rows + r * a.pitch + 4 * q;
-        __stcs(reinterpret_cast<float4 *>(out + (int64_t)r * a.C) + q, make_float4(from[0], from[1], from[2], from[3]));
-      }
-  } else {
-    for (int r = warp; r < rows; r += kWarps)
-      for (int c = lane; c < a.C; c += 32) __stcs(out + (int64_t)r * a.C + c, tile_rows[r * a.pitch + c]);
-  }
+  // (a number per lane: 16 bytes per lane would take every row of four banks four times)
+  for (int r = warp; r < rows; r += kWarps)
+    for (int c = lane; c < a.C; c += 32) __stcs(out + (int64_t)r * a.C + c, tile_rows[r * a.pitch + c]);
 }
 
 inline size_t row_x_smem(int64_t C) { return (size_t)kXRows * (C | 1) * 4; }
