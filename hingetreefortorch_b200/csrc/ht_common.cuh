@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <type_traits>
 
 #include "hingetree_b200.h"
@@ -156,6 +157,45 @@ struct WideOrdinals {
     return (uint64_t)o < (uint64_t)channels ? (int)o : 0;
   }
   __device__ __forceinline__ bool valid(int64_t e) const { return (uint64_t)__ldg(at + e) < (uint64_t)channels; }
+};
+
+// V adjacent numbers as one load or store.
+template <typename Real, int V>
+struct alignas(sizeof(Real) * V) Vec {
+  Real v[V];
+};
+template <typename Real, int V>
+__device__ __forceinline__ Vec<Real, V> load_vec(const Real *p) {
+  Vec<Real, V> r;
+  if constexpr (sizeof(Real) * V == 16) {
+    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
+    r = *reinterpret_cast<const Vec<Real, V> *>(&q);
+  } else if constexpr (sizeof(Real) * V == 8) {
+    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
+    r = *reinterpret_cast<const Vec<Real, V> *>(&q);
+  } else {
+    r.v[0] = __ldg(p);
+  }
+  return r;
+}
+// The widest load and store that the rows of M numbers and the tensors' addresses allow.
+inline int vector_width(int64_t M, size_t real_bytes, std::initializer_list<const void *> tensors) {
+  uintptr_t bits = (uintptr_t)M * real_bytes;
+  for (const void *t : tensors) bits |= reinterpret_cast<uintptr_t>(t);
+  const int most = real_bytes == 8 ? 2 : 4;
+  int v = 1;
+  while (v < most && (bits & (uintptr_t)(2 * v * real_bytes - 1)) == 0) v *= 2;
+  return v;
+}
+
+// Quotients by a number that stays the same for a launch (numerators below 2^31).
+struct Divisor {
+  uint32_t number, factor, shift;
+  Divisor(uint32_t d = 1) : number(d), factor(0), shift(0) {
+    while ((1ull << shift) < d) ++shift;
+    factor = (uint32_t)(((1ull << (31 + shift)) + d - 1) / d);  // ceil(2^(31 + shift) / d), 2^31 <= factor < 2^32
+  }
+  __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return (uint32_t)(((uint64_t)n * factor) >> (31 + shift)); }
 };
 
 // Memory to be zeroed before the kernels of a call add into it.

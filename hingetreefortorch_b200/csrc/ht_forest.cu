@@ -9,6 +9,7 @@
 
 #include "ht_common.cuh"
 #include "ht_forest_multi.cuh"
+#include "ht_forest_rows.cuh"
 #include "ht_forest_tiled.cuh"
 
 namespace ht {
@@ -471,6 +472,22 @@ static bool ordered_from_paths(const ht_forest_problem *p) {
   return (p->flags & HT_DETERMINISTIC) != 0 && (p->M > 1 || p->B * p->T * p->K <= (1 << 26)) && ordered_list_bytes(p, sizeof(float)) > 0;
 }
 
+// Whether the walk goes past resident trees row by row (ht_forest_rows.cu) rather than past resident tiles of samples, or with
+// a thread per evaluation: where the estimates say so by a margin that covers their error.  It does for samples of many
+// features, which leave room for small tiles only (8192 x 784 under 800 trees of depth 8, 10 outputs: 254 against 485 us), and
+// for batches that give few tiles.
+static bool rows_are_better(const ht_forest_problem *p) {
+  const double rows = rows_forward_cost(p);
+  if (rows < 0.0 || p->B * p->T < 32768) return false;
+  double other = forward_tiled_cost(p);
+  if (other < 0.0) {
+    if (p->kind == FERN) return false;
+    const double evals = (double)(p->B * p->T);
+    other = 5.1 + evals * (3.1e-6 * p->depth + 3.7e-6 * (double)p->M);
+  }
+  return rows < 0.85 * other;
+}
+
 // What a backward keeps per evaluation: the records of the tile kernels (one output per leaf), or the paths (several) and,
 // in fixed-order mode, their lists.
 static size_t records_bytes(const ht_forest_problem *p) {
@@ -506,16 +523,23 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
   }
   const WideOrdinals wide = {ord, p->C};
   int32_t *packed = static_cast<int32_t *>(workspace);
-  rc = forward_tiled(p, x, thr, packed, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream, &wide);
-  if (rc != HT_ERR_UNSUPPORTED) return rc;
-  if (eval_records == nullptr && small_enough_for_wide(pr)) {
+  const bool by_rows = rows_are_better(p);
+  if (!by_rows) {
+    rc = forward_tiled(p, x, thr, packed, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream, &wide);
+    if (rc != HT_ERR_UNSUPPORTED) return rc;
+  }
+  if (eval_records == nullptr && !by_rows && small_enough_for_wide(pr)) {
     rc = multi_forward(p, x, thr, nullptr, w, out, PathRecordsOf<float>{nullptr, nullptr}, pr.stream, &wide, status_word);
     if (rc != HT_ERR_UNSUPPORTED) return rc;
   }
   rc = pack_now(pr, ord, status_word);
   if (rc != HT_OK) return rc;
+  const PathRecordsOf<float> paths = eval_records != nullptr ? saved_paths(p, eval_records) : PathRecordsOf<float>{nullptr, nullptr};
+  if (by_rows) {
+    rc = rows_forward(p, x, thr, packed, w, out, paths.margin, paths.where, status_word, pr.stream);
+    if (rc != HT_ERR_UNSUPPORTED) return rc;
+  }
   if (p->M > 1 || eval_records != nullptr) {
-    const PathRecordsOf<float> paths = eval_records != nullptr ? saved_paths(p, eval_records) : PathRecordsOf<float>{nullptr, nullptr};
     rc = multi_forward(p, x, thr, packed, w, out, paths, pr.stream);
     if (rc != HT_ERR_UNSUPPORTED || eval_records != nullptr) return rc;
   }
@@ -598,10 +622,13 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
     }
     if ((p->M > 1 || ordered) && eval_records != nullptr) {
       if (!kept && (!ordered || gthr != nullptr || gw != nullptr)) {  // the paths first
-        int prc = p->M == 1 ? HT_ERR_UNSUPPORTED
-                            : forward_tiled(p, x, thr, static_cast<int32_t *>(workspace), w, none, ws + ordinals_bytes(p), eval_records,
-                                          status_word, pr.stream);
-        if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, saved_paths(p, eval_records), pr.stream);
+        const PathRecordsOf<float> paths = saved_paths(p, eval_records);
+        int prc = HT_ERR_UNSUPPORTED;
+        if (rows_are_better(p)) prc = rows_forward(p, x, thr, a.ord, w, none, paths.margin, paths.where, status_word, pr.stream);
+        if (prc == HT_ERR_UNSUPPORTED && p->M > 1)
+          prc = forward_tiled(p, x, thr, static_cast<int32_t *>(workspace), w, none, ws + ordinals_bytes(p), eval_records, status_word,
+                              pr.stream);
+        if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, paths, pr.stream);
         if (prc != HT_OK) return prc;
       }
       if (ordered) {

@@ -214,7 +214,7 @@ int with_outputs(int64_t outputs, F &&f) {
 }  // namespace
 
 bool linear_tiled_takes(const ht_forest_problem *p, int64_t outputs) {
-  return p->M == 1 && outputs >= 1 && outputs <= kMostOutputs && rows_paths_takes(p) && rows_x_gradient_takes(p) &&
+  return p->M == 1 && outputs >= 1 && outputs <= kMostOutputs && rows_forward_takes(p) && rows_x_gradient_takes(p) &&
          backward_smem(p->T, padded_outputs(outputs)) <= tile::kSmemBudget;
 }
 
@@ -228,7 +228,7 @@ int linear_tiled_forward(const ht_forest_problem *p, int64_t outputs, const floa
   if (!linear_tiled_takes(p, outputs)) return HT_ERR_UNSUPPORTED;
   LinearArgs a = {};
   a.r = eval_record_arrays(p, area);
-  const int rc = rows_paths(p, x, thr, ord, a.r.dx, a.r.where, status_word, stream);
+  const int rc = rows_forward(p, x, thr, ord, w, nullptr, a.r.dx, a.r.where, status_word, stream);
   if (rc != HT_OK) return rc;
   a.w = w;
   a.lin = lin;
@@ -250,7 +250,7 @@ int linear_tiled_backward(const ht_forest_problem *p, int64_t outputs, const flo
   LinearArgs a = {};
   a.r = eval_record_arrays(p, area);
   if (!kept) {
-    const int rc = rows_paths(p, x, thr, ord, a.r.dx, a.r.where, status_word, stream);
+    const int rc = rows_forward(p, x, thr, ord, w, nullptr, a.r.dx, a.r.where, status_word, stream);
     if (rc != HT_OK) return rc;
   }
   a.w = w;

@@ -19,25 +19,6 @@ constexpr uint32_t kSlice = 1024;  // evaluations per CTA
 constexpr int kMaxSortDepth = 12;
 constexpr int64_t kMaxDivisor = 4096;
 
-// V adjacent numbers as one load or store.
-template <typename Real, int V>
-struct alignas(sizeof(Real) * V) Vec {
-  Real v[V];
-};
-template <typename Real, int V>
-__device__ __forceinline__ Vec<Real, V> load_vec(const Real *p) {
-  Vec<Real, V> r;
-  if constexpr (sizeof(Real) * V == 16) {
-    const uint4 q = __ldg(reinterpret_cast<const uint4 *>(p));
-    r = *reinterpret_cast<const Vec<Real, V> *>(&q);
-  } else if constexpr (sizeof(Real) * V == 8) {
-    const uint2 q = __ldg(reinterpret_cast<const uint2 *>(p));
-    r = *reinterpret_cast<const Vec<Real, V> *>(&q);
-  } else {
-    r.v[0] = __ldg(p);
-  }
-  return r;
-}
 template <int V>
 __device__ __forceinline__ void red_add(float *p, const float (&v)[V]) {
   if constexpr (V == 4) red_add_quad(p, v[0], v[1], v[2], v[3]);
@@ -48,16 +29,6 @@ template <int V>
 __device__ __forceinline__ void red_add(double *p, const double (&v)[V]) {
 #pragma unroll
   for (int k = 0; k < V; ++k) atomicAdd(p + k, v[k]);
-}
-
-// The widest load and store that the rows of M numbers and the tensors' addresses allow.
-inline int vector_width(int64_t M, size_t real_bytes, std::initializer_list<const void *> tensors) {
-  uintptr_t bits = (uintptr_t)M * real_bytes;
-  for (const void *t : tensors) bits |= reinterpret_cast<uintptr_t>(t);
-  const int most = real_bytes == 8 ? 2 : 4;
-  int v = 1;
-  while (v < most && (bits & (uintptr_t)(2 * v * real_bytes - 1)) == 0) v *= 2;
-  return v;
 }
 
 template <typename Real>
@@ -137,16 +108,6 @@ __global__ void __launch_bounds__(kForwardThreads) multi_forward_kernel(const __
 }
 
 // ---- backward, default mode ------------------------------------------------------------------------------------------
-
-// Quotients by a number that stays the same for a launch (numerators below 2^31).
-struct Divisor {
-  uint32_t number, factor, shift;
-  Divisor(uint32_t d = 1) : number(d), factor(0), shift(0) {
-    while ((1ull << shift) < d) ++shift;
-    factor = (uint32_t)(((1ull << (31 + shift)) + d - 1) / d);  // ceil(2^(31 + shift) / d), 2^31 <= factor < 2^32
-  }
-  __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return (uint32_t)(((uint64_t)n * factor) >> (31 + shift)); }
-};
 
 template <typename Real>
 struct SortedArgs {

@@ -32,7 +32,7 @@ inline size_t row_smem(int64_t N, int64_t C, int rows, int trees) {
 }
 
 bool make_row_plan(const ht_forest_problem *p, RowPlan &plan) {
-  if (p->K != 1 || p->C > 65536 || p->depth > 12 || p->T < 1 || p->B < 1 || p->B > 0x7fffffff || p->T > 0x7fffff) return false;
+  if (p->K != 1 || p->M < 1 || p->M > 64 || p->C > 65536 || p->depth > 12 || p->T < 1 || p->B < 1 || p->B > 0x7fffffff || p->T > 0x7fffff) return false;
   const int64_t N = threshold_count(p->kind, p->depth);
   for (int rows = 16; rows >= 4; rows /= 2) {
     // as many trees as fit, but groups of the same size; a warp walks 32 trees at a time
@@ -54,7 +54,11 @@ bool make_row_plan(const ht_forest_problem *p, RowPlan &plan) {
 }
 
 struct RowArgs {
-  const float *x, *thr;
+  const float *x, *thr, *w;
+  float *out;
+  Divisor by_M;
+  int64_t L;
+  int M, width;
   const int32_t *ord;
   float *margin;
   void *where;
@@ -73,7 +77,7 @@ struct RowArgs {
 // HEADS: a lane meets the same (up to four) trees in every row, so their roots' and the roots' children's decisions, two of
 // the levels, stay in registers.
 template <int KIND, typename WhereT, bool HEADS>
-__global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid_constant__ RowArgs a) {
+__global__ void __launch_bounds__(kRowThreads, 1) rows_forward_kernel(const __grid_constant__ RowArgs a) {
   extern __shared__ __align__(128) unsigned char smem[];
   const int R = a.rows, G = a.trees, C = a.C, N = a.N;
   float *thr = reinterpret_cast<float *>(smem);
@@ -127,6 +131,24 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid
       }
     }
   }
+  // the outputs of the group's trees are one run in every row: V numbers per thread, consecutive threads along the run
+  auto write_outputs = [&](int64_t s, int here, const uint2 *staged, auto vector) {
+    constexpr int V = decltype(vector)::value;
+    const int pieces = trees * a.M / V;
+    float *to = a.out + ((step0 + s) * R * a.T + j0) * a.M;
+    for (int r = my_row; r < here; r += R)
+#pragma unroll 4
+      for (int q = part * 32 + lane; q < pieces; q += per_row * 32) {
+        const uint32_t element = (uint32_t)q * V, t = a.by_M.quotient(element);
+        const uint2 path = staged[t * R + r];
+        const float size = fabsf(__uint_as_float(path.x));
+        const uint32_t key = sizeof(WhereT) == 2 ? path.y >> 8 : path.y >> 16;
+        Vec<float, V> v = load_vec<float, V>(a.w + ((j0 + t) * a.L + key) * a.M + (element - t * (uint32_t)a.M));
+#pragma unroll
+        for (int u = 0; u < V; ++u) v.v[u] = mul_rn(size, v.v[u]);
+        *reinterpret_cast<Vec<float, V> *>(to + (int64_t)r * a.T * a.M + element) = v;
+      }
+  };
   bool poisoned = false;
   for (int64_t s = 0; s < steps; ++s) {
     const int here = rows_of(s);
@@ -192,6 +214,12 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid
     }
     __syncthreads();  // rows read, results staged
     if (tid == 0) issue(s + 2);
+    if (a.out != nullptr) {
+      if (a.width == 4) write_outputs(s, here, out, std::integral_constant<int, 4>{});
+      else if (a.width == 2) write_outputs(s, here, out, std::integral_constant<int, 2>{});
+      else write_outputs(s, here, out, std::integral_constant<int, 1>{});
+    }
+    if (a.margin == nullptr) continue;
     // four rows of a tree per thread: they are consecutive samples of one record block
     const int64_t sample = (step0 + s) * R;
     const int64_t at0 = record_index(sample, j0, a.T);
@@ -214,8 +242,8 @@ __global__ void __launch_bounds__(kRowThreads, 1) rows_paths_kernel(const __grid
 template <typename WhereT>
 int launch_rows(const RowArgs &a, int kind, size_t smem, cudaStream_t stream) {
   const bool heads = a.trees <= 128 * (kRowWarps / a.rows);
-  auto kernel = kind == TREE ? (heads ? rows_paths_kernel<TREE, WhereT, true> : rows_paths_kernel<TREE, WhereT, false>)
-                             : (heads ? rows_paths_kernel<FERN, WhereT, true> : rows_paths_kernel<FERN, WhereT, false>);
+  auto kernel = kind == TREE ? (heads ? rows_forward_kernel<TREE, WhereT, true> : rows_forward_kernel<TREE, WhereT, false>)
+                             : (heads ? rows_forward_kernel<FERN, WhereT, true> : rows_forward_kernel<FERN, WhereT, false>);
   HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   kernel<<<(unsigned)(a.groups * a.slices), kRowThreads, smem, stream>>>(a);
   HT_CHECK_LAUNCH();
@@ -283,13 +311,33 @@ inline size_t row_x_smem(int64_t C) { return (size_t)kXRows * (C | 1) * 4; }
 
 }  // namespace
 
-bool rows_paths_takes(const ht_forest_problem *p) {
+// One CTA per SM, and a CTA fetches its parameters once: groups x slices as close below 148 as it gets.
+static int row_slices(const ht_forest_problem *p, const RowPlan &plan) {
+  const int64_t steps = (p->B + plan.rows - 1) / plan.rows, groups = (p->T + plan.trees - 1) / plan.trees;
+  return (int)std::max<int64_t>(1, std::min<int64_t>(148 / std::min<int64_t>(groups, 148), steps));
+}
+
+// Rounds of CTAs, each of them steps x (levels of the walks that a warp does one after another, outputs, row copies) behind
+// the fetch of its parameters; the coefficients are a least-squares fit to 342 measured forwards (B 1000 .. 65536, C 32 ..
+// 1500, T 40 .. 800, depth 5 .. 10, M 1 .. 10; 19 % off on average).
+double rows_forward_cost(const ht_forest_problem *p) {
+  RowPlan plan;
+  if (!make_row_plan(p, plan)) return -1.0;
+  const int64_t groups = (p->T + plan.trees - 1) / plan.trees, slices = row_slices(p, plan);
+  const double waves = (double)((groups * slices + 147) / 148);
+  const double steps = (double)(((p->B + plan.rows - 1) / plan.rows + slices - 1) / slices);
+  const int at_once = 128 * (kRowWarps / plan.rows), rounds = (plan.trees + at_once - 1) / at_once;
+  return 6.1 + waves * (steps * (0.34 * rounds * p->depth + 0.22e-3 * plan.rows * plan.trees * (double)p->M + 0.008e-3 * plan.rows * (double)p->C) +
+                        0.13e-3 * plan.trees * (double)threshold_count(p->kind, p->depth));
+}
+
+bool rows_forward_takes(const ht_forest_problem *p) {
   RowPlan plan;
   return make_row_plan(p, plan);
 }
 
-int rows_paths(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, float *margin, void *where,
-               uint32_t *status_word, cudaStream_t stream) {
+int rows_forward(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w, float *out,
+                 float *margin, void *where, uint32_t *status_word, cudaStream_t stream) {
   RowPlan plan;
   if (!make_row_plan(p, plan) || (reinterpret_cast<uintptr_t>(x) & 15u) != 0) return HT_ERR_UNSUPPORTED;
   RowArgs a = {};
@@ -298,6 +346,12 @@ int rows_paths(const ht_forest_problem *p, const float *x, const float *thr, con
   a.ord = ord;
   a.margin = margin;
   a.where = where;
+  a.w = w;
+  a.out = out;
+  a.M = (int)p->M;
+  a.L = ((int64_t)1) << p->depth;
+  a.by_M = Divisor((uint32_t)std::max<int64_t>(p->M, 1));
+  a.width = out != nullptr ? vector_width(p->M, sizeof(float), {w, out}) : 1;
   a.status_word = status_word;
   a.B = p->B;
   a.T = p->T;
@@ -307,9 +361,7 @@ int rows_paths(const ht_forest_problem *p, const float *x, const float *thr, con
   a.rows = plan.rows;
   a.trees = plan.trees;
   a.groups = (int)((p->T + plan.trees - 1) / plan.trees);
-  // one CTA per SM, and a CTA fetches its parameters once: groups x slices as close below 148 as it gets
-  const int64_t steps = (p->B + plan.rows - 1) / plan.rows;
-  a.slices = (int)std::max<int64_t>(1, std::min<int64_t>(148 / std::min(a.groups, 148), steps));
+  a.slices = row_slices(p, plan);
   return where_bytes(p->depth) == 2 ? launch_rows<unsigned short>(a, p->kind, plan.smem, stream)
                                     : launch_rows<uint32_t>(a, p->kind, plan.smem, stream);
 }

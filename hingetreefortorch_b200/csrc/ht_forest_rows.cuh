@@ -7,11 +7,13 @@
 
 namespace ht {
 
-// The paths of all evaluations (threshold - feature at the deciding vertex; vertex and leaf key in the packing of the
-// evaluation records) with the tree parameters in shared memory and the rows streaming past them.
-bool rows_paths_takes(const ht_forest_problem *p);
-int rows_paths(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, float *margin, void *where,
-               uint32_t *status_word, cudaStream_t stream);
+// The walk with the tree parameters in shared memory and the rows streaming past them.  What it leaves: the paths of all
+// evaluations (threshold - feature at the deciding vertex; vertex and leaf key in the packing of the evaluation records)
+// where `margin` and `where` are given, and the forest's output [B, T, M] where `out` is.
+bool rows_forward_takes(const ht_forest_problem *p);
+double rows_forward_cost(const ht_forest_problem *p);  // estimated microseconds; negative: not taken
+int rows_forward(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w, float *out,
+                 float *margin, void *where, uint32_t *status_word, cudaStream_t stream);
 
 // gx [B, C] from records that hold the x-gradient terms (EvalRecords::dx), every element written; sums in free order.
 bool rows_x_gradient_takes(const ht_forest_problem *p);

@@ -68,10 +68,6 @@ __host__ __device__ inline size_t results_bytes(bool one_output, int S, int G) {
   return (bytes + 1023) & ~(size_t)1023;
 }
 
-// 16-byte loads a thread keeps in flight while it stages the feature tile (1, 2, 4, 8 measured on the benchmark shape:
-// 3.86, 3.80, 3.89, 3.80 ms; 8 spills a register)
-constexpr int kStageLoads = 2;
-
 bool make_plan(const ht_forest_problem *p, TilePlan &plan) {
   if (p->K != 1 || p->M < 1 || p->M > 64) return false;
   if (p->C > 65536 || p->depth > 12) return false;
@@ -181,40 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1) forest_forward_tiled_kernel(const
     if (num_groups > 1) issue(1);
   }
 
-  // Stage the tile's features: lanes run along samples so that the shared-memory writes are
-  // conflict free; each lane fetches 16 bytes of its row at a time when the row allows it.
-  if ((C & 3) == 0) {
-    // several 16-byte loads in flight per thread before the first is stored: the tile comes from HBM, and a loop that
-    // waits for each load in turn spends a memory round trip per pass
-    const int quads = C >> 2;
-    const int total = S * quads;
-    for (int idx0 = tid; idx0 < total; idx0 += kStageLoads * kThreads) {
-      float4 v[kStageLoads];
-#pragma unroll
-      for (int u = 0; u < kStageLoads; ++u) {
-        const int idx = idx0 + u * kThreads;
-        const int s = idx % S, q = idx / S;
-        v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (idx < total && row0 + s < a.B) v[u] = __ldg(reinterpret_cast<const float4 *>(a.x + (row0 + s) * C) + q);
-      }
-#pragma unroll
-      for (int u = 0; u < kStageLoads; ++u) {
-        const int idx = idx0 + u * kThreads;
-        if (idx < total) {
-          const int s = idx % S, q = idx / S;
-          xs[(4 * q + 0) * S + s] = v[u].x;
-          xs[(4 * q + 1) * S + s] = v[u].y;
-          xs[(4 * q + 2) * S + s] = v[u].z;
-          xs[(4 * q + 3) * S + s] = v[u].w;
-        }
-      }
-    }
-  } else {
-    for (int idx = tid; idx < S * C; idx += kThreads) {
-      const int s = idx % S, c = idx / S;
-      xs[c * S + s] = (row0 + s < a.B) ? __ldg(a.x + (row0 + s) * C + c) : 0.f;
-    }
-  }
+  stage_rows(xs, a.x, row0, a.B, C, S, tid);
   __syncthreads();  // features staged; barrier initialisation visible
 
   const uint32_t xl_addr = smem_addr(xs + sample_group * 32 + lane);
@@ -687,6 +650,21 @@ size_t forward_tiled_workspace_bytes(const ht_forest_problem *p) {
   TilePlan plan;
   if (!(p->K > 1 ? make_inner_plan(p, plan) : make_plan(p, plan))) return 0;
   return align_up((size_t)p->T * plan.rec.bytes, 256);
+}
+
+// Rounds of CTAs, each staging its tile and walking its share of the tree groups; one, two or four trees per warp at once
+// differ in what a group costs (few in flight leave the shared memory's latency in the open).  Fitted like
+// rows_forward_cost(): 9 to 16 % off on average.
+double forward_tiled_cost(const ht_forest_problem *p) {
+  TilePlan plan;
+  if (!make_plan(p, plan)) return -1.0;
+  const int64_t tiles = (p->B + plan.S - 1) / plan.S, groups = (p->T + plan.G - 1) / plan.G;
+  const int splits = choose_splits(tiles, groups);
+  const double waves = (double)((tiles * splits + 147) / 148), per_cta = (double)((groups + splits - 1) / splits);
+  const double level = plan.per_warp == 1 ? 0.18 : plan.per_warp == 2 ? 0.23 : 0.41;
+  const double output = plan.per_warp == 1 ? 3.6e-4 : plan.per_warp == 2 ? 1.9e-4 : 1.6e-4;
+  return 4.5 + waves * (2.0e-4 * plan.S * (double)p->C +
+                        per_cta * (level * p->depth + (p->M > 1 ? output * plan.G * plan.S * (double)p->M : 0.0)));
 }
 
 bool forward_saves(const ht_forest_problem *p) {

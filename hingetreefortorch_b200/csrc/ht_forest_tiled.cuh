@@ -8,6 +8,9 @@ namespace ht {
 // Bytes of per-tree records the tile kernel needs in the workspace (0 when the shape does not qualify).
 size_t forward_tiled_workspace_bytes(const ht_forest_problem *p);
 
+// Estimated microseconds of the tile kernel on tabular data; negative: not taken.
+double forward_tiled_cost(const ht_forest_problem *p);
+
 // Runs the forward with the tile kernel when the shape qualifies; returns HT_ERR_UNSUPPORTED
 // (and launches nothing) when it does not, so that the caller can use the any-shape kernel.
 // `ord` are the compact (validated, clamped) int32 ordinals; `records` is 256-byte aligned

@@ -26,6 +26,11 @@ SHAPES = [
     (513, 11, (2,), 33, 4, 33),
     (5, 16, (900,), 9, 11, 63),
     (2, 100, (24, 24), 30, 7, 64),
+    # many features: the walk goes row by row (last rows not a whole step; groups of trees; two trees' worth of outputs per lane)
+    (1003, 333, (), 40, 5, 10),
+    (1001, 784, (), 48, 5, 3),
+    (2050, 784, (), 300, 8, 1),
+    (8195, 200, (), 4, 3, 2),
     # too few evaluations for the sorted backward, but not for the fixed order; one output, more than a buffer of terms holds
     (31, 5, (), 3, 2, 2),
     (700, 20, (), 6, 7, 1),
