@@ -119,6 +119,8 @@ struct TiledArgs {
   uint32_t *status_word;
   int64_t B, T, K;
   int C, S, G, per_warp, M;
+  int width;                 // several outputs per leaf: numbers per load and store
+  Divisor by_M, by_pieces;   // ... and what a place in a warp's outputs is divided by
   int tma_store;  // results of full groups leave through the TMA engine (G is 16 or 32)
   // a forward that saves its traversal for the backward (SAVE kernels): threshold - feature at the deciding
   // vertex, and the packed vertex / leaf key, in the evaluation-record layout
@@ -416,35 +418,31 @@ __global__ void __launch_bounds__(kThreads, 1) forest_forward_tiled_kernel(const
         pairs[lane * 4 + u] = make_float2(result[u], __uint_as_float(__brev(path[u] - kL) >> (32 - DEPTH)));
       __syncwarp();
       if (trees_here > 0 && (!SAVE || a.out != nullptr)) {
-        const int run = trees_here * M;  // outputs of one sample that this warp owns, contiguous
         const int64_t first_row = row0 + sample_group * 32;
-        const int rows_here = (int)min((int64_t)32, a.B - first_row);
+        const int rows_here = (int)max((int64_t)0, min((int64_t)32, a.B - first_row));
         const float *w_first = a.w + (col0 + t_first) * (int64_t)kL * M;
         float *dst = a.out + first_row * row_pitch + (col0 + t_first) * M;
-        // Lane l writes element l, l + 32, ... of every sample's run: which tree and which output
-        // that is does not depend on the sample, so it is worked out once per pass and the loop
-        // over the samples is a pair load, a weight load, a multiply and a store.
-        for (int e = lane; e < run; e += 32) {
-          const int u = (e >= M) + (e >= 2 * M) + (e >= 3 * M), m = e - u * M;  // run <= 4 * M
-          const float *w_tree = w_first + (int64_t)u * kL * M + m;
-          const float2 *pair_of = pairs + u;
-          float *to = dst + e;
-          int sample = 0;
-          for (; sample + 4 <= rows_here; sample += 4) {
-            float2 pr[4];
-            float weight[4];
+        // The outputs of all 32 samples, V at a time, are dealt out to the lanes one after another: a run of one or two trees
+        // with few outputs would leave most lanes idle (10007 x 257 trees, 3 outputs, one tree per warp: 1055 instructions per
+        // evaluation of 32 samples with a pass per sample: 118 us, dealt out 77).
+        auto write_out = [&](auto vector) {
+          constexpr int V = decltype(vector)::value;
+          const uint32_t pieces = (uint32_t)(trees_here * M) / V, total = (uint32_t)rows_here * pieces;
+          const bool whole = trees_here == per_warp;
+#pragma unroll 4
+          for (uint32_t e = (uint32_t)lane; e < total; e += 32) {
+            const uint32_t sample = whole ? a.by_pieces.quotient(e) : e / pieces, element = (e - sample * pieces) * V;
+            const uint32_t u = a.by_M.quotient(element);
+            const float2 pr = pairs[sample * 4 + u];
+            Vec<float, V> v = load_vec<float, V>(w_first + ((u << DEPTH) + __float_as_uint(pr.y)) * (uint32_t)M + (element - u * (uint32_t)M));
 #pragma unroll
-            for (int k = 0; k < 4; ++k) pr[k] = pair_of[(sample + k) * 4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) weight[k] = __ldg(w_tree + (int64_t)__float_as_uint(pr[k].y) * M);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) to[(int64_t)(sample + k) * row_pitch] = pr[k].x * weight[k];
+            for (int k = 0; k < V; ++k) v.v[k] = pr.x * v.v[k];
+            *reinterpret_cast<Vec<float, V> *>(dst + (int64_t)sample * row_pitch + element) = v;
           }
-          for (; sample < rows_here; ++sample) {
-            const float2 pr = pair_of[sample * 4];
-            to[(int64_t)sample * row_pitch] = pr.x * __ldg(w_tree + (int64_t)__float_as_uint(pr.y) * M);
-          }
-        }
+        };
+        if (a.width == 4) write_out(std::integral_constant<int, 4>{});
+        else if (a.width == 2) write_out(std::integral_constant<int, 2>{});
+        else write_out(std::integral_constant<int, 1>{});
       }
       continue;
     }
@@ -662,7 +660,7 @@ double forward_tiled_cost(const ht_forest_problem *p) {
   const int splits = choose_splits(tiles, groups);
   const double waves = (double)((tiles * splits + 147) / 148), per_cta = (double)((groups + splits - 1) / splits);
   const double level = plan.per_warp == 1 ? 0.18 : plan.per_warp == 2 ? 0.23 : 0.41;
-  const double output = plan.per_warp == 1 ? 3.6e-4 : plan.per_warp == 2 ? 1.9e-4 : 1.6e-4;
+  const double output = 1.5e-4;
   return 4.5 + waves * (2.0e-4 * plan.S * (double)p->C +
                         per_cta * (level * p->depth + (p->M > 1 ? output * plan.G * plan.S * (double)p->M : 0.0)));
 }
@@ -700,6 +698,9 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
   a.records = rec;
   a.w = w;
   a.M = (int)p->M;
+  a.width = vector_width(p->M, sizeof(float), {w, out});
+  a.by_M = Divisor((uint32_t)p->M);
+  a.by_pieces = Divisor((uint32_t)(plan.per_warp * p->M / a.width));
   a.out = out;
   a.status_word = status_word;
   a.B = p->B;
