@@ -163,6 +163,7 @@ struct PipelineNode : public torch::autograd::Function<PipelineNode> {
     ctx->save_for_backward({x, w, z[0], stats[0], stats[2], thr, ord, leaves, r[1], r[2]});
     ctx->saved_data["kind"] = kind;
     ctx->mark_non_differentiable({stats[0], stats[1]});
+    ctx->set_materialize_grads(false);  // no zeros for the gradients of mean and variance
     return {r[0], stats[0], stats[1]};
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {

@@ -345,6 +345,23 @@ __global__ void __launch_bounds__(kSortThreads) sorted_backward_kernel(const __g
       for (int t0 = begin; t0 < begin + share; t0 += kAhead) walk_list(t0, std::true_type{});
     else
       for (int t0 = begin; t0 < begin + share; t0 += kAhead) walk_list(t0, std::false_type{});
+    // groups of the warp that end in the same leaf hand in one sum (23 million evaluations of 22 trees of depth 4, 2 outputs:
+    // 495 us; 1293 when all 256 groups of a slice met in 16 leaves)
+    if constexpr (kGroupsPerWarp > 1) {
+#pragma unroll
+      for (int d = 1; d < kGroupsPerWarp; d <<= 1) {
+        const bool join = __shfl_down_sync(0xffffffffu, current, d * LANES) == current && group_in_warp + d < kGroupsPerWarp;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int v = 0; v < V; ++v) {
+            const Real other = __shfl_down_sync(0xffffffffu, sums[r][v], d * LANES);
+            if (join) sums[r][v] += other;
+          }
+      }
+      const uint32_t before = __shfl_up_sync(0xffffffffu, current, LANES);
+      if (group_in_warp > 0 && before == current) current = kNone;
+    }
     leave();
   }
   if (a.gx == nullptr && a.gthr == nullptr) return;

@@ -52,6 +52,7 @@ namespace {
 
 
 struct TilePlan {
+  bool weights;    // the records carry the leaf weights (one output per leaf)
   int S;           // samples per tile
   int G;           // trees per parameter group
   int per_warp;    // trees a warp walks at once: G / slots
@@ -73,18 +74,23 @@ bool make_plan(const ht_forest_problem *p, TilePlan &plan) {
   if (p->C > 65536 || p->depth > 12) return false;
   if (p->B * p->T < 32 * 1024) return false;  // too small to fill the machine with sample tiles
   plan.ord_bytes = p->C <= 256 ? 1 : 2;
-  plan.rec = record_layout(p->kind, p->depth, (uint32_t)plan.ord_bytes, p->M == 1,
-                           paired_ordinals(p->kind, p->depth, (uint32_t)plan.ord_bytes));
-  for (int S = 256; S >= 32; S >>= 1) {
-    const int slots = kWarps / (S / 32);
-    for (int per_warp = 4; per_warp >= 1; per_warp >>= 1) {
-      const int G = slots * per_warp;
-      plan.S = S;
-      plan.G = G;
-      plan.per_warp = per_warp;
-      // results: a staging row per sample (one output per leaf), or the warps' (margin, leaf) pairs
-      plan.smem = 1024 + results_bytes(p->M == 1, S, G) + (size_t)p->C * S * 4 + 2 * (size_t)G * plan.rec.bytes + 64;
-      if (plan.smem <= kSmemBudget) return true;
+  // One output per leaf: weights in the records first; where those do not fit beside a tile (ferns of depth 10 on 579 features:
+  // 121336 x 241 forwards 297 us, 444 with a thread per evaluation) they are read from global memory like several outputs'.
+  for (int weights = p->M == 1 ? 1 : 0; weights >= 0; --weights) {
+    plan.weights = weights != 0;
+    plan.rec = record_layout(p->kind, p->depth, (uint32_t)plan.ord_bytes, plan.weights,
+                             paired_ordinals(p->kind, p->depth, (uint32_t)plan.ord_bytes));
+    for (int S = 256; S >= 32; S >>= 1) {
+      const int slots = kWarps / (S / 32);
+      for (int per_warp = 4; per_warp >= 1; per_warp >>= 1) {
+        const int G = slots * per_warp;
+        plan.S = S;
+        plan.G = G;
+        plan.per_warp = per_warp;
+        // results: a staging row per sample (one output per leaf), or the warps' (margin, leaf) pairs
+        plan.smem = 1024 + results_bytes(plan.weights, S, G) + (size_t)p->C * S * 4 + 2 * (size_t)G * plan.rec.bytes + 64;
+        if (plan.smem <= kSmemBudget) return true;
+      }
     }
   }
   return false;
@@ -100,6 +106,7 @@ bool make_inner_plan(const ht_forest_problem *p, TilePlan &plan) {
   plan.ord_bytes = p->C <= 256 ? 1 : 2;
   plan.rec = record_layout(p->kind, p->depth, (uint32_t)plan.ord_bytes, true,
                            paired_ordinals(p->kind, p->depth, (uint32_t)plan.ord_bytes));
+  plan.weights = true;
   plan.per_warp = 4;
   for (int S = 256; S >= 32; S >>= 1) {
     plan.S = S;
@@ -603,7 +610,7 @@ int launch_depth(const TilePlan &plan, const TiledArgs &a, dim3 grid, cudaStream
     if (plan.ord_bytes == 1) return launch_one(forest_forward_tiled_inner_kernel<KIND, DEPTH, uint8_t>, plan, a, grid, stream);
     return launch_one(forest_forward_tiled_inner_kernel<KIND, DEPTH, uint16_t>, plan, a, grid, stream);
   }
-  const bool wrec = a.M == 1;
+  const bool wrec = plan.weights;
   if (a.save_margin != nullptr) {
     if (plan.ord_bytes == 1)
       return wrec ? launch_one(forest_forward_tiled_kernel<KIND, DEPTH, uint8_t, true, true>, plan, a, grid, stream)
@@ -647,7 +654,10 @@ int launch_kind(int depth, const TilePlan &plan, const TiledArgs &a, dim3 grid, 
 size_t forward_tiled_workspace_bytes(const ht_forest_problem *p) {
   TilePlan plan;
   if (!(p->K > 1 ? make_inner_plan(p, plan) : make_plan(p, plan))) return 0;
-  return align_up((size_t)p->T * plan.rec.bytes, 256);
+  // one output per leaf: the backward's records carry the leaf weights whatever the forward's do
+  const size_t with_weights =
+      p->M == 1 ? record_layout(p->kind, p->depth, (uint32_t)plan.ord_bytes, true, plan.rec.paired).bytes : 0;
+  return align_up((size_t)p->T * std::max<size_t>(plan.rec.bytes, with_weights), 256);
 }
 
 // Rounds of CTAs, each staging its tile and walking its share of the tree groups; one, two or four trees per warp at once
@@ -662,7 +672,7 @@ double forward_tiled_cost(const ht_forest_problem *p) {
   const double level = plan.per_warp == 1 ? 0.18 : plan.per_warp == 2 ? 0.23 : 0.41;
   const double output = 1.5e-4;
   return 4.5 + waves * (2.0e-4 * plan.S * (double)p->C +
-                        per_cta * (level * p->depth + (p->M > 1 ? output * plan.G * plan.S * (double)p->M : 0.0)));
+                        per_cta * (level * p->depth + (!plan.weights ? output * plan.G * plan.S * (double)p->M : 0.0)));
 }
 
 bool forward_saves(const ht_forest_problem *p) {
@@ -670,7 +680,7 @@ bool forward_saves(const ht_forest_problem *p) {
   if (p->K != 1 || p->M != 1 || !make_plan(p, plan)) return false;
   // every tree group takes the kernel's streamlined body: 4 trees per warp, no short last group
   // ... and the kernel that expands the records fits its tables into shared memory
-  return plan.per_warp == 4 && p->T % plan.G == 0 && p->B <= 0x7fffffff && backward_records_bytes(p) > 0 &&
+  return plan.weights && plan.per_warp == 4 && p->T % plan.G == 0 && p->B <= 0x7fffffff && backward_records_bytes(p) > 0 &&
          saved_samples_per_cta(p) != 0;
 }
 
@@ -724,7 +734,7 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
   // Full groups of 16 or 32 trees leave as tiled TMA stores when the output admits a tensor map
   // (rows of a multiple of 16 bytes); otherwise, and for a short last group, as row segments.
   a.tma_store = 0;
-  if (p->K == 1 && p->M == 1 && plan.per_warp == 4 && (plan.G == 16 || plan.G == 32) && (p->T & 3) == 0 &&
+  if (p->K == 1 && plan.weights && plan.per_warp == 4 && (plan.G == 16 || plan.G == 32) && (p->T & 3) == 0 &&
       p->T >= plan.G && tma::encode_matrix_f32(&a.out_map, out, p->B, p->T, 32, plan.G))
     a.tma_store = 1;
   // With few sample tiles the tree groups are split among CTAs (grid.y) so that the SMs are busy in

@@ -383,7 +383,7 @@ __device__ __forceinline__ void lanes_in_order_per_key(bool valid, uint32_t key,
 // threshold, the likeliest leaves) collect a third of the lanes of a typical chunk.
 template <bool ORDERED, typename WT>
 __global__ void __launch_bounds__(512) reduce_parameter_records_kernel(EvalRecords r, int64_t B, int64_t T, int64_t N,
-                                                                       int64_t L, float *gthr, float *gw) {
+                                                                       int64_t L, int64_t per_split, float *gthr, float *gw) {
   extern __shared__ float all_bins[];
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
   float *bins = all_bins + (size_t)warp * (N + L);
@@ -408,7 +408,9 @@ __global__ void __launch_bounds__(512) reduce_parameter_records_kernel(EvalRecor
       fw[u] = valid ? load_where<WT>(r.where, first + 32 * u) : 1u;
     }
   };
-  int64_t i0 = (int64_t)warp * 32 * kAhead;
+  // a split's samples are whole record blocks
+  int64_t i0 = (int64_t)blockIdx.y * per_split + (int64_t)warp * 32 * kAhead;
+  B = min(B, (int64_t)(blockIdx.y + 1) * per_split);
   if (i0 < B) fetch(i0, a, b, wh);
   for (; i0 < B; i0 += stride) {
     if (i0 + stride < B) fetch(i0 + stride, na, nb, nwh);
@@ -446,11 +448,12 @@ __global__ void __launch_bounds__(512) reduce_parameter_records_kernel(EvalRecor
   for (int64_t t = threadIdx.x; t < N + L; t += blockDim.x) {
     float sum = all_bins[t];
     for (int wi = 1; wi < warps; ++wi) sum = __fadd_rn(sum, all_bins[(size_t)wi * (N + L) + t]);
-    if (t < N) {
-      if (gthr != nullptr) gthr[j * N + t] = sum;
-    } else if (gw != nullptr) {
-      gw[j * L + (t - N)] = sum;
-    }
+    float *to = t < N ? (gthr == nullptr ? nullptr : gthr + j * N + t) : (gw == nullptr ? nullptr : gw + j * L + (t - N));
+    if (to == nullptr) continue;
+    if (gridDim.y == 1)
+      *to = sum;
+    else if (sum != 0.0f)
+      atomicAdd(to, sum);
   }
 }
 
@@ -462,7 +465,7 @@ __global__ void __launch_bounds__(512) reduce_parameter_records_kernel(EvalRecor
 // warps' columns are summed in a fixed order at the end: reproducible, another association.
 template <int CHUNKS, typename WT>
 __global__ void __launch_bounds__(512, 1) reduce_parameter_records_columns_kernel(EvalRecords r, int64_t B, int64_t T,
-                                                                                  int64_t N, int64_t L, int columns,
+                                                                                  int64_t N, int64_t L, int columns, int64_t per_split,
                                                                                   float *gthr, float *gw) {
   extern __shared__ float all_bins[];  // [warp][bin][column]
   const int warps = blockDim.x >> 5, warp = threadIdx.x >> 5;
@@ -488,7 +491,8 @@ __global__ void __launch_bounds__(512, 1) reduce_parameter_records_columns_kerne
       fw[u] = valid ? load_where<WT>(r.where, first + 32 * u) : 1u;
     }
   };
-  int64_t i0 = (int64_t)warp * 32 * CHUNKS;
+  int64_t i0 = (int64_t)blockIdx.y * per_split + (int64_t)warp * 32 * CHUNKS;
+  B = min(B, (int64_t)(blockIdx.y + 1) * per_split);
   if (i0 < B) fetch(i0, a, b, wh);
   for (; i0 < B; i0 += stride) {
     if (i0 + stride < B) fetch(i0 + stride, na, nb, nwh);
@@ -522,11 +526,12 @@ __global__ void __launch_bounds__(512, 1) reduce_parameter_records_columns_kerne
     float sum = 0.0f;
     for (int wi = 0; wi < warps; ++wi)
       for (int c = 0; c < columns; ++c) sum = __fadd_rn(sum, all_bins[((size_t)wi * bins_per_tree + t) * columns + c]);
-    if (t < N) {
-      if (gthr != nullptr) gthr[j * N + t] = sum;
-    } else if (gw != nullptr) {
-      gw[j * L + (t - N)] = sum;
-    }
+    float *to = t < N ? (gthr == nullptr ? nullptr : gthr + j * N + t) : (gw == nullptr ? nullptr : gw + j * L + (t - N));
+    if (to == nullptr) continue;
+    if (gridDim.y == 1)
+      *to = sum;
+    else if (sum != 0.0f)
+      atomicAdd(to, sum);
   }
 }
 
@@ -1004,10 +1009,18 @@ int reduce_parameters(const ht_forest_problem *p, const EvalRecords &evals, int6
   if ((p->flags & HT_DETERMINISTIC) != 0) {
     HT_CUDA_TRY(cudaFuncSetAttribute(reduce_parameter_records_kernel<true, WT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)kSmemBudget));
-    reduce_parameter_records_kernel<true, WT><<<(unsigned)p->T, 32 * warps, smem, stream>>>(evals, samples, p->T, N, L, gthr, gw);
+    reduce_parameter_records_kernel<true, WT><<<(unsigned)p->T, 32 * warps, smem, stream>>>(
+        evals, samples, p->T, N, L, samples, gthr, gw);
     HT_CHECK_LAUNCH();
     return HT_OK;
   }
+  // Few trees leave SMs idle: their samples are split over gridDim.y as far as CTAs fit at once, each split with `least`
+  // samples or more to pay for handing in its bins (173584 samples, 11 trees of depth 10: 497 us on 11 SMs, 25 now).
+  auto split_of = [&](int64_t ctas_per_sm, int64_t least) {
+    const int64_t splits = std::max<int64_t>(1, std::min<int64_t>({148 * ctas_per_sm / std::max<int64_t>(p->T, 1), samples / least, 65535}));
+    return ((samples + splits - 1) / splits + kRecordBlock - 1) / kRecordBlock * kRecordBlock;
+  };
+  auto split_grid = [&](int64_t per_split) { return dim3((unsigned)p->T, (unsigned)((samples + per_split - 1) / per_split)); };
   // copies of the bins per warp (a power of two, at most one per lane) that `column_warps` warps can hold
   const int column_warps = kColumnWarps;
   int columns = 32;
@@ -1031,12 +1044,15 @@ int reduce_parameters(const ht_forest_problem *p, const EvalRecords &evals, int6
     const size_t column_smem = (size_t)column_warps * (N + L) * columns * 4;
     HT_CUDA_TRY(cudaFuncSetAttribute(reduce_parameter_records_columns_kernel<8, WT>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    reduce_parameter_records_columns_kernel<8, WT><<<(unsigned)p->T, 32 * column_warps, column_smem, stream>>>(
-        evals, samples, p->T, N, L, columns, gthr, gw);
+    const int64_t per_split = split_of(1, (int64_t)column_warps * 512);
+    reduce_parameter_records_columns_kernel<8, WT><<<split_grid(per_split), 32 * column_warps, column_smem, stream>>>(
+        evals, samples, p->T, N, L, columns, per_split, gthr, gw);
   } else {
     HT_CUDA_TRY(cudaFuncSetAttribute(reduce_parameter_records_kernel<false, WT>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-    reduce_parameter_records_kernel<false, WT><<<(unsigned)p->T, 32 * warps, smem, stream>>>(evals, samples, p->T, N, L, gthr, gw);
+    const int64_t per_split = split_of(std::max<int64_t>(1, std::min<int64_t>(200 * 1024 / (int64_t)smem, 64 / warps)), (int64_t)warps * 256);
+    reduce_parameter_records_kernel<false, WT><<<split_grid(per_split), 32 * warps, smem, stream>>>(evals, samples, p->T, N, L, per_split,
+                                                                                                  gthr, gw);
   }
   HT_CHECK_LAUNCH();
   return HT_OK;
