@@ -28,7 +28,7 @@ SYMBOLS = [
     "ht_forest_static_scratch_bytes", "ht_forest_forward_static_f32",
     "ht_forest_fusion_workspace_bytes", "ht_forest_fusion_forward_f32", "ht_forest_fusion_backward_f32",
     "ht_forest_linear_workspace_bytes", "ht_forest_linear_forward_f32", "ht_forest_linear_backward_f32",
-    "ht_conv_output_size", "ht_conv_workspace_bytes", "ht_conv_forward_f32", "ht_conv_backward_f32",
+    "ht_conv_output_size", "ht_conv_workspace_bytes", "ht_conv_backward_workspace_bytes", "ht_conv_forward_f32", "ht_conv_backward_f32",
     "ht_contract", "ht_expand",
     "ht_trie_forward_f32", "ht_trie_backward_f32", "ht_forest_touched_f32", "ht_linear_tf32_stats_f32",
     "ht_forest_linear_workspace_bytes_f64", "ht_forest_fusion_forward_f64", "ht_forest_fusion_backward_f64",
@@ -55,7 +55,7 @@ def _triple(values, fill):
 class Conv:
     """Convolutional hinge trees through the C ABI: x [B,Ci,*size], thr/ord [Co,Ci,N], w [Co,Ci,L,*extra]."""
 
-    def __init__(self, kind, x, w, kernel, stride, padding, dilation):
+    def __init__(self, kind, x, w, kernel, stride, padding, dilation, code_share=1.0):
         import math
         import torch
         dims = x.dim() - 2
@@ -68,7 +68,10 @@ class Conv:
         osize = (ctypes.c_int64 * 3)()
         _check(lib.ht_conv_output_size(ctypes.byref(self.problem), osize))
         self.out_shape = (x.shape[0], w.shape[0]) + tuple(osize[:dims]) + tuple(w.shape[3:])
+        lib.ht_conv_backward_workspace_bytes.restype = ctypes.c_size_t
         nbytes = lib.ht_conv_workspace_bytes(ctypes.byref(self.problem))
+        # code_share: of the scratch through which the backward's kernels share one walk
+        nbytes += int(code_share * (lib.ht_conv_backward_workspace_bytes(ctypes.byref(self.problem)) - nbytes))
         self.workspace = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=x.device)
         self.status = torch.zeros(1, dtype=torch.int32, device=x.device)
 

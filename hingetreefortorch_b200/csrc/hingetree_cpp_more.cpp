@@ -568,7 +568,15 @@ std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bo
   if (need_x) grads[0] = fresh_like(x);
   if (need_thr) grads[1] = fresh_like(thr);
   if (need_w) grads[3] = fresh_like(w);
-  torch::Tensor ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);
+  torch::Tensor ws;
+  try {
+    ws = make_workspace(x.scalar_type() == torch::kFloat32 && need_x && (need_thr || need_w)
+                            ? ht_conv_backward_workspace_bytes(&call.problem)
+                            : ht_conv_workspace_bytes(&call.problem),
+                        x);
+  } catch (const c10::OutOfMemoryError &) {  // no room for the shared walk
+    ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);
+  }
   OrdinalGuard og(ord, call.window_cells);
   dispatch_real(x, [&](auto real) {
     using Real = decltype(real);

@@ -536,8 +536,11 @@ int conv_backward(const ht_conv_problem *p, const Real *x, const Real *thr, cons
     if (tile_problem(p, a, t)) {
       const size_t records = conv_backward_tiled_workspace_bytes(t);
       if (records != 0 && workspace_bytes >= conv_ordinal_bytes(a) + records + 256) {
-        const int tiled = conv_backward_tiled(t, x, thr, a.ord, w, g, gx, gthr, gw,
-                                              static_cast<unsigned char *>(workspace) + conv_ordinal_bytes(a), status_word, s);
+        unsigned char *ws = static_cast<unsigned char *>(workspace);
+        const size_t codes_at = conv_ordinal_bytes(a) + conv_records_bytes(p, a) + 256;
+        const size_t code_bytes = workspace_bytes > codes_at ? workspace_bytes - codes_at : 0;
+        const int tiled = conv_backward_tiled(t, x, thr, a.ord, w, g, gx, gthr, gw, ws + conv_ordinal_bytes(a),
+                                              code_bytes > 0 ? ws + codes_at : nullptr, code_bytes, status_word, s);
         if (tiled != HT_ERR_UNSUPPORTED) return tiled;
       }
     }
@@ -570,6 +573,18 @@ size_t ht_conv_workspace_bytes(const ht_conv_problem *p) {
   ConvArgs a;
   if (check_conv(p, a) != HT_OK) return 0;
   return conv_ordinal_bytes(a) + conv_records_bytes(p, a) + 256;
+}
+
+size_t ht_conv_backward_workspace_bytes(const ht_conv_problem *p) {
+  ConvArgs a;
+  ConvTileProblem t;
+  const size_t base = ht_conv_workspace_bytes(p);
+  if (base == 0 || check_conv(p, a) != HT_OK || !tile_problem(p, a, t)) return base;
+  const size_t per_sample = conv_code_bytes(t);
+  if (per_sample == 0) return base;
+  // whole batches up to 8 GiB of codes, then a part of the batch at a time
+  const size_t samples = std::min<size_t>((size_t)p->B, std::max<size_t>(1, ((size_t)8 << 30) / per_sample));
+  return base + samples * per_sample;
 }
 
 int ht_conv_forward_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,

@@ -17,6 +17,8 @@ struct ConvTileProblem {
 // take the problem.
 size_t conv_tiled_workspace_bytes(const ConvTileProblem &p);
 size_t conv_backward_tiled_workspace_bytes(const ConvTileProblem &p);
+// Bytes per sample of the codes through which the backward's kernels hand on one walk; 0: they walk for themselves.
+size_t conv_code_bytes(const ConvTileProblem &p);
 
 // HT_ERR_UNSUPPORTED when the tile kernel does not take the problem (the caller falls back to the
 // thread-per-output kernel).  `ord` holds validated window-cell indices, `records` is scratch of
@@ -24,10 +26,11 @@ size_t conv_backward_tiled_workspace_bytes(const ConvTileProblem &p);
 int conv_forward_tiled(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w,
                        float *out, void *records, uint32_t *status_word, cudaStream_t stream);
 
-// Gradients are ADDED to gx, gthr, gw (the caller clears them); any of the three may be null.
+// Gradients are ADDED to gx, gthr, gw (the caller clears them); any of the three may be null.  `codes`: code_bytes bytes of
+// scratch for the codes of as many samples as that is enough for (none with null).
 int conv_backward_tiled(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w,
-                        const float *g, float *gx, float *gthr, float *gw, void *records, uint32_t *status_word,
-                        cudaStream_t stream);
+                        const float *g, float *gx, float *gthr, float *gw, void *records, void *codes, size_t code_bytes,
+                        uint32_t *status_word, cudaStream_t stream);
 
 namespace conv_tile {
 

@@ -35,17 +35,26 @@ using namespace conv_tile;
 
 namespace {
 
+// What the image gradient needs of an evaluation, in 16 bits: leaf in path order (7 bits), window cell of the deciding vertex
+// (7 bits), and on top the factor sign(margin) as the first two bits of a float (2, -2, or 0 for a margin of zero or none).
+constexpr uint32_t kCodeCellShift = 7;
+constexpr int kCodeCells = 128, kCodeDepth = 7;
+
 // ---- records with one 8-byte entry per vertex --------------------------------------------------------
 //
 // The backward's traversal needs the threshold and the patch offset of every vertex it visits, from addresses
 // that differ from lane to lane.  In this form of the record vertex v (1-based; ferns: level + 1) has the
 // entry {threshold, offset as a 32-bit word} at byte 8 v (bytes 0..7 are unused), so that one address and one
 // 8-byte load bring both; the leaf weights follow in path order as in the other records.  Larger than the
-// packed form (8 against 5 or 6 bytes a vertex): the plans below take it where it fits.
+// packed form (8 against 5 or 6 bytes a vertex): the plans below take it where it fits.  Behind the leaf weights stands, for
+// every vertex, what its window cell contributes to a code (below).
 __host__ __device__ constexpr RecordLayout vertex_pair_layout(int kind, int depth) {
   const uint32_t n = kind == FERN ? (uint32_t)depth : (1u << depth) - 1u;
   const uint32_t w = round16(8u * (n + 1u));
-  return RecordLayout{0u, 4u, w, round16(w + 4u * (1u << depth)), false};
+  return RecordLayout{0u, 4u, w, round16(w + 4u * (1u << depth) + 2u * (n + 1u)), false};
+}
+__host__ __device__ constexpr uint32_t vertex_pair_cells(int kind, int depth) {
+  return vertex_pair_layout(kind, depth).w + 4u * (1u << depth);
 }
 
 __global__ void repack_vertex_pairs_kernel(const float *__restrict__ thr, const int32_t *__restrict__ ord,
@@ -66,6 +75,8 @@ __global__ void repack_vertex_pairs_kernel(const float *__restrict__ thr, const 
     entry.x = __float_as_uint(t);
     entry.y = map.feature((uint32_t)ord[j * N + r]);
     reinterpret_cast<uint2 *>(rec)[r + 1] = entry;
+    reinterpret_cast<unsigned short *>(rec + vertex_pair_cells(kind, depth))[r + 1] =
+        (unsigned short)(((uint32_t)ord[j * N + r] << kCodeCellShift) - (uint32_t)L);  // wraps: the path's leading one goes
     if (r == 0) reinterpret_cast<uint2 *>(rec)[0] = make_uint2(0u, 0u);
   } else {
     const int64_t h = r - N;
@@ -411,6 +422,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_backward_tiled_kernel(ConvBw
 // come in three buffers: a warp runs up to two groups ahead of the slowest before it waits.
 
 struct ParamGradPlan {
+  bool flat;    // see ParamGradArgs
   int R;        // tile rows
   int columns;  // lanes' columns per bin: 16, 8 or 4
   int staged;   // input channels whose patches are staged together
@@ -423,16 +435,19 @@ struct ParamGradPlan {
 // Record groups in flight or in use: with three, a warp runs up to two groups ahead of the slowest before it waits.
 constexpr int kParamBuffers = 3;
 
-bool make_param_plan(const ConvTileProblem &p, ParamGradPlan &plan, bool pairs) {
+bool make_param_plan(const ConvTileProblem &p, ParamGradPlan &plan, bool pairs, bool flat = false) {
   plan.pairs = pairs;
+  plan.flat = flat;
   if (p.depth > 7 || p.Ci < 1 || p.Co < 1 || p.B < 1 || p.Ho < 1 || p.Wo < 1) return false;
   if ((double)p.B * p.Ho * p.Wo * (double)p.Co * p.Ci < 1048576.0) return false;
+  if (p.Ho * (int64_t)p.Wo > (1 << 30)) return false;  // positions in 32 bits
   // a warp's bins: 2^depth rows of {threshold bin, leaf bin}, `columns` lanes' columns each
   const int bins_per_tree = 2 << p.depth;
   plan.columns = 16;
   while (plan.columns > 4 && bins_per_tree * plan.columns * 4 > 4096) plan.columns >>= 1;
-  plan.R = std::min(16, (p.Ho + 3) & ~3);
-  const PatchShape shape = patch_shape(p, plan.R);
+  plan.R = std::min(16, ((flat ? (p.Wo + kTileColumns - 1) / kTileColumns : p.Ho) + 3) & ~3);
+  PatchShape shape = patch_shape(p, flat ? 1 : plan.R);
+  if (flat) shape.w += (plan.R - 1) * kTileColumns * p.sx;
   if (shape.far > 16383) return false;
   plan.patch_h = shape.h;
   plan.patch_w = shape.w;
@@ -455,7 +470,18 @@ struct ParamGradArgs {
   uint32_t *status_word;
   int Ci, Co, H, W, Ho, Wo, sy, sx, py, px;
   int R, columns, staged, patch_h, patch_w, tiles_x, row_blocks;
+  int flat;              // one row of outputs: the "rows" of a tile are runs of 32 columns, one after another
+  uint2 *codes;          // or null
+  int64_t code_groups;   // groups of four rows per (sample, channels)
+  int code_columns;
 };
+
+__device__ __forceinline__ uint32_t lds_u16(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(addr));
+  return v;
+}
+
 
 template <int KIND, int DEPTH, typename OrdT, bool PAIRS>
 __global__ void __launch_bounds__(kThreads, 1) conv_backward_params_tiled_kernel(ParamGradArgs a) {
@@ -479,7 +505,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_backward_params_tiled_kernel
   const int tiles = a.tiles_x * a.row_blocks;
   const int64_t b = blockIdx.x / tiles;
   const int tile = (int)(blockIdx.x - b * tiles);
-  const int oy0 = (tile / a.tiles_x) * R, ox0 = (tile % a.tiles_x) * kTileColumns;
+  const int oy0 = a.flat ? 0 : (tile / a.tiles_x) * R, ox0 = (tile % a.tiles_x) * kTileColumns * (a.flat ? R : 1);
 
   // blockIdx.y splits the rounds (32 output channels, one per warp) among CTAs; `it` counts this
   // CTA's groups, input channel outermost
@@ -513,11 +539,15 @@ __global__ void __launch_bounds__(kThreads, 1) conv_backward_params_tiled_kernel
 
   const int ox = ox0 + lane;
   const uint32_t lane_addr = smem_addr(patch) + (uint32_t)(lane * a.sx) * 4u;
-  const uint32_t row_bytes = (uint32_t)(a.sy * a.patch_w) * 4u;
+  const uint32_t row_bytes = (uint32_t)(a.flat ? kTileColumns * a.sx : a.sy * a.patch_w) * 4u;
   const uint32_t my_bins_addr = smem_addr(bins) + (uint32_t)(warp * 2 * (int)kL * columns + lane % columns) * 4u;
   const uint32_t bin_bytes = (uint32_t)columns * 4u, row_bytes_of_bins = 2u * bin_bytes;
   const int turns = 32 / columns, group = lane / columns;
-  const int rows_here = min(R, a.Ho - oy0);
+  const int rows_here = a.flat ? min(R, (a.Wo - ox0 + kTileColumns - 1) / kTileColumns) : min(R, a.Ho - oy0);
+  // outputs of this lane: row r is at out0 + r * out_pitch, and those past out_last (rows or columns off the output) repeat it
+  const int out0 = a.flat ? ox : oy0 * a.Wo + min(ox, a.Wo - 1), out_pitch = a.flat ? kTileColumns : a.Wo;
+  const int out_last = a.flat ? a.Wo - 1 : out0 + (rows_here - 1) * a.Wo;
+  const int valid_rows = ox >= a.Wo ? 0 : a.flat ? (a.Wo - ox + kTileColumns - 1) / kTileColumns : rows_here;
   const float *image = a.x + b * a.Ci * (int64_t)a.H * a.W;
   const bool want_thr = a.gthr != nullptr, want_w = a.gw != nullptr;
   bool poisoned = false;
@@ -544,8 +574,13 @@ __global__ void __launch_bounds__(kThreads, 1) conv_backward_params_tiled_kernel
     const int j = (round0 + round) * kWarps + warp;
     if (j < a.Co && !poisoned) {
       const uint32_t record = params_addr + (uint32_t)(it % kParamBuffers) * buffer_bytes + (uint32_t)warp * lay.bytes;
-      // lanes and rows off the output read the last valid element instead and have their terms cleared below
-      const float *g_rows = a.g + ((b * a.Co + j) * a.Ho + oy0) * (int64_t)a.Wo + min(ox, a.Wo - 1);
+      // lanes and rows off the output read another's upstream gradient and have their terms cleared below
+      const float *g_tree = a.g + (b * a.Co + j) * a.Ho * (int64_t)a.Wo;
+      // four rows' codes are 8 bytes: [sample][input channel][output channel][group of four rows][column]
+      uint2 *code_quads = nullptr;
+      if (PAIRS && a.codes != nullptr && (a.flat || ox < a.Wo))
+        code_quads = a.codes + (((b * a.Ci + c) * a.Co + j) * a.code_groups + (a.flat ? ox0 >> 7 : oy0 >> 2)) * (int64_t)a.code_columns +
+                     (a.flat ? lane : ox);
       for (int row0 = 0; row0 < rows_here; row0 += 4) {
         uint32_t rec[4], x_addr[4];
         float gval[4];
@@ -553,13 +588,25 @@ __global__ void __launch_bounds__(kThreads, 1) conv_backward_params_tiled_kernel
         for (int u = 0; u < 4; ++u) {
           rec[u] = record;
           x_addr[u] = channel_addr + (uint32_t)(row0 + u) * row_bytes;
-          gval[u] = __ldg(g_rows + (int64_t)min(row0 + u, rows_here - 1) * a.Wo);
+          gval[u] = __ldg(g_tree + min(out0 + (row0 + u) * out_pitch, out_last));
         }
         Walked wk[4];
         if constexpr (PAIRS)
           walk_vertex_pairs<KIND, DEPTH, 4>(rec, x_addr, wk);
         else
           walk_full<KIND, DEPTH, OrdT, 4>(rec, x_addr, 4u, wk);
+        if constexpr (PAIRS) {
+          if (code_quads != nullptr) {
+            uint32_t code[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const uint32_t factor = fabsf(wk[u].nm) > 0.0f ? ((__float_as_uint(wk[u].nm) >> 16) & 0x8000u) ^ 0xc000u : 0u;
+              code[u] = lds_u16(record + 2u * wk[u].v + vertex_pair_cells(KIND, DEPTH)) + wk[u].path + factor;
+            }
+            __stcs(code_quads, make_uint2(prmt(code[0], code[1], 0x5410u), prmt(code[2], code[3], 0x5410u)));
+            code_quads += a.code_columns;
+          }
+        }
         float term_thr[4], term_w[4];
         uint32_t at_thr[4], at_w[4];
 #pragma unroll
@@ -569,7 +616,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_backward_params_tiled_kernel
           // the threshold term is -sign(margin) * w * g with margin = -nm
           term_thr[u] = -signed_term(wk[u].nm, wg);
           term_w[u] = __fmul_rn(fabsf(wk[u].nm), gval[u]);
-          if (!(row0 + u < rows_here && ox < a.Wo)) term_thr[u] = term_w[u] = 0.0f;
+          if (row0 + u >= valid_rows) term_thr[u] = term_w[u] = 0.0f;
           at_thr[u] = my_bins_addr + (wk[u].v - 1u) * row_bytes_of_bins;
           at_w[u] = my_bins_addr + bin_bytes + (wk[u].path - kL) * row_bytes_of_bins;
         }
@@ -642,6 +689,115 @@ __global__ void __launch_bounds__(kThreads, 1) conv_backward_params_tiled_kernel
         atomicExch(&finished[it % kParamBuffers], 0u);
         __threadfence_block();
         if (it + kParamBuffers < num_groups) issue(it + kParamBuffers);
+      }
+    }
+  }
+}
+
+// ---- image gradient from the codes of the parameter kernel ------------------------------------------------
+//
+// Lane = four output positions (a code quad) x two input channels (which share the upstream gradient), over the output
+// channels: no walk (a thread that takes one position and channel pair per 2-byte load spends 33 instructions per evaluation and
+// ran 5.8 ms below).  A lane adds
+// sign * w * g into its own columns of [channel][position][window cell][lane], eight independent additions at a time; one
+// global reduction per touched pixel at the end.  x [64, 64, 64, 64], 3 x 3, 128 trees of depth 5: 2.1 ms where the walking
+// kernel takes 6.9, and the parameter kernel 9.0 instead of 8.4 for writing the codes.
+struct ImageArgs {
+  const uint2 *codes;
+  const unsigned char *records;
+  const float *g;
+  float *gx;
+  int64_t positions, quads, quad_blocks, channel_pairs;
+  int Ci, Co, H, W, Wo, sy, sx, py, px, dy, dx, kw, cells, splits, flat, code_columns;
+  uint32_t record_bytes, weights_at, leaf_mask;
+};
+
+__global__ void __launch_bounds__(128) conv_image_from_codes_kernel(const __grid_constant__ ImageArgs a) {
+  extern __shared__ float cell_columns[];  // [warp][2][4][cells][32]
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  int64_t at = blockIdx.x;
+  const int64_t quad_block = at % a.quad_blocks;
+  at /= a.quad_blocks;
+  const int split = (int)(at % a.splits);
+  at /= a.splits;
+  const int64_t pair = at % a.channel_pairs, b = at / a.channel_pairs;
+  const int c0 = (int)pair * 2, c1 = min(c0 + 1, a.Ci - 1);
+  const int share = (a.Co + a.splits - 1) / a.splits;
+  const int j0 = split * share, j_end = min(j0 + share, a.Co);
+
+  float *mine = cell_columns + (size_t)warp * 8 * a.cells * 32 + lane;
+  for (int q = 0; q < 8 * a.cells; ++q) mine[32 * q] = 0.0f;
+  // lanes past the last quad, and rows or columns past the output, repeat others and hand nothing in
+  const int64_t my_quad = quad_block * blockDim.x + threadIdx.x, quad = min(my_quad, a.quads - 1);
+  const int64_t group = quad / a.code_columns;
+  const int column = (int)(quad - group * a.code_columns);
+  const int64_t position0 = a.flat ? group * 128 + column : 4 * group * a.Wo + column;
+  const int step = a.flat ? 32 : a.Wo;
+  const float *up_at[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) up_at[u] = a.g + (b * a.Co + j0) * a.positions + min(position0 + u * step, a.positions - 1);
+  const uint2 *codes0 = a.codes + ((b * a.Ci + c0) * a.Co + j0) * a.quads + quad;
+  const uint2 *codes1 = a.codes + ((b * a.Ci + c1) * a.Co + j0) * a.quads + quad;
+  const unsigned char *leaves0 = a.records + ((int64_t)c0 * a.Co + j0) * a.record_bytes + a.weights_at;
+  const unsigned char *leaves1 = a.records + ((int64_t)c1 * a.Co + j0) * a.record_bytes + a.weights_at;
+  const uint32_t columns = smem_addr(mine), column_bytes = (uint32_t)a.cells * 128u, last_cell = column_bytes - 128u;
+
+  constexpr int kAhead = 4;  // output channels whose codes are under way
+  uint2 next[kAhead][2];
+  auto fetch = [&](int n, int j) {
+    if (j < j_end) {
+      next[n][0] = __ldcs(codes0);
+      next[n][1] = __ldcs(codes1);
+      codes0 += a.quads;
+      codes1 += a.quads;
+    }
+  };
+#pragma unroll
+  for (int n = 0; n < kAhead; ++n) fetch(n, j0 + n);
+  for (int j = j0; j < j_end; j += kAhead) {
+#pragma unroll
+    for (int n = 0; n < kAhead; ++n) {
+      if (j + n >= j_end) break;
+      const uint32_t code[8] = {next[n][0].x, next[n][0].x >> 16, next[n][0].y, next[n][0].y >> 16,
+                                next[n][1].x, next[n][1].x >> 16, next[n][1].y, next[n][1].y >> 16};
+      fetch(n, j + n + kAhead);
+      float up[4], weight[8], sum[8];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        up[u] = 0.5f * __ldg(up_at[u]);  // the factors of the codes are twice the sign
+        up_at[u] += a.positions;
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e)
+        weight[e] = __ldg(reinterpret_cast<const float *>(e < 4 ? leaves0 : leaves1) + (code[e] & a.leaf_mask));
+      leaves0 += a.record_bytes;
+      leaves1 += a.record_bytes;
+      uint32_t cell[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        // (clamped: a parameter kernel that gave up on a lost copy leaves codes unwritten)
+        cell[e] = columns + (uint32_t)e * column_bytes + min(code[e] & (127u << kCodeCellShift), last_cell);
+        sum[e] = lds_f32(cell[e]);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float factor = __uint_as_float((code[e] << 16) & 0xc0000000u);
+        sts_f32(cell[e], __fmaf_rn(factor, __fmul_rn(weight[e], up[e & 3]), sum[e]));
+      }
+    }
+  }
+  if (my_quad >= a.quads) return;
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int oy = a.flat ? 0 : (int)(4 * group) + u, ox = a.flat ? (int)position0 + 32 * u : column;
+    if (position0 + (int64_t)u * step >= a.positions) break;
+    const int wy = oy * a.sy - a.py, wx = ox * a.sx - a.px;
+    for (int h = 0; h < 2 && c0 + h < a.Ci; ++h) {
+      float *image = a.gx + (b * a.Ci + c0 + h) * (int64_t)a.H * a.W;
+      for (int q = 0; q < a.cells; ++q) {
+        const float v = lds_f32(columns + (uint32_t)(4 * h + u) * column_bytes + (uint32_t)q * 128u);
+        const int iy = wy + (q / a.kw) * a.dy, ix = wx + (q % a.kw) * a.dx;
+        if (v != 0.0f && iy >= 0 && iy < a.H && ix >= 0 && ix < a.W) atomicAdd(image + (int64_t)iy * a.W + ix, v);  // padding has no gradient
       }
     }
   }
@@ -737,6 +893,67 @@ bool choose_plans(const ConvTileProblem &p, ConvBwdPlan &plan, ParamGradPlan &pp
   return true;
 }
 
+// The parameter kernel with records of its own: 8-byte entries, and outputs of a single row taken 32 columns per "row" (four
+// rows walk at a time whether they exist or not).  Some channels' patches have to fit at a time.
+bool codes_plan(const ConvTileProblem &p, ParamGradPlan &plan) {
+  const bool flat = p.Ho == 1 && p.H == 1 && p.kh == 1;
+  return p.depth <= kCodeDepth && (int64_t)p.kh * p.kw <= kCodeCells && make_param_plan(p, plan, true, flat) &&
+         plan.staged >= std::min<int64_t>(p.Ci, 4);
+}
+// Groups of four rows and columns of the codes per (sample, input channel, output channel).
+struct CodeShape {
+  int64_t groups;
+  int columns;
+};
+inline CodeShape code_shape(const ConvTileProblem &p, const ParamGradPlan &plan) {
+  if (plan.flat) return {(p.Wo + 4 * kTileColumns - 1) / (4 * kTileColumns), kTileColumns};
+  return {(p.Ho + 3) / 4, p.Wo};
+}
+
+// The parameter gradients of samples b0 .. b0 + p.B - 1 (p, x and g are theirs); with `codes` it leaves those too.
+int launch_parameters(const ConvTileProblem &p, const ParamGradPlan &pplan, const float *x, const unsigned char *rec, const float *g,
+                      float *gthr, float *gw, uint2 *codes, uint32_t *status_word, cudaStream_t stream) {
+  ParamGradArgs pa;
+  const CodeShape shape = code_shape(p, pplan);
+  pa.flat = pplan.flat ? 1 : 0;
+  pa.code_groups = shape.groups;
+  pa.code_columns = shape.columns;
+  pa.x = x;
+  pa.records = rec;
+  pa.g = g;
+  pa.gthr = gthr;
+  pa.gw = gw;
+  pa.status_word = status_word;
+  pa.Ci = (int)p.Ci;
+  pa.Co = (int)p.Co;
+  pa.H = p.H;
+  pa.W = p.W;
+  pa.Ho = p.Ho;
+  pa.Wo = p.Wo;
+  pa.sy = p.sy;
+  pa.sx = p.sx;
+  pa.py = p.py;
+  pa.px = p.px;
+  pa.R = pplan.R;
+  pa.columns = pplan.columns;
+  pa.staged = pplan.staged;
+  pa.patch_h = pplan.patch_h;
+  pa.patch_w = pplan.patch_w;
+  pa.codes = codes;
+  const int tile_columns = kTileColumns * (pplan.flat ? pplan.R : 1);
+  pa.tiles_x = (p.Wo + tile_columns - 1) / tile_columns;
+  pa.row_blocks = pplan.flat ? 1 : (p.Ho + pplan.R - 1) / pplan.R;
+  const int64_t tiles = p.B * pa.tiles_x * pa.row_blocks;
+  if (tiles > 0x7fffffff) return HT_ERR_UNSUPPORTED;
+  // enough CTAs for about seven rounds of the machine, so that the last round's idle SMs cost little
+  const int64_t rounds = (p.Co + kWarps - 1) / kWarps;
+  int64_t splits = 1;
+  if (tiles < 7 * 148) splits = std::min<int64_t>(rounds, (7 * 148 + tiles - 1) / tiles);
+  const dim3 pgrid((unsigned)tiles, (unsigned)std::max<int64_t>(splits, 1));
+  return p.kind == TREE ? launch_params_kind<TREE>(p.depth, pplan, pa, pgrid, stream)
+                        : launch_params_kind<FERN>(p.depth, pplan, pa, pgrid, stream);
+}
+
 }  // namespace
 
 size_t conv_backward_tiled_workspace_bytes(const ConvTileProblem &p) {
@@ -744,12 +961,100 @@ size_t conv_backward_tiled_workspace_bytes(const ConvTileProblem &p) {
   ParamGradPlan pplan;
   bool with_params;
   if (!choose_plans(p, plan, pplan, with_params)) return 0;
-  return align_up((size_t)(p.Co * p.Ci) * plan.rec.bytes, 256);
+  size_t record = plan.rec.bytes;
+  if (codes_plan(p, pplan)) record = std::max<size_t>(record, pplan.rec.bytes);
+  return align_up((size_t)(p.Co * p.Ci) * record, 256);
+}
+
+size_t conv_code_bytes(const ConvTileProblem &p) {
+  ConvBwdPlan plan;
+  ParamGradPlan pplan;
+  bool with_params;
+  if (!choose_plans(p, plan, pplan, with_params) || !codes_plan(p, pplan)) return 0;
+  const CodeShape shape = code_shape(p, pplan);
+  return (size_t)(p.Ci * p.Co) * (size_t)(shape.groups * shape.columns) * sizeof(uint2);
+}
+
+// The parameter gradients, and with gx the image gradient from their codes: as many samples at a time as the scratch for
+// codes holds, but not with less than an eighth of the batch, where a launch would leave SMs idle more often than not.
+static int backward_by_codes(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w,
+                             const float *g, float *gx, float *gthr, float *gw, void *records, void *codes, size_t code_bytes,
+                             uint32_t *status_word, cudaStream_t stream) {
+  ParamGradPlan pplan;
+  const size_t per_sample = conv_code_bytes(p);
+  if (per_sample == 0 || !codes_plan(p, pplan)) return HT_ERR_UNSUPPORTED;
+  int64_t at_once = p.B;
+  if (gx != nullptr) {
+    at_once = codes == nullptr ? 0 : std::min<int64_t>(p.B, (int64_t)(code_bytes / per_sample));
+    if (at_once < 1 || at_once * 8 < p.B) return HT_ERR_UNSUPPORTED;
+  }
+  const int64_t trees = p.Co * p.Ci, positions = p.Ho * (int64_t)p.Wo, image = p.H * (int64_t)p.W;
+  const int64_t elements = trees * (threshold_count(p.kind, p.depth) + (((int64_t)1) << p.depth));
+  const CodeShape shape = code_shape(p, pplan);
+  ImageArgs ia = {};
+  ia.cells = p.kh * p.kw;
+  int warps = 4;  // of a CTA: their columns of sums have to fit
+  while (warps > 1 && (size_t)warps * ia.cells * 1024 > 100 * 1024) warps /= 2;
+  const size_t smem = (size_t)warps * ia.cells * 1024;
+  ia.positions = positions;
+  ia.quads = shape.groups * shape.columns;
+  ia.quad_blocks = (ia.quads + 32 * warps - 1) / (32 * warps);
+  ia.channel_pairs = (p.Ci + 1) / 2;
+  if (ia.quad_blocks * ia.channel_pairs * at_once * 16 > 0x7fffffff) return HT_ERR_UNSUPPORTED;
+  unsigned char *rec = static_cast<unsigned char *>(records);
+  RecordMap map;
+  map.columns = p.kw;
+  map.row_step = p.dy * pplan.patch_w;
+  map.column_step = p.dx;
+  map.inner = p.Ci;  // tree (j, c) goes to record c * Co + j
+  map.outer_count = p.Co;
+  repack_vertex_pairs_kernel<<<(unsigned)((elements + 255) / 256), 256, 0, stream>>>(thr, ord, w, rec, p.kind, p.depth, trees, pplan.rec, map);
+  HT_CHECK_LAUNCH();
+  ia.codes = static_cast<const uint2 *>(codes);
+  ia.records = rec;
+  ia.record_bytes = pplan.rec.bytes;
+  ia.weights_at = pplan.rec.w;
+  ia.leaf_mask = (1u << p.depth) - 1u;
+  ia.flat = pplan.flat ? 1 : 0;
+  ia.code_columns = shape.columns;
+  ia.Ci = (int)p.Ci;
+  ia.Co = (int)p.Co;
+  ia.H = p.H;
+  ia.W = p.W;
+  ia.Wo = p.Wo;
+  ia.sy = p.sy;
+  ia.sx = p.sx;
+  ia.py = p.py;
+  ia.px = p.px;
+  ia.dy = p.dy;
+  ia.dx = p.dx;
+  ia.kw = p.kw;
+  HT_CUDA_TRY(cudaFuncSetAttribute(conv_image_from_codes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+  for (int64_t b0 = 0; b0 < p.B; b0 += at_once) {
+    ConvTileProblem part = p;
+    part.B = std::min<int64_t>(at_once, p.B - b0);
+    const float *part_g = g + b0 * p.Co * positions;
+    const int rc = launch_parameters(part, pplan, x + b0 * p.Ci * image, rec, part_g, gthr, gw,
+                                     gx != nullptr ? static_cast<uint2 *>(codes) : nullptr, status_word, stream);
+    if (rc != HT_OK) return rc;
+    if (gx == nullptr) continue;
+    ia.g = part_g;
+    ia.gx = gx + b0 * p.Ci * image;
+    const int64_t blocks = ia.quad_blocks * ia.channel_pairs * part.B;
+    ia.splits = (int)std::max<int64_t>(1, std::min<int64_t>({16, p.Co / 16, 148 * 6 / blocks}));
+    conv_image_from_codes_kernel<<<(unsigned)(blocks * ia.splits), 32 * warps, smem, stream>>>(ia);
+    HT_CHECK_LAUNCH();
+  }
+  return HT_OK;
 }
 
 int conv_backward_tiled(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w,
-                        const float *g, float *gx, float *gthr, float *gw, void *records, uint32_t *status_word,
-                        cudaStream_t stream) {
+                        const float *g, float *gx, float *gthr, float *gw, void *records, void *codes, size_t code_bytes,
+                        uint32_t *status_word, cudaStream_t stream) {
+  if (gthr != nullptr || gw != nullptr) {
+    const int rc = backward_by_codes(p, x, thr, ord, w, g, gx, gthr, gw, records, codes, code_bytes, status_word, stream);
+    if (rc != HT_ERR_UNSUPPORTED) return rc;
+  }
   ConvBwdPlan plan;
   ParamGradPlan pplan;
   bool with_params;
@@ -780,41 +1085,9 @@ int conv_backward_tiled(const ConvTileProblem &p, const float *x, const float *t
   // Shallow trees: the parameter gradients come from the kernel built for them, and the kernel
   // below is left with the image gradient.
   if ((gthr != nullptr || gw != nullptr) && with_params) {
-    ParamGradArgs pa;
-    pa.x = x;
-    pa.records = rec;
-    pa.g = g;
-    pa.gthr = gthr;
-    pa.gw = gw;
-    pa.status_word = status_word;
-    pa.Ci = (int)p.Ci;
-    pa.Co = (int)p.Co;
-    pa.H = p.H;
-    pa.W = p.W;
-    pa.Ho = p.Ho;
-    pa.Wo = p.Wo;
-    pa.sy = p.sy;
-    pa.sx = p.sx;
-    pa.py = p.py;
-    pa.px = p.px;
-    pa.R = pplan.R;
-    pa.columns = pplan.columns;
-    pa.staged = pplan.staged;
-    pa.patch_h = pplan.patch_h;
-    pa.patch_w = pplan.patch_w;
-    pa.tiles_x = tiles_x;
-    pa.row_blocks = (p.Ho + pplan.R - 1) / pplan.R;
-    const int64_t tiles = p.B * pa.tiles_x * pa.row_blocks;
-    if (tiles <= 0x7fffffff) {
-      // enough CTAs for about seven rounds of the machine, so that the last round's idle SMs cost little
-      const int64_t rounds = (p.Co + kWarps - 1) / kWarps;
-      int64_t splits = 1;
-      if (tiles < 7 * 148) splits = std::min<int64_t>(rounds, (7 * 148 + tiles - 1) / tiles);
-      const dim3 pgrid((unsigned)tiles, (unsigned)std::max<int64_t>(splits, 1));
-      const int rc = p.kind == TREE ? launch_params_kind<TREE>(p.depth, pplan, pa, pgrid, stream)
-                                    : launch_params_kind<FERN>(p.depth, pplan, pa, pgrid, stream);
-      if (rc != HT_OK) return rc;
-      if (gx == nullptr) return HT_OK;
+    const int rc = launch_parameters(p, pplan, x, rec, g, gthr, gw, nullptr, status_word, stream);
+    if (rc != HT_ERR_UNSUPPORTED) {
+      if (rc != HT_OK || gx == nullptr) return rc;
       gthr = nullptr;
       gw = nullptr;
     }

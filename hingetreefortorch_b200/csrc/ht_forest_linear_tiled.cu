@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(kBackwardBlock) linear_rows_backward_kernel(co
   for (int e = tid; e < (int)a.T * OP; e += kBackwardBlock) sums[e] = 0.0f;
   for (int e = tid; e < OP * kPitch; e += kBackwardBlock) gt[e] = 0.0f;
   const int64_t blocks = (a.B + kBackwardBlock - 1) / kBackwardBlock;
+  const int64_t share = (a.T + gridDim.y - 1) / gridDim.y;  // few record blocks: their trees are split over gridDim.y
+  const int64_t tree0 = blockIdx.y * share, tree_end = min(tree0 + share, a.T);
   const int O = (int)a.O;
   for (int64_t block = blockIdx.x; block < blocks; block += gridDim.x) {
     __syncthreads();
@@ -111,7 +113,7 @@ __global__ void __launch_bounds__(kBackwardBlock) linear_rows_backward_kernel(co
       gt[o * kPitch + s] = s < here ? __ldg(a.g + i0 * O + e) : 0.0f;
     }
     __syncthreads();
-    for (int64_t j = warp; j < a.T; j += kBackwardBlock / 32) {
+    for (int64_t j = tree0 + warp; j < tree_end; j += kBackwardBlock / 32) {
       const int64_t at0 = (block * a.T + j) * kRecordBlock + lane;
       const float *leaves = a.w + j * a.L;
       float l[OP], gl[OP];
@@ -195,7 +197,9 @@ int launch_backward(const LinearArgs &a, cudaStream_t stream) {
   const size_t smem = backward_smem(a.T, OP);
   if (smem > 48 * 1024) HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int64_t blocks = (a.B + kBackwardBlock - 1) / kBackwardBlock;
-  kernel<<<(unsigned)std::min<int64_t>(blocks, 148 * 4), kBackwardBlock, smem, stream>>>(a);
+  // four CTAs per SM, and a tree for every warp
+  const int64_t splits = std::max<int64_t>(1, std::min<int64_t>(148 * 4 / blocks, (a.T + 7) / 8));
+  kernel<<<dim3((unsigned)std::min<int64_t>(blocks, 148 * 4), (unsigned)splits), kBackwardBlock, smem, stream>>>(a);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }

@@ -275,6 +275,9 @@ typedef struct ht_conv_problem {
 
 int ht_conv_output_size(const ht_conv_problem *p, int64_t *osize /* [dims] */);
 size_t ht_conv_workspace_bytes(const ht_conv_problem *p);
+/* For a single precision backward that walks once for all gradients: room for 2 bytes per evaluation beyond
+ * ht_conv_workspace_bytes(p) (at most 8 GiB; the batch then goes in parts).  With less the kernels walk for themselves. */
+size_t ht_conv_backward_workspace_bytes(const ht_conv_problem *p);
 int ht_conv_forward_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
                         float *out, void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream);
 int ht_conv_backward_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
