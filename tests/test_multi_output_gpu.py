@@ -71,3 +71,20 @@ def test_forward_and_backward(kind, shape):
     got = f.forward(dev(x)[0], dthr, dord, dw).cpu().numpy()
     assert np.array_equal(got, ho.forward(kind, x, thr, ord_, w), equal_nan=True)
     assert f.ordinal_flags() == 0
+
+
+@pytest.mark.parametrize("depth", [5, 8])
+def test_terms_formed_in_the_reduction(depth):
+    """One output per leaf, many samples: the expansion hands on the upstream gradient and the reduction forms the terms."""
+    B, C, T = 65537 + 30, 20, 16
+    x, thr, ord_, w = random_forest_inputs(400 + depth, "tree", B, C, (), T, depth, (), quantise=True)
+    g = np.random.default_rng(6).standard_normal((B, T)).astype(np.float32)
+    ref = ho.backward("tree", x, thr, ord_, w, g)
+    sizes = ho.backward_magnitudes("tree", x, thr, ord_, w, g)
+    dx, dthr, dord, dw, dg = dev(x, thr, ord_, w, g)
+    f = _cabi.Forest("tree", dx, dw)
+    assert f.saves_forward()
+    for need in ((True, True, True), (True, True, False), (True, False, True)):
+        f.forward(dx, dthr, dord, dw, save=True)
+        for wanted, got, r, s in zip(need, f.backward(dx, dthr, dord, dw, dg, need=need, saved=True), ref, sizes):
+            assert (got is None) if not wanted else grad_close(got, r, s)
