@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(kBackwardBlock) linear_rows_backward_kernel(co
   for (int e = tid; e < (int)a.T * OP; e += kBackwardBlock) sums[e] = 0.0f;
   for (int e = tid; e < OP * kPitch; e += kBackwardBlock) gt[e] = 0.0f;
   const int64_t blocks = (a.B + kBackwardBlock - 1) / kBackwardBlock;
-  const int64_t share = (a.T + gridDim.y - 1) / gridDim.y;  // few record blocks: their trees are split over gridDim.y
-  const int64_t tree0 = blockIdx.y * share, tree_end = min(tree0 + share, a.T);
+  const int share = ((int)a.T + (int)gridDim.y - 1) / (int)gridDim.y;  // few record blocks: their trees are split over gridDim.y
+  const int tree0 = (int)blockIdx.y * share, tree_end = min(tree0 + share, (int)a.T);
   const int O = (int)a.O;
   for (int64_t block = blockIdx.x; block < blocks; block += gridDim.x) {
     __syncthreads();
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(kBackwardBlock) linear_rows_backward_kernel(co
       gt[o * kPitch + s] = s < here ? __ldg(a.g + i0 * O + e) : 0.0f;
     }
     __syncthreads();
-    for (int64_t j = tree0 + warp; j < tree_end; j += kBackwardBlock / 32) {
+    for (int j = tree0 + warp; j < tree_end; j += kBackwardBlock / 32) {
       const int64_t at0 = (block * a.T + j) * kRecordBlock + lane;
       const float *leaves = a.w + j * a.L;
       float l[OP], gl[OP];

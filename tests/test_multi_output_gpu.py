@@ -32,7 +32,7 @@ SHAPES = [
     (2050, 784, (), 300, 8, 1),
     (8195, 200, (), 4, 3, 2),
     # leaf weights that do not fit beside a tile; few trees whose samples are split among blocks
-    (1100, 579, (), 30, 12, 1),
+    (9500, 719, (), 6, 12, 1),
     (9000, 30, (), 4, 10, 1),
     (33000, 12, (), 3, 4, 1),
     # too few evaluations for the sorted backward, but not for the fixed order; one output, more than a buffer of terms holds
