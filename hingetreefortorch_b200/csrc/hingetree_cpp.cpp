@@ -388,6 +388,12 @@ std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torc
   return {out, saved ? ws : fresh({0}, ws)};
 }
 
+// Bytes of the scratch that a saving forward returns in the given mode; 0: it keeps nothing.
+static size_t kept_bytes(ht_forest_problem problem, bool deterministic) {
+  problem.flags = HT_WORKSPACE_FOR_BACKWARD | (deterministic ? HT_DETERMINISTIC : 0u);
+  return ht_forest_forward_saves(&problem) != 0 ? ht_forest_workspace_bytes(&problem) : 0;
+}
+
 std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, torch::Tensor x, bool need_x,
                                                  torch::Tensor thr, bool need_thr, torch::Tensor ord, bool need_ord,
                                                  torch::Tensor w, bool need_w, torch::Tensor g, torch::Tensor saved) {
@@ -396,14 +402,16 @@ std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, t
   c10::DeviceGuard guard(x.device());
   std::vector<torch::Tensor> grads(4);
   if (!need_x && !need_thr && !need_w) return grads;
-  if (deterministic) call.problem.flags |= HT_DETERMINISTIC;
-  call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD | HT_SAVED_FORWARD;
-  if (saved.defined() && deterministic && (size_t)saved.numel() < ht_forest_workspace_bytes(&call.problem))
-    // the mode was switched on after the forward, which kept less than the fixed order needs
-    return forest_backward(kind, deterministic, x, need_x, thr, need_thr, ord, need_ord, w, need_w, g);
-  if (!saved.defined() || saved.device() != x.device() || saved.scalar_type() != torch::kUInt8 ||
-      (size_t)saved.numel() < ht_forest_workspace_bytes(&call.problem) || ht_forest_forward_saves(&call.problem) == 0)
+  // Each mode keeps what its own backward needs, and one may keep where the other does not.  Where the mode was switched after
+  // the forward and its scratch does not serve this one, the trees are walked again.
+  const auto holds = [&](bool mode) {
+    const size_t bytes = kept_bytes(call.problem, mode);
+    return bytes != 0 && (size_t)saved.numel() >= bytes;
+  };
+  if (!saved.defined() || saved.device() != x.device() || saved.scalar_type() != torch::kUInt8 || !(holds(false) || holds(true)))
     bad_argument("Error: `saved` is not the scratch a saving forward returned for these tensors.");
+  if (!holds(deterministic)) return forest_backward(kind, deterministic, x, need_x, thr, need_thr, ord, need_ord, w, need_w, g);
+  call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD | HT_SAVED_FORWARD | (deterministic ? HT_DETERMINISTIC : 0u);
   if (need_x) grads[0] = fresh_like(x);
   if (need_thr) grads[1] = fresh_like(thr);
   if (need_w) grads[3] = fresh_like(w);

@@ -218,6 +218,44 @@ def test_backward_scratch_limit_switches_to_scatters(ext):
         ext.set_backward_scratch_limit(-1)
 
 
+# B, C, T, depth, outputs per leaf: the forward keeps its paths in fixed-order mode only (too few evaluations; more than 64
+# outputs), in both modes (several outputs; one), in neither
+SWITCHED = [(100, 1000, 100, 7, 10), (700, 20, 50, 4, 70), (1100, 40, 31, 6, 3), (2048, 64, 32, 6, 1), (200, 16, 6, 3, 1)]
+
+
+@pytest.mark.parametrize("shape", SWITCHED, ids=[str(s) for s in SWITCHED])
+@pytest.mark.parametrize("forward_mode", [False, True], ids=["off_then_on", "on_then_off"])
+def test_fixed_order_switched_between_forward_and_backward(shape, forward_mode):
+    """torch.use_deterministic_algorithms changed between the two: the backward runs in the mode that is set when it runs."""
+    from hingetreefortorch_b200.HingeTree import HingeTree
+    B, C, T, depth, M = shape
+    x, thr, ord_, w = random_forest_inputs(31, "tree", B, C, (), T, depth, (M,))
+    g = np.random.default_rng(9).standard_normal((B, T, M)).astype(np.float32)
+    ref, mags = ho.backward("tree", x, thr, ord_, w, g), ho.backward_magnitudes("tree", x, thr, ord_, w, g)
+    dx, dthr, dord, dw, dg = dev(x, thr, ord_, w, g)
+    for t in (dx, dthr, dw):
+        t.requires_grad_(True)
+    try:
+        torch.use_deterministic_algorithms(forward_mode)
+        out = HingeTree.apply(dx, dthr, dord, dw)
+        torch.use_deterministic_algorithms(not forward_mode)
+        grads = torch.autograd.grad(out, (dx, dthr, dw), dg)
+    finally:
+        torch.use_deterministic_algorithms(False)
+    assert np.array_equal(out.detach().cpu().numpy(), ho.forward("tree", x, thr, ord_, w))
+    for got, r, m in zip(grads, ref, mags):
+        assert np.array_equal(got.cpu().numpy(), r) if not forward_mode else grad_close(got, r, m)
+
+
+def test_scratch_of_no_saving_forward_is_refused(ext):
+    x, thr, ord_, w = random_forest_inputs(32, "tree", 100, 30, (), 20, 5, (4,))
+    dx, dthr, dord, dw = dev(x, thr, ord_, w)
+    g = torch.ones(100, 20, 4, device="cuda")
+    for scratch in (torch.empty(0, dtype=torch.uint8, device="cuda"), torch.empty(1 << 20, device="cuda"), torch.empty(1 << 20, dtype=torch.uint8)):
+        with pytest.raises(ValueError, match="saving forward"):
+            ext.tree_backward_saved(dx, True, dthr, True, dord, False, dw, True, g, scratch, False)
+
+
 def test_speedtest_sweeps_like_the_reference(ext, capfd):
     """The reference's own benchmark operator: trees 1..512 by powers of two, depth 1..12, rows = trees, depth,
     forward ms, backward ms (hingetree.cpp:1361-1438)."""
