@@ -12,6 +12,7 @@
 #include <c10/cuda/CUDAStream.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <limits>
 #include <mutex>
@@ -193,11 +194,11 @@ void selftest_bounded_wait() {
                "selftest_bounded_wait");
 }
 
-// Most scratch a backward call may take for its per-evaluation records (12 bytes per tree
-// evaluation).  Beyond it the call runs without them: atomic scatters instead of ordered sums.
-// Default: whatever fits (an allocation that fails falls back to the path without records); a caller may
-// set a smaller figure.
-static int64_t g_backward_scratch_limit = INT64_MAX;
+// Most scratch a plain forest's backward may take, or a forward may keep for it.  Per tree evaluation that is 10 or 12 bytes
+// with one output per leaf, 6 or 8 with several, and in fixed-order mode 16 more for the lists.  A call that would need
+// more runs with less: the same results, from kernels that are slower.  Default: whatever fits (an allocation that fails
+// counts as one beyond the limit); a caller may set a smaller figure.  Read by backward threads, too.
+static std::atomic<int64_t> g_backward_scratch_limit{INT64_MAX};
 
 void set_backward_scratch_limit(int64_t bytes) {
   if (bytes < 0) bad_argument("Error: the scratch limit is a number of bytes >= 0.");
@@ -302,6 +303,32 @@ torch::Tensor forest_forward(int kind, torch::Tensor x, torch::Tensor thr, torch
   return out;
 }
 
+namespace {
+
+// Bytes of the workspace with room for what a backward keeps per evaluation: all that it can use; or what still serves it
+// (one output per leaf in fixed-order mode: the default mode's records, without the lists); or none of it.
+enum class Scratch { All, Records, None };
+size_t scratch_bytes(ht_forest_problem problem, Scratch scratch) {
+  problem.flags &= scratch == Scratch::All ? HT_DETERMINISTIC : 0u;
+  if (scratch == Scratch::All || (scratch == Scratch::Records && problem.M == 1)) problem.flags |= HT_WORKSPACE_FOR_BACKWARD;
+  return ht_forest_workspace_bytes(&problem);
+}
+
+// The largest of these workspaces that the limit and the device's memory admit.
+torch::Tensor backward_workspace(const ht_forest_problem &problem, const torch::Tensor &like) {
+  for (const Scratch scratch : {Scratch::All, Scratch::Records}) {
+    const size_t bytes = scratch_bytes(problem, scratch);
+    if ((int64_t)bytes > g_backward_scratch_limit) continue;
+    try {
+      return make_workspace(bytes, like);
+    } catch (const c10::OutOfMemoryError &) {
+    }
+  }
+  return make_workspace(scratch_bytes(problem, Scratch::None), like);
+}
+
+}  // namespace
+
 std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::Tensor x, bool need_x, torch::Tensor thr,
                                            bool need_thr, torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w,
                                            torch::Tensor g) {
@@ -327,19 +354,7 @@ std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::
     og.finish();
     return grads;
   }
-  call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD;
-  if ((int64_t)ht_forest_workspace_bytes(&call.problem) > g_backward_scratch_limit && !deterministic)
-    call.problem.flags &= ~HT_WORKSPACE_FOR_BACKWARD;
-  torch::Tensor ws;
-  try {
-    ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
-  } catch (const c10::OutOfMemoryError &) {
-    // no room for the evaluation records (10 to 12 bytes per tree evaluation): the default mode can do
-    // without them (the reference allocates nothing for its backward either); the fixed-order mode cannot
-    if (deterministic || (call.problem.flags & HT_WORKSPACE_FOR_BACKWARD) == 0) throw;
-    call.problem.flags &= ~HT_WORKSPACE_FOR_BACKWARD;
-    ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
-  }
+  torch::Tensor ws = backward_workspace(call.problem, x);
   OrdinalGuard og(ord, call.problem.C);
   raise_status(
       ht_forest_backward_f32(&call.problem, x.data_ptr<float>(), thr.data_ptr<float>(), ord.data_ptr<int64_t>(),
@@ -356,7 +371,13 @@ std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::
 // Not part of the reference's operator set: the reference's backward walks every tree again (three times).  These
 // two let the autograd layer walk them once per training step.  `saved` is the call's scratch, which holds the
 // traversal; it is empty when the library does not save for this problem (the caller then uses the plain backward).
-static bool g_save_forward = true;
+static std::atomic<bool> g_save_forward{true};
+
+// Bytes that a saving forward's scratch has at least, in the problem's mode; 0: nothing is kept.
+static size_t kept_bytes(const ht_forest_problem &problem) {
+  if (ht_forest_forward_saves(&problem) == 0) return 0;
+  return scratch_bytes(problem, problem.M == 1 ? Scratch::Records : Scratch::All);
+}
 
 std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torch::Tensor thr, torch::Tensor ord,
                                                  torch::Tensor w) {
@@ -365,33 +386,18 @@ std::vector<torch::Tensor> forest_forward_saving(int kind, torch::Tensor x, torc
   ForestCall call(kind, x, thr, ord, w, nullptr);
   c10::DeviceGuard guard(x.device());
   if (at::globalContext().deterministicAlgorithms()) call.problem.flags |= HT_DETERMINISTIC;  // the scratch its backward needs
-  const bool saves = g_save_forward && ht_forest_forward_saves(&call.problem) != 0;
-  if (saves) call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD | HT_SAVE_FOR_BACKWARD;
-  if (saves && (int64_t)ht_forest_workspace_bytes(&call.problem) > g_backward_scratch_limit)
-    call.problem.flags &= ~(HT_WORKSPACE_FOR_BACKWARD | HT_SAVE_FOR_BACKWARD);
   torch::Tensor out = fresh(call.out_sizes, x);
-  torch::Tensor ws;
-  try {
-    ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
-  } catch (const c10::OutOfMemoryError &) {
-    if ((call.problem.flags & HT_SAVE_FOR_BACKWARD) == 0) throw;
-    call.problem.flags &= ~(HT_WORKSPACE_FOR_BACKWARD | HT_SAVE_FOR_BACKWARD);  // no room: a plain forward
-    ws = make_workspace(ht_forest_workspace_bytes(&call.problem), x);
-  }
+  const bool saves = g_save_forward && ht_forest_forward_saves(&call.problem) != 0;
+  torch::Tensor ws = saves ? backward_workspace(call.problem, x) : make_workspace(scratch_bytes(call.problem, Scratch::None), x);
+  const bool saved = saves && (size_t)ws.numel() > scratch_bytes(call.problem, Scratch::None);
+  if (saved) call.problem.flags |= HT_SAVE_FOR_BACKWARD;
   OrdinalGuard og(ord, call.problem.C);
   raise_status(ht_forest_forward_f32(&call.problem, x.data_ptr<float>(), thr.data_ptr<float>(), ord.data_ptr<int64_t>(),
                                      w.data_ptr<float>(), out.data_ptr<float>(), ws.data_ptr(), ws.numel(), og.word(),
                                      current_stream(x)),
                "forest forward");
   og.finish();
-  const bool saved = (call.problem.flags & HT_SAVE_FOR_BACKWARD) != 0;
   return {out, saved ? ws : fresh({0}, ws)};
-}
-
-// Bytes of the scratch that a saving forward returns in the given mode; 0: it keeps nothing.
-static size_t kept_bytes(ht_forest_problem problem, bool deterministic) {
-  problem.flags = HT_WORKSPACE_FOR_BACKWARD | (deterministic ? HT_DETERMINISTIC : 0u);
-  return ht_forest_forward_saves(&problem) != 0 ? ht_forest_workspace_bytes(&problem) : 0;
 }
 
 std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, torch::Tensor x, bool need_x,
@@ -404,14 +410,17 @@ std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, t
   if (!need_x && !need_thr && !need_w) return grads;
   // Each mode keeps what its own backward needs, and one may keep where the other does not.  Where the mode was switched after
   // the forward and its scratch does not serve this one, the trees are walked again.
-  const auto holds = [&](bool mode) {
-    const size_t bytes = kept_bytes(call.problem, mode);
+  const auto holds_paths = [&](bool mode) {
+    if (!saved.defined() || saved.device() != x.device() || saved.scalar_type() != torch::kUInt8) return false;
+    call.problem.flags = mode ? HT_DETERMINISTIC : 0u;
+    const size_t bytes = kept_bytes(call.problem);
     return bytes != 0 && (size_t)saved.numel() >= bytes;
   };
-  if (!saved.defined() || saved.device() != x.device() || saved.scalar_type() != torch::kUInt8 || !(holds(false) || holds(true)))
+  if (!holds_paths(deterministic)) {
+    if (holds_paths(!deterministic)) return forest_backward(kind, deterministic, x, need_x, thr, need_thr, ord, need_ord, w, need_w, g);
     bad_argument("Error: `saved` is not the scratch a saving forward returned for these tensors.");
-  if (!holds(deterministic)) return forest_backward(kind, deterministic, x, need_x, thr, need_thr, ord, need_ord, w, need_w, g);
-  call.problem.flags |= HT_WORKSPACE_FOR_BACKWARD | HT_SAVED_FORWARD | (deterministic ? HT_DETERMINISTIC : 0u);
+  }
+  call.problem.flags |= HT_SAVED_FORWARD;
   if (need_x) grads[0] = fresh_like(x);
   if (need_thr) grads[1] = fresh_like(thr);
   if (need_w) grads[3] = fresh_like(w);
@@ -866,8 +875,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "Initialize thresholds and ordinals by random decision tree learning on class labels (CPU only).");
   m.def("seed_init", &seed_init, "Seed the generator tree_init_greedy draws from.");
   m.def("set_backward_scratch_limit", &set_backward_scratch_limit,
-        "Upper bound in bytes on the scratch a default-mode backward call allocates for its per-evaluation records "
-        "(12 bytes per tree evaluation); above it the gradients are scattered with atomics instead. Default: no bound.");
+        "Upper bound in bytes on the scratch a forest's backward allocates for what it keeps per tree evaluation (6 to 12 bytes, "
+        "in fixed-order mode 22 to 28) and its forward keeps for it; above it slower kernels give the same results. Default: no "
+        "bound.");
   m.def("batchnorm_statistics", &batchnorm_statistics,
         "[mean, biased variance, 1 / sqrt(variance + eps)] per column from the columns' sums and sums of squares over `rows` rows.");
   m.def("linear_tf32_stats", &linear_tf32_stats,

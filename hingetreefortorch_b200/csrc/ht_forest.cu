@@ -495,6 +495,9 @@ static size_t records_bytes(const ht_forest_problem *p) {
   return p->M > 1 ? multi_area_bytes(p, sizeof(float)) : backward_records_bytes(p);
 }
 
+// What still serves the fixed order without the lists.
+static size_t records_without_lists(const ht_forest_problem *p) { return p->M == 1 ? backward_records_bytes(p) : 0; }
+
 int ht_forest_forward_saves(const ht_forest_problem *p) {
   if (check_forest_problem(p) != HT_OK) return 0;
   return p->M == 1 ? forward_saves(p) : records_bytes(p) > 0;
@@ -519,7 +522,8 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
   void *eval_records = nullptr;
   if ((p->flags & HT_SAVE_FOR_BACKWARD) != 0 && ht_forest_forward_saves(p)) {
     const size_t records_at = ordinals_bytes(p) + forward_tiled_workspace_bytes(p);
-    if (workspace_bytes >= records_at + records_bytes(p)) eval_records = ws + records_at;
+    const size_t kept = p->M == 1 ? records_without_lists(p) : records_bytes(p);
+    if (workspace_bytes >= records_at + kept) eval_records = ws + records_at;
   }
   const WideOrdinals wide = {ord, p->C};
   int32_t *packed = static_cast<int32_t *>(workspace);
@@ -596,9 +600,14 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
     // they serve both modes (that path is fixed-order), without it only the default mode.
     unsigned char *ws = static_cast<unsigned char *>(workspace);
     const size_t records_at = ordinals_bytes(p) + forward_tiled_workspace_bytes(p);
-    const size_t eval_bytes = records_bytes(p);
+    size_t eval_bytes = records_bytes(p);
+    bool ordered = ordered_from_paths(p);
+    if (ordered && workspace_bytes < records_at + eval_bytes) {
+      // no room for the lists: the same order from the tile kernels' records, or from kernels that keep nothing
+      ordered = false;
+      eval_bytes = records_without_lists(p);
+    }
     void *eval_records = eval_bytes > 0 && workspace_bytes >= records_at + eval_bytes ? ws + records_at : nullptr;
-    const bool ordered = ordered_from_paths(p);
     // what a saving forward left in the workspace: the paths, and the packed ordinals
     const bool kept = (p->flags & HT_SAVED_FORWARD) != 0 && eval_records != nullptr && ht_forest_forward_saves(p);
     const int64_t *to_pack = kept ? nullptr : ord;

@@ -78,22 +78,24 @@ uint64_t ht_launch_count(void); /* kernels this library has launched in this pro
 int ht_selftest_bounded_wait(uint32_t *status_word, ht_stream_t stream);
 
 /* Scratch bytes ht_forest_* calls need for this problem: compact ordinals and the tile kernel's
- * per-tree records.  With HT_WORKSPACE_FOR_BACKWARD in p->flags the figure also covers 12 bytes
- * per (sample, tree) of evaluation records (10 up to depth 8), which let ht_forest_backward_f32 run its fastest,
- * fixed-order path on tabular one-output-per-leaf problems (up to 32 GiB; beyond that, and
- * whenever the workspace passed is smaller, the backward uses its other paths).  The workspace
- * must be 256-byte aligned device memory. */
+ * per-tree records.  With HT_WORKSPACE_FOR_BACKWARD in p->flags the figure also covers what ht_forest_backward_f32
+ * keeps per tree evaluation on its fastest paths: with one output per leaf 10 bytes (12 beyond depth 8), with several
+ * 6 (8), each up to 32 GiB and none where those paths do not take the problem; with HT_DETERMINISTIC 16 bytes more (one
+ * output per leaf: up to 2^26 evaluations), and no bound.  The results do not depend on it: whenever the workspace passed
+ * is smaller, the backward uses its other paths (in fixed-order mode with one output per leaf a workspace of the default
+ * mode's size still serves the record path).  The workspace must be 256-byte aligned device memory. */
 size_t ht_forest_workspace_bytes(const ht_forest_problem *p);
 
 /* Saving the forward's traversal for the backward.  The reference's backward walks every tree again, three
  * times (hingetree_gpu.cu:699-727); here a training step can walk them once: ht_forest_forward_f32 called with
- * HT_SAVE_FOR_BACKWARD and a workspace sized with HT_WORKSPACE_FOR_BACKWARD leaves, per (sample, tree), the
+ * HT_SAVE_FOR_BACKWARD and a workspace sized with HT_WORKSPACE_FOR_BACKWARD leaves, per evaluation, the
  * signed margin and the deciding vertex / leaf in the workspace (6 or 8 bytes), and ht_forest_backward_f32
  * called with HT_SAVED_FORWARD on the SAME x, thr, ord, w and workspace — nothing else having used the
  * workspace in between — computes the gradients from them.  ht_forest_forward_saves() tells whether the
- * forward does so for a problem (tabular input, one output per leaf, shapes the tile kernel takes with whole
- * tree groups); where it returns 0 both flags are ignored.  Both modes: with HT_DETERMINISTIC the sums are
- * the reference's, bit for bit, as without saving. */
+ * forward does so for a problem: with one output per leaf tabular shapes that the tile kernel takes with whole
+ * tree groups; with several any shape, from 32768 evaluations and up to 64 outputs on in default mode, up to depth 12
+ * (so it can differ between the modes of one problem).  Where it returns 0 both flags are ignored.  Both modes: with
+ * HT_DETERMINISTIC the sums are the reference's, bit for bit, as without saving. */
 int ht_forest_forward_saves(const ht_forest_problem *p);
 
 /* out[i,j,k,m] = |margin(i,j,k)| * w[j, leaf(i,j,k), m]

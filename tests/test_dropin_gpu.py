@@ -218,6 +218,63 @@ def test_backward_scratch_limit_switches_to_scatters(ext):
         ext.set_backward_scratch_limit(-1)
 
 
+# B, C, T, depth, outputs per leaf: one output with and without tile records, several
+@pytest.mark.parametrize("shape", [(4096, 64, 32, 6, 1), (7000, 20, 4, 7, 1), (3000, 30, 20, 6, 3)], ids=str)
+@pytest.mark.parametrize("room", ["all", "records", "none"])
+def test_scratch_limit_in_fixed_order_mode(ext, shape, room):
+    """The fixed-order mode stays within the limit, and its sums keep their order with any scratch: with the lists, with the
+    default mode's records (one output per leaf) and with none."""
+    from hingetreefortorch_b200.HingeTree import HingeTree
+    B, C, T, depth, M = shape
+    x, thr, ord_, w = random_forest_inputs(33, "tree", B, C, (), T, depth, (M,))
+    g = np.random.default_rng(10).standard_normal((B, T, M)).astype(np.float32)
+    ref = ho.backward("tree", x, thr, ord_, w, g)
+    dx, dthr, dord, dw, dg = dev(x, thr, ord_, w, g)
+    ext.tree_forward(dx, dthr, dord, dw)  # the ordinals' check takes memory of its own
+    for t in (dx, dthr, dw):
+        t.requires_grad_(True)
+    parameters = 16 * thr.size + 8 * w.size + 65536  # packed ordinals, tree records
+    limit = {"all": 2 ** 62, "records": 12 * B * T + parameters, "none": parameters}[room]
+    results = x.nbytes + thr.nbytes + w.nbytes + g.nbytes + 65536
+    torch.use_deterministic_algorithms(True)
+    ext.set_backward_scratch_limit(limit)
+    try:
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before = torch.cuda.memory_allocated()
+        out = HingeTree.apply(dx, dthr, dord, dw)
+        assert torch.cuda.memory_allocated() - before <= g.nbytes + limit
+        grads = torch.autograd.grad(out, (dx, dthr, dw), dg)
+        peak = torch.cuda.max_memory_allocated() - before
+    finally:
+        ext.set_backward_scratch_limit(2 ** 62)
+        torch.use_deterministic_algorithms(False)
+    assert np.array_equal(out.detach().cpu().numpy(), ho.forward("tree", x, thr, ord_, w))
+    for got, r in zip(grads, ref):
+        assert np.array_equal(got.cpu().numpy(), r)
+    assert peak <= results + limit if room != "all" else peak > results + 16 * B * T
+
+
+def test_fixed_order_mode_without_memory_for_its_lists(ext):
+    """An allocation that fails is like a limit: the step goes on without the lists."""
+    B, C, T, depth, M = 40000, 20, 100, 4, 2
+    x, thr, ord_, w = random_forest_inputs(34, "tree", B, C, (), T, depth, (M,))
+    g = np.random.default_rng(11).standard_normal((B, T, M)).astype(np.float32)
+    ref = ho.backward("tree", x, thr, ord_, w, g)
+    dx, dthr, dord, dw, dg = dev(x, thr, ord_, w, g)
+    ext.tree_forward(dx, dthr, dord, dw)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(0).total_memory
+    torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved() + 40 * 2 ** 20) / total)  # the lists take 88 MB
+    try:
+        grads = ext.tree_backward_deterministic(dx, True, dthr, True, dord, False, dw, True, dg)
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    for got, r in zip((grads[0], grads[1], grads[3]), ref):
+        assert np.array_equal(got.cpu().numpy(), r)
+
+
 # B, C, T, depth, outputs per leaf: the forward keeps its paths in fixed-order mode only (too few evaluations; more than 64
 # outputs), in both modes (several outputs; one), in neither
 SWITCHED = [(100, 1000, 100, 7, 10), (700, 20, 50, 4, 70), (1100, 40, 31, 6, 3), (2048, 64, 32, 6, 1), (200, 16, 6, 3, 1)]
