@@ -194,11 +194,14 @@ void selftest_bounded_wait() {
                "selftest_bounded_wait");
 }
 
-// Most scratch a plain forest's backward may take, or a forward may keep for it.  Per tree evaluation that is 10 or 12 bytes
-// with one output per leaf, 6 or 8 with several, and in fixed-order mode 16 more for the lists.  A call that would need
-// more runs with less: the same results, from kernels that are slower.  Default: whatever fits (an allocation that fails
-// counts as one beyond the limit); a caller may set a smaller figure.  Read by backward threads, too.
+// Most scratch a backward may take beyond what it cannot do without, or a forward may keep for it.  Per tree evaluation the
+// plain forest takes 10 or 12 bytes with one output per leaf, 6 or 8 with several, and in fixed-order mode 16 more for the
+// lists; the convolution 2.  A call that would need more runs with less: the same results, from kernels that are slower.
+// Default: whatever fits (an allocation that fails counts as one beyond the limit); a caller may set a smaller figure.  Read
+// by backward threads, too.
 static std::atomic<int64_t> g_backward_scratch_limit{INT64_MAX};
+
+int64_t backward_scratch_limit() { return g_backward_scratch_limit; }
 
 void set_backward_scratch_limit(int64_t bytes) {
   if (bytes < 0) bad_argument("Error: the scratch limit is a number of bytes >= 0.");
@@ -875,9 +878,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "Initialize thresholds and ordinals by random decision tree learning on class labels (CPU only).");
   m.def("seed_init", &seed_init, "Seed the generator tree_init_greedy draws from.");
   m.def("set_backward_scratch_limit", &set_backward_scratch_limit,
-        "Upper bound in bytes on the scratch a forest's backward allocates for what it keeps per tree evaluation (6 to 12 bytes, "
-        "in fixed-order mode 22 to 28) and its forward keeps for it; above it slower kernels give the same results. Default: no "
-        "bound.");
+        "Upper bound in bytes on the scratch a backward allocates for what it keeps per tree evaluation (forest: 6 to 12 bytes, in "
+        "fixed-order mode 22 to 28; convolution: 2) and a forward keeps for it; above it slower kernels give the same results. "
+        "Default: no bound.");
   m.def("batchnorm_statistics", &batchnorm_statistics,
         "[mean, biased variance, 1 / sqrt(variance + eps)] per column from the columns' sums and sums of squares over `rows` rows.");
   m.def("linear_tf32_stats", &linear_tf32_stats,

@@ -4,6 +4,7 @@
 // RuntimeError for depth / ordinal range), allocate, call the C ABI on the current stream.
 #include <c10/core/DeviceGuard.h>
 
+#include <algorithm>
 #include <sstream>
 
 #include "hingetree_cpp_ops.h"
@@ -568,15 +569,19 @@ std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bo
   if (need_x) grads[0] = fresh_like(x);
   if (need_thr) grads[1] = fresh_like(thr);
   if (need_w) grads[3] = fresh_like(w);
+  // Room for the codes through which both kinds of gradients share one walk, as far as the limit allows: the batch goes in
+  // parts that fit, or without codes.
+  const size_t needed = ht_conv_workspace_bytes(&call.problem);
+  size_t bytes = needed;
+  if (x.scalar_type() == torch::kFloat32 && need_x && (need_thr || need_w))
+    bytes = std::max(needed, std::min(ht_conv_backward_workspace_bytes(&call.problem), (size_t)backward_scratch_limit()));
   torch::Tensor ws;
   try {
-    ws = make_workspace(x.scalar_type() == torch::kFloat32 && need_x && (need_thr || need_w)
-                            ? ht_conv_backward_workspace_bytes(&call.problem)
-                            : ht_conv_workspace_bytes(&call.problem),
-                        x);
-  } catch (const c10::OutOfMemoryError &) {  // no room for the shared walk
-    ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);
+    ws = make_workspace(bytes, x);
+  } catch (const c10::OutOfMemoryError &) {
+    if (bytes == needed) throw;
   }
+  if (!ws.defined()) ws = make_workspace(needed, x);
   OrdinalGuard og(ord, call.window_cells);
   dispatch_real(x, [&](auto real) {
     using Real = decltype(real);

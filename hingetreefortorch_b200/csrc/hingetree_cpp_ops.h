@@ -26,6 +26,7 @@ torch::Tensor make_workspace(size_t bytes, const torch::Tensor &like);
 torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like, c10::ScalarType type);
 inline torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like) { return fresh(sizes, like, like.scalar_type()); }
 inline torch::Tensor fresh_like(const torch::Tensor &like) { return fresh(like.sizes(), like); }
+int64_t backward_scratch_limit();  // set by the caller; see hingetree_cpp.cpp
 void set_ordinal_check(const std::string &mode);
 int64_t pipeline_status();
 

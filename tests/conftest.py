@@ -53,3 +53,10 @@ def grad_close(t, ref, scale, rel=1e-5):
     got = t.detach().cpu().numpy() if hasattr(t, "detach") else np.asarray(t)
     got = got.astype(np.float64)
     return bool(np.all(np.abs(got - np.asarray(ref, dtype=np.float64)) <= rel * np.asarray(scale, dtype=np.float64) + 1e-30))
+
+
+def requested_bytes(peak=False):
+    """Device memory that tensors have asked for, now or at the most since torch.cuda.reset_peak_memory_stats() (what the
+    allocator hands out is rounded up by as much as 1 MiB)."""
+    import torch
+    return torch.cuda.memory_stats()["requested_bytes.all." + ("peak" if peak else "current")]

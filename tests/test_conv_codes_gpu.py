@@ -2,9 +2,10 @@
 kernel walks); single rows of outputs, rows and columns off the tiles, odd channel counts, the widest and deepest codes."""
 import numpy as np
 import pytest
+import torch
 
 import hingetreefortorch_b200._cabi as _cabi
-from conftest import grad_close
+from conftest import grad_close, requested_bytes
 from oracle import hinge_oracle as ho
 from test_conv_gpu import dev
 
@@ -41,3 +42,33 @@ def test_backward_through_codes(kind, case):
         for got, r, s in zip(conv.backward(*tensors), ref, sizes):
             assert grad_close(got, r, s)
         assert int(conv.status.item()) == 0
+
+
+@pytest.mark.parametrize("samples", [5, 2, 0])
+def test_backward_within_the_scratch_limit(samples):
+    """The operator's codes stay within the limit that the caller set: the whole batch, two samples at a time, none."""
+    from hingetreefortorch_b200._ext import hingetree_cpp as ext
+    dims, xs, Co, depth, kernel, stride, padding, dilation = CASES[0]
+    rng = np.random.default_rng(80)
+    x = rng.standard_normal(xs).astype(np.float32)
+    thr = rng.uniform(-1, 1, (Co, xs[1], 2 ** depth - 1)).astype(np.float32)
+    ord_ = rng.integers(0, int(np.prod(kernel)), thr.shape).astype(np.int64)
+    w = rng.standard_normal((Co, xs[1], 2 ** depth)).astype(np.float32)
+    g = rng.standard_normal((xs[0], Co, 33, 65)).astype(np.float32)
+    ref = ho.conv_backward("tree", x, thr, ord_, w, g, kernel, stride, padding, dilation)
+    sizes = ho.magnitudes(ho.conv_backward, "tree", x, thr, ord_, w, g, kernel, stride, padding, dilation)
+    dx, dthr, dord, dw, dg = dev(x, thr, ord_, w, g)
+    ext.tree_conv2d_forward(dx, dthr, dord, dw, kernel, stride, padding, dilation)  # checks the ordinals
+    code_bytes = 2 * Co * xs[1] * 36 * 68 + 65536  # of a sample: rows and columns rounded up to groups; tree records
+    limit = samples * code_bytes
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = requested_bytes()
+    ext.set_backward_scratch_limit(limit)
+    try:
+        grads = ext.tree_conv2d_backward(dx, True, dthr, True, dord, False, dw, True, dg, kernel, stride, padding, dilation)
+    finally:
+        ext.set_backward_scratch_limit(2 ** 62)
+    assert requested_bytes(peak=True) - before <= x.nbytes + thr.nbytes + w.nbytes + max(limit, 16 * thr.size + 4 * w.size + 65536)
+    for got, r, s in zip((grads[0], grads[1], grads[3]), ref, sizes):
+        assert grad_close(got, r, s)

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import grad_close, random_forest_inputs
+from conftest import grad_close, random_forest_inputs, requested_bytes
 from oracle import hinge_oracle as ho
 
 pytestmark = pytest.mark.gpu
@@ -241,11 +241,11 @@ def test_scratch_limit_in_fixed_order_mode(ext, shape, room):
     try:
         torch.cuda.synchronize()
         torch.cuda.reset_peak_memory_stats()
-        before = torch.cuda.memory_allocated()
+        before = requested_bytes()
         out = HingeTree.apply(dx, dthr, dord, dw)
-        assert torch.cuda.memory_allocated() - before <= g.nbytes + limit
+        assert requested_bytes() - before <= g.nbytes + limit
         grads = torch.autograd.grad(out, (dx, dthr, dw), dg)
-        peak = torch.cuda.max_memory_allocated() - before
+        peak = requested_bytes(peak=True) - before
     finally:
         ext.set_backward_scratch_limit(2 ** 62)
         torch.use_deterministic_algorithms(False)
