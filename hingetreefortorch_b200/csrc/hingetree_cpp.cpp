@@ -203,6 +203,10 @@ static std::atomic<int64_t> g_backward_scratch_limit{INT64_MAX};
 
 int64_t backward_scratch_limit() { return g_backward_scratch_limit; }
 
+static std::atomic<bool> g_save_forward{true};
+
+bool may_keep(const torch::Tensor &scratch) { return g_save_forward && scratch.numel() <= g_backward_scratch_limit; }
+
 void set_backward_scratch_limit(int64_t bytes) {
   if (bytes < 0) bad_argument("Error: the scratch limit is a number of bytes >= 0.");
   g_backward_scratch_limit = bytes;
@@ -374,8 +378,6 @@ std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::
 // Not part of the reference's operator set: the reference's backward walks every tree again (three times).  These
 // two let the autograd layer walk them once per training step.  `saved` is the call's scratch, which holds the
 // traversal; it is empty when the library does not save for this problem (the caller then uses the plain backward).
-static std::atomic<bool> g_save_forward{true};
-
 // Bytes that a saving forward's scratch has at least, in the problem's mode; 0: nothing is kept.
 static size_t kept_bytes(const ht_forest_problem &problem) {
   if (ht_forest_forward_saves(&problem) == 0) return 0;
@@ -887,7 +889,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "z = x @ w.T on the tensor cores (TF32 products, fp32 accumulation) and the column sums of z and z*z: "
         "[z, sum, sumsq]. K and N must be multiples of 4.");
   m.def("set_save_forward", [](bool on) { g_save_forward = on; },
-        "Whether tree_/fern_forward_saving keep the traversal for the backward (default) or act as the plain forward.");
+        "Whether a forward keeps the traversal for the backward (default; tree_/fern_forward_saving, the autograd Functions of the "
+        "plain and the fused-linear forest) or the backward walks the trees again.");
   m.def("selftest_bounded_wait", &selftest_bounded_wait,
         "Runs a one-warp kernel whose bounded wait has to run out (nothing faults): the next pipeline_status() raises.");
   m.def("pipeline_status", &pipeline_status,

@@ -73,7 +73,7 @@ struct LinearNode : public torch::autograd::Function<LinearNode> {
     ctx->saved_data["kind"] = kind;
     torch::Tensor scratch;
     const torch::Tensor out = linear_forward((int)kind, x, nullptr, thr, ord, w, lin, bias, &scratch);
-    ctx->saved_data["kept"] = scratch;
+    if (scratch.defined()) ctx->saved_data["kept"] = scratch;
     return out;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {

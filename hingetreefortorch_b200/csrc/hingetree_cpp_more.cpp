@@ -234,7 +234,7 @@ torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *
                  "fused linear forward");
   });
   og.finish();
-  if (scratch != nullptr) *scratch = ws;
+  if (scratch != nullptr && may_keep(ws)) *scratch = ws;
   return out;
 }
 

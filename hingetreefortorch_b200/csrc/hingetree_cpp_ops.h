@@ -26,7 +26,8 @@ torch::Tensor make_workspace(size_t bytes, const torch::Tensor &like);
 torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like, c10::ScalarType type);
 inline torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like) { return fresh(sizes, like, like.scalar_type()); }
 inline torch::Tensor fresh_like(const torch::Tensor &like) { return fresh(like.sizes(), like); }
-int64_t backward_scratch_limit();  // set by the caller; see hingetree_cpp.cpp
+int64_t backward_scratch_limit();              // set by the caller; see hingetree_cpp.cpp
+bool may_keep(const torch::Tensor &scratch);  // from a forward to its backward, by the caller's settings
 void set_ordinal_check(const std::string &mode);
 int64_t pipeline_status();
 
@@ -64,8 +65,8 @@ std::vector<torch::Tensor> forest_backward(int kind, bool deterministic, torch::
 std::vector<torch::Tensor> forest_backward_saved(int kind, bool deterministic, torch::Tensor x, bool need_x, torch::Tensor thr,
                                                  bool need_thr, torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w,
                                                  torch::Tensor g, torch::Tensor saved);
-// `scratch`: receives the forward's workspace, which holds the paths of all evaluations; given to the backward it saves it
-// another walk.
+// `scratch`: receives the forward's workspace, which holds the paths of all evaluations, where it may be kept; given to the
+// backward it saves it another walk.
 torch::Tensor linear_forward(int kind, torch::Tensor data, const torch::Tensor *vec, torch::Tensor thr, torch::Tensor ord,
                              torch::Tensor w, torch::Tensor lin, torch::Tensor bias, torch::Tensor *scratch = nullptr);
 std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool need_data, const torch::Tensor *vec, bool need_vec,

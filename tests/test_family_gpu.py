@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import grad_close, random_forest_inputs
+from conftest import grad_close, random_forest_inputs, requested_bytes
 from oracle import hinge_oracle as ho
 
 pytestmark = pytest.mark.gpu
@@ -71,6 +71,38 @@ def test_fused_linear_and_fusion(case):
         aimg, avec, athr, aw = ho.magnitudes(ho.backward, kind, x, thr, ord_, w, g2, vec=vec)
         assert grad_close(gimg, rimg, aimg) and grad_close(gvec, rvec, avec)
         assert grad_close(gthr, rthr, athr) and grad_close(gw, rw, aw)
+
+
+@pytest.mark.parametrize("setting", ["keep", "limit", "off"])
+def test_fused_linear_keeps_its_paths_as_the_caller_allows(setting):
+    """The forward's scratch stays until the backward, unless the scratch limit or the switch for keeping rules it out; the
+    gradients are the same sums either way."""
+    from hingetreefortorch_b200._ext import hingetree_cpp as ext
+    from hingetreefortorch_b200.HingeTree import HingeTreeFusedLinear
+    B, C, T, depth, O = 900, 24, 40, 6, 7
+    rng = np.random.default_rng(3)
+    x, thr, ord_, w = random_forest_inputs(60, "tree", B, C, (), T, depth, ())
+    lin, bias, g = [rng.standard_normal(s).astype(np.float32) for s in ((O, T), O, (B, O))]
+    ref = ho.linear_backward("tree", x, thr, ord_, w, lin, g)
+    sizes = ho.magnitudes(ho.linear_backward, "tree", x, thr, ord_, w, lin, g)
+    dx, dthr, dord, dw, dlin, dbias, dg = dev(x, thr, ord_, w, lin, bias, g)
+    ext.tree_fused_linear_forward(dx, dthr, dord, dw, dlin, dbias)  # checks the ordinals
+    wrt = [t.requires_grad_(True) for t in (dx, dthr, dw, dlin, dbias)]
+    before = requested_bytes()
+    try:
+        if setting == "limit":
+            ext.set_backward_scratch_limit(10 * B * T)
+        elif setting == "off":
+            ext.set_save_forward(False)
+        out = HingeTreeFusedLinear.apply(dx, dthr, dord, dw, dlin, dbias)
+        held = requested_bytes() - before - 4 * out.numel()
+        grads = torch.autograd.grad(out, wrt, dg)
+    finally:
+        ext.set_backward_scratch_limit(2 ** 62)
+        ext.set_save_forward(True)
+    assert held >= 10 * B * T if setting == "keep" else held == 0
+    for got, r, s in zip(grads, ref, sizes):
+        assert grad_close(got, r, s)
 
 
 def test_modules_fused_linear_and_fusion():
