@@ -224,9 +224,10 @@ size_t path_scratch_bytes(const ht_forest_problem *p, size_t real_bytes) {
   return real_bytes == 4 && p->M == 1 && p->K == 1 ? std::max(paths, linear_tiled_bytes(p)) : paths;
 }
 
-// Whether the kernels of ht_forest_linear_tiled.cu take the call (tabular data without a vector beside it).
-bool tiled_takes(const ht_forest_problem *p, const float *vec, int64_t outputs, const float *x) {
-  return vec == nullptr && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && p->B * p->T > 0 && linear_tiled_takes(p, outputs);
+// Whether the kernels of ht_forest_linear_tiled.cu take the call (tabular data without a vector beside it).  A matter of sizes
+// alone: the paths that the forward leaves are read by a backward whose x may lie elsewhere (a copy made by saved-tensor hooks).
+bool tiled_takes(const ht_forest_problem *p, const float *vec, int64_t outputs) {
+  return vec == nullptr && p->B * p->T > 0 && linear_tiled_takes(p, outputs);
 }
 
 template <typename Real>
@@ -349,7 +350,7 @@ int linear_forward(const ht_forest_problem *p, int64_t out_channels, const Real 
   if (elements == 0) return HT_OK;
   if (out == nullptr || bias == nullptr || (lin == nullptr && p->T > 0)) return HT_ERR_INVALID_ARGUMENT;
   if constexpr (std::is_same<Real, float>::value) {
-    if (tiled_takes(p, vec, out_channels, img)) {
+    if (tiled_takes(p, vec, out_channels)) {
       const int trc = linear_tiled_forward(p, out_channels, img, thr, pr.args.ord, w, lin, bias, out,
                                            static_cast<unsigned char *>(workspace) + ordinal_bytes(p), status_word, pr.stream);
       if (trc != HT_ERR_UNSUPPORTED) return trc;
@@ -371,7 +372,7 @@ int linear_backward(const ht_forest_problem *p, int64_t out_channels, const Real
   // the workspace of the forward on these tensors: packed ordinals and paths are there
   const bool kept = p != nullptr && (p->flags & HT_SAVED_FORWARD) != 0;
   bool tiled = false;
-  if constexpr (std::is_same<Real, float>::value) tiled = check_forest_problem(p) == HT_OK && tiled_takes(p, vec, out_channels, img);
+  if constexpr (std::is_same<Real, float>::value) tiled = check_forest_problem(p) == HT_OK && tiled_takes(p, vec, out_channels);
   const int rc = prepare<Real>(p, img, vec, vec_channels, thr, ord, w, true, workspace, workspace_bytes, status_word, stream, pr,
                                gradients<Real>(p, vec_channels, tiled ? nullptr : gimg, gvec, gthr, gw, glin, out_channels), kept);
   if (rc != HT_OK) return rc;

@@ -3,6 +3,7 @@
 // The paths (margin; deciding vertex and leaf) lie [block of 256 samples][tree][256]: a thread that stays with its sample
 // reads them in runs, whatever order it takes the trees in.
 #include "ht_forest_linear_tiled.cuh"
+#include "ht_forest_multi.cuh"
 #include "ht_forest_rows.cuh"
 #include "ht_forest_tiled.cuh"
 #include "ht_tile_common.cuh"
@@ -215,6 +216,14 @@ int with_outputs(int64_t outputs, F &&f) {
   }
 }
 
+// The paths: row by row, or with a thread per evaluation where x is not aligned for the row copies.
+int walk_paths(const ht_forest_problem *p, const float *x, const float *thr, const int32_t *ord, const float *w, const EvalRecords &r,
+               uint32_t *status_word, cudaStream_t stream) {
+  const int rc = rows_forward(p, x, thr, ord, w, nullptr, r.dx, r.where, status_word, stream);
+  if (rc != HT_ERR_UNSUPPORTED) return rc;
+  return multi_forward<float>(p, x, thr, ord, w, nullptr, PathRecordsOf<float>{r.dx, r.where}, stream);
+}
+
 }  // namespace
 
 bool linear_tiled_takes(const ht_forest_problem *p, int64_t outputs) {
@@ -232,7 +241,7 @@ int linear_tiled_forward(const ht_forest_problem *p, int64_t outputs, const floa
   if (!linear_tiled_takes(p, outputs)) return HT_ERR_UNSUPPORTED;
   LinearArgs a = {};
   a.r = eval_record_arrays(p, area);
-  const int rc = rows_forward(p, x, thr, ord, w, nullptr, a.r.dx, a.r.where, status_word, stream);
+  const int rc = walk_paths(p, x, thr, ord, w, a.r, status_word, stream);
   if (rc != HT_OK) return rc;
   a.w = w;
   a.lin = lin;
@@ -254,7 +263,7 @@ int linear_tiled_backward(const ht_forest_problem *p, int64_t outputs, const flo
   LinearArgs a = {};
   a.r = eval_record_arrays(p, area);
   if (!kept) {
-    const int rc = rows_forward(p, x, thr, ord, w, nullptr, a.r.dx, a.r.where, status_word, stream);
+    const int rc = walk_paths(p, x, thr, ord, w, a.r, status_word, stream);
     if (rc != HT_OK) return rc;
   }
   a.w = w;
