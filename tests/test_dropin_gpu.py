@@ -304,6 +304,45 @@ def test_fixed_order_switched_between_forward_and_backward(shape, forward_mode):
         assert np.array_equal(got.cpu().numpy(), r) if not forward_mode else grad_close(got, r, m)
 
 
+@pytest.mark.parametrize("call", ["tile", "several", "ordered", "linear", "conv"])
+def test_second_backward_through_the_same_node(call):
+    """retain_graph: the first backward uses up what the forward kept, the second walks the trees again."""
+    from hingetreefortorch_b200 import HingeTree as F
+    rng = np.random.default_rng(12)
+    B, C, T, depth, M = 1030, 48, 32, 6, {"tile": 1, "several": 3, "ordered": 2}.get(call, 1)
+    if call == "conv":
+        x = rng.standard_normal((9, 4, 40, 41)).astype(np.float32)
+        thr, w = rng.uniform(-1, 1, (20, 4, 31)).astype(np.float32), rng.standard_normal((20, 4, 32)).astype(np.float32)
+        ord_ = rng.integers(0, 9, thr.shape).astype(np.int64)
+        geometry = ((3, 3), (1, 1), (1, 1), (1, 1))
+        g = rng.standard_normal((9, 20, 40, 41)).astype(np.float32)
+        inputs, extra, function = (x, thr, ord_, w), [list(v) for v in geometry], F.HingeTreeConv2d
+        ref, sizes = ho.conv_backward("tree", *inputs, g, *geometry), ho.magnitudes(ho.conv_backward, "tree", *inputs, g, *geometry)
+    else:
+        inputs = random_forest_inputs(35, "tree", B, C, (), T, depth, () if call == "linear" else (M,))
+        if call == "linear":
+            lin, bias, g = [rng.standard_normal(s).astype(np.float32) for s in ((5, T), 5, (B, 5))]
+            inputs, extra, function = (*inputs, lin, bias), [], F.HingeTreeFusedLinear
+            ref = ho.linear_backward("tree", *inputs[:5], g)
+            sizes = ho.magnitudes(ho.linear_backward, "tree", *inputs[:5], g)
+        else:
+            g = rng.standard_normal((B, T, M)).astype(np.float32)
+            extra, function = [], F.HingeTree
+            ref, sizes = ho.backward("tree", *inputs, g), ho.backward_magnitudes("tree", *inputs, g)
+    tensors = dev(*inputs)
+    dg, = dev(g)
+    wrt = [t.requires_grad_(True) for t in tensors if t.is_floating_point()]
+    torch.use_deterministic_algorithms(call == "ordered")
+    try:
+        out = function.apply(*tensors, *extra)
+        for again in (True, False):
+            grads = torch.autograd.grad(out, wrt, dg, retain_graph=again)
+            for got, r, s in zip(grads, ref, sizes):
+                assert np.array_equal(got.cpu().numpy(), r) if call == "ordered" else grad_close(got, r, s)
+    finally:
+        torch.use_deterministic_algorithms(False)
+
+
 def test_scratch_of_no_saving_forward_is_refused(ext):
     x, thr, ord_, w = random_forest_inputs(32, "tree", 100, 30, (), 20, 5, (4,))
     dx, dthr, dord, dw = dev(x, thr, ord_, w)

@@ -135,6 +135,56 @@ def test_fused_linear_on_data_off_the_copies_alignment(offset_then):
         assert grad_close(got, r, s)
 
 
+# kind, B, C, T, depth, O of tabular calls with one output per leaf.  Linear outputs up to the last that the row kernels take and one
+# beyond; more than 592 blocks of 256 samples (a block of threads takes several); records of 16 + 16 bits; last rows, and trees
+# split among blocks; the narrowest x, an odd one, the widest whose gradient rows fit and one beyond.
+LINEAR = [
+    ("tree", 1000, 24, 33, 7, 16),
+    ("fern", 1000, 24, 33, 7, 13),
+    ("tree", 700, 24, 20, 6, 17),
+    ("tree", 593 * 256 + 1, 6, 9, 4, 3),
+    ("fern", 2 * 592 * 256 + 77, 5, 3, 3, 1),
+    ("tree", 515, 40, 12, 9, 4),
+    ("fern", 515, 40, 12, 12, 5),
+    ("tree", 333, 1, 100, 5, 10),
+    ("tree", 257, 783, 50, 7, 8),
+    ("tree", 70, 1815, 17, 6, 2),
+    ("tree", 70, 1900, 17, 6, 2),
+    ("tree", 31, 10, 1, 1, 1),
+]
+
+
+@pytest.mark.parametrize("case", LINEAR, ids=[str(c) for c in LINEAR])
+def test_fused_linear_on_tabular_data(case):
+    """Through the operators (the backward walks again), through autograd from the forward's paths, and some gradients only."""
+    from hingetreefortorch_b200 import HingeTree as F, _cabi
+    kind, B, C, T, depth, O = case
+    rng = np.random.default_rng(90 + LINEAR.index(case))
+    x, thr, ord_, w = random_forest_inputs(90 + LINEAR.index(case), kind, B, C, (), T, depth, (), quantise=True)
+    lin, bias, g = [rng.standard_normal(s).astype(np.float32) for s in ((O, T), O, (B, O))]
+    ref = ho.linear_backward(kind, x, thr, ord_, w, lin, g)
+    sizes = ho.magnitudes(ho.linear_backward, kind, x, thr, ord_, w, lin, g)
+    tensors = dev(x, thr, ord_, w, lin, bias)
+    dx, dthr, dord, dw, dlin, dbias = tensors
+    dg, = dev(g)
+    fam = _cabi.ForestFamily(kind, dx, dw, lin=dlin)
+    want = ho.linear_forward(kind, x, thr, ord_, w, lin, bias)
+    assert np.array_equal(fam.linear_forward(dx, None, dthr, dord, dw, dlin, dbias).cpu().numpy(), want)
+    gx, _, gthr, gw, glin = fam.linear_backward(dx, None, dthr, dord, dw, dlin, dg)
+    for got, r, s in zip((gx, gthr, gw, glin), ref, sizes):
+        assert grad_close(got, r, s)
+    assert fam.status.item() == 0
+    function = F.HingeTreeFusedLinear if kind == "tree" else F.HingeFernFusedLinear
+    for wanted in ((0, 1, 3, 4, 5), (0,), (4,), (1, 3)):
+        wrt = [tensors[n].detach().requires_grad_(True) if n in wanted else tensors[n] for n in range(6)]
+        out = function.apply(*wrt)
+        assert np.array_equal(out.detach().cpu().numpy(), want)
+        grads = torch.autograd.grad(out, [wrt[n] for n in wanted], dg)
+        for n, got in zip(wanted, grads):
+            at = n - (n > 2)  # the ordinals have none
+            assert grad_close(got, ref[at], sizes[at])
+
+
 def test_modules_fused_linear_and_fusion():
     from hingetreefortorch_b200 import RandomHingeForest as R
     torch.manual_seed(1)
