@@ -472,10 +472,16 @@ static bool ordered_from_paths(const ht_forest_problem *p) {
   return (p->flags & HT_DETERMINISTIC) != 0 && (p->M > 1 || p->B * p->T * p->K <= (1 << 26)) && ordered_list_bytes(p, sizeof(float)) > 0;
 }
 
-// Whether the walk goes past resident trees row by row (ht_forest_rows.cu) rather than past resident tiles of samples, or with
-// a thread per evaluation: where the estimates say so by a margin that covers their error.  It does for samples of many
-// features, which leave room for small tiles only (8192 x 784 under 800 trees of depth 8, 10 outputs: 254 against 485 us), and
-// for batches that give few tiles.
+// Whether the walk goes past resident trees row by row (ht_forest_rows.cu) rather than past resident tiles of samples or with a
+// thread per evaluation: where the estimates have it cheaper by 15 %.  It is for samples of many features, which leave room for
+// small tiles only (8192 x 784 under 800 trees of depth 8, 10 outputs: 254 against 485 us), and for batches that give few tiles.
+// How good the choice is, on 1104 forwards of random sizes timed every way (profiles/forward_kernel_choice.csv):
+//   * against the tile kernel (808 of them) it costs 0.9 % over the better of the two on average and more than 20 % in 5 cases;
+//     always tiles 9.1 %, always rows 29 %.  The 15 % are where that loss is least: 2.0 % with a margin of 30 %, 1.4 % with none;
+//   * against a thread per evaluation (296) the third estimate is a rough one (it has the right order of magnitude, and a spread
+//     of 1.6 to 1.8 times), and the choice costs 3.2 %, never taking rows 3.4 % (with the time of all these calls added up 12
+//     and 13 %: rows win in the long calls).  Ferns stay with the threads there: the estimate is too high for them, and chosen
+//     by it they lose 2.4 % instead of 1.5.
 static bool rows_are_better(const ht_forest_problem *p) {
   const double rows = rows_forward_cost(p);
   if (rows < 0.0 || p->B * p->T < 32768) return false;

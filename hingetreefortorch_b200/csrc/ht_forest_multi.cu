@@ -466,6 +466,8 @@ bool multi_takes(const ht_forest_problem *p, size_t real_bytes) {
   return p->B * p->K * p->T >= 32768;
 }
 
+// Up to 32 GiB, like the records of one output per leaf: the forward keeps the paths until the backward, and in between the
+// program needs its memory for what it computes from the outputs.  Larger problems scatter; a caller's limit may be lower.
 size_t multi_area_bytes(const ht_forest_problem *p, size_t real_bytes) {
   if (!multi_takes(p, real_bytes)) return 0;
   const size_t bytes = path_bytes(p, real_bytes);

@@ -318,8 +318,9 @@ static int row_slices(const ht_forest_problem *p, const RowPlan &plan) {
 }
 
 // Rounds of CTAs, each of them steps x (levels of the walks that a warp does one after another, outputs, row copies) behind
-// the fetch of its parameters; the coefficients are a least-squares fit to 342 measured forwards (B 1000 .. 65536, C 32 ..
-// 1500, T 40 .. 800, depth 5 .. 10, M 1 .. 10; 19 % off on average).
+// the fetch of its parameters.  The coefficients are a least-squares fit to forwards in a loop (B 1000 .. 65536, C 32 .. 1500, T 40
+// .. 800, depth 5 .. 10, M 1 .. 10).  Single calls on cold caches (profiles/forward_kernel_choice.csv) take 1.3 times the estimate,
+// give or take 28 %; the choice between the kernels needs the ratio of two estimates, and forward_tiled_cost() is off likewise.
 double rows_forward_cost(const ht_forest_problem *p) {
   RowPlan plan;
   if (!make_row_plan(p, plan)) return -1.0;

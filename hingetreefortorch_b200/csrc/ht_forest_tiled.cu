@@ -664,7 +664,7 @@ size_t forward_tiled_workspace_bytes(const ht_forest_problem *p) {
 
 // Rounds of CTAs, each staging its tile and walking its share of the tree groups; one, two or four trees per warp at once
 // differ in what a group costs (few in flight leave the shared memory's latency in the open).  Fitted like
-// rows_forward_cost(): 9 to 16 % off on average.
+// rows_forward_cost(); single calls on cold caches take 1.25 times the estimate, give or take 25 %.
 double forward_tiled_cost(const ht_forest_problem *p) {
   TilePlan plan;
   if (!make_plan(p, plan)) return -1.0;

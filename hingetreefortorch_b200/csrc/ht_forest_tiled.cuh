@@ -26,7 +26,7 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
                   float *out, void *records, void *eval_records, uint32_t *status_word, cudaStream_t stream,
                   const WideOrdinals *wide = nullptr);
 
-// The backward from the records a saving forward left (default mode; forward_saves(p) must hold and the inputs must
+// The backward from the records a saving forward left (either mode; forward_saves(p) must hold and the inputs must
 // be the forward's).  `ord` are the compact ordinals.  Any of gx / gthr / gw may be null; the others must have been
 // cleared.
 int backward_saved(const ht_forest_problem *p, const int32_t *ord, const float *w, const float *g, float *gx, float *gthr,

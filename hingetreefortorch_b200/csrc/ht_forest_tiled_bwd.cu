@@ -8,11 +8,12 @@
 // (the reference runs three kernels that each repeat it, hingetree_gpu.cu:699-727); it keeps the
 // signed margin and the deciding vertex, with the reference's strict `<` so that the shallowest
 // minimum wins.  What happens to the terms depends on the workspace the caller gave:
-//   * with room for 12 bytes per evaluation (the record path, both modes): the kernel writes one
+//   * with room for 10 bytes per evaluation, 12 beyond depth 8 (the record path, both modes): the kernel writes one
 //     record per evaluation and two reductions further down add the records in a fixed order —
 //     reduce_x_records_kernel for the x gradient, reduce_parameter_records_* for thresholds and
-//     leaf weights.  No floating-point atomics anywhere; in fixed-order mode the sums are the
-//     reference's sequential CPU sums bit for bit;
+//     leaf weights.  In fixed-order mode the sums are the reference's sequential CPU sums bit for bit (its parameter sums
+//     come from lists instead, ht_forest_ordered.cu, where there is room for those); in default mode a tree's samples may be
+//     split, each split adding its bins with one reduction;
 //   * without it (default mode only): fire-and-forget global reductions (red.global.add.f32) from
 //     the traversal kernel itself.
 // There is no block-wide barrier after the feature tile has been staged.
