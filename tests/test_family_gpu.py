@@ -105,17 +105,19 @@ def test_fused_linear_keeps_its_paths_as_the_caller_allows(setting):
         assert grad_close(got, r, s)
 
 
+@pytest.mark.parametrize("kind,depth", [("tree", 6), ("tree", 9), ("fern", 8), ("fern", 11)])
 @pytest.mark.parametrize("offset_then", ["aligned", "moved"])
-def test_fused_linear_on_data_off_the_copies_alignment(offset_then):
+def test_fused_linear_on_data_off_the_copies_alignment(offset_then, kind, depth):
     """x that starts between two 16-byte boundaries, and a backward whose x is a copy elsewhere (saved-tensor hooks): the paths
     that the forward kept mean the same wherever x lies."""
-    from hingetreefortorch_b200.HingeTree import HingeTreeFusedLinear
-    B, C, T, depth, O = 300, 24, 40, 6, 7
+    from hingetreefortorch_b200.HingeTree import HingeFernFusedLinear, HingeTreeFusedLinear
+    B, C, T, O = 300, 24, 40, 7
+    function = HingeTreeFusedLinear if kind == "tree" else HingeFernFusedLinear
     rng = np.random.default_rng(4)
-    x, thr, ord_, w = random_forest_inputs(61, "tree", B, C, (), T, depth, ())
+    x, thr, ord_, w = random_forest_inputs(61, kind, B, C, (), T, depth, ())
     lin, bias, g = [rng.standard_normal(s).astype(np.float32) for s in ((O, T), O, (B, O))]
-    ref = ho.linear_backward("tree", x, thr, ord_, w, lin, g)
-    sizes = ho.magnitudes(ho.linear_backward, "tree", x, thr, ord_, w, lin, g)
+    ref = ho.linear_backward(kind, x, thr, ord_, w, lin, g)
+    sizes = ho.magnitudes(ho.linear_backward, kind, x, thr, ord_, w, lin, g)
     dthr, dord, dw, dlin, dbias, dg = dev(thr, ord_, w, lin, bias, g)
     dx = torch.empty(B * C + 1, device="cuda")[1:].view(B, C).copy_(torch.from_numpy(x))
     assert dx.is_contiguous() and dx.data_ptr() % 16 == 4
@@ -128,9 +130,9 @@ def test_fused_linear_on_data_off_the_copies_alignment(offset_then):
         dx = dx.clone()
     wrt = [t.requires_grad_(True) for t in (dx, dthr, dw, dlin, dbias)]
     with torch.autograd.graph.saved_tensors_hooks(lambda t: t.detach(), elsewhere):
-        out = HingeTreeFusedLinear.apply(dx, dthr, dord, dw, dlin, dbias)
+        out = function.apply(dx, dthr, dord, dw, dlin, dbias)
         grads = torch.autograd.grad(out, wrt, dg)
-    assert np.array_equal(out.detach().cpu().numpy(), ho.linear_forward("tree", x, thr, ord_, w, lin, bias))
+    assert np.array_equal(out.detach().cpu().numpy(), ho.linear_forward(kind, x, thr, ord_, w, lin, bias))
     for got, r, s in zip(grads, ref, sizes):
         assert grad_close(got, r, s)
 
