@@ -16,10 +16,11 @@ namespace {
 using torch::autograd::AutogradContext;
 using torch::autograd::variable_list;
 
+// Forward-mode derivatives count, with or without grad mode: the nodes refuse them, the plain forward would drop the tangents.
 bool differentiated(std::initializer_list<const torch::Tensor *> tensors) {
-  if (!at::GradMode::is_enabled()) return false;
+  const bool backward = at::GradMode::is_enabled();
   for (const torch::Tensor *t : tensors)
-    if (t->requires_grad()) return true;
+    if ((backward && t->requires_grad()) || t->_fw_grad(/*level=*/0).defined()) return true;
   return false;
 }
 

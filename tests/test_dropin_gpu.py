@@ -343,6 +343,36 @@ def test_second_backward_through_the_same_node(call):
         torch.use_deterministic_algorithms(False)
 
 
+def _small_modules():
+    from hingetreefortorch_b200 import RandomHingeForest as R
+    torch.manual_seed(5)
+    tabular = torch.randn(12, 8, device="cuda")
+    front = R.LinearBatchNorm1d(8, 4 * 7)
+    return {
+        "forest": (R.RandomHingeForest(8, 6, 3).cuda(), tabular),
+        "linear": (R.RandomHingeFernFusedLinear(8, 6, 3, 4).cuda(), tabular),
+        "conv": (R.HingeTreeConv1d(2, 3, 3, 3).cuda(), torch.randn(2, 2, 9, device="cuda")),
+        "pipeline": (R.LinearBatchNormForest(front, R.RandomHingeForest(28, 4, 3, init_type="sequential")).cuda(), tabular),
+    }
+
+
+@pytest.mark.parametrize("name", ["forest", "linear", "conv", "pipeline"])
+@pytest.mark.parametrize("grad", [True, False])
+def test_forward_mode_and_vmap_are_refused(name, grad):
+    """The operators have neither; a call that is not differentiated backward must not drop a tangent."""
+    from torch.autograd import forward_ad
+    m, x = _small_modules()[name]
+    m(x)
+    m.requires_grad_(False)
+    with torch.set_grad_enabled(grad):
+        with forward_ad.dual_level(), pytest.raises((RuntimeError, NotImplementedError), match="jvp"):
+            m(forward_ad.make_dual(x, torch.ones_like(x)))
+        with pytest.raises(RuntimeError):
+            torch.func.vmap(m)(torch.stack([x, x + 1]))
+        with pytest.raises(RuntimeError):
+            torch.func.jvp(m, (x,), (x,))
+
+
 def test_scratch_of_no_saving_forward_is_refused(ext):
     x, thr, ord_, w = random_forest_inputs(32, "tree", 100, 30, (), 20, 5, (4,))
     dx, dthr, dord, dw = dev(x, thr, ord_, w)
