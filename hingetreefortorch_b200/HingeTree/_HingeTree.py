@@ -118,6 +118,26 @@ class Expand(torch.nn.Module):
         return _Patches.apply(inData, None, self.padding)
 
 
+class _Traced(torch.autograd.Function):
+    """One of the extension's `*_apply` as torch.jit.trace records it: a Python operation, which calls it again whenever the
+    trace runs.  The backward differentiates another such call."""
+
+    @staticmethod
+    def forward(ctx, name, *args):
+        ctx.name, ctx.others = name, [None if isinstance(a, torch.Tensor) else a for a in args]
+        ctx.save_for_backward(*[a for a in args if isinstance(a, torch.Tensor)])
+        return _op(name)(*args)
+
+    @staticmethod
+    def backward(ctx, grad):
+        tensors, needs = iter(ctx.saved_tensors), ctx.needs_input_grad[1:]
+        with torch.enable_grad():
+            args = [next(tensors).detach().requires_grad_(need) if a is None else a for a, need in zip(ctx.others, needs)]
+            out = _op(ctx.name)(*args)
+        grads = iter(torch.autograd.grad(out, [a for a, need in zip(args, needs) if need], grad))
+        return (None, *[next(grads) if need else None for need in needs])
+
+
 # ---- Function templates --------------------------------------------------------------------
 
 _UTILITIES = ("check_thresholds", "fix_thresholds", "reachability", "leafmap", "marginmap", "init_medians")

@@ -81,6 +81,13 @@ class LinearBatchNorm1d(nn.Module):
         if not self.training:
             return _LinearBatchNorm.apply(x, self.weight, self.eps, self.running_mean, self.running_var)[0]
         y, mean, var = _LinearBatchNorm.apply(x, self.weight, self.eps, None, None)
+        if torch.jit.is_tracing():  # in operations that a trace records
+            with torch.no_grad():
+                rows = x.shape[0]
+                self.num_batches_tracked += 1
+                self.running_mean.lerp_(mean, self.momentum)
+                self.running_var.lerp_(var * (rows / max(rows - 1, 1)), self.momentum)
+            return y
         hingetree_cpp.batchnorm_running(mean, var, x.shape[0], self.momentum, self.running_mean, self.running_var,
                                         self.num_batches_tracked)
         return y
@@ -94,7 +101,7 @@ class LinearBatchNormForest(nn.Module):
     """A LinearBatchNorm1d front and a RandomHingeForest / RandomHingeFern behind it as one step: in training mode the
     normalised activations are never materialised (hingetree_cpp.linear_batchnorm_forest: the forest normalises the
     features it visits, bit-identical to the forest behind a materialised normalisation, and its backward gives the
-    normalisation's one entry per (sample, tree)); in evaluation mode the two modules run one after the other.  The parameters stay those of the two modules (``front.weight``, ``forest.thresholds``,
+    normalisation's one entry per (sample, tree)); in evaluation mode, and while torch.jit.trace records, the two modules run one after the other.  The parameters stay those of the two modules (``front.weight``, ``forest.thresholds``,
     ``forest.ordinals``, ``forest.weights``), so checkpoints of the unfused pair load as they are."""
 
     def __init__(self, front, forest):
@@ -106,7 +113,7 @@ class LinearBatchNormForest(nn.Module):
         self.front, self.forest = front, forest
 
     def forward(self, x):
-        if not self.training:
+        if not self.training or torch.jit.is_tracing():
             return self.forest(self.front(x))
         front, forest = self.front, self.forest
         return hingetree_cpp.linear_batchnorm_forest(x, front.weight, forest.thresholds, forest.ordinals, forest.weights, front.eps,

@@ -6,6 +6,7 @@
 
 #include <ATen/Context.h>
 #include <c10/core/DeviceGuard.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include "hingetree_cpp_ops.h"
 
@@ -198,21 +199,48 @@ torch::Tensor pipeline_apply(const torch::Tensor &x, const torch::Tensor &w, con
   return out[0];
 }
 
+// While torch.jit.trace records, what the extension computes by itself would end up in the trace as a constant.  A Python
+// Function is recorded as an operation, so the call is made through one (_HingeTree.py, _Traced), which calls `name` again: then,
+// and whenever the trace runs, straight through.
+thread_local bool recording = false;
+template <typename Compute, typename... Args>
+torch::Tensor traceable(const std::string &name, Compute &&compute, const Args &...args) {
+  if (!torch::jit::tracer::isTracing()) return compute(args...);
+  if (recording) {  // the result stands for something the recorder has seen made
+    const torch::Tensor out = compute(args...);
+    torch::jit::tracer::setValueTrace(out, torch::jit::tracer::getValueTrace(at::empty({0}, out.options())));
+    return out;
+  }
+  struct Recording {
+    Recording() { recording = true; }
+    ~Recording() { recording = false; }
+  } scope;
+  return pybind11::module_::import("hingetreefortorch_b200.HingeTree._HingeTree")
+      .attr("_Traced")
+      .attr("apply")(name, args...)
+      .template cast<torch::Tensor>();
+}
+
 }  // namespace
 
 void bind_autograd(pybind11::module_ &m) {
   for (const int kind : {HT_KIND_TREE, HT_KIND_FERN}) {
-    const std::string prefix = name_of(kind);
-    m.def((prefix + "_apply").c_str(), [kind](const torch::Tensor &x, const torch::Tensor &t, const torch::Tensor &o,
-                                              const torch::Tensor &w) { return plain_apply(kind, x, t, o, w); });
-    m.def((prefix + "_fused_linear_apply").c_str(),
-          [kind](const torch::Tensor &x, const torch::Tensor &t, const torch::Tensor &o, const torch::Tensor &w, const torch::Tensor &l,
-                 const torch::Tensor &b) { return linear_apply(kind, x, t, o, w, l, b); });
-    for (int dims = 1; dims <= 3; ++dims)
-      m.def((prefix + "_conv" + std::to_string(dims) + "d_apply").c_str(),
-            [kind, dims](const torch::Tensor &x, const torch::Tensor &t, const torch::Tensor &o, const torch::Tensor &w,
-                         const std::vector<int64_t> &k, const std::vector<int64_t> &s, const std::vector<int64_t> &p,
-                         const std::vector<int64_t> &d) { return conv_apply(kind, dims, x, t, o, w, k, s, p, d); });
+    const std::string prefix = name_of(kind), plain = prefix + "_apply", linear = prefix + "_fused_linear_apply";
+    m.def(plain.c_str(), [kind, plain](const torch::Tensor &x, const torch::Tensor &t, const torch::Tensor &o, const torch::Tensor &w) {
+      return traceable(plain, [kind](auto &...a) { return plain_apply(kind, a...); }, x, t, o, w);
+    });
+    m.def(linear.c_str(), [kind, linear](const torch::Tensor &x, const torch::Tensor &t, const torch::Tensor &o, const torch::Tensor &w,
+                                         const torch::Tensor &l, const torch::Tensor &b) {
+      return traceable(linear, [kind](auto &...a) { return linear_apply(kind, a...); }, x, t, o, w, l, b);
+    });
+    for (int dims = 1; dims <= 3; ++dims) {
+      const std::string conv = prefix + "_conv" + std::to_string(dims) + "d_apply";
+      m.def(conv.c_str(), [kind, dims, conv](const torch::Tensor &x, const torch::Tensor &t, const torch::Tensor &o,
+                                             const torch::Tensor &w, const std::vector<int64_t> &k, const std::vector<int64_t> &s,
+                                             const std::vector<int64_t> &p, const std::vector<int64_t> &d) {
+        return traceable(conv, [kind, dims](auto &...a) { return conv_apply(kind, dims, a...); }, x, t, o, w, k, s, p, d);
+      });
+    }
   }
   m.def("linear_batchnorm_forest", &pipeline_apply,
         "One training-mode step forward of Linear -> BatchNorm1d(affine=False) -> forest / fern, differentiable; advances the "

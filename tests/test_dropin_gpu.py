@@ -1,5 +1,7 @@
 """The reference-facing surface on a GPU: the `hingetree_cpp` operators, the autograd
 Functions and the nn.Modules, checked against the CPU oracle."""
+import copy
+
 import numpy as np
 import pytest
 import torch
@@ -371,6 +373,38 @@ def test_forward_mode_and_vmap_are_refused(name, grad):
             torch.func.vmap(m)(torch.stack([x, x + 1]))
         with pytest.raises(RuntimeError):
             torch.func.jvp(m, (x,), (x,))
+
+
+@pytest.mark.parametrize("name", ["forest", "linear", "conv", "pipeline"])
+@pytest.mark.parametrize("grad", [True, False])
+def test_a_traced_module_computes_on_new_data(name, grad):
+    """torch.jit.trace records the operators (as Python operations), not what they gave on the example."""
+    m, x = _small_modules()[name]
+    m(x)
+
+    class Around(torch.nn.Module):
+        def __init__(self):
+            super().__init__()
+            self.inner = m
+
+        def forward(self, v):
+            return 3 * self.inner(v + 1)
+
+    net = Around()
+    with torch.set_grad_enabled(grad):
+        traced = torch.jit.trace(net, x, check_trace=False)
+        eager = copy.deepcopy(net)
+        y = torch.randn_like(x).requires_grad_(grad)
+        got, want = traced(y), eager(y)
+        assert torch.allclose(got, want, atol=1e-5) and not torch.allclose(got, eager(x), atol=1e-2)
+    traced(x)
+    for a, b in zip(net.state_dict().values(), eager.state_dict().values()):  # running statistics, too
+        assert torch.allclose(a.double(), b.double(), atol=1e-6)
+    if grad:
+        g = torch.randn_like(want)
+        grads = [torch.autograd.grad(out, [y] + [p for p in n.parameters() if p.requires_grad], g) for out, n in ((got, net), (want, eager))]
+        for a, b in zip(*grads):
+            assert torch.allclose(a, b, rtol=1e-4, atol=1e-4 * float(b.abs().max()) + 1e-6)
 
 
 def test_scratch_of_no_saving_forward_is_refused(ext):
