@@ -6,6 +6,7 @@
 
 #include <ATen/Context.h>
 #include <c10/core/DeviceGuard.h>
+#include <torch/csrc/autograd/forward_grad.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include "hingetree_cpp_ops.h"
@@ -19,9 +20,12 @@ using torch::autograd::variable_list;
 
 // Forward-mode derivatives count, with or without grad mode: the nodes refuse them, the plain forward would drop the tangents.
 bool differentiated(std::initializer_list<const torch::Tensor *> tensors) {
-  const bool backward = at::GradMode::is_enabled();
-  for (const torch::Tensor *t : tensors)
-    if ((backward && t->requires_grad()) || t->_fw_grad(/*level=*/0).defined()) return true;
+  if (at::GradMode::is_enabled())
+    for (const torch::Tensor *t : tensors)
+      if (t->requires_grad()) return true;
+  if (torch::autograd::ForwardADLevel::try_get_by_idx(0) != nullptr)  // a dual level is open
+    for (const torch::Tensor *t : tensors)
+      if (t->_fw_grad(/*level=*/0).defined()) return true;
   return false;
 }
 
