@@ -29,6 +29,7 @@ SYMBOLS = [
     "ht_forest_fusion_workspace_bytes", "ht_forest_fusion_forward_f32", "ht_forest_fusion_backward_f32",
     "ht_forest_linear_workspace_bytes", "ht_forest_linear_forward_f32", "ht_forest_linear_backward_f32",
     "ht_conv_output_size", "ht_conv_workspace_bytes", "ht_conv_backward_workspace_bytes", "ht_conv_forward_f32", "ht_conv_backward_f32",
+    "ht_conv_saved_bytes", "ht_conv_forward_saving_f32", "ht_conv_backward_saved_f32",
     "ht_contract", "ht_expand",
     "ht_trie_forward_f32", "ht_trie_backward_f32", "ht_forest_touched_f32", "ht_linear_tf32_stats_f32",
     "ht_forest_linear_workspace_bytes_f64", "ht_forest_fusion_forward_f64", "ht_forest_fusion_backward_f64",
@@ -84,6 +85,27 @@ class Conv:
         _check(library().ht_conv_forward_f32(ctypes.byref(self.problem), _ptr(x), _ptr(thr), _ptr(ord_), _ptr(w),
                                              _ptr(out), *self._tail(x)))
         return out
+
+    def saved_bytes(self):
+        """Bytes a forward keeps for the backward; 0: nothing."""
+        library().ht_conv_saved_bytes.restype = ctypes.c_size_t
+        return library().ht_conv_saved_bytes(ctypes.byref(self.problem))
+
+    def forward_saving(self, x, thr, ord_, w):
+        import torch
+        out = torch.empty(self.out_shape, dtype=torch.float32, device=x.device)
+        kept = torch.empty(self.saved_bytes(), dtype=torch.uint8, device=x.device)
+        _check(library().ht_conv_forward_saving_f32(ctypes.byref(self.problem), _ptr(x), _ptr(thr), _ptr(ord_), _ptr(w),
+                                                    _ptr(out), _ptr(kept), *self._tail(x)))
+        return out, kept
+
+    def backward_saved(self, x, thr, ord_, w, g, kept, need=(True, True, True)):
+        import torch
+        outs = [torch.empty_like(t) if n else None for t, n in zip((x, thr, w), need)]
+        _check(library().ht_conv_backward_saved_f32(ctypes.byref(self.problem), _ptr(x), _ptr(thr), _ptr(ord_), _ptr(w), _ptr(g),
+                                                    *[_ptr(t) if t is not None else None for t in outs], _ptr(kept),
+                                                    *self._tail(x)))
+        return outs
 
     def backward(self, x, thr, ord_, w, g):
         import torch

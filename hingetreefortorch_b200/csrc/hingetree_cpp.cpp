@@ -205,7 +205,8 @@ int64_t backward_scratch_limit() { return g_backward_scratch_limit; }
 
 static std::atomic<bool> g_save_forward{true};
 
-bool may_keep(const torch::Tensor &scratch) { return g_save_forward && scratch.numel() <= g_backward_scratch_limit; }
+bool may_keep(int64_t bytes) { return g_save_forward && bytes <= g_backward_scratch_limit; }
+bool may_keep(const torch::Tensor &scratch) { return may_keep(scratch.numel()); }
 
 void set_backward_scratch_limit(int64_t bytes) {
   if (bytes < 0) bad_argument("Error: the scratch limit is a number of bytes >= 0.");
@@ -895,7 +896,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
         "[z, sum, sumsq]. K and N must be multiples of 4.");
   m.def("set_save_forward", [](bool on) { g_save_forward = on; },
         "Whether a forward keeps the traversal for the backward (default; tree_/fern_forward_saving, the autograd Functions of the "
-        "plain and the fused-linear forest) or the backward walks the trees again.");
+        "plain and the fused-linear forest and of the convolutions) or the backward walks the trees again.");
   m.def("selftest_bounded_wait", &selftest_bounded_wait,
         "Runs a one-warp kernel whose bounded wait has to run out (nothing faults): the next pipeline_status() raises.");
   m.def("pipeline_status", &pipeline_status,

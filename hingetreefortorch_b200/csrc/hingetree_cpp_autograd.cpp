@@ -115,16 +115,21 @@ struct ConvNode : public torch::autograd::Function<ConvNode> {
     ctx->saved_data["kind"] = kind;
     ctx->saved_data["geometry"] = geometry;
     const Geometry g(geometry);
-    return conv_forward((int)kind, g.dims, x, thr, ord, w, g.part(0), g.part(1), g.part(2), g.part(3));
+    torch::Tensor kept;  // serves every backward through this node
+    const torch::Tensor out = conv_forward((int)kind, g.dims, x, thr, ord, w, g.part(0), g.part(1), g.part(2), g.part(3), &kept);
+    if (kept.defined()) ctx->saved_data["kept"] = kept;
+    return out;
   }
   static variable_list backward(AutogradContext *ctx, variable_list grads) {
     const variable_list s = ctx->get_saved_variables();
     const int64_t kind = ctx->saved_data["kind"].toInt();
     refuse_deterministic(grads[0], "backpropagation for hinge " + name_of(kind) + " convolution");
     const Geometry g(ctx->saved_data["geometry"].toIntVector());
+    const auto at = ctx->saved_data.find("kept");
+    const torch::Tensor kept = at != ctx->saved_data.end() ? at->second.toTensor() : torch::Tensor();
     std::vector<torch::Tensor> r = conv_backward((int)kind, g.dims, s[0], ctx->needs_input_grad(0), s[1], ctx->needs_input_grad(1), s[2],
                                                  false, s[3], ctx->needs_input_grad(3), grads[0].contiguous(), g.part(0), g.part(1),
-                                                 g.part(2), g.part(3));
+                                                 g.part(2), g.part(3), &kept);
     return {r[0], r[1], torch::Tensor(), r[3], torch::Tensor(), torch::Tensor()};
   }
   struct Geometry {  // kernel size, stride, padding and dilation one after another

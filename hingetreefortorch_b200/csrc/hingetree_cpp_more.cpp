@@ -540,12 +540,30 @@ struct ConvCall {
 
 torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w,
                            std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
-                           std::vector<int64_t> dilation) {
+                           std::vector<int64_t> dilation, torch::Tensor *kept) {
   ConvCall call(kind, dims, x, thr, ord, w, nullptr, kernel, stride, padding, dilation);
   c10::DeviceGuard guard(x.device());
   torch::Tensor out = fresh(call.out_sizes, x);
+  if (kept != nullptr && x.scalar_type() == torch::kFloat32) {
+    constexpr int64_t kMostKept = (int64_t)8 << 30;  // as much as the codes of a backward that walks may take
+    const int64_t bytes = (int64_t)ht_conv_saved_bytes(&call.problem);
+    if (bytes > 0 && bytes <= kMostKept && may_keep(bytes)) {
+      try {
+        *kept = make_workspace((size_t)bytes, x);
+      } catch (const c10::OutOfMemoryError &) {
+      }
+    }
+  }
   torch::Tensor ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.window_cells);
+  if (kept != nullptr && kept->defined()) {
+    raise_status(ht_conv_forward_saving_f32(&call.problem, x.data_ptr<float>(), thr.data_ptr<float>(), ord.data_ptr<int64_t>(),
+                                            w.data_ptr<float>(), out.data_ptr<float>(), kept->data_ptr(), ws.data_ptr(), ws.numel(),
+                                            og.word(), current_stream(x)),
+                 "convolution forward");
+    og.finish();
+    return out;
+  }
   dispatch_real(x, [&](auto real) {
     using Real = decltype(real);
     raise_status(abi::conv_forward(&call.problem, x.data_ptr<Real>(), thr.data_ptr<Real>(), ord.data_ptr<int64_t>(),
@@ -560,7 +578,7 @@ torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor th
 std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bool need_x, torch::Tensor thr, bool need_thr,
                                          torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w, torch::Tensor g,
                                          std::vector<int64_t> kernel, std::vector<int64_t> stride,
-                                         std::vector<int64_t> padding, std::vector<int64_t> dilation) {
+                                         std::vector<int64_t> padding, std::vector<int64_t> dilation, const torch::Tensor *kept) {
   if (need_ord) bad_runtime("Error: Gradient on inOrdinals is requested, but inOrdinals never has a gradient.");
   ConvCall call(kind, dims, x, thr, ord, w, &g, kernel, stride, padding, dilation);
   c10::DeviceGuard guard(x.device());
@@ -572,6 +590,17 @@ std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bo
   // Room for the codes through which both kinds of gradients share one walk, as far as the limit allows: the batch goes in
   // parts that fit, or without codes.
   const size_t needed = ht_conv_workspace_bytes(&call.problem);
+  if (kept != nullptr && kept->defined()) {
+    torch::Tensor ws = make_workspace(needed, x);
+    OrdinalGuard og(ord, call.window_cells);
+    raise_status(ht_conv_backward_saved_f32(&call.problem, x.data_ptr<float>(), thr.data_ptr<float>(), ord.data_ptr<int64_t>(),
+                                            w.data_ptr<float>(), g.data_ptr<float>(), ptr_or_null<float>(grads[0]),
+                                            ptr_or_null<float>(grads[1]), ptr_or_null<float>(grads[3]), kept->data_ptr(), ws.data_ptr(),
+                                            ws.numel(), og.word(), current_stream(x)),
+                 "convolution backward");
+    og.finish();
+    return grads;
+  }
   size_t bytes = needed;
   if (x.scalar_type() == torch::kFloat32 && need_x && (need_thr || need_w))
     bytes = std::max(needed, std::min(ht_conv_backward_workspace_bytes(&call.problem), (size_t)backward_scratch_limit()));

@@ -27,7 +27,8 @@ torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like, c10::Scal
 inline torch::Tensor fresh(c10::IntArrayRef sizes, const torch::Tensor &like) { return fresh(sizes, like, like.scalar_type()); }
 inline torch::Tensor fresh_like(const torch::Tensor &like) { return fresh(like.sizes(), like); }
 int64_t backward_scratch_limit();              // set by the caller; see hingetree_cpp.cpp
-bool may_keep(const torch::Tensor &scratch);  // from a forward to its backward, by the caller's settings
+bool may_keep(int64_t bytes);                  // from a forward to its backward, by the caller's settings
+bool may_keep(const torch::Tensor &scratch);
 void set_ordinal_check(const std::string &mode);
 int64_t pipeline_status();
 
@@ -73,13 +74,15 @@ std::vector<torch::Tensor> linear_backward(int kind, torch::Tensor data, bool ne
                                            torch::Tensor thr, bool need_thr, torch::Tensor ord, bool need_ord, torch::Tensor w,
                                            bool need_w, torch::Tensor lin, bool need_lin, torch::Tensor bias, bool need_bias,
                                            torch::Tensor g, const torch::Tensor *scratch = nullptr);
+// `kept`: receives the codes of all evaluations where the library and the caller's settings provide for that; a backward that is
+// given them does not walk, and leaves them as they are.
 torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w,
                            std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
-                           std::vector<int64_t> dilation);
+                           std::vector<int64_t> dilation, torch::Tensor *kept = nullptr);
 std::vector<torch::Tensor> conv_backward(int kind, int dims, torch::Tensor x, bool need_x, torch::Tensor thr, bool need_thr,
                                          torch::Tensor ord, bool need_ord, torch::Tensor w, bool need_w, torch::Tensor g,
                                          std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
-                                         std::vector<int64_t> dilation);
+                                         std::vector<int64_t> dilation, const torch::Tensor *kept = nullptr);
 std::vector<torch::Tensor> linear_tf32_stats(torch::Tensor x, torch::Tensor w);
 std::vector<torch::Tensor> batchnorm_statistics(torch::Tensor sum, torch::Tensor sumsq, int64_t rows, double eps);
 void batchnorm_running(torch::Tensor mean, torch::Tensor var, int64_t rows, double momentum, torch::Tensor running_mean,

@@ -394,7 +394,7 @@ bool tile_problem(const ht_conv_problem *p, const ConvShape &a, ConvTileProblem 
 size_t conv_records_bytes(const ht_conv_problem *p, const ConvShape &a) {
   ConvTileProblem t;
   if (!tile_problem(p, a, t)) return 0;
-  return std::max(conv_tiled_workspace_bytes(t), conv_backward_tiled_workspace_bytes(t));
+  return std::max({conv_tiled_workspace_bytes(t), conv_rows_workspace_bytes(t), conv_backward_tiled_workspace_bytes(t)});
 }
 
 template <typename Real>
@@ -493,7 +493,7 @@ int run_patches(bool contract, int dims, int elem_bytes, const void *in, void *o
 // Forward / backward for either precision; the shared-memory tile kernels are single precision only.
 template <typename Real>
 int conv_forward(const ht_conv_problem *p, const Real *x, const Real *thr, const int64_t *ord, const Real *w, Real *out,
-                 void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {
+                 void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream, void *codes = nullptr) {
   ConvArgsOf<Real> a;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int rc = prepare_conv<Real>(p, x, thr, ord, w, workspace, workspace_bytes, status_word, s, a);
@@ -504,10 +504,15 @@ int conv_forward(const ht_conv_problem *p, const Real *x, const Real *thr, const
   if constexpr (std::is_same<Real, float>::value) {
     ConvTileProblem t;
     if (tile_problem(p, a, t)) {
+      unsigned char *records_at = static_cast<unsigned char *>(workspace) + conv_ordinal_bytes(a);
+      const size_t rows_records = conv_rows_workspace_bytes(t);
+      if (rows_records != 0 && workspace_bytes >= conv_ordinal_bytes(a) + rows_records + 256) {
+        const int by_rows = conv_forward_rows(t, x, thr, a.ord, w, out, records_at, codes, status_word, s);
+        if (by_rows != HT_ERR_UNSUPPORTED || codes != nullptr) return by_rows;
+      }
       const size_t records = conv_tiled_workspace_bytes(t);
       if (records != 0 && workspace_bytes >= conv_ordinal_bytes(a) + records + 256) {
-        const int tiled = conv_forward_tiled(t, x, thr, a.ord, w, out,
-                                             static_cast<unsigned char *>(workspace) + conv_ordinal_bytes(a), status_word, s);
+        const int tiled = conv_forward_tiled(t, x, thr, a.ord, w, out, records_at, status_word, s);
         if (tiled != HT_ERR_UNSUPPORTED) return tiled;
       }
     }
@@ -523,7 +528,7 @@ int conv_forward(const ht_conv_problem *p, const Real *x, const Real *thr, const
 template <typename Real>
 int conv_backward(const ht_conv_problem *p, const Real *x, const Real *thr, const int64_t *ord, const Real *w, const Real *g,
                   Real *gx, Real *gthr, Real *gw, void *workspace, size_t workspace_bytes, uint32_t *status_word,
-                  ht_stream_t stream) {
+                  ht_stream_t stream, const void *saved_codes = nullptr) {
   ConvArgsOf<Real> a;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   const int rc = prepare_conv<Real>(p, x, thr, ord, w, workspace, workspace_bytes, status_word, s, a, gx, gthr, gw);
@@ -533,6 +538,14 @@ int conv_backward(const ht_conv_problem *p, const Real *x, const Real *thr, cons
   if (g == nullptr) return HT_ERR_INVALID_ARGUMENT;
   if constexpr (std::is_same<Real, float>::value) {
     ConvTileProblem t;
+    if (saved_codes != nullptr) {
+      unsigned char *records_at = static_cast<unsigned char *>(workspace) + conv_ordinal_bytes(a);
+      if (!tile_problem(p, a, t) || conv_saved_code_bytes(t) == 0) return HT_ERR_INVALID_ARGUMENT;
+      if (workspace_bytes < conv_ordinal_bytes(a) + conv_rows_workspace_bytes(t) + 256) return HT_ERR_WORKSPACE;
+      const int params = conv_params_from_codes(t, x, thr, a.ord, w, g, gthr, gw, records_at, saved_codes, s);
+      if (params != HT_OK || gx == nullptr) return params;
+      return conv_image_from_saved_codes(t, g, gx, records_at, saved_codes, s);
+    }
     if (tile_problem(p, a, t)) {
       const size_t records = conv_backward_tiled_workspace_bytes(t);
       if (records != 0 && workspace_bytes >= conv_ordinal_bytes(a) + records + 256) {
@@ -591,6 +604,25 @@ size_t ht_conv_backward_workspace_bytes(const ht_conv_problem *p) {
 int ht_conv_forward_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
                         float *out, void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {
   return conv_forward<float>(p, x, thr, ord, w, out, workspace, workspace_bytes, status_word, stream);
+}
+size_t ht_conv_saved_bytes(const ht_conv_problem *p) {
+  ConvShape a;
+  ConvTileProblem t;
+  if (check_conv(p, a) != HT_OK || !tile_problem(p, a, t)) return 0;
+  return conv_saved_code_bytes(t);
+}
+int ht_conv_forward_saving_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
+                               float *out, void *kept, void *workspace, size_t workspace_bytes, uint32_t *status_word,
+                               ht_stream_t stream) {
+  if (kept == nullptr || (reinterpret_cast<uintptr_t>(kept) & 15u) != 0 || ht_conv_saved_bytes(p) == 0) return HT_ERR_INVALID_ARGUMENT;
+  if (workspace_bytes < ht_conv_workspace_bytes(p)) return HT_ERR_WORKSPACE;
+  return conv_forward<float>(p, x, thr, ord, w, out, workspace, workspace_bytes, status_word, stream, kept);
+}
+int ht_conv_backward_saved_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
+                               const float *g, float *gx, float *gthr, float *gw, const void *kept, void *workspace,
+                               size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {
+  if (kept == nullptr || (reinterpret_cast<uintptr_t>(kept) & 15u) != 0 || ht_conv_saved_bytes(p) == 0) return HT_ERR_INVALID_ARGUMENT;
+  return conv_backward<float>(p, x, thr, ord, w, g, gx, gthr, gw, workspace, workspace_bytes, status_word, stream, kept);
 }
 int ht_conv_forward_f64(const ht_conv_problem *p, const double *x, const double *thr, const int64_t *ord, const double *w,
                         double *out, void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream) {

@@ -1,5 +1,5 @@
 // Shared-memory tile kernel for the forward of 1-D / 2-D convolutional hinge trees and ferns
-// (one output per leaf).
+// (one output per leaf), where ht_conv_rows.cu does not take the problem: trees of one level or of more than seven.
 //
 // out[b, j, p] = sum over input channels c (ascending) of tree (j, c) evaluated on the kernel
 // window of channel c at output position p.  Work decomposition (one CTA of 1024 threads per SM):

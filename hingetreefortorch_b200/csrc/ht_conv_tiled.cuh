@@ -20,6 +20,12 @@ size_t conv_backward_tiled_workspace_bytes(const ConvTileProblem &p);
 // Bytes per sample of the codes through which the backward's kernels hand on one walk; 0: they walk for themselves.
 size_t conv_code_bytes(const ConvTileProblem &p);
 
+// The forward that takes four rows of outputs at a time (ht_conv_rows.cu), used where it takes the problem.  With `codes`
+// (conv_saved_code_bytes bytes) it leaves there what the backward needs of every evaluation.
+size_t conv_rows_workspace_bytes(const ConvTileProblem &p);
+int conv_forward_rows(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w, float *out,
+                      void *records, void *codes, uint32_t *status_word, cudaStream_t stream);
+
 // HT_ERR_UNSUPPORTED when the tile kernel does not take the problem (the caller falls back to the
 // thread-per-output kernel).  `ord` holds validated window-cell indices, `records` is scratch of
 // conv_tiled_workspace_bytes.
@@ -31,6 +37,15 @@ int conv_forward_tiled(const ConvTileProblem &p, const float *x, const float *th
 int conv_backward_tiled(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w,
                         const float *g, float *gx, float *gthr, float *gw, void *records, void *codes, size_t code_bytes,
                         uint32_t *status_word, cudaStream_t stream);
+
+// Scratch for those codes, for the whole batch; 0: the forward leaves none.  From them, without a walk: the gradients of thresholds
+// and leaf weights (ht_conv_codes.cu; either may be null, the records are written all the same) and, after that, the image's.
+// All are added to.
+size_t conv_saved_code_bytes(const ConvTileProblem &p);
+int conv_params_from_codes(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w,
+                           const float *g, float *gthr, float *gw, void *records, const void *codes, cudaStream_t stream);
+int conv_image_from_saved_codes(const ConvTileProblem &p, const float *g, float *gx, const void *records, const void *codes,
+                                cudaStream_t stream);
 
 namespace conv_tile {
 

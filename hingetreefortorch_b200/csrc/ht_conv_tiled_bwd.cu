@@ -23,6 +23,7 @@
 // kernel is launched for the image gradient only.  A fused form of the two with 16 warps per CTA
 // (both kinds of lane-owned arrays need the shared memory of a whole SM) was measured slower than
 // the pair: half the warps hide too little of the traversal's latency.
+#include "ht_conv_rows.cuh"
 #include "ht_conv_tiled.cuh"
 #include "ht_tile_common.cuh"
 
@@ -37,7 +38,7 @@ namespace {
 
 // What the image gradient needs of an evaluation, in 16 bits: leaf in path order (7 bits), window cell of the deciding vertex
 // (7 bits), and on top the factor sign(margin) as the first two bits of a float (2, -2, or 0 for a margin of zero or none).
-constexpr uint32_t kCodeCellShift = 7;
+using conv_rows::kCodeCellShift;
 constexpr int kCodeCells = 128, kCodeDepth = 7;
 
 // ---- records with one 8-byte entry per vertex --------------------------------------------------------
@@ -712,6 +713,8 @@ struct ImageArgs {
   uint32_t record_bytes, weights_at, leaf_mask;
 };
 
+// CELL_BITS: of the codes' window cells (a known number costs 6 % less than a mask in the arguments).
+template <int CELL_BITS>
 __global__ void __launch_bounds__(128) conv_image_from_codes_kernel(const __grid_constant__ ImageArgs a) {
   extern __shared__ float cell_columns[];  // [warp][2][4][cells][32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -776,7 +779,7 @@ __global__ void __launch_bounds__(128) conv_image_from_codes_kernel(const __grid
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         // (clamped: a parameter kernel that gave up on a lost copy leaves codes unwritten)
-        cell[e] = columns + (uint32_t)e * column_bytes + min(code[e] & (127u << kCodeCellShift), last_cell);
+        cell[e] = columns + (uint32_t)e * column_bytes + min(code[e] & (((1u << CELL_BITS) - 1u) << kCodeCellShift), last_cell);
         sum[e] = lds_f32(cell[e]);
       }
 #pragma unroll
@@ -975,6 +978,62 @@ size_t conv_code_bytes(const ConvTileProblem &p) {
   return (size_t)(p.Ci * p.Co) * (size_t)(shape.groups * shape.columns) * sizeof(uint2);
 }
 
+// The image gradient of samples `codes`, g and gx are the first of, added to gx.
+static int launch_image(const ConvTileProblem &p, const float *g, float *gx, const unsigned char *records, uint32_t record_bytes,
+                        uint32_t weights_at, int cell_bits, bool flat, const void *codes, cudaStream_t stream) {
+  ImageArgs ia = {};
+  ia.cells = p.kh * p.kw;
+  int warps = 4;  // of a CTA: their columns of sums have to fit
+  while (warps > 1 && (size_t)warps * ia.cells * 1024 > 100 * 1024) warps /= 2;
+  const size_t smem = (size_t)warps * ia.cells * 1024;
+  ia.positions = p.Ho * (int64_t)p.Wo;
+  ia.code_columns = flat ? kTileColumns : p.Wo;
+  ia.quads = (int64_t)(flat ? (p.Wo + 4 * kTileColumns - 1) / (4 * kTileColumns) : (p.Ho + 3) / 4) * ia.code_columns;
+  ia.quad_blocks = (ia.quads + 32 * warps - 1) / (32 * warps);
+  ia.channel_pairs = (p.Ci + 1) / 2;
+  if (ia.quad_blocks * ia.channel_pairs * p.B * 16 > 0x7fffffff) return HT_ERR_UNSUPPORTED;
+  ia.codes = static_cast<const uint2 *>(codes);
+  ia.records = records;
+  ia.record_bytes = record_bytes;
+  ia.weights_at = weights_at;
+  ia.leaf_mask = (1u << p.depth) - 1u;
+  ia.flat = flat ? 1 : 0;
+  ia.Ci = (int)p.Ci;
+  ia.Co = (int)p.Co;
+  ia.H = p.H;
+  ia.W = p.W;
+  ia.Wo = p.Wo;
+  ia.sy = p.sy;
+  ia.sx = p.sx;
+  ia.py = p.py;
+  ia.px = p.px;
+  ia.dy = p.dy;
+  ia.dx = p.dx;
+  ia.kw = p.kw;
+  ia.g = g;
+  ia.gx = gx;
+  auto kernel = cell_bits <= 4   ? conv_image_from_codes_kernel<4>
+                : cell_bits == 5 ? conv_image_from_codes_kernel<5>
+                : cell_bits == 6 ? conv_image_from_codes_kernel<6>
+                                 : conv_image_from_codes_kernel<7>;
+  HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+  const int64_t blocks = ia.quad_blocks * ia.channel_pairs * p.B;
+  ia.splits = (int)std::max<int64_t>(1, std::min<int64_t>({16, p.Co / 16, 148 * 6 / blocks}));
+  kernel<<<(unsigned)(blocks * ia.splits), 32 * warps, smem, stream>>>(ia);
+  HT_CHECK_LAUNCH();
+  return HT_OK;
+}
+
+int conv_image_from_saved_codes(const ConvTileProblem &p, const float *g, float *gx, const void *records, const void *codes,
+                                cudaStream_t stream) {
+  const conv_rows::Layout lay = conv_rows::rows_layout(p.kind, p.depth);
+  const conv_rows::CodeFormat format = conv_rows::code_format(p.depth, (int64_t)p.kh * p.kw);
+  // (above the cell stand bits of the height, but for shallow trees, which leave room for them below)
+  const int cell_bits = format.low_shift == p.depth && format.low_bits == 3 ? 7 : format.cell_bits;
+  return launch_image(p, g, gx, static_cast<const unsigned char *>(records), lay.bytes, lay.w,
+                      cell_bits, p.Ho == 1 && p.H == 1 && p.kh == 1, codes, stream);
+}
+
 // The parameter gradients, and with gx the image gradient from their codes: as many samples at a time as the scratch for
 // codes holds, but not with less than an eighth of the batch, where a launch would leave SMs idle more often than not.
 static int backward_by_codes(const ConvTileProblem &p, const float *x, const float *thr, const int32_t *ord, const float *w,
@@ -990,17 +1049,7 @@ static int backward_by_codes(const ConvTileProblem &p, const float *x, const flo
   }
   const int64_t trees = p.Co * p.Ci, positions = p.Ho * (int64_t)p.Wo, image = p.H * (int64_t)p.W;
   const int64_t elements = trees * (threshold_count(p.kind, p.depth) + (((int64_t)1) << p.depth));
-  const CodeShape shape = code_shape(p, pplan);
-  ImageArgs ia = {};
-  ia.cells = p.kh * p.kw;
-  int warps = 4;  // of a CTA: their columns of sums have to fit
-  while (warps > 1 && (size_t)warps * ia.cells * 1024 > 100 * 1024) warps /= 2;
-  const size_t smem = (size_t)warps * ia.cells * 1024;
-  ia.positions = positions;
-  ia.quads = shape.groups * shape.columns;
-  ia.quad_blocks = (ia.quads + 32 * warps - 1) / (32 * warps);
-  ia.channel_pairs = (p.Ci + 1) / 2;
-  if (ia.quad_blocks * ia.channel_pairs * at_once * 16 > 0x7fffffff) return HT_ERR_UNSUPPORTED;
+  if (((positions + 127) / 32) * ((p.Ci + 1) / 2) * at_once * 16 > 0x7fffffff) return HT_ERR_UNSUPPORTED;
   unsigned char *rec = static_cast<unsigned char *>(records);
   RecordMap map;
   map.columns = p.kw;
@@ -1010,40 +1059,16 @@ static int backward_by_codes(const ConvTileProblem &p, const float *x, const flo
   map.outer_count = p.Co;
   repack_vertex_pairs_kernel<<<(unsigned)((elements + 255) / 256), 256, 0, stream>>>(thr, ord, w, rec, p.kind, p.depth, trees, pplan.rec, map);
   HT_CHECK_LAUNCH();
-  ia.codes = static_cast<const uint2 *>(codes);
-  ia.records = rec;
-  ia.record_bytes = pplan.rec.bytes;
-  ia.weights_at = pplan.rec.w;
-  ia.leaf_mask = (1u << p.depth) - 1u;
-  ia.flat = pplan.flat ? 1 : 0;
-  ia.code_columns = shape.columns;
-  ia.Ci = (int)p.Ci;
-  ia.Co = (int)p.Co;
-  ia.H = p.H;
-  ia.W = p.W;
-  ia.Wo = p.Wo;
-  ia.sy = p.sy;
-  ia.sx = p.sx;
-  ia.py = p.py;
-  ia.px = p.px;
-  ia.dy = p.dy;
-  ia.dx = p.dx;
-  ia.kw = p.kw;
-  HT_CUDA_TRY(cudaFuncSetAttribute(conv_image_from_codes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   for (int64_t b0 = 0; b0 < p.B; b0 += at_once) {
     ConvTileProblem part = p;
     part.B = std::min<int64_t>(at_once, p.B - b0);
     const float *part_g = g + b0 * p.Co * positions;
-    const int rc = launch_parameters(part, pplan, x + b0 * p.Ci * image, rec, part_g, gthr, gw,
-                                     gx != nullptr ? static_cast<uint2 *>(codes) : nullptr, status_word, stream);
+    int rc = launch_parameters(part, pplan, x + b0 * p.Ci * image, rec, part_g, gthr, gw,
+                               gx != nullptr ? static_cast<uint2 *>(codes) : nullptr, status_word, stream);
+    if (rc == HT_OK && gx != nullptr)
+      rc = launch_image(part, part_g, gx + b0 * p.Ci * image, rec, pplan.rec.bytes, pplan.rec.w,
+                        7, pplan.flat, codes, stream);
     if (rc != HT_OK) return rc;
-    if (gx == nullptr) continue;
-    ia.g = part_g;
-    ia.gx = gx + b0 * p.Ci * image;
-    const int64_t blocks = ia.quad_blocks * ia.channel_pairs * part.B;
-    ia.splits = (int)std::max<int64_t>(1, std::min<int64_t>({16, p.Co / 16, 148 * 6 / blocks}));
-    conv_image_from_codes_kernel<<<(unsigned)(blocks * ia.splits), 32 * warps, smem, stream>>>(ia);
-    HT_CHECK_LAUNCH();
   }
   return HT_OK;
 }

@@ -285,6 +285,16 @@ int ht_conv_forward_f32(const ht_conv_problem *p, const float *x, const float *t
 int ht_conv_backward_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
                          const float *g, float *gx, float *gthr, float *gw, void *workspace, size_t workspace_bytes,
                          uint32_t *status_word, ht_stream_t stream);
+/* A forward that keeps, in ht_conv_saved_bytes(p) bytes of the caller's (2 per evaluation, 16-byte aligned), what the backward
+ * of the same problem and parameters needs of every evaluation, and the backward that reads it instead of walking; it leaves the
+ * bytes as they are.  0 bytes: the forward keeps nothing of this problem, and both are refused (HT_ERR_INVALID_ARGUMENT). */
+size_t ht_conv_saved_bytes(const ht_conv_problem *p);
+int ht_conv_forward_saving_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
+                               float *out, void *kept, void *workspace, size_t workspace_bytes, uint32_t *status_word,
+                               ht_stream_t stream);
+int ht_conv_backward_saved_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
+                               const float *g, float *gx, float *gthr, float *gw, const void *kept, void *workspace,
+                               size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream);
 
 /* ---- contract / expand -------------------------------------------------------------------------
  * contract: image [BC, size...] -> non-overlapping windows [BC, osize..., window...], zero padded,
