@@ -473,25 +473,22 @@ static bool ordered_from_paths(const ht_forest_problem *p) {
 }
 
 // Whether the walk goes past resident trees row by row (ht_forest_rows.cu) rather than past resident tiles of samples or with a
-// thread per evaluation: where the estimates have it cheaper by 15 %.  It is for samples of many features, which leave room for
-// small tiles only (8192 x 784 under 800 trees of depth 8, 10 outputs: 254 against 485 us), and for batches that give few tiles.
-// How good the choice is, on 1104 forwards of random sizes timed every way (profiles/forward_kernel_choice.csv):
-//   * against the tile kernel (808 of them) it costs 0.9 % over the better of the two on average and more than 20 % in 5 cases;
-//     always tiles 9.1 %, always rows 29 %.  The 15 % are where that loss is least: 2.0 % with a margin of 30 %, 1.4 % with none;
-//   * against a thread per evaluation (296) the third estimate is a rough one (it has the right order of magnitude, and a spread
-//     of 1.6 to 1.8 times), and the choice costs 3.2 %, never taking rows 3.4 % (with the time of all these calls added up 12
-//     and 13 %: rows win in the long calls).  Ferns stay with the threads there: the estimate is too high for them, and chosen
-//     by it they lose 2.4 % instead of 1.5.
-static bool rows_are_better(const ht_forest_problem *p) {
+// thread per evaluation: where the estimates, all three of single calls on cold caches, have it cheaper by 10 %.  It is for samples of
+// many features, which leave room for small tiles only, and for batches that give few tiles.  How good the choice is, on 1104
+// forwards of random sizes timed every way (profiles/forward_kernel_choice.csv):
+//   * against the tile kernel (808 of them) it costs 1.3 % over the better of the two on average and more than 20 % in 18 cases;
+//     always tiles 9.4 %, always rows 25 %; with no margin it costs 1.1 %, but calls in a loop, on warm caches, gain from tiles what
+//     the estimates do not know (12407 x 342, 34 trees of depth 8, 26 outputs: a ratio of 0.905, a training step of 88 against 82 us);
+//   * against a thread per evaluation (296) 3 % (trees) and 0.4 % (ferns); never taking rows 6.2 and 2.6 %.
+// `keep`: the paths leave, too.
+static bool rows_are_better(const ht_forest_problem *p, bool keep) {
   const double rows = rows_forward_cost(p);
   if (rows < 0.0 || p->B * p->T < 32768) return false;
   double other = forward_tiled_cost(p);
-  if (other < 0.0) {
-    if (p->kind == FERN) return false;
-    const double evals = (double)(p->B * p->T);
-    other = 5.1 + evals * (3.1e-6 * p->depth + 3.7e-6 * (double)p->M);
-  }
-  return rows < 0.85 * other;
+  if (other < 0.0)
+    other = 10.8 + (double)(p->B * p->T) * ((p->kind == FERN ? 2.0e-6 : 4.3e-6) * p->depth + 0.74e-6 * (double)p->M + (keep ? 16.2e-6 : 0.0)) +
+            0.31e-6 * (double)p->B * (double)p->C;
+  return rows < 0.9 * other;
 }
 
 // What a backward keeps per evaluation: the records of the tile kernels (one output per leaf), or the paths (several) and,
@@ -533,7 +530,7 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
   }
   const WideOrdinals wide = {ord, p->C};
   int32_t *packed = static_cast<int32_t *>(workspace);
-  const bool by_rows = rows_are_better(p);
+  const bool by_rows = rows_are_better(p, eval_records != nullptr);
   if (!by_rows) {
     rc = forward_tiled(p, x, thr, packed, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream, &wide);
     if (rc != HT_ERR_UNSUPPORTED) return rc;
@@ -639,7 +636,7 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
       if (!kept && (!ordered || gthr != nullptr || gw != nullptr)) {  // the paths first
         const PathRecordsOf<float> paths = saved_paths(p, eval_records);
         int prc = HT_ERR_UNSUPPORTED;
-        if (rows_are_better(p)) prc = rows_forward(p, x, thr, a.ord, w, none, paths.margin, paths.where, status_word, pr.stream);
+        if (rows_are_better(p, true)) prc = rows_forward(p, x, thr, a.ord, w, none, paths.margin, paths.where, status_word, pr.stream);
         if (prc == HT_ERR_UNSUPPORTED && p->M > 1)
           prc = forward_tiled(p, x, thr, static_cast<int32_t *>(workspace), w, none, ws + ordinals_bytes(p), eval_records, status_word,
                               pr.stream);

@@ -187,6 +187,37 @@ def test_fused_linear_on_tabular_data(case):
             assert grad_close(got, ref[at], sizes[at])
 
 
+# Rows of x streaming past resident trees: pitches that are padded and that are not, 16, 8 and 4 rows at a time, from fewer sets of
+# trees than warps to several rounds of them, several groups of trees, more steps than row buffers and a last step that is short.
+ROWS = [
+    ("tree", 16 * 148 * 10 + 5, 64, 100, 7),
+    ("tree", 16 * 148 * 3 + 16, 41, 9, 3),
+    ("fern", 5000, 90, 113, 8),
+    ("tree", 2400, 24, 250, 2),
+    ("tree", 700, 1500, 65, 6),
+    ("tree", 600, 3004, 40, 6),
+    ("tree", 150, 5002, 70, 9),
+    ("fern", 300, 6008, 20, 10),
+]
+
+
+@pytest.mark.parametrize("case", ROWS, ids=[str(c) for c in ROWS])
+def test_rows_past_resident_trees(case):
+    from hingetreefortorch_b200 import _cabi
+    kind, B, C, T, depth = case
+    rng = np.random.default_rng(190 + ROWS.index(case))
+    x, thr, ord_, w = random_forest_inputs(190 + ROWS.index(case), kind, B, C, (), T, depth, (), quantise=True)
+    x[0, :] = np.nan
+    x[B - 1, ::2] = np.inf
+    lin, bias = [rng.standard_normal(s).astype(np.float32) for s in ((2, T), 2)]
+    dx, dthr, dord, dw, dlin, dbias = dev(x, thr, ord_, w, lin, bias)
+    fam = _cabi.ForestFamily(kind, dx, dw, lin=dlin)
+    got = fam.linear_forward(dx, None, dthr, dord, dw, dlin, dbias).cpu().numpy()
+    with np.errstate(all="ignore"):
+        assert np.array_equal(got, ho.linear_forward(kind, x, thr, ord_, w, lin, bias), equal_nan=True)
+    assert fam.status.item() == 0
+
+
 def test_modules_fused_linear_and_fusion():
     from hingetreefortorch_b200 import RandomHingeForest as R
     torch.manual_seed(1)
