@@ -6,6 +6,7 @@
 // rows of x stream past them as they lie in memory, by bulk async copies.
 #include "ht_forest_rows.cuh"
 #include "ht_tile_common.cuh"
+#include "ht_tma.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -333,7 +334,8 @@ int launch_rows(const RowArgs &a, int kind, size_t smem, cudaStream_t stream) {
 
 // ---- x gradient ------------------------------------------------------------------------------------------------------
 
-constexpr int kXRows = 32;
+constexpr int kXRows = 16;
+constexpr int kXTrees = 32 / kXRows;  // of a warp at a time
 constexpr int kXThreads = 512;
 
 struct RowXArgs {
@@ -345,50 +347,74 @@ struct RowXArgs {
   int C, N, pitch;
 };
 
-// CTA = 32 rows of gx in shared memory (lane = row, so that records are read in runs), a warp per tree.  Two warps may add
+// CTA = 16 rows of gx in shared memory (a warp is 16 rows on two trees, so that records are read in runs).  Two warps may add
 // into an element at the same time, hence atomics; on different rows they do not meet.  Every element of gx is written once,
-// where scattering into cleared global memory touches it twice and half of it in 32-byte pieces.
-// Bound by writing gx: two CTAs per SM for rows of up to 880 features, so that one adds while the other writes.
-// 262144 x 784, 100 trees: 234 us, 3.5 TB/s (clearing and scattering took over 500).
-template <typename WhereT>
+// where scattering into cleared global memory touches it twice and half of it in 32-byte pieces.  The records of a warp's first
+// sets of trees are under way while the rows are cleared.
+// BULK: rows leave by bulk copies (they lie on 16-byte boundaries here and there).
+// Bound by writing gx: four CTAs per SM for rows of up to 880 features, so that some add while others write.
+// 262144 x 784, 100 trees: 203 us, 4.8 TB/s (237 with 32 rows, four trees at a time after the clearing, and rows written by the threads;
+// clearing and scattering took over 500).
+template <typename WhereT, bool BULK>
 __global__ void __launch_bounds__(kXThreads) rows_x_gradient_kernel(const __grid_constant__ RowXArgs a) {
   extern __shared__ __align__(16) float tile_rows[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t row0 = (int64_t)blockIdx.x * kXRows;
   const int rows = (int)min((int64_t)kXRows, a.B - row0);
-  for (int e = tid; e < kXRows * a.pitch; e += kXThreads) tile_rows[e] = 0.0f;
+  constexpr int kAhead = 4, kApart = kXThreads / 32 * kXTrees;  // trees between a lane's
+  const int my_row = lane % kXRows, first = warp * kXTrees + lane / kXRows;
+  const int64_t at0 = record_index(row0, 0, a.T) + my_row;
+  const int T = (int)a.T;
+  float d[kAhead];
+  uint32_t vertex[kAhead];
+  auto fetch = [&](int j0) {
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      const int j = j0 + u * kApart;
+      d[u] = 0.0f;
+      vertex[u] = 1u;
+      if (j < T && my_row < rows) {
+        d[u] = stream_f32(a.dx + at0 + (int64_t)j * kRecordBlock);
+        vertex[u] = stream_raw_where<WhereT>(a.where, at0 + (int64_t)j * kRecordBlock);
+      }
+    }
+  };
+  fetch(first);
+  for (int e = tid; e < kXRows * a.pitch / 4; e += kXThreads) reinterpret_cast<float4 *>(tile_rows)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   __syncthreads();
-  constexpr int kAhead = 4, kWarps = kXThreads / 32;
-  const int64_t at0 = record_index(row0, 0, a.T) + lane;
-  float *mine = tile_rows + lane * a.pitch;
-  for (int64_t j0 = warp; j0 < a.T; j0 += kWarps * kAhead) {
-    float d[kAhead];
-    uint32_t vertex[kAhead];
+  float *mine = tile_rows + my_row * a.pitch;
+  for (int j0 = first; j0 - lane / kXRows < T; j0 += kApart * kAhead) {
+    if (j0 != first) fetch(j0);
     int feature[kAhead];
 #pragma unroll
     for (int u = 0; u < kAhead; ++u) {
-      const int64_t j = j0 + u * kWarps;
-      const bool on = j < a.T && lane < rows;
-      d[u] = on ? __ldcs(a.dx + at0 + j * kRecordBlock) : 0.0f;
-      vertex[u] = on ? load_where<WhereT>(a.where, at0 + j * kRecordBlock) & 0xffffu : 1u;
-    }
-#pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      const int64_t j = min(j0 + u * kWarps, a.T - 1);
-      feature[u] = __ldg(a.ord + j * a.N + vertex[u] - 1);
+      const int j = min(j0 + u * kApart, T - 1);
+      feature[u] = __ldg(a.ord + (int64_t)j * a.N + (unpack_where<WhereT>(vertex[u]) & 0xffffu) - 1);
     }
 #pragma unroll
     for (int u = 0; u < kAhead; ++u)
       if (d[u] != 0.0f) atomicAdd(mine + feature[u], d[u]);  // (a NaN is not equal to 0)
   }
-  __syncthreads();
   float *out = a.gx + row0 * a.C;
-  // (a number per lane: 16 bytes per lane would take every row of four banks four times)
-  for (int r = warp; r < rows; r += kWarps)
-    for (int c = lane; c < a.C; c += 32) __stcs(out + (int64_t)r * a.C + c, tile_rows[r * a.pitch + c]);
+  if constexpr (BULK) {
+    tma::fence_async_shared();
+    __syncthreads();
+    if (warp == 0) {
+      if (lane < rows) tma::store_rows(out + (int64_t)lane * a.C, smem_addr(mine), (uint32_t)a.C * 4u);  // (lane < 16: its own row)
+      tma::commit_group();
+      tma::wait_stores_read();
+    }
+  } else {
+    __syncthreads();
+    // (a number per lane: 16 bytes per lane would take every row of four banks four times)
+    for (int r = warp; r < rows; r += kXThreads / 32)
+      for (int c = lane; c < a.C; c += 32) __stcs(out + (int64_t)r * a.C + c, tile_rows[r * a.pitch + c]);
+  }
 }
 
-inline size_t row_x_smem(int64_t C) { return (size_t)kXRows * (C | 1) * 4; }
+// Rows that leave by bulk copies start on 16-byte boundaries, four banks apart or a multiple of that; others at an odd distance.
+inline int64_t row_x_pitch(int64_t C, bool bulk) { return bulk ? row_pitch(C) : C | 1; }
+inline size_t row_x_smem(int64_t C) { return (size_t)kXRows * std::max(row_x_pitch(C, (C & 3) == 0), C | 1) * 4; }
 
 }  // namespace
 
@@ -456,8 +482,11 @@ bool rows_x_gradient_takes(const ht_forest_problem *p) {
 
 int rows_x_gradient(const ht_forest_problem *p, const int32_t *ord, const float *dx, const void *where, float *gx, cudaStream_t stream) {
   if (!rows_x_gradient_takes(p)) return HT_ERR_UNSUPPORTED;
-  RowXArgs a = {dx, where, ord, gx, p->B, p->T, (int)p->C, (int)threshold_count(p->kind, p->depth), (int)(p->C | 1)};
-  auto kernel = where_bytes(p->depth) == 2 ? rows_x_gradient_kernel<unsigned short> : rows_x_gradient_kernel<uint32_t>;
+  const bool bulk = (p->C & 3) == 0 && (reinterpret_cast<uintptr_t>(gx) & 15u) == 0;
+  RowXArgs a = {dx, where, ord, gx, p->B, p->T, (int)p->C, (int)threshold_count(p->kind, p->depth), (int)row_x_pitch(p->C, bulk)};
+  auto kernel = where_bytes(p->depth) == 2
+                    ? (bulk ? rows_x_gradient_kernel<unsigned short, true> : rows_x_gradient_kernel<unsigned short, false>)
+                    : (bulk ? rows_x_gradient_kernel<uint32_t, true> : rows_x_gradient_kernel<uint32_t, false>);
   HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
   kernel<<<(unsigned)((p->B + kXRows - 1) / kXRows), kXThreads, row_x_smem(p->C), stream>>>(a);
   HT_CHECK_LAUNCH();

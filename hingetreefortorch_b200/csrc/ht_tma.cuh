@@ -77,6 +77,10 @@ __device__ __forceinline__ void store_2d(const CUtensorMap *map, uint32_t src, i
                "r"(src)
                : "memory");
 }
+// The same for contiguous bytes: both addresses and the size are multiples of 16.
+__device__ __forceinline__ void store_rows(float *dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
 __device__ __forceinline__ void commit_group() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Until the issuing thread's earlier stores have finished READING shared memory (the source may be reused).
 __device__ __forceinline__ void wait_stores_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
