@@ -16,6 +16,9 @@
 // 3.58.
 #include "ht_conv_rows.cuh"
 
+#include <cstring>
+#include <type_traits>
+
 namespace ht {
 
 using namespace tile;
@@ -38,7 +41,7 @@ struct RowsPlan {
   int rows() const { return 4 * quads * row_groups; }
 };
 
-bool make_plan(const ConvTileProblem &p, RowsPlan &plan) {
+bool find_plan(const ConvTileProblem &p, RowsPlan &plan) {
   if (p.depth < 2 || p.depth > kMaxDepth || p.Ci < 1 || p.Co < 1 || p.B < 1 || p.Ho < 1 || p.Wo < 1) return false;
   if ((double)p.B * p.Ho * p.Wo * (double)p.Co * p.Ci < 1048576.0) return false;  // not worth a 1024-thread CTA
   plan.flat = p.Ho == 1 && p.H == 1 && p.kh == 1;
@@ -82,6 +85,21 @@ bool make_plan(const ConvTileProblem &p, RowsPlan &plan) {
         }
       }
   return best != 0.0 && plan.smem <= kSmemBudget;
+}
+
+// A call asks for its plan several times (scratch, what is kept, the launch): the last one is at hand (3 us to find one).
+bool make_plan(const ConvTileProblem &p, RowsPlan &plan) {
+  static_assert(std::has_unique_object_representations<ConvTileProblem>::value, "compared byte by byte");
+  thread_local ConvTileProblem last = {};
+  thread_local RowsPlan found = {};
+  thread_local bool known = false, takes = false;
+  if (!known || std::memcmp(&last, &p, sizeof p) != 0) {
+    takes = find_plan(p, found);
+    last = p;
+    known = true;
+  }
+  plan = found;
+  return takes;
 }
 
 struct RowsArgs {
