@@ -482,8 +482,9 @@ static bool ordered_from_paths(const ht_forest_problem *p) {
 //   * against a thread per evaluation (296) 3 % (trees) and 0.4 % (ferns); never taking rows 6.2 and 2.6 %.
 // `keep`: the paths leave, too.
 static bool rows_are_better(const ht_forest_problem *p, bool keep) {
+  if (p->B * p->T < 32768) return false;
   const double rows = rows_forward_cost(p);
-  if (rows < 0.0 || p->B * p->T < 32768) return false;
+  if (rows < 0.0) return false;
   double other = forward_tiled_cost(p);
   if (other < 0.0)
     other = 10.8 + (double)(p->B * p->T) * ((p->kind == FERN ? 2.0e-6 : 4.3e-6) * p->depth + 0.74e-6 * (double)p->M + (keep ? 16.2e-6 : 0.0)) +

@@ -172,7 +172,15 @@ __device__ __forceinline__ Real chain(const Real *t, int n, Real acc, int stride
     for (int u = 0; u < kAhead; ++u) acc = add_rn(acc, now[u]);
     e += kAhead;
   }
-  for (; e < n; ++e) acc = add_rn(acc, t[e * stride]);
+  while (e < n) {  // the rest: loads together, none past the end
+    Real rest[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) rest[u] = t[min(e + u, n - 1) * stride];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (e + u < n) acc = add_rn(acc, rest[u]);
+    e += kAhead;
+  }
   return acc;
 }
 
@@ -181,8 +189,10 @@ __device__ __forceinline__ Real chain(const Real *t, int n, Real acc, int stride
 // position, 32 outputs per CTA.  Thresholds (kind 1): a position's M terms follow one another in the same chain.  A bin is
 // in one part only: the part that its first position falls into when the list is cut evenly.
 // Bound by the chain of the fullest bin, 4 clocks per addition (data in [0, 1] under thresholds in [-3, 3]: many samples
-// decide at one vertex).  8192 x 784, 100 trees of depth 7, 10 outputs: 261 us, of which the longest
-// chain (81920 terms at one vertex) is 170; one warp per tree that walked and added in turn took 7476.
+// decide at one vertex).  8192 x 784, 100 trees of depth 7, 10 outputs: 248 us, of which the longest
+// chain (81920 terms at one vertex) is 172 (266 with seven producing warps and the adding one always the first); one warp per
+// tree that walked and added in turn took 7476.  Measured and not faster: three CTAs per SM instead of two (284), one (313), the outcomes
+// of pieces of a chain worked out ahead for the binade that the sum is in (270 to 460).
 template <typename Real>
 __global__ void __launch_bounds__(kSumBlock) ordered_sum_kernel(const __grid_constant__ OrderedArgs<Real> a) {
   __shared__ __align__(16) unsigned char buffers[2][kTermBytes];
@@ -191,17 +201,24 @@ __global__ void __launch_bounds__(kSumBlock) ordered_sum_kernel(const __grid_con
   const int m0 = kind == 0 ? 32 * ((int)blockIdx.z - 1) : 0;
   const int width = kind == 0 ? (int)min((int64_t)32, a.M - m0) : (int)a.M;  // terms per position
   const int bins = (int)(kind == 0 ? a.L : a.N);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x, lane = tid & 31;
+  // Which warp does what: 0 adds, kIdle would share its scheduler (a warp's number modulo 4) and with it the issue slots that the
+  // chain of additions asks for every fourth clock, the others produce.  CTAs that are likely to share an SM (148 are launched at
+  // a time) add on different schedulers.
+  constexpr int kIdle = 4;
+  const uint32_t cta = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  const int warp = ((tid >> 5) + (int)((cta / 148) & 3u)) & (kSumBlock / 32 - 1);
+  const bool produces = warp != 0 && warp != kIdle;
   const int64_t j = blockIdx.x;
   const uint32_t *list = a.lists.list[kind] + j * a.P, *first = a.lists.first[kind] + j * (bins + 1);
-  auto bin_at = [&](int64_t part) {  // the first bin that begins at or after part / parts of the list
-    int lo = 0, hi = bins;
-    while (lo < hi) {
-      const int mid = (lo + hi) / 2;
-      if ((int64_t)__ldg(first + mid) * a.parts >= part * a.P) hi = mid;
-      else lo = mid + 1;
+  // the first bin that begins at or after part / parts of the list: as many as begin before it
+  auto bin_at = [&](int64_t part) {
+    int before = 0;
+    for (int b0 = 0; b0 < bins; b0 += kSumBlock) {
+      const int b = b0 + tid;
+      before += __syncthreads_count(b < bins && (int64_t)__ldg(first + b) * a.parts < part * a.P);
     }
-    return lo;
+    return before;
   };
   const Real *sizes = static_cast<const Real *>(a.lists.value[0]) + j * a.P;
   const uint32_t *keys = static_cast<const uint32_t *>(a.lists.value[1]) + j * a.P;
@@ -215,7 +232,8 @@ __global__ void __launch_bounds__(kSumBlock) ordered_sum_kernel(const __grid_con
   const int piece = min(width, kTerms), pieces = (width + piece - 1) / piece;
   int lanes = 1;
   while (lanes < 32 && lanes < piece) lanes *= 2;
-  const int pitch = kind == 0 ? lanes : piece, rows = max(1, kTerms / pitch);
+  // (whole loads and whole turns of the adding loop, where a bin goes on)
+  const int pitch = kind == 0 ? lanes : piece, room = max(1, kTerms / pitch), rows = room >= 32 ? room & ~31 : room;
   const int64_t steps = ((end - begin + rows - 1) / rows) * pieces;
 
   auto produce = [&](int64_t step) {
@@ -223,9 +241,9 @@ __global__ void __launch_bounds__(kSumBlock) ordered_sum_kernel(const __grid_con
     const int64_t row0 = begin + step / pieces * rows;
     const int count = (int)min((int64_t)rows, end - row0);
     const int from = (int)(step % pieces) * piece, here = min(piece, width - from);
-    constexpr int kAhead = 8, kWarps = kSumBlock / 32 - 1;
+    constexpr int kAhead = 8, kWarps = kSumBlock / 32 - 2;
     const int per_warp = 32 / lanes;
-    const int m_lane = lane % lanes, first_row = (warp - 1) * per_warp + lane / lanes;
+    const int m_lane = lane % lanes, first_row = (warp < kIdle ? warp - 1 : warp - 2) * per_warp + lane / lanes;
     for (int m = m_lane; m - m_lane < here; m += lanes) {
       const bool on = m < here;
       const int mc = min(m, here - 1);  // lanes and rows past the end load what their neighbours load, and store nothing
@@ -259,7 +277,7 @@ __global__ void __launch_bounds__(kSumBlock) ordered_sum_kernel(const __grid_con
     }
   };
 
-  if (warp != 0) produce(0);
+  if (produces) produce(0);
   __syncthreads();
   Real acc = (Real)0;
   int64_t row = begin, bin_end = __ldg(first + bin + 1);  // the adding warp's place in the list
@@ -279,7 +297,7 @@ __global__ void __launch_bounds__(kSumBlock) ordered_sum_kernel(const __grid_con
   if (warp == 0) next_bin();
   for (int64_t step = 0; step < steps; ++step) {
     if (warp != 0) {
-      if (step + 1 < steps) produce(step + 1);
+      if (produces && step + 1 < steps) produce(step + 1);
     } else {
       const Real *from = reinterpret_cast<const Real *>(buffers[step & 1]);
       const int64_t row0 = begin + step / pieces * rows;
