@@ -211,7 +211,7 @@ __global__ void __launch_bounds__(kThreads, 1) conv_forward_rows_kernel(const __
       uint2 *codes = nullptr;
       if constexpr (CODES) codes = a.codes + ((b * a.Ci + lot0) * a.Co + j) * code_quads + code_at;
       for (int c = 0; c < lot && !poisoned; c += a.CC) {
-        if (!mbar_wait(&my_full[stage], phase)) {
+        if (!__all_sync(0xffffffffu, mbar_wait(&my_full[stage], phase))) {  // (the lanes leave together or not at all)
           poisoned = true;
           if (lane == 0 && a.status_word != nullptr) atomicOr(a.status_word, HT_FLAG_PIPELINE_TIMEOUT);
           break;
