@@ -7,6 +7,7 @@
 #include <ATen/Context.h>
 #include <c10/core/DeviceGuard.h>
 #include <torch/csrc/autograd/forward_grad.h>
+#include <torch/csrc/autograd/graph_task.h>
 #include <torch/csrc/jit/frontend/tracer.h>
 
 #include "hingetree_cpp_ops.h"
@@ -115,7 +116,7 @@ struct ConvNode : public torch::autograd::Function<ConvNode> {
     ctx->saved_data["kind"] = kind;
     ctx->saved_data["geometry"] = geometry;
     const Geometry g(geometry);
-    torch::Tensor kept;  // serves every backward through this node
+    torch::Tensor kept;
     const torch::Tensor out = conv_forward((int)kind, g.dims, x, thr, ord, w, g.part(0), g.part(1), g.part(2), g.part(3), &kept);
     if (kept.defined()) ctx->saved_data["kept"] = kept;
     return out;
@@ -125,8 +126,14 @@ struct ConvNode : public torch::autograd::Function<ConvNode> {
     const int64_t kind = ctx->saved_data["kind"].toInt();
     refuse_deterministic(grads[0], "backpropagation for hinge " + name_of(kind) + " convolution");
     const Geometry g(ctx->saved_data["geometry"].toIntVector());
+    // The codes serve every backward through this node.  They go with the graph's buffers: saved_data lives as long as the output
+    // is referenced, which in a training loop is until the next step's forward has taken as much again.
     const auto at = ctx->saved_data.find("kept");
-    const torch::Tensor kept = at != ctx->saved_data.end() ? at->second.toTensor() : torch::Tensor();
+    torch::Tensor kept;
+    if (at != ctx->saved_data.end()) {
+      kept = at->second.toTensor();
+      if (!torch::autograd::get_current_graph_task_keep_graph()) ctx->saved_data.erase(at);
+    }
     std::vector<torch::Tensor> r = conv_backward((int)kind, g.dims, s[0], ctx->needs_input_grad(0), s[1], ctx->needs_input_grad(1), s[2],
                                                  false, s[3], ctx->needs_input_grad(3), grads[0].contiguous(), g.part(0), g.part(1),
                                                  g.part(2), g.part(3), &kept);

@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import hingetreefortorch_b200._cabi as _cabi
-from conftest import grad_close
+from conftest import grad_close, requested_bytes
 from oracle import hinge_oracle as ho
 from test_conv_gpu import dev
 
@@ -95,3 +95,36 @@ def test_autograd_keeps_the_codes_by_the_callers_settings(setting):
     finally:
         ext.set_save_forward(True)
         ext.set_backward_scratch_limit(2 ** 62)
+
+
+def layer(x_shape=(4, 32, 32, 64), Co=32, depth=5):
+    """The call of a 3 x 3 convolution, what it is differentiated by, an upstream gradient, and the bytes that a forward keeps."""
+    from hingetreefortorch_b200._ext import hingetree_cpp as ext
+    geometry = ((3, 3), (1, 1), (1, 1), (1, 1))
+    x, w = torch.randn(x_shape, device="cuda"), torch.randn(Co, x_shape[1], 2 ** depth, device="cuda")
+    thr = torch.rand(Co, x_shape[1], 2 ** depth - 1, device="cuda") - 0.5
+    ord_ = torch.randint(0, 9, thr.shape, device="cuda")
+    g = torch.randn_like(ext.tree_conv2d_forward(x, thr, ord_, w, *geometry))  # (which checks the ordinals)
+    leaves = [t.requires_grad_() for t in (x, thr, w)]
+    return lambda: ext.tree_conv2d_apply(x, thr, ord_, w, *geometry), leaves, g, _cabi.Conv("tree", x, w, *geometry).saved_bytes()
+
+
+def test_a_backward_gives_back_what_the_forward_kept():
+    """The output still referenced, as a training loop holds it until the next step's forward has run: of both steps' codes only
+    one is ever there.  A graph that is retained holds on to them until the backward that does not retain it."""
+    call, leaves, g, codes = layer()
+    before = requested_bytes()
+    out = call()
+    assert requested_bytes() - before >= codes + out.numel() * 4
+    torch.autograd.grad(out, leaves, g)
+    assert requested_bytes() - before <= out.numel() * 4
+    torch.cuda.reset_peak_memory_stats()
+    second = call()
+    assert requested_bytes(peak=True) - before < 2 * codes
+    first = torch.autograd.grad(second, leaves, g, retain_graph=True)
+    held = requested_bytes() - before
+    again = torch.autograd.grad(second, leaves, g, retain_graph=True)
+    assert requested_bytes() - held - before == sum(t.numel() * 4 for t in again)
+    del again
+    torch.autograd.grad(second, leaves, g)
+    assert requested_bytes() - before <= 2 * out.numel() * 4 + sum(t.numel() * 4 for t in first)
