@@ -134,9 +134,19 @@ struct ConvNode : public torch::autograd::Function<ConvNode> {
       kept = at->second.toTensor();
       if (!torch::autograd::get_current_graph_task_keep_graph()) ctx->saved_data.erase(at);
     }
-    std::vector<torch::Tensor> r = conv_backward((int)kind, g.dims, s[0], ctx->needs_input_grad(0), s[1], ctx->needs_input_grad(1), s[2],
-                                                 false, s[3], ctx->needs_input_grad(3), grads[0].contiguous(), g.part(0), g.part(1),
-                                                 g.part(2), g.part(3), &kept);
+    auto from = [&](const torch::Tensor *codes) {
+      return conv_backward((int)kind, g.dims, s[0], ctx->needs_input_grad(0), s[1], ctx->needs_input_grad(1), s[2], false, s[3],
+                           ctx->needs_input_grad(3), grads[0].contiguous(), g.part(0), g.part(1), g.part(2), g.part(3), codes);
+    };
+    std::vector<torch::Tensor> r;
+    try {
+      r = from(&kept);
+    } catch (const c10::OutOfMemoryError &) {  // the codes may be in the way of what the backward cannot do without
+      if (!kept.defined()) throw;
+      kept.reset();
+      ctx->saved_data.erase("kept");
+    }
+    if (r.empty()) r = from(nullptr);
     return {r[0], r[1], torch::Tensor(), r[3], torch::Tensor(), torch::Tensor()};
   }
   struct Geometry {  // kernel size, stride, padding and dilation one after another

@@ -544,6 +544,7 @@ torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor th
   ConvCall call(kind, dims, x, thr, ord, w, nullptr, kernel, stride, padding, dilation);
   c10::DeviceGuard guard(x.device());
   torch::Tensor out = fresh(call.out_sizes, x);
+  torch::Tensor ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);  // before what the call can do without
   if (kept != nullptr && x.scalar_type() == torch::kFloat32) {
     constexpr int64_t kMostKept = (int64_t)8 << 30;  // as much as the codes of a backward that walks may take
     const int64_t bytes = (int64_t)ht_conv_saved_bytes(&call.problem);
@@ -554,7 +555,6 @@ torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor th
       }
     }
   }
-  torch::Tensor ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);
   OrdinalGuard og(ord, call.window_cells);
   if (kept != nullptr && kept->defined()) {
     raise_status(ht_conv_forward_saving_f32(&call.problem, x.data_ptr<float>(), thr.data_ptr<float>(), ord.data_ptr<int64_t>(),

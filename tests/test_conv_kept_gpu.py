@@ -128,3 +128,40 @@ def test_a_backward_gives_back_what_the_forward_kept():
     del again
     torch.autograd.grad(second, leaves, g)
     assert requested_bytes() - before <= 2 * out.numel() * 4 + sum(t.numel() * 4 for t in first)
+
+
+def within(room, what):
+    """The call under a limit of that much more device memory than is in use."""
+    torch.cuda.empty_cache()
+    room += torch.cuda.memory_reserved()
+    torch.cuda.set_per_process_memory_fraction(room / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        return what()
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+
+
+def test_codes_give_way_to_the_forwards_scratch():
+    """4.7 MB, from a segment of 20 MB, under a limit that results and codes alone would fill."""
+    call, leaves, g, codes = layer((32, 16, 32, 32), 128, 7)
+    before, segment = requested_bytes(), 2 ** 21
+    out = within((-(-g.numel() * 4 // segment) - (-codes // segment)) * segment + 2 ** 20, call)
+    assert requested_bytes() - before < codes
+    assert torch.equal(out, call())
+
+
+def test_codes_give_way_to_the_gradients():
+    """The image's gradient, 17 MB, under a limit that leaves no room beside the codes; after that a second backward, which walks."""
+    torch.cuda.empty_cache()
+    call, leaves, g, codes = layer((64, 16, 64, 64), 16, 5)
+    expected = torch.autograd.grad(call(), leaves, g)
+    torch.cuda.empty_cache()
+    out = call()
+    torch.cuda.empty_cache()
+    held = requested_bytes()
+    assert torch.cuda.memory_reserved() - held < leaves[0].numel() * 4  # (else the gradient fits into what is cached)
+    got = within(2 ** 20, lambda: torch.autograd.grad(out, leaves, g, retain_graph=True))
+    assert requested_bytes() < held  # the codes are gone
+    for grads in (got, torch.autograd.grad(out, leaves, g)):
+        for a, b in zip(grads, expected):  # sums in another order, the bar of the module's cases
+            assert (a - b).norm() <= 1e-5 * b.norm()
