@@ -5,6 +5,10 @@
 #include <c10/core/DeviceGuard.h>
 
 #include <algorithm>
+#include <array>
+#include <atomic>
+#include <limits>
+#include <memory>
 #include <sstream>
 
 #include "hingetree_cpp_ops.h"
@@ -538,6 +542,27 @@ struct ConvCall {
 
 }  // namespace
 
+// Memory for what a forward keeps, or an undefined tensor.  All forwards on a device together hold at most as much as one backward
+// that walks may take for its codes, however many layers there are: each such tensor counts until it is freed.
+static torch::Tensor kept_codes(int64_t bytes, const torch::Tensor &like) {
+  static std::array<std::atomic<int64_t>, std::numeric_limits<c10::DeviceIndex>::max() + 1> held_on;  // (zero)
+  constexpr int64_t kMostKept = (int64_t)8 << 30;
+  std::atomic<int64_t> &held = held_on.at((size_t)like.device().index());
+  const int64_t together = held += bytes;
+  const std::shared_ptr<void> share(nullptr, [&held, bytes](void *) { held -= bytes; });
+  if (together > kMostKept || !may_keep(together)) return torch::Tensor();
+  try {
+    const torch::Tensor memory = make_workspace((size_t)bytes, like);
+    return at::for_blob(memory.data_ptr(), memory.sizes())
+        .deleter([memory, share](void *) {})
+        .target_device(like.device())
+        .options(memory.options())
+        .make_tensor();
+  } catch (const c10::OutOfMemoryError &) {
+    return torch::Tensor();
+  }
+}
+
 torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor thr, torch::Tensor ord, torch::Tensor w,
                            std::vector<int64_t> kernel, std::vector<int64_t> stride, std::vector<int64_t> padding,
                            std::vector<int64_t> dilation, torch::Tensor *kept) {
@@ -546,14 +571,8 @@ torch::Tensor conv_forward(int kind, int dims, torch::Tensor x, torch::Tensor th
   torch::Tensor out = fresh(call.out_sizes, x);
   torch::Tensor ws = make_workspace(ht_conv_workspace_bytes(&call.problem), x);  // before what the call can do without
   if (kept != nullptr && x.scalar_type() == torch::kFloat32) {
-    constexpr int64_t kMostKept = (int64_t)8 << 30;  // as much as the codes of a backward that walks may take
     const int64_t bytes = (int64_t)ht_conv_saved_bytes(&call.problem);
-    if (bytes > 0 && bytes <= kMostKept && may_keep(bytes)) {
-      try {
-        *kept = make_workspace((size_t)bytes, x);
-      } catch (const c10::OutOfMemoryError &) {
-      }
-    }
+    if (bytes > 0) *kept = kept_codes(bytes, x);
   }
   OrdinalGuard og(ord, call.window_cells);
   if (kept != nullptr && kept->defined()) {

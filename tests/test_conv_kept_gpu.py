@@ -130,6 +130,26 @@ def test_a_backward_gives_back_what_the_forward_kept():
     assert requested_bytes() - before <= 2 * out.numel() * 4 + sum(t.numel() * 4 for t in first)
 
 
+def test_layers_together_keep_no_more_than_the_limit():
+    from hingetreefortorch_b200._ext import hingetree_cpp as ext
+    call, leaves, g, codes = layer()
+    expected = torch.autograd.grad(call(), leaves, g)
+    ext.set_backward_scratch_limit(2 * codes + codes // 2)
+    try:
+        before = requested_bytes()
+        stack = [call() for _ in range(4)]
+        assert 2 * codes <= requested_bytes() - before - 4 * g.numel() * 4 < 3 * codes
+        for out in stack + [call()]:  # the last one keeps its codes again
+            for a, b in zip(torch.autograd.grad(out, leaves, g), expected):
+                assert (a - b).norm() <= 1e-5 * b.norm()
+        before = requested_bytes()
+        out = call()
+        assert requested_bytes() - before >= codes
+        del out, stack
+    finally:
+        ext.set_backward_scratch_limit(2 ** 62)
+
+
 def within(room, what):
     """The call under a limit of that much more device memory than is in use."""
     torch.cuda.empty_cache()
