@@ -39,7 +39,7 @@ struct CodesPlan {
   size_t smem;
 };
 
-bool make_plan(const ConvTileProblem &p, CodesPlan &plan) {
+bool find_plan(const ConvTileProblem &p, CodesPlan &plan) {
   plan.flat = p.Ho == 1 && p.H == 1 && p.kh == 1;
   plan.record = rows_layout(p.kind, p.depth);
   plan.trees = 1;
@@ -74,6 +74,8 @@ bool make_plan(const ConvTileProblem &p, CodesPlan &plan) {
       }
   return largest != 0 && plan.smem <= kSmemBudget;
 }
+
+bool make_plan(const ConvTileProblem &p, CodesPlan &plan) { return plan_at_hand(p, plan, find_plan); }
 
 struct CodesArgs {
   const float *x, *g;

@@ -16,7 +16,6 @@
 // 3.58.
 #include "ht_conv_rows.cuh"
 
-#include <cstring>
 #include <type_traits>
 
 namespace ht {
@@ -87,20 +86,7 @@ bool find_plan(const ConvTileProblem &p, RowsPlan &plan) {
   return best != 0.0 && plan.smem <= kSmemBudget;
 }
 
-// A call asks for its plan several times (scratch, what is kept, the launch): the last one is at hand (3 us to find one).
-bool make_plan(const ConvTileProblem &p, RowsPlan &plan) {
-  static_assert(std::has_unique_object_representations<ConvTileProblem>::value, "compared byte by byte");
-  thread_local ConvTileProblem last = {};
-  thread_local RowsPlan found = {};
-  thread_local bool known = false, takes = false;
-  if (!known || std::memcmp(&last, &p, sizeof p) != 0) {
-    takes = find_plan(p, found);
-    last = p;
-    known = true;
-  }
-  plan = found;
-  return takes;
-}
+bool make_plan(const ConvTileProblem &p, RowsPlan &plan) { return plan_at_hand(p, plan, find_plan); }
 
 struct RowsArgs {
   const float *x;

@@ -3,6 +3,7 @@ import ctypes
 import glob
 import os
 import re
+import threading
 
 from conftest import ROOT
 from hingetreefortorch_b200 import _build, _cabi
@@ -48,3 +49,26 @@ def test_workspace_query_and_argument_screening():
     assert rc == -1
     rc = lib.ht_forest_forward_f32(None, None, None, None, None, None, None, ctypes.c_size_t(0), None, None)
     assert rc == -1
+
+
+def test_convolution_plans_at_hand_are_those_of_the_question():
+    """Sizes asked for in turn, and each in a thread of its own, which has no earlier plan at hand: the same answers."""
+    lib = _cabi.library()
+    lib.ht_conv_saved_bytes.restype = lib.ht_conv_workspace_bytes.restype = ctypes.c_size_t
+    t = _cabi._triple
+    problems = [_cabi.ConvProblem(kind, depth, 2, 0, 4, ci, co, 1, t((h, h), 1), t((k, k), 1), t((1, 1), 1), t((p, p), 0), t((1, 1), 1))
+                for kind, depth, ci, co, h, k, p in [(0, 5, 64, 128, 64, 3, 1), (1, 5, 64, 128, 64, 3, 1), (0, 7, 8, 16, 128, 3, 1),
+                                                     (0, 4, 3, 64, 224, 5, 2), (0, 7, 8, 16, 128, 5, 2), (0, 5, 2, 2, 8, 3, 1)]]
+
+    def sizes(p):
+        return lib.ht_conv_saved_bytes(ctypes.byref(p)), lib.ht_conv_workspace_bytes(ctypes.byref(p))
+
+    alone = []
+    for p in problems:
+        thread = threading.Thread(target=lambda p=p: alone.append(sizes(p)))
+        thread.start()
+        thread.join()
+    assert [a[0] > 0 for a in alone] == [True, True, True, True, False, False]
+    for order in (range(len(problems)), reversed(range(len(problems)))):
+        for k in order:
+            assert sizes(problems[k]) == alone[k] == sizes(problems[k])
