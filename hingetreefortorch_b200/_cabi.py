@@ -20,7 +20,7 @@ HT_FLAG_PIPELINE_TIMEOUT = 0x80000000  # a bounded wait inside a kernel ran out:
 
 # every symbol include/hingetree_b200.h declares (checked by the CPU test-suite)
 SYMBOLS = [
-    "ht_version", "ht_status_string", "ht_last_cuda_error", "ht_forest_workspace_bytes", "ht_forest_forward_saves", "ht_launch_count", "ht_selftest_bounded_wait",
+    "ht_version", "ht_status_string", "ht_last_cuda_error", "ht_forest_workspace_bytes", "ht_forest_forward_saves", "ht_forest_forward_kernel", "ht_launch_count", "ht_selftest_bounded_wait",
     "ht_forest_forward_f32", "ht_forest_leafmap_f32", "ht_forest_marginmap_f32",
     "ht_forest_reachability_f32", "ht_forest_backward_f32",
     "ht_forest_forward_f64", "ht_forest_leafmap_f64", "ht_forest_marginmap_f64", "ht_forest_reachability_f64",

@@ -472,24 +472,33 @@ static bool ordered_from_paths(const ht_forest_problem *p) {
   return (p->flags & HT_DETERMINISTIC) != 0 && (p->M > 1 || p->B * p->T * p->K <= (1 << 26)) && ordered_list_bytes(p, sizeof(float)) > 0;
 }
 
-// Whether the walk goes past resident trees row by row (ht_forest_rows.cu) rather than past resident tiles of samples or with a
-// thread per evaluation: where the estimates, all three of single calls on cold caches, have it cheaper by 10 %.  It is for samples of
-// many features, which leave room for small tiles only, and for batches that give few tiles.  How good the choice is, on 1104
-// forwards of random sizes timed every way (profiles/forward_kernel_choice.csv):
-//   * against the tile kernel (808 of them) it costs 1.3 % over the better of the two on average and more than 20 % in 18 cases;
-//     always tiles 9.4 %, always rows 25 %; with no margin it costs 1.1 %, but calls in a loop, on warm caches, gain from tiles what
-//     the estimates do not know (12407 x 342, 34 trees of depth 8, 26 outputs: a ratio of 0.905, a training step of 88 against 82 us);
-//   * against a thread per evaluation (296) 3 % (trees) and 0.4 % (ferns); never taking rows 6.2 and 2.6 %.
-// `keep`: the paths leave, too.
+// Microseconds of a single forward on cold caches with a thread per evaluation (tabular data).  A warp's lanes are on 32 trees, so a
+// level whose vertices of all trees (8 bytes each) do not fit the 128 KB of L1 that x leaves them costs gathers from L2, three and a
+// half times a level in L1.  Long calls turn on that term: with it the logarithm of estimate over time has a spread of 0.12 above
+// 100 us, without it 0.20.  (A fern's decisions lie together, and do fit.)  `keep`: the paths leave, too.
+static double thread_forward_cost(const ht_forest_problem *p, bool keep) {
+  int near = p->kind == FERN ? p->depth : 0;
+  while (near < p->depth && p->T * 8 * ((((int64_t)2) << near) - 1) <= 128 * 1024) ++near;
+  const double evals = (double)p->B * (double)p->T;
+  return 11.5 + evals * ((p->kind == FERN ? 1.87e-6 : 2.67e-6) * p->depth + 6.92e-6 * (p->depth - near) + 0.583e-6 * (double)p->M + (keep ? 14.4e-6 : 0.0)) +
+         0.392e-6 * (double)p->B * (double)p->C;
+}
+
+// Whether the walk goes past resident trees row by row (ht_forest_rows.cu) rather than past resident tiles of samples or, where the
+// tile kernel does not take the sizes, with a thread per evaluation: where its estimate is the lower one.  It is for samples of many
+// features, which leave room for small tiles only, and for batches that give few tiles.  The three estimates are fits to 1904 forwards
+// of random sizes, all timed all ways in one session (profiles/forward_kernel_choice.csv), with residuals weighed so that long calls
+// count: absolute over time to the power 3/4.  Time of the chosen kernels over that of the better ones, all calls together (always
+// rows, never rows), and chosen for those above 100 us alone:
+//   * beside the tile kernel, 808 trees 1.003 (1.51, 1.06), 1.001; 423 ferns 1.005 (1.45, 1.08), 1.003;
+//   * beside a thread per evaluation, 441 trees 1.007 (1.15, 1.35), 1.007; 232 ferns 1.026 (1.15, 1.12), 1.027.
+// Calls in a loop, on warm caches, give 1.002, 1.004, 1.007 and 1.027.  No margin: one of 10 % costs 1.006, 1.010, 1.016 and 1.028.
 static bool rows_are_better(const ht_forest_problem *p, bool keep) {
   if (p->B * p->T < 32768) return false;
   const double rows = rows_forward_cost(p);
   if (rows < 0.0) return false;
-  double other = forward_tiled_cost(p);
-  if (other < 0.0)
-    other = 10.8 + (double)(p->B * p->T) * ((p->kind == FERN ? 2.0e-6 : 4.3e-6) * p->depth + 0.74e-6 * (double)p->M + (keep ? 16.2e-6 : 0.0)) +
-            0.31e-6 * (double)p->B * (double)p->C;
-  return rows < 0.9 * other;
+  const double tiles = forward_tiled_cost(p);
+  return rows < (tiles < 0.0 ? thread_forward_cost(p, keep) : tiles);
 }
 
 // What a backward keeps per evaluation: the records of the tile kernels (one output per leaf), or the paths (several) and,
@@ -505,6 +514,14 @@ static size_t records_without_lists(const ht_forest_problem *p) { return p->M ==
 int ht_forest_forward_saves(const ht_forest_problem *p) {
   if (check_forest_problem(p) != HT_OK) return 0;
   return p->M == 1 ? forward_saves(p) : records_bytes(p) > 0;
+}
+
+int ht_forest_forward_kernel(const ht_forest_problem *p) {
+  const int rc = check_forest_problem(p);
+  if (rc != HT_OK) return rc;
+  const bool keep = (p->flags & HT_SAVE_FOR_BACKWARD) != 0 && ht_forest_forward_saves(p);
+  if (rows_are_better(p, keep)) return HT_FORWARD_ROWS;
+  return forward_tiled_workspace_bytes(p) > 0 ? HT_FORWARD_TILES : HT_FORWARD_THREADS;
 }
 
 size_t ht_forest_workspace_bytes(const ht_forest_problem *p) {

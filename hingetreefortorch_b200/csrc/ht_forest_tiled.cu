@@ -664,16 +664,17 @@ size_t forward_tiled_workspace_bytes(const ht_forest_problem *p) {
 
 // Rounds of CTAs, each staging its tile and walking its share of the tree groups; one, two or four trees per warp at once
 // differ in what a group costs (few in flight leave the shared memory's latency in the open).  Fitted like
-// rows_forward_cost(): single calls on cold caches, spread 0.12.
+// rows_forward_cost(): single calls on cold caches, spread 0.09.
 double forward_tiled_cost(const ht_forest_problem *p) {
   TilePlan plan;
   if (!make_plan(p, plan)) return -1.0;
   const int64_t tiles = (p->B + plan.S - 1) / plan.S, groups = (p->T + plan.G - 1) / plan.G;
   const int splits = choose_splits(tiles, groups);
   const double waves = (double)((tiles * splits + 147) / 148), per_cta = (double)((groups + splits - 1) / splits);
-  const double level = plan.per_warp == 1 ? 0.036 : plan.per_warp == 2 ? 0.108 : 0.207;
-  return 10.9 + waves * (1.3 + 1.77e-4 * plan.S * (double)p->C +
-                         per_cta * (1.37 + level * p->depth + (!plan.weights ? 0.95e-4 * plan.G * plan.S * (double)p->M : 0.0)));
+  const double level = plan.per_warp == 1 ? 0.0167 : plan.per_warp == 2 ? 0.0681 : 0.141;
+  const double output = plan.weights ? 0.0 : 0.0293e-3 + 0.181e-3 / vector_width(p->M, sizeof(float), {});
+  return 11.1 + waves * (1.45 + 0.177e-3 * plan.S * (double)p->C +
+                         per_cta * (1.37 + level * p->depth + output * plan.G * plan.S * (double)p->M));
 }
 
 bool forward_saves(const ht_forest_problem *p) {

@@ -98,6 +98,12 @@ size_t ht_forest_workspace_bytes(const ht_forest_problem *p);
  * HT_DETERMINISTIC the sums are the reference's, bit for bit, as without saving. */
 int ht_forest_forward_saves(const ht_forest_problem *p);
 
+/* Which kernel ht_forest_forward_f32 takes for a problem (with HT_SAVE_FOR_BACKWARD: the forward that saves), x and out on 16-byte
+ * boundaries: a thread per evaluation, tiles of samples in shared memory with the trees streaming past, or trees in shared memory
+ * with rows of x streaming past.  The results are the same bits. */
+enum { HT_FORWARD_THREADS = 0, HT_FORWARD_TILES = 1, HT_FORWARD_ROWS = 2 };
+int ht_forest_forward_kernel(const ht_forest_problem *p);
+
 /* out[i,j,k,m] = |margin(i,j,k)| * w[j, leaf(i,j,k), m]
  * Replaces hingetree_gpu_forward / ForwardKernel (hingetree_gpu.cu:416-498, 58-87) and the
  * traversal templates it instantiates (HingeTreeCommon.cuh:60-79 fern, 133-154 tree). */
