@@ -1,5 +1,9 @@
 // Shared-memory tile kernel for the forward of 1-D / 2-D convolutional hinge trees and ferns
-// (one output per leaf), where ht_conv_rows.cu does not take the problem: trees of one level or of more than seven.
+// (one output per leaf), where ht_conv_rows.cu does not take the problem: trees of one level or of more than seven; and, whatever the
+// depth, strides or windows so large that the pixels under four rows of outputs do not fit beside the records (or lie too far
+// apart for these) while those under one row do, for all input channels.  What that is worth there depends on the sizes: 8 x 8 windows 40
+// x 16 apart on [8, 2, 1024, 1024], 512 trees of depth 5: 172 us, 310 with a thread per output; 1 x 8 windows 64 x 16 apart on
+// [64, 1, 1024, 1024], 64 trees of depth 4: 215 against 103.
 //
 // out[b, j, p] = sum over input channels c (ascending) of tree (j, c) evaluated on the kernel
 // window of channel c at output position p.  Work decomposition (one CTA of 1024 threads per SM):

@@ -41,6 +41,9 @@ CONV_CASES = [
     # kernel collects the parameter gradients in its shared bins as well
     (2, (2, 8, 48, 64), 24, 7, (), (3, 3), (1, 1), (1, 1), (1, 1)),
     (2, (2, 8, 48, 64), 24, 8, (), (3, 3), (1, 1), (1, 1), (1, 1)),
+    # shallow trees that only the tile kernel's single row of outputs has room for: window offsets of two bytes and of one
+    (2, (2, 1, 256, 1024), 512, 7, (), (16, 16), (16, 16), (0, 0), (1, 1)),
+    (2, (16, 1, 1024, 1024), 64, 4, (), (1, 8), (64, 16), (0, 0), (1, 1)),
 ]
 
 
