@@ -6,7 +6,7 @@ import pytest
 import torch
 
 import hingetreefortorch_b200._cabi as _cabi
-from conftest import grad_close, requested_bytes
+from conftest import grad_close, grad_same, requested_bytes
 from oracle import hinge_oracle as ho
 from test_conv_gpu import dev
 
@@ -55,11 +55,22 @@ def test_forward_and_backward_from_kept_codes(kind, case):
         for wanted, got, r, s in zip(need, conv.backward_saved(*tensors, kept, need=need), ref, sizes):
             assert (got is None) if not wanted else grad_close(got, r, s)
     assert int(conv.status.item()) == 0
+    # infinite pixels and one that is no number, in the first channels; the upstream gradient too
     x.reshape(-1)[:3] = [np.inf, -np.inf, np.nan]
-    dx = dev(x)[0]
-    want = ho.conv_forward(kind, x, thr, ord_, w, *geometry)
+    g.reshape(-1)[[0, 5]] = [np.inf, np.nan]
+    dx, dg = dev(x, g)
+    with np.errstate(all="ignore"):
+        want = ho.conv_forward(kind, x, thr, ord_, w, *geometry)
+        ref = ho.conv_backward(kind, x, thr, ord_, w, g, *geometry)
+        sizes = ho.magnitudes(ho.conv_backward, kind, x, thr, ord_, w, g, *geometry)
+    assert not all(np.isfinite(r).all() for r in ref) and all(np.isfinite(r).any() for r in ref)
     assert np.array_equal(conv.forward(dx, *tensors[1:4]).cpu().numpy(), want, equal_nan=True)
-    assert np.array_equal(conv.forward_saving(dx, *tensors[1:4])[0].cpu().numpy(), want, equal_nan=True)
+    out, kept = conv.forward_saving(dx, *tensors[1:4])
+    assert np.array_equal(out.cpu().numpy(), want, equal_nan=True)
+    for grads in (conv.backward_saved(dx, *tensors[1:4], dg, kept), conv.backward(dx, *tensors[1:4], dg)):
+        for got, r, s in zip(grads, ref, sizes):
+            assert grad_same(got, r, s)
+    assert int(conv.status.item()) == 0
 
 
 def test_codes_without_room_for_the_height_are_not_kept():

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from conftest import grad_close, random_forest_inputs, requested_bytes
+from conftest import grad_close, grad_same, random_forest_inputs, requested_bytes
 from oracle import hinge_oracle as ho
 
 pytestmark = pytest.mark.gpu
@@ -215,6 +215,20 @@ def test_rows_past_resident_trees(case):
     got = fam.linear_forward(dx, None, dthr, dord, dw, dlin, dbias).cpu().numpy()
     with np.errstate(all="ignore"):
         assert np.array_equal(got, ho.linear_forward(kind, x, thr, ord_, w, lin, bias), equal_nan=True)
+    assert fam.status.item() == 0
+    # Gradients, the upstream one infinite and no number in places.  One linear output: with several their gradients are summed before
+    # they meet the margin, and an infinite margin stays one where the reference's terms of opposite signs leave no number.
+    lin, g = lin[:1].copy(), rng.standard_normal((B, 1)).astype(np.float32)
+    g[B // 2], g[B // 3] = np.inf, np.nan
+    dlin, dg = dev(lin, g)
+    with np.errstate(all="ignore"):
+        ref = ho.linear_backward(kind, x, thr, ord_, w, lin, g)
+        sizes = ho.magnitudes(ho.linear_backward, kind, x, thr, ord_, w, lin, g)
+    assert not np.isfinite(ref[0]).all() and np.isfinite(ref[0]).any()
+    fam = _cabi.ForestFamily(kind, dx, dw, lin=dlin)
+    gx, _, gthr, gw, glin = fam.linear_backward(dx, None, dthr, dord, dw, dlin, dg)
+    for grad, r, s in zip((gx, gthr, gw, glin), ref, sizes):
+        assert grad_same(grad, r, s)
     assert fam.status.item() == 0
 
 
