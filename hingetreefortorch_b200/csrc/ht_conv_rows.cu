@@ -3,8 +3,8 @@
 // out[b, j, p] = sum over input channels c (ascending) of tree (j, c) evaluated on the kernel window of channel c at output
 // position p.  A CTA owns a tile of output positions of one sample and holds the pixels under it in shared memory, for as many
 // input channels at a time as fit.  A warp is (four or eight rows, one output channel) and walks ONE tree at four rows x 32
-// columns at a time: the entries of the root and of its children serve all four, and where the backward wants the paths, four
-// rows' codes make one 8-byte store.  Every warp has a ring of records of its own, filled by bulk copies, and waits for no other
+// columns at a time: the root's entry serves all four, and its children's where no codes are left; where the backward wants the
+// paths, four rows' codes make one 8-byte store.  Every warp has a ring of records of its own, filled by bulk copies, and waits for no other
 // warp but where pixels are staged.  The sums of an output go to memory and back between two lots of input channels.  Outputs
 // of a single row are taken as rows of 32 columns.
 //

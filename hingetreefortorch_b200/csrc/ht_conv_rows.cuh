@@ -136,8 +136,8 @@ __device__ __forceinline__ uint32_t opaque(uint32_t known) {
 }
 
 // Walks the tree at `rec` on four windows: value[u] = |least margin| * leaf weight, and with CODES the evaluation's code.
-// The root and its children, the same for all windows, are loaded once for the four; another vertex's threshold and offset come
-// in one load from the address that the path makes.
+// The root's entry, the same for all windows, is loaded once for the four, and without CODES its children's are; another vertex's
+// threshold and offset come in one load from the address that the path makes.
 // Window u's origin is x_addr + u * row_bytes; ROW_BYTES, if not 0, says how many those are and joins the loads' immediates.
 template <int KIND, int DEPTH, bool CODES, uint32_t ROW_BYTES>
 __device__ __forceinline__ void walk_rows(uint32_t rec, uint32_t x_addr, uint32_t row_bytes, uint32_t eight, float (&value)[4],

@@ -46,7 +46,7 @@ bool make_row_plan(const ht_forest_problem *p, RowPlan &plan, bool outputs = tru
   if (p->K != 1 || p->M < 1 || p->M > 64 || p->C > 65536 || p->depth > 12 || p->T < 1 || p->B < 1 || p->B > 0x7fffffff || p->T > 0x7fffff) return false;
   const int64_t N = threshold_count(p->kind, p->depth);
   for (int rows = 16; rows >= 4; rows /= 2) {
-    // as many trees as fit, but groups of the same size; a warp walks 32 trees at a time
+    // as many trees as fit, but groups of the same size
     int64_t fit = 0;
     for (int64_t groups = 1; groups <= p->T; ++groups) {
       fit = (p->T + groups - 1) / groups;
@@ -61,8 +61,9 @@ bool make_row_plan(const ht_forest_problem *p, RowPlan &plan, bool outputs = tru
       // A copy takes longer to arrive than a step takes to walk: what room is left goes to more copies under way.
       while (plan.buffers < kMostBuffers && row_smem(N, p->C, rows, (int)fit, plan.buffers + 1, outputs) <= kSmemBudget) ++plan.buffers;
       plan.smem = row_smem(N, p->C, rows, (int)fit, plan.buffers, outputs);
-      // A step lasts as long as its busiest warp: as many warps as give all the same number of sets of trees (262144 x 784, 100
-      // trees, 50 sets: 25 warps walk two each: 215 us; 234 with 24, two of which walk three).
+      // A step lasts as long as its busiest warp: as few warps as give all the same number of sets of trees.  262144 x 784, 100
+      // trees, 50 sets: 25 warps walk two each, 204 us; 263 with 20 and 284 with 24 (some walk three), 217 with 28.  Over 16 sizes and
+      // every count from 12 to 28 the rule takes at most 5 % more than the best count, 2 % on average (profiles/conv_rows_codes_ncu.md).
       const int sets = (int)((fit + 32 / rows - 1) / (32 / rows)), rounds = (sets + kAtOnce * kMostWalkers - 1) / (kAtOnce * kMostWalkers);
       plan.walkers = sets <= kMostWalkers ? std::max(sets, 16) : (sets + kAtOnce * rounds - 1) / (kAtOnce * rounds);
       return true;
@@ -86,13 +87,14 @@ struct RowArgs {
 };
 
 // CTA (one per SM) = a group of trees and a slice of the rows.  A step is `rows` rows; a warp's lanes are those rows on 32 / rows
-// trees, and it walks up to four such sets of trees at once.  Rows are copied as they lie, so features are gathered at random
+// trees, and it walks up to two such sets of trees at once.  Rows are copied as they lie, so features are gathered at random
 // banks (3.4 wavefronts for 32 lanes on average where the vertices differ), but lanes on one tree share its thresholds and
 // feature indices, nothing is transposed and the copies run under the walk.  The paths leave from registers, runs of consecutive
 // samples; outputs through a staging area.
-// Bound by shared-memory wavefronts.  262144 x 784, 100 trees of depth 7: 215 us, 4.5 TB/s and 64 % of the wavefronts (358 with 32 trees on one row per warp, whose
-// thresholds and indices lay at random banks as well; 608 with a thread per evaluation gathering through L1).
-// HEADS: a lane meets the same (up to four) trees in every step, so their roots' and the roots' children's decisions, two of
+// Bound by shared-memory wavefronts and the rows' arrival.  262144 x 784, 100 trees of depth 7, paths only: 204 us, 4.8 TB/s (358 with
+// 32 trees on one row per warp, whose thresholds and indices lay at random banks as well; 608 with a thread per evaluation gathering
+// through L1).
+// HEADS: a lane meets the same (one or two) trees in every step, so their roots' and the roots' children's decisions, two of
 // the levels, stay in registers.
 // DEPTH: of the trees, 0 for any.
 template <int KIND, int DEPTH, typename WhereT, bool HEADS>
