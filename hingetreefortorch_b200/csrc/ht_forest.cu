@@ -473,15 +473,16 @@ static bool ordered_from_paths(const ht_forest_problem *p) {
 }
 
 // Microseconds of a single forward on cold caches with a thread per evaluation (tabular data).  A warp's lanes are on 32 trees, so a
-// level whose vertices of all trees (8 bytes each) do not fit the 128 KB of L1 that x leaves them costs gathers from L2, three and a
-// half times a level in L1.  Long calls turn on that term: with it the logarithm of estimate over time has a spread of 0.12 above
-// 100 us, without it 0.20.  (A fern's decisions lie together, and do fit.)  `keep`: the paths leave, too.
+// level whose vertices of all trees (8 bytes each) do not fit the 128 KB of L1 that x leaves them costs gathers from L2, three to four
+// times a level in L1; wide rows leave L1 the sooner.  Long calls turn on the first term: with it the logarithm of estimate over time
+// has a spread of 0.12 above 100 us, without it 0.20, with both 0.105.  (A fern's decisions lie together, and do fit.)  `keep`: the paths leave, too.
 static double thread_forward_cost(const ht_forest_problem *p, bool keep) {
   int near = p->kind == FERN ? p->depth : 0;
   while (near < p->depth && p->T * 8 * ((((int64_t)2) << near) - 1) <= 128 * 1024) ++near;
   const double evals = (double)p->B * (double)p->T;
-  return 11.5 + evals * ((p->kind == FERN ? 1.87e-6 : 2.67e-6) * p->depth + 6.92e-6 * (p->depth - near) + 0.583e-6 * (double)p->M + (keep ? 14.4e-6 : 0.0)) +
-         0.392e-6 * (double)p->B * (double)p->C;
+  return 11.6 + evals * (((p->kind == FERN ? 1.22e-6 : 2.26e-6) + 0.262e-9 * (double)p->C) * p->depth + 7.07e-6 * (p->depth - near) +
+                         0.565e-6 * (double)p->M + (keep ? 13.8e-6 : 0.0)) +
+         0.359e-6 * (double)p->B * (double)p->C;
 }
 
 // Whether the walk goes past resident trees row by row (ht_forest_rows.cu) rather than past resident tiles of samples or, where the
@@ -490,9 +491,9 @@ static double thread_forward_cost(const ht_forest_problem *p, bool keep) {
 // of random sizes, all timed all ways in one session (profiles/forward_kernel_choice.csv), with residuals weighed so that long calls
 // count: absolute over time to the power 3/4.  Time of the chosen kernels over that of the better ones, all calls together (always
 // rows, never rows), and chosen for those above 100 us alone:
-//   * beside the tile kernel, 808 trees 1.003 (1.51, 1.06), 1.001; 423 ferns 1.005 (1.45, 1.08), 1.003;
-//   * beside a thread per evaluation, 441 trees 1.007 (1.15, 1.35), 1.007; 232 ferns 1.026 (1.15, 1.12), 1.027.
-// Calls in a loop, on warm caches, give 1.002, 1.004, 1.007 and 1.027.  No margin: one of 10 % costs 1.006, 1.010, 1.016 and 1.028.
+//   * beside the tile kernel, 808 trees 1.002 (1.51, 1.06), 1.001; 423 ferns 1.005 (1.45, 1.08), 1.003;
+//   * beside a thread per evaluation, 441 trees 1.003 (1.15, 1.35), 1.002; 232 ferns 1.021 (1.15, 1.12), 1.022.
+// Calls in a loop, on warm caches, give 1.002, 1.004, 1.003 and 1.022.  No margin: one of 10 % costs 1.006, 1.008, 1.010 and 1.025.
 static bool rows_are_better(const ht_forest_problem *p, bool keep) {
   if (p->B * p->T < 32768) return false;
   const double rows = rows_forward_cost(p);

@@ -427,10 +427,10 @@ static int row_slices(const ht_forest_problem *p, const RowPlan &plan) {
 }
 
 // Microseconds of a single call on cold caches: rounds of CTAs, each of them steps x (levels of the sets of trees walked, paths and
-// outputs, the latter by bytes and by the stores they go in, row copies by bytes and by what of them comes from memory rather than
+// outputs, the latter by bytes and by the stores they go in (a third more for these where the leaf weights exceed 10 MB), row copies by bytes and by what of them comes from memory rather than
 // from L2, where groups of trees share the rows) behind the fetch of its parameters.  A fit to profiles/forward_kernel_choice.csv (the
-// logarithm of estimate over time has a spread of 0.13), as are forward_tiled_cost() (0.09) and the estimate for a thread per evaluation
-// (0.14); rows_are_better() says how good the choice between them is.
+// logarithm of estimate over time has a spread of 0.12), as are forward_tiled_cost() (0.09) and the estimate for a thread per evaluation
+// (0.13); rows_are_better() says how good the choice between them is.
 double rows_forward_cost(const ht_forest_problem *p) {
   RowPlan plan;
   if (!make_row_plan(p, plan)) return -1.0;
@@ -440,10 +440,11 @@ double rows_forward_cost(const ht_forest_problem *p) {
   const int per_set = 32 / plan.rows, sets = (plan.trees + per_set - 1) / per_set;
   const int rounds = (sets + kAtOnce * kMostWalkers - 1) / (kAtOnce * kMostWalkers);
   const double paths = (double)plan.rows * plan.trees, outputs = paths * (double)p->M;
-  return 13.6 + waves * (steps * (0.42 + (2.45e-3 * sets + 0.0711 * rounds) * p->depth + 0.321e-3 * paths +
-                                  (0.0437e-3 + 0.328e-3 / vector_width(p->M, sizeof(float), {})) * outputs +
-                                  (0.0118e-3 + 0.027e-3 * slices / 148.0) * plan.rows * (double)p->C) +
-                         0.713e-3 * plan.trees * (double)threshold_count(p->kind, p->depth));
+  const bool far_leaves = (double)p->T * (double)(((int64_t)1) << p->depth) * (double)p->M > 2.5e6;
+  return 13.7 + waves * (steps * (0.446 + (2.34e-3 * sets + 0.0675 * rounds) * p->depth + 0.369e-3 * paths +
+                                  (0.0356e-3 + (far_leaves ? 0.444e-3 : 0.329e-3) / vector_width(p->M, sizeof(float), {})) * outputs +
+                                  (0.0112e-3 + 0.0276e-3 * slices / 148.0) * plan.rows * (double)p->C) +
+                         0.71e-3 * plan.trees * (double)threshold_count(p->kind, p->depth));
 }
 
 bool rows_forward_takes(const ht_forest_problem *p) {

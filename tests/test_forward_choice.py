@@ -29,7 +29,7 @@ def test_the_table_says_what_the_library_chooses():
 @pytest.mark.parametrize("column", ["", "_loop"], ids=["cold caches", "in a loop"])
 def test_long_and_short_forwards_take_the_kernel_that_costs_less(column):
     """By the time that calls cost, not by their number: together within 1 % of the better kernel, those above 100 us as well, and
-    no kind beyond 3 % of the better of its two kernels."""
+    no kind beyond 2.5 % of the better of its two kernels."""
     total = {}
     for row in forwards():
         other = "tile" if row["tile"] else "thread"
@@ -42,7 +42,7 @@ def test_long_and_short_forwards_take_the_kernel_that_costs_less(column):
             total[group] = (chosen + times[row["takes"]], least + best)
     ratios = {group: chosen / least for group, (chosen, least) in total.items()}
     assert ratios["all",] < 1.01 and ratios["long",] < 1.01, ratios
-    assert max(ratios.values()) < 1.03, ratios
+    assert max(ratios.values()) < 1.025, ratios
 
 
 @pytest.mark.parametrize("B,C,T,depth,M", [(3146, 1194, 616, 8, 8), (3334, 1212, 718, 7, 16), (1716, 1173, 791, 7, 16),
