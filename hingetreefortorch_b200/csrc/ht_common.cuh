@@ -196,6 +196,8 @@ struct Divisor {
     factor = (uint32_t)(((1ull << (31 + shift)) + d - 1) / d);  // ceil(2^(31 + shift) / d), 2^31 <= factor < 2^32
   }
   __device__ __forceinline__ uint32_t quotient(uint32_t n) const { return (uint32_t)(((uint64_t)n * factor) >> (31 + shift)); }
+  // the same for divisors of two and more, from the product's upper half alone
+  __device__ __forceinline__ uint32_t quotient_above_one(uint32_t n) const { return __umulhi(n, factor) >> (shift - 1); }
 };
 
 // Memory to be zeroed before the kernels of a call add into it.

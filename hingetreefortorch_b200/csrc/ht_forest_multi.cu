@@ -15,20 +15,55 @@ namespace {
 
 constexpr int kForwardThreads = 256;
 constexpr int kSortThreads = 256;
-constexpr uint32_t kSlice = 1024;  // evaluations per CTA
 constexpr int kMaxSortDepth = 12;
 constexpr int64_t kMaxDivisor = 4096;
 
+// p[0 .. V) += v where `now` is set, without a branch.
 template <int V>
-__device__ __forceinline__ void red_add(float *p, const float (&v)[V]) {
-  if constexpr (V == 4) red_add_quad(p, v[0], v[1], v[2], v[3]);
-  else if constexpr (V == 2) red_add_pair(p, v[0], v[1]);
-  else atomicAdd(p, v[0]);
+__device__ __forceinline__ void red_add_if(float *p, const float (&v)[V], bool now) {
+  if constexpr (V == 4)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"l"(p), "f"(v[0]),
+                 "f"(v[1]), "f"(v[2]), "f"(v[3]), "r"((int)now)
+                 : "memory");
+  else if constexpr (V == 2)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t@p red.global.add.v2.f32 [%0], {%1, %2};\n\t}" ::"l"(p), "f"(v[0]),
+                 "f"(v[1]), "r"((int)now)
+                 : "memory");
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p red.global.add.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v[0]), "r"((int)now)
+                 : "memory");
+}
+// base + index without the second instruction that a 64-bit sum of two registers takes
+template <typename Real>
+__device__ __forceinline__ const Real *element(const Real *base, uint32_t index) {
+  uint64_t at;
+  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(at) : "r"(index), "n"((int)sizeof(Real)), "l"(base));
+  return reinterpret_cast<const Real *>(at);
+}
+// r = p[0 .. V) where `now` is set, without a branch
+template <int V>
+__device__ __forceinline__ void load_if(Vec<float, V> &r, const float *p, bool now) {
+  if constexpr (V == 4)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %5, 0;\n\t@p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "+f"(r.v[0]), "+f"(r.v[1]), "+f"(r.v[2]), "+f"(r.v[3])
+                 : "l"(p), "r"((int)now));
+  else if constexpr (V == 2)
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %3, 0;\n\t@p ld.global.nc.v2.f32 {%0, %1}, [%2];\n\t}"
+                 : "+f"(r.v[0]), "+f"(r.v[1])
+                 : "l"(p), "r"((int)now));
+  else
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}" : "+f"(r.v[0]) : "l"(p), "r"((int)now));
 }
 template <int V>
-__device__ __forceinline__ void red_add(double *p, const double (&v)[V]) {
+__device__ __forceinline__ void load_if(Vec<double, V> &r, const double *p, bool now) {
+  if (now) r = load_vec<double, V>(p);
+}
+template <int V>
+__device__ __forceinline__ void red_add_if(double *p, const double (&v)[V], bool now) {
+  if (now) {
 #pragma unroll
-  for (int k = 0; k < V; ++k) atomicAdd(p + k, v[k]);
+    for (int k = 0; k < V; ++k) atomicAdd(p + k, v[k]);
+  }
 }
 
 template <typename Real>
@@ -120,23 +155,30 @@ struct SortedArgs {
   Divisor K;           // positions per sample
   uint32_t P;          // evaluations per tree
   int M, depth, fern, narrow;
-  int exclusive;       // a CTA has all the evaluations of its tree
 };
 
+// CTAs per SM that the registers are shared out for
+template <typename Real>
+__host__ __device__ constexpr int sort_blocks(int numbers) {
+  return numbers * (int)sizeof(Real) > 8 ? 3 : 4;
+}
 // g rows (and rows of weights) in flight per group of lanes, as far as registers go
 template <typename Real>
 __host__ __device__ constexpr int sort_ahead(int numbers) {
   return numbers * (int)sizeof(Real) > 16 ? 2 : 4;
 }
 
-// Turns counts[0 .. size) into the sums of what is before each (a run of them per thread).  All threads of the block.
+// Turns counts[0 .. 4 * quads) into the sums of what is before each.  All threads of the block; partial: a number per warp.
 template <int THREADS>
-__device__ __forceinline__ void exclusive_sums(uint32_t *counts, int size, uint32_t *partial) {
+__device__ __forceinline__ void exclusive_sums(uint4 *counts, int quads, uint32_t *partial) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int per = (size + THREADS - 1) / THREADS;
-  const int first = min(tid * per, size), last = min(first + per, size);
+  const int per = (quads + THREADS - 1) / THREADS;  // 16 bytes each: one up to 1024 numbers
+  const int first = min(tid * per, quads), last = min(first + per, quads);
   uint32_t mine = 0;
-  for (int b = first; b < last; ++b) mine += counts[b];
+  for (int b = first; b < last; ++b) {
+    const uint4 c = counts[b];
+    mine += c.x + c.y + c.z + c.w;
+  }
   uint32_t sum = mine;
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
@@ -146,291 +188,432 @@ __device__ __forceinline__ void exclusive_sums(uint32_t *counts, int size, uint3
   if (lane == 31) partial[warp] = sum;
   __syncthreads();
   uint32_t base = sum - mine;
-  for (int k = 0; k < warp; ++k) base += partial[k];
+#pragma unroll
+  for (int k = 0; k < THREADS / 32 - 1; ++k) base += k < warp ? partial[k] : 0u;
   for (int b = first; b < last; ++b) {
-    const uint32_t count = counts[b];
-    counts[b] = base;
-    base += count;
+    uint4 c = counts[b], before;
+    before.x = base;
+    before.y = before.x + c.x;
+    before.z = before.y + c.y;
+    before.w = before.z + c.z;
+    base = before.w + c.w;
+    counts[b] = before;
   }
   __syncthreads();
 }
 
+// Evaluations per CTA: whole rounds for every group of lanes (three and five lanes per evaluation leave 80 and 48 groups).
+__host__ __device__ constexpr uint32_t sort_slice(int lanes) { return lanes == 3 || lanes == 5 ? 960u : 1024u; }
+
+// Place of the list entries without an evaluation, which fill up the last parts: they read the slice's first g row.
+constexpr uint32_t kNobody = 1024;
+
+// Lanes of three and five leave their parts of D to the evaluation's own thread; others add them up.
+__host__ __device__ constexpr int sort_dots(int lanes) { return (lanes & (lanes - 1)) == 0 ? 1 : lanes; }
+
+// Rows of eight lanes and more: the list holds the places of the g row and of the weights, so that no lane works them out
+// (64 outputs: 56 -> 53 us).  Shorter rows are bound by the shared memory's wavefronts, to which a list of 16-byte entries adds
+// (3 and 10 outputs: 56 us each, 60 with it).
+__host__ __device__ constexpr bool sort_rows_listed(int lanes) { return lanes >= 8; }
+
+// Where the arrays of sorted_backward_kernel lie in its shared memory; the counts, whose number varies, come last.
+struct SortedPlaces {
+  uint32_t sizes, dots, partial, bins;
+};
+__host__ __device__ constexpr SortedPlaces sorted_places(uint32_t real_bytes, int lanes) {
+  SortedPlaces at = {};
+  const uint32_t slice = sort_slice(lanes), entries = slice + (uint32_t)(32 / lanes * (kSortThreads / 32));
+  const uint32_t columns = kMaxSortDepth * kSortThreads * real_bytes;  // of the ferns' thresholds, in the list's place after the walk
+  at.sizes = entries * (sort_rows_listed(lanes) ? 16u : 8u);
+  at.dots = at.sizes + (real_bytes == 4 ? 0u : (entries * real_bytes + 15u) & ~15u);
+  at.dots = at.dots < slice * (real_bytes + 4u) ? slice * (real_bytes + 4u) : at.dots;  // terms and vertices, after the walk as well
+  at.dots = at.dots < columns ? columns : at.dots;
+  at.partial = at.dots + (((kNobody + 1u) * (uint32_t)sort_dots(lanes) * real_bytes + 15u) & ~15u);
+  at.bins = at.partial + ((4u * (kSortThreads / 32) + 15u) & ~15u);
+  return at;
+}
+__host__ __device__ inline int sorted_bin_quads(int L, int N, bool fern) { return (L + (fern ? 0 : N) + 1 + 3) / 4; }
+
+// Sums of dot[0 .. LEFT) over groups of 2 D lanes, D a power of two: lanes hand each other the halves of the list that they drop,
+// as long as there is more than one number, so that sum u ends in the lanes whose upper bits (of the lane in its group) say u.
+// Those bits are appended to `mine`; the lane is left with dot[0 .. LEFT / 2 D), at least one.
+template <int D, int LEFT, typename Real, int A>
+__device__ __forceinline__ void sums_over_lanes(Real (&dot)[A], int q, int &mine) {
+  if constexpr (D >= 1) {
+    if constexpr (LEFT > 1) {
+      const bool upper = (q & D) != 0;
+#pragma unroll
+      for (int u = 0; u < LEFT / 2; ++u) {
+        const Real away = upper ? dot[u] : dot[u + LEFT / 2], kept = upper ? dot[u + LEFT / 2] : dot[u];
+        dot[u] = kept + __shfl_xor_sync(0xffffffffu, away, D);
+      }
+      mine = mine * 2 + (upper ? 1 : 0);
+    } else {
+      dot[0] += __shfl_xor_sync(0xffffffffu, dot[0], D);
+    }
+    sums_over_lanes<D / 2, (LEFT > 1 ? LEFT / 2 : 1)>(dot, q, mine);
+  }
+}
+
 // CTA per (tree, slice of its evaluations).
 //
-// The slice's paths are sorted by leaf, root decision first, by counting in shared memory.  `lanes` lanes share an
-// evaluation (R pieces of V of its M outputs each), and every such group of lanes walks a contiguous part of the list:
-//   * an evaluation of the same leaf as the one before adds |margin| * g to the leaf's sums in registers; only where the
-//     leaf changes do they go to memory, so the leaf-weight gradient costs one reduction per leaf and group instead of
-//     one per evaluation, and a plain store where nobody else can have a part of that leaf;
-//   * the leaf's weights stay in registers as long as the leaf does, and D = sum over m of w * g needs no gather.
-// D replaces the margin in the list.  Then a thread per evaluation adds it to the x gradient, and a second sort, by
-// deciding vertex, gives every threshold gradient as a sum over a run of the list (scatters would meet at the root and its
-// neighbours: 28 us of reductions into 257 x 511 thresholds for 2.6 million evaluations, CAS loops in shared memory 30).
+// The slice's paths are sorted by leaf by counting in shared memory.  LANES lanes share an evaluation (R pieces of V of its M
+// outputs each), and every such group of lanes walks a contiguous part of the list: the evaluations of a leaf follow one
+// another, so their |margin| * g are summed in registers and the leaf-weight gradient costs one reduction per leaf and group;
+// the leaf's weights are loaded with the first of them, and D = sum over m of w * g comes from the same registers.  Where a
+// leaf begins and ends is marked in the list when it is written, so that a step is straight code: two list loads, the g row,
+// two products per output and a predicated reduction.
+// D goes back to the evaluation's own thread, which adds it to the x gradient (neighbouring threads are neighbouring positions)
+// and to the threshold sums: for trees through a second list, by deciding vertex, whose places were counted together with the
+// leaves' (scatters would meet at the root and its neighbours); for ferns, whose few thresholds everybody meets in, through a
+// column of shared memory per thread.
 //
-// What bounds it: for long rows the latency of the g rows (x [8, 100, 32, 32], 100 trees, 64 outputs: 68 us for 210 MB,
-// 228 us with a reduction per weight term), for short ones the issue slots (4096 x 500 ferns of depth 10, 10 outputs: 83 us
-// against 95; 10007 x 257 trees of depth 9, 3 outputs: 68 against 164) and the L1's rate of one row per cycle: three
-// pieces per lane instead of five lanes with one each cost 73 us for the first pass of the ferns, not 45.
-// Slices of 1024 evaluations: the counts and the lists take 16 KB and the evaluations of a thread stay in registers;
-// 4096 (16 evaluations per thread: 121 registers) run the ferns in 137 us.
-template <typename Real, int V, int LANES, int R, int PER>
-__global__ void __launch_bounds__(kSortThreads) sorted_backward_kernel(const __grid_constant__ SortedArgs<Real> a) {
+// What bounds it: issue slots (60 % used by 32 warps per SM) and the shared memory's wavefronts for short rows, the latency of
+// the g rows for long ones.  4096 x 500 ferns of depth 10, 10 outputs: 83 -> 57 us; 10007 x 257 trees of depth 9, 3 outputs:
+// 74 -> 57; x [8, 100, 32, 32], 100 trees of depth 7, 64 outputs (210 MB of g): 62 -> 53.  What had cost that: a test and a
+// branch at every change of leaf, which with five or ten groups in a warp is every step (a predicated load and a predicated
+// reduction instead; 24 -> 17.5 warp instructions per evaluation for the ferns), parts of the list that begin in the same bank,
+// a batch of g rows that is waited for before the next is asked for (a ring instead), a second count for the vertices.
+// Slices of 2048 and 4096 evaluations: ferns 98 and 137 us against 83 in the earlier form (registers).  Asking for the rows
+// ahead of the sort (prefetches into L2): 65 -> 73 us.  Two rows in flight instead of four, in exchange for five or six CTAs per
+// SM: ferns 57 and 73 us, 64 outputs 71 and 61.
+template <typename Real, int V, int LANES, int R>
+__global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted_backward_kernel(const __grid_constant__ SortedArgs<Real> a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr uint32_t S = PER * kSortThreads;
-  Real *values = reinterpret_cast<Real *>(smem);                 // by leaf: |margin|, later D
-  uint32_t *offsets = reinterpret_cast<uint32_t *>(values + S);  // by leaf: g row, in numbers from the slice's first
-  uint32_t *tags = offsets + S;                                  // by leaf: sign | level << 24 | path << 12 | place in the slice
-  uint32_t *bins = tags + S;                                     // [L]: counts, then first places
-  uint32_t *partial = bins + a.L;                                // [kSortThreads / 32]
+  constexpr int kAhead = sort_ahead<Real>(R * V), kGroupsPerWarp = 32 / LANES, kGroups = kGroupsPerWarp * (kSortThreads / 32);
+  constexpr uint32_t S = sort_slice(LANES);
+  constexpr int PER = (int)((S + kSortThreads - 1) / kSortThreads);
+  constexpr int kParts = sort_dots(LANES);
+  static_assert(S % (kGroups * kAhead) == 0, "whole rounds");
+  constexpr SortedPlaces at = sorted_places((uint32_t)sizeof(Real), LANES);
+  constexpr bool kListed = sort_rows_listed(LANES);
+  using Entry = typename std::conditional<kListed, uint4, uint2>::type;
+  Entry *list = reinterpret_cast<Entry *>(smem);              // by leaf: {tag, |margin| (float)}, and where listed {g row, weight row}
+  [[maybe_unused]] Real *sizes = reinterpret_cast<Real *>(smem + at.sizes);  // by leaf: |margin| (double)
+  Real *dots = reinterpret_cast<Real *>(smem + at.dots);      // by place in the slice: D, or its parts
+  uint32_t *partial = reinterpret_cast<uint32_t *>(smem + at.partial);
+  uint32_t *bins = reinterpret_cast<uint32_t *>(smem + at.bins);  // leaves, then vertices: counts, then first places
+  Real *by_vertex = reinterpret_cast<Real *>(smem);               // after the walk: signed D by vertex, or the ferns' columns
+  uint32_t *vertices = reinterpret_cast<uint32_t *>(by_vertex + S);  // ... and the vertices
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t j = blockIdx.x % (uint32_t)a.T;  // neighbouring trees run together: their g rows share sectors
   const uint32_t p0 = (uint32_t)(blockIdx.x / (uint32_t)a.T) * S;
   const int n = (int)min(S, a.P - p0);
-  const int depth = a.depth, L = 1 << depth;
-  const uint32_t i0 = a.K.quotient(p0), k0 = p0 - i0 * a.K.number;
+  const int L = (int)a.L, N = a.fern ? 0 : (int)a.N;  // N: vertices that are counted
+  const uint32_t K = a.K.number, M = (uint32_t)a.M;
+  const uint32_t i0 = K == 1 ? p0 : a.K.quotient_above_one(p0);
+  // tag: place in the slice | leaf << 12, whether there is an evaluation, and whether it is the first or the last of its leaf
+  constexpr uint32_t kHere = 1u << 29, kFirst = 1u << 30, kLast = 1u << 31;
+  // what a thread keeps of each of its evaluations: vertex (1-based) | place by vertex << 13 | sign of the margin
   constexpr uint32_t kPositive = 1u << 28, kNegative = 1u << 29;
 
-  // every thread's evaluations tid, tid + 256, ... are loaded at once and stay in registers while they are counted
-  uint32_t where[PER];
+  // every thread's evaluations tid, tid + 256, ... are loaded at once and stay in registers; `whole`: a full slice, all of them there
+  uint32_t where[PER], keep[PER];
   Real margin[PER];
+  const int quads = sorted_bin_quads(L, N, a.fern != 0);
+  const int share = ((n + kGroups - 1) / kGroups + kAhead - 1) / kAhead * kAhead;
+  auto here = [&](int u, bool whole) {
+    if (whole && (uint32_t)(u + 1) * kSortThreads <= S) return true;
+    return tid + u * kSortThreads < (whole ? (int)S : n);
+  };
+  // g rows, from the one of sample i0's first position: evaluation p of the tree is row p + (samples before it) * (T - 1) * K
+  const uint32_t from_first = p0 - i0 * K, skipped = ((uint32_t)a.T - 1u) * K;
+  auto g_row = [&](uint32_t p) { return (p + (K == 1 ? p : a.K.quotient_above_one(p)) * skipped) * M; };
+  auto make_list = [&](auto whole_slice) {
+    constexpr bool whole = decltype(whole_slice)::value;
+    const uint32_t sample = p0 + (uint32_t)tid, blocks = (uint32_t)a.T * kRecordBlock;
+    const int64_t from = (int64_t)(sample / kRecordBlock) * blocks + j * kRecordBlock + sample % kRecordBlock;
+    static_assert(kSortThreads == kRecordBlock, "a thread's evaluations are one record block apart");
+    const Real *margins = a.margin + from;
 #pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int t = tid + u * kSortThreads;
-    const int64_t at = record_index((int64_t)p0 + t, j, a.T);
-    where[u] = 0;
-    margin[u] = (Real)0;
-    if (t < n) {
-      where[u] = a.narrow ? __ldg(static_cast<const unsigned short *>(a.where) + at) : __ldg(static_cast<const uint32_t *>(a.where) + at);
-      margin[u] = -__ldg(a.margin + at);
-    }
-  }
-  for (int b = tid; b < L; b += kSortThreads) bins[b] = 0;
-  __syncthreads();
+    for (int u = 0; u < PER; ++u) margin[u] = here(u, whole) ? -__ldg(margins + (int64_t)u * blocks) : (Real)0;
+    if (a.narrow) {
+      const unsigned short *wheres = static_cast<const unsigned short *>(a.where) + from;
 #pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    if (tid + u * kSortThreads < n) {
-      const uint32_t packed = a.narrow ? unpack_where<unsigned short>(where[u]) : where[u];
-      const uint32_t path = tile::bit_reverse(packed >> 16, depth), vertex = packed & 0xffffu;
-      const uint32_t level = a.fern ? vertex - 1 : 31 - __clz((int)vertex);
-      where[u] = level << 24 | path << 12 | atomicAdd(&bins[path], 1u);
-    }
-  }
-  __syncthreads();
-  exclusive_sums<kSortThreads>(bins, L, partial);
+      for (int u = 0; u < PER; ++u) {
+        where[u] = here(u, whole) ? __ldg(wheres + (int64_t)u * blocks) : 0u;
+        where[u] = (where[u] & 0xffu) | (where[u] >> 8) << 16;
+      }
+    } else {
+      const uint32_t *wheres = static_cast<const uint32_t *>(a.where) + from;
 #pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int t = tid + u * kSortThreads;
-    if (t < n) {
-      const uint32_t to = bins[(where[u] >> 12) & 0xfffu] + (where[u] & 0xfffu);
-      const uint32_t sign = margin[u] > (Real)0 ? kPositive : margin[u] < (Real)0 ? kNegative : 0u;
-      const uint32_t i = a.K.quotient(p0 + t), k = p0 + t - i * a.K.number;
-      values[to] = abs_of(margin[u]);
-      offsets[to] = ((i - i0) * (uint32_t)a.T * a.K.number + k - k0) * (uint32_t)a.M;
-      tags[to] = sign | (where[u] & 0xffff000u) | (uint32_t)t;
+      for (int u = 0; u < PER; ++u) where[u] = here(u, whole) ? __ldg(wheres + (int64_t)u * blocks) : 0u;
     }
-  }
+    for (int b = tid; b < quads; b += kSortThreads) reinterpret_cast<uint4 *>(bins)[b] = make_uint4(0u, 0u, 0u, 0u);
+    __syncthreads();
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const uint32_t leaf = where[u] >> 16, vertex = where[u] & 0xffffu;
+      keep[u] = vertex | (margin[u] > (Real)0 ? kPositive : 0u) | (margin[u] < (Real)0 ? kNegative : 0u);
+      if (here(u, whole)) {
+        if (N > 0) keep[u] |= atomicAdd(&bins[L - 1 + vertex], 1u) << 13;
+        where[u] = leaf << 12 | atomicAdd(&bins[leaf], 1u);
+      }
+    }
+    __syncthreads();
+    exclusive_sums<kSortThreads>(reinterpret_cast<uint4 *>(bins), quads, partial);  // bins[L] = n, the first vertex's place + n
+    const float per_share = 1.0f / (float)share;
+    // the groups' parts lie one entry further apart than they are long: their reads fall into different banks
+    auto slot_of = [&](uint32_t to) { return to + (uint32_t)(((float)to + 0.5f) * per_share); };
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      if (here(u, whole)) {
+        const int t = tid + u * kSortThreads;
+        const uint32_t leaf = where[u] >> 12, rank = where[u] & 0xfffu, next = bins[leaf + 1];
+        const uint32_t to = bins[leaf] + rank, slot = slot_of(to);
+        Entry entry = {};
+        entry.x = (uint32_t)t | leaf << 12 | kHere | (rank == 0 ? kFirst : 0u) | (to + 1 == next ? kLast : 0u);
+        if constexpr (kListed) {
+          entry.z = g_row(from_first + (uint32_t)t);
+          entry.w = leaf * M;
+        }
+        if constexpr (sizeof(Real) == 4)
+          entry.y = __float_as_uint(fabsf((float)margin[u]));
+        else
+          sizes[slot] = abs_of(margin[u]);
+        list[slot] = entry;
+        if (N > 0) keep[u] += (bins[L - 1 + (keep[u] & 0x1fffu)] - (uint32_t)n) << 13;
+      }
+    }
+    if constexpr (!whole) {  // entries without an evaluation fill the last parts
+      for (uint32_t to = (uint32_t)(n + tid); to < (uint32_t)(share * kGroups); to += kSortThreads) {
+        Entry nobody = {};
+        nobody.x = kNobody;
+        if constexpr (kListed) nobody.z = g_row(from_first);
+        list[slot_of(to)] = nobody;
+        if constexpr (sizeof(Real) != 4) sizes[slot_of(to)] = (Real)0;
+      }
+    }
+  };
+  if (n == (int)S)
+    make_list(std::true_type{});
+  else
+    make_list(std::false_type{});
   __syncthreads();
 
   {
-    constexpr int kAhead = sort_ahead<Real>(R * V), kGroupsPerWarp = 32 / LANES, groups = kGroupsPerWarp * (kSortThreads / 32);
-    const int group_in_warp = lane / LANES, q = lane % LANES;
-    const int share = ((n + groups - 1) / groups + kAhead - 1) / kAhead * kAhead;
-    const bool idle = group_in_warp >= kGroupsPerWarp;  // lanes left over
-    const int begin = idle ? n : min((warp * kGroupsPerWarp + group_in_warp) * share, n);
-    const int end = min(begin + share, n);
-    const Real *g_first = a.g + (((int64_t)i0 * a.T + j) * a.K.number + k0) * a.M + q * V;
-    Real sums[R][V], weight[R][V];
+    // lanes left over (32 is no multiple of LANES) accompany the last group, and lanes beyond a row's end its first; neither
+    // hands anything in
+    const int group_in_warp = min(lane / LANES, kGroupsPerWarp - 1), q = lane - group_in_warp * LANES;
+    const int part = warp * kGroupsPerWarp + group_in_warp;
+    const Entry *my_list = list + part * (share + 1);
+    [[maybe_unused]] const Real *my_sizes = sizes + part * (share + 1);
     bool on[R];
+    uint32_t piece[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      on[r] = (q + r * LANES) * V < a.M;
+      on[r] = q < LANES && (q + r * LANES) * V < a.M;
+      piece[r] = on[r] ? (uint32_t)((q + r * LANES) * V) : 0u;
+    }
+    const Real *g_first = a.g + ((int64_t)i0 * a.T + j) * K * M;
+    const Real *w_first = a.w + j * L * M;
+    const Real *gw_first = a.gw + j * L * M;
+    const bool want_w = a.gw != nullptr;
+    Real sums[R][V], weight[R][V];
+#pragma unroll
+    for (int r = 0; r < R; ++r)
 #pragma unroll
       for (int v = 0; v < V; ++v) sums[r][v] = weight[r][v] = (Real)0;
-    }
-    constexpr uint32_t kNone = 0xffffffffu;
-    uint32_t current = kNone;  // the leaf (path) whose sums are in the registers
-    bool whole = false;        // all of its evaluations are in this group's part
-
-    auto leave = [&]() {
-      if (a.gw == nullptr || current == kNone) return;
-      Real *row = a.gw + (j * L + tile::bit_reverse(current, depth)) * a.M + q * V;
+    auto hand_in = [&](uint32_t leaf_row, bool now) {
 #pragma unroll
-      for (int r = 0; r < R; ++r)
-        if (on[r]) {
-          Real *to = row + r * LANES * V;
-          if (whole) {
-            Vec<Real, V> out;
-#pragma unroll
-            for (int v = 0; v < V; ++v) out.v[v] = sums[r][v];
-            *reinterpret_cast<Vec<Real, V> *>(to) = out;
-          } else {
-            red_add<V>(to, sums[r]);
-          }
-        }
+      for (int r = 0; r < R; ++r) red_add_if<V>(const_cast<Real *>(element(gw_first, leaf_row + piece[r])), sums[r], now && on[r]);
     };
-    auto walk_list = [&](int t0, auto no_bounds) {
-      constexpr bool full = decltype(no_bounds)::value;
-      Vec<Real, V> rows[kAhead][R], entered[kAhead][R];  // g rows, and the weights of the leaves that this round enters
-      uint32_t path[kAhead];
+    // a ring of kAhead evaluations: their list entries, g rows, and the weights of the leaves that they enter
+    Vec<Real, V> rows[kAhead][R], entered[kAhead][R] = {};
+    uint32_t tag[kAhead], leaf_row[kAhead];
+    Real size[kAhead];
+    auto fetch = [&](int u, int t, bool enters) {
+      const Entry entry = my_list[t];
+      tag[u] = entry.x | (enters ? kFirst : 0u);
+      if constexpr (sizeof(Real) == 4)
+        size[u] = __uint_as_float(entry.y);
+      else
+        size[u] = my_sizes[t];
+      uint32_t row;
+      if constexpr (kListed) {
+        row = entry.z;
+        leaf_row[u] = entry.w;
+      } else {
+        row = g_row(from_first + (entry.x & (kNobody - 1u)));
+        leaf_row[u] = ((entry.x >> 12) & 0xfffu) * M;
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        rows[u][r] = load_vec<Real, V>(element(g_first, row + piece[r]));
+        load_if<V>(entered[u][r], element(w_first, leaf_row[u] + piece[r]), (tag[u] & kFirst) != 0);
+      }
+    };
+    auto round = [&](int t0, auto more) {
+      uint32_t place[kAhead];
       Real dot[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
-        const int t = t0 + u;
-        path[u] = full || t < end ? (tags[t] >> 12) & 0xfffu : kNone;
-        if (full || t < end) {
-          const Real *row = g_first + (int32_t)offsets[t];
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-            if (on[r]) rows[u][r] = load_vec<Real, V>(row + r * LANES * V);
-          if (path[u] != (u == 0 ? current : path[u == 0 ? 0 : u - 1])) {
-            const Real *leaf = a.w + (j * L + tile::bit_reverse(path[u], depth)) * a.M + q * V;
-#pragma unroll
-            for (int r = 0; r < R; ++r)
-              if (on[r]) entered[u][r] = load_vec<Real, V>(leaf + r * LANES * V);
-          }
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < kAhead; ++u) {
-        const int t = t0 + u;
+        place[u] = tag[u];
         dot[u] = (Real)0;
-        if (full || t < end) {
-          if (path[u] != current) {
-            leave();
-            current = path[u];
-            if (a.exclusive) {
-              const int run_end = current + 1 < (uint32_t)L ? (int)bins[current + 1] : n;
-              whole = run_end <= end && (int)bins[current] >= begin;
-            }
 #pragma unroll
-            for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R; ++r) {
+          Real mine = (Real)0;
 #pragma unroll
-              for (int v = 0; v < V; ++v) {
-                sums[r][v] = (Real)0;
-                weight[r][v] = entered[u][r].v[v];
-              }
+          for (int v = 0; v < V; ++v) {
+            weight[r][v] = (tag[u] & kFirst) ? entered[u][r].v[v] : weight[r][v];
+            sums[r][v] += size[u] * rows[u][r].v[v];
+            mine += weight[r][v] * rows[u][r].v[v];
           }
-          const Real size = values[t];
-#pragma unroll
-          for (int r = 0; r < R; ++r)
-            if (on[r]) {
-#pragma unroll
-              for (int v = 0; v < V; ++v) {
-                sums[r][v] += size * rows[u][r].v[v];
-                dot[u] += weight[r][v] * rows[u][r].v[v];
-              }
-            }
+          dot[u] += kParts > 1 || on[r] ? mine : (Real)0;
         }
-      }
-#pragma unroll
-      for (int d = 16; d >= 1; d >>= 1) {
-        if (d >= LANES) continue;
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u) {
-          const Real other = __shfl_down_sync(0xffffffffu, dot[u], d);
-          if (q + d < LANES || (LANES & (LANES - 1)) == 0) dot[u] += other;  // (powers of two: only lane q = 0 is read)
-        }
-      }
-      __syncwarp();  // the margins of this round have been read
-      if (q == 0) {
-#pragma unroll
-        for (int u = 0; u < kAhead; ++u)
-          if (full || t0 + u < end) values[t0 + u] = dot[u];
-      }
-    };
-    // the groups of a warp go through their parts together; only a warp that holds the list's end, or lanes left over,
-    // has short parts
-    if (__all_sync(0xffffffffu, begin + share == end))
-      for (int t0 = begin; t0 < begin + share; t0 += kAhead) walk_list(t0, std::true_type{});
-    else
-      for (int t0 = begin; t0 < begin + share; t0 += kAhead) walk_list(t0, std::false_type{});
-    // groups of the warp that end in the same leaf hand in one sum (23 million evaluations of 22 trees of depth 4, 2 outputs:
-    // 495 us; 1293 when all 256 groups of a slice met in 16 leaves)
-    if constexpr (kGroupsPerWarp > 1) {
-#pragma unroll
-      for (int d = 1; d < kGroupsPerWarp; d <<= 1) {
-        const bool join = __shfl_down_sync(0xffffffffu, current, d * LANES) == current && group_in_warp + d < kGroupsPerWarp;
+        hand_in(leaf_row[u], want_w && (tag[u] & kLast) != 0);
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-          for (int v = 0; v < V; ++v) {
-            const Real other = __shfl_down_sync(0xffffffffu, sums[r][v], d * LANES);
-            if (join) sums[r][v] += other;
-          }
+          for (int v = 0; v < V; ++v) sums[r][v] = (tag[u] & kLast) ? (Real)0 : sums[r][v];
+        if constexpr (decltype(more)::value) fetch(u, t0 + u + kAhead, false);
       }
-      const uint32_t before = __shfl_up_sync(0xffffffffu, current, LANES);
-      if (group_in_warp > 0 && before == current) current = kNone;
+      if constexpr (kParts > 1) {
+        if (q < LANES) {
+#pragma unroll
+          for (int u = 0; u < kAhead; ++u) dots[(place[u] & (2u * kNobody - 1u)) * kParts + q] = dot[u];
+        }
+      } else {
+        constexpr int kLists = LANES < kAhead ? LANES : kAhead, kEach = kAhead / kLists;  // sums that a lane is left with
+        int mine = 0;
+        sums_over_lanes<LANES / 2, kAhead>(dot, q, mine);
+        if ((q & (LANES / kLists - 1)) == 0) {
+#pragma unroll
+          for (int e = 0; e < kEach; ++e) {
+            uint32_t whose = place[e];
+#pragma unroll
+            for (int l = 1; l < kLists; ++l) whose = mine == l ? place[l * kEach + e] : whose;
+            dots[whose & (2u * kNobody - 1u)] = dot[e];
+          }
+        }
+      }
+    };
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) fetch(u, u, u == 0);
+    int t0 = 0;
+    for (; t0 + kAhead < share; t0 += kAhead) round(t0, std::true_type{});
+    round(t0, std::false_type{});
+    if (want_w) {
+      constexpr uint32_t kNone = 0xffffffffu;
+      const uint32_t final = my_list[share - 1].x;
+      // the leaf (its row) whose evaluations go on behind this group's part
+      uint32_t current = (final & (kHere | kLast)) == kHere ? ((final >> 12) & 0xfffu) * M : kNone;
+      // groups of the warp that end in the same leaf hand in one sum (23 million evaluations of 22 trees of depth 4, 2 outputs:
+      // 495 us; 1293 when all 256 groups of a slice met in 16 leaves)
+      if constexpr (kGroupsPerWarp > 1) {
+#pragma unroll
+        for (int d = 1; d < kGroupsPerWarp; d <<= 1) {
+          const bool join = __shfl_down_sync(0xffffffffu, current, d * LANES) == current && group_in_warp + d < kGroupsPerWarp;
+#pragma unroll
+          for (int r = 0; r < R; ++r)
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              const Real other = __shfl_down_sync(0xffffffffu, sums[r][v], d * LANES);
+              sums[r][v] += join ? other : (Real)0;
+            }
+        }
+        const uint32_t before = __shfl_up_sync(0xffffffffu, current, LANES);
+        if (group_in_warp > 0 && before == current) current = kNone;
+      }
+      hand_in(current, current != kNone);
     }
-    leave();
   }
   if (a.gx == nullptr && a.gthr == nullptr) return;
   __syncthreads();
 
-  // thread per evaluation: x gradient, and the evaluations of every vertex are counted
-  for (int b = tid; b < L; b += kSortThreads) bins[b] = 0;
-  __syncthreads();
+  // thread per evaluation again
+  if (a.fern && a.gthr != nullptr)
+    for (int l = 0; l < (int)a.N; ++l) by_vertex[l * kSortThreads + tid] = (Real)0;
+  auto finish = [&](auto whole_slice) {
+    constexpr bool whole = decltype(whole_slice)::value;
+    const int32_t *features = a.ord + j * a.N - 1;
 #pragma unroll
-  for (int u = 0; u < PER; ++u) {
-    const int t = tid + u * kSortThreads;
-    if (t < n) {
-      const uint32_t tag = tags[t];
-      const Real d = values[t];
-      margin[u] = (tag & kPositive) ? d : (tag & kNegative) ? -d : (Real)0 * d;  // sign(margin) * D
-      const int level = (int)(tag >> 24) & 0xf;
-      const uint32_t vertex = a.fern ? (uint32_t)level : (1u << level | ((tag >> 12) & 0xfffu) >> (depth - level)) - 1u;
-      if (a.gx != nullptr) {
-        const uint32_t p = p0 + (tag & 0xfffu);
-        const uint32_t i = a.K.quotient(p), k = p - i * a.K.number;
-        atomicAdd(a.gx + ((int64_t)i * a.C + __ldg(a.ord + j * a.N + vertex)) * a.K.number + k, margin[u]);
+    for (int u = 0; u < PER; ++u) {
+      if (here(u, whole)) {
+        const int t = tid + u * kSortThreads;
+        Real d = dots[t * kParts];
+#pragma unroll
+        for (int part = 1; part < kParts; ++part) d += dots[t * kParts + part];
+        const uint32_t vertex = keep[u] & 0x1fffu;
+        Real term = (keep[u] & kPositive) ? d : -d;  // sign(margin) * D
+        if ((keep[u] & (kPositive | kNegative)) == 0) term = (Real)0 * d;
+        if (a.gx != nullptr) {
+          const uint32_t f = (uint32_t)__ldg(features + vertex);
+          if (K == 1) {
+            atomicAdd(a.gx + (int64_t)(p0 + (uint32_t)t) * a.C + f, term);
+          } else {
+            const uint32_t i = a.K.quotient_above_one(p0 + t), k = p0 + t - i * K;
+            atomicAdd(a.gx + ((int64_t)i * a.C + f) * K + k, term);
+          }
+        }
+        if (a.gthr != nullptr) {
+          if (a.fern) {
+            by_vertex[(vertex - 1) * kSortThreads + tid] += term;
+          } else {
+            const uint32_t to = (keep[u] >> 13) & 0x7fffu;
+            by_vertex[to] = term;
+            vertices[to] = vertex - 1;
+          }
+        }
       }
-      if (a.gthr != nullptr) where[u] = vertex << 12 | atomicAdd(&bins[vertex], 1u);
     }
-  }
+  };
+  if (n == (int)S)
+    finish(std::true_type{});
+  else
+    finish(std::false_type{});
   if (a.gthr == nullptr) return;
   __syncthreads();
-  const int N = (int)a.N;
-  exclusive_sums<kSortThreads>(bins, N, partial);
+  if (a.fern) {
+    for (int l = warp; l < (int)a.N; l += kSortThreads / 32) {
+      Real sum = (Real)0;
 #pragma unroll
-  for (int u = 0; u < PER; ++u)
-    if (tid + u * kSortThreads < n) {
-      const uint32_t to = bins[where[u] >> 12] + (where[u] & 0xfffu);
-      values[to] = margin[u];  // every D and tag is in registers by now
-      tags[to] = where[u] >> 12;
+      for (int e = 0; e < kSortThreads; e += 32) sum += by_vertex[l * kSortThreads + e + lane];
+#pragma unroll
+      for (int d = 16; d >= 1; d >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, d);
+      if (lane == 0) atomicAdd(a.gthr + j * a.N + l, -sum);
     }
-  __syncthreads();
+    return;
+  }
   // warps sum runs of 32: a lane adds what is d lanes above while that is the same vertex
   for (int e0 = warp * 32; e0 < n; e0 += kSortThreads) {
     const int e = e0 + lane;
-    Real sum = e < n ? values[e] : (Real)0;
-    const uint32_t vertex = e < n ? tags[e] : 0xffffu;
+    Real sum = e < n ? by_vertex[e] : (Real)0;
+    const uint32_t vertex = e < n ? vertices[e] : 0xffffu;
+    const uint32_t before = __shfl_up_sync(0xffffffffu, vertex, 1);
+    const bool leads = lane == 0 || before != vertex;
+    const uint32_t leaders = __ballot_sync(0xffffffffu, leads) & ~((2u << lane) - 1u);  // of the runs above this lane's
+    const int last = (leaders != 0u ? __ffs((int)leaders) - 1 : 32) - lane;             // lanes to the end of the run
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const Real other = __shfl_down_sync(0xffffffffu, sum, d);
-      const uint32_t whose = __shfl_down_sync(0xffffffffu, vertex, d);
-      if (lane + d < 32 && whose == vertex) sum += other;
+      if (d < last) sum += other;
     }
-    const uint32_t before = __shfl_up_sync(0xffffffffu, vertex, 1);
-    if (e < n && (lane == 0 || before != vertex)) atomicAdd(a.gthr + j * N + vertex, -sum);
+    if (e < n && leads) atomicAdd(a.gthr + j * a.N + vertex, -sum);
   }
 }
 
 template <typename Real, int V, int LANES, int R>
-int launch_sorted(const SortedArgs<Real> &a, unsigned grid, size_t smem, cudaStream_t stream) {
-  auto kernel = sorted_backward_kernel<Real, V, LANES, R, kSlice / kSortThreads>;
+int launch_sorted(const SortedArgs<Real> &a, cudaStream_t stream) {
+  constexpr uint32_t slice = sort_slice(LANES);
+  const int64_t grid = (int64_t)((a.P + slice - 1) / slice) * a.T;
+  if (grid > 0x7fffffff) return HT_ERR_UNSUPPORTED;
+  auto kernel = sorted_backward_kernel<Real, V, LANES, R>;
+  const size_t smem = sorted_places((uint32_t)sizeof(Real), LANES).bins + 16 * (size_t)sorted_bin_quads((int)a.L, (int)a.N, a.fern != 0);
   if (smem > 48 * 1024) HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kernel<<<grid, kSortThreads, smem, stream>>>(a);
+  kernel<<<(unsigned)grid, kSortThreads, smem, stream>>>(a);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }
 
 template <typename Real, int V>
-int launch_sorted_width(const SortedArgs<Real> &a, unsigned grid, size_t smem, cudaStream_t stream) {
+int launch_sorted_width(const SortedArgs<Real> &a, cudaStream_t stream) {
   // one load per lane and row up to half a warp per row (64 outputs: 68 us, with two loads and 8 lanes 78)
   const int pieces = (a.M + V - 1) / V;
   const bool one = pieces <= 16;
 #define HT_SORTED(LANES, R) \
-  if (pieces <= LANES * R && one == (R == 1)) return launch_sorted<Real, V, LANES, R>(a, grid, smem, stream);
+  if (pieces <= LANES * R && one == (R == 1)) return launch_sorted<Real, V, LANES, R>(a, stream);
   HT_SORTED(1, 1)
   HT_SORTED(2, 1)
   HT_SORTED(3, 1)
@@ -530,16 +713,11 @@ int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w
   a.depth = p->depth;
   a.fern = p->kind == FERN;
   a.narrow = where_bytes(p->depth) == 2;
-  constexpr uint32_t slice = kSlice;
-  a.exclusive = a.P <= slice;
-  const int64_t grid = (int64_t)((a.P + slice - 1) / slice) * p->T;
-  if (grid > 0x7fffffff) return HT_ERR_UNSUPPORTED;
-  if ((int64_t)slice * p->T * p->M + (int64_t)p->T * p->K * p->M > 0x7fffffff) return HT_ERR_UNSUPPORTED;  // g row offsets
-  const size_t smem = (size_t)slice * (sizeof(Real) + 8) + 4 * (size_t)(a.L + kSortThreads / 32);
+  if ((int64_t)1024 * p->T * p->M + (int64_t)p->T * p->K * p->M > 0x7fffffff) return HT_ERR_UNSUPPORTED;  // g row offsets
   const int width = vector_width(p->M, sizeof(Real), {w, g, gw});
-  if (width == 1) return launch_sorted_width<Real, 1>(a, (unsigned)grid, smem, stream);
-  if (width == 2) return launch_sorted_width<Real, 2>(a, (unsigned)grid, smem, stream);
-  if constexpr (sizeof(Real) == 4) return launch_sorted_width<Real, 4>(a, (unsigned)grid, smem, stream);
+  if (width == 1) return launch_sorted_width<Real, 1>(a, stream);
+  if (width == 2) return launch_sorted_width<Real, 2>(a, stream);
+  if constexpr (sizeof(Real) == 4) return launch_sorted_width<Real, 4>(a, stream);
   return HT_ERR_UNSUPPORTED;
 }
 

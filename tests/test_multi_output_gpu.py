@@ -2,6 +2,7 @@
 positions, both ways to the paths (kept by the forward, or walked again)."""
 import numpy as np
 import pytest
+import torch
 
 import hingetreefortorch_b200._cabi as _cabi
 from conftest import grad_close
@@ -71,6 +72,28 @@ def test_forward_and_backward(kind, shape):
     got = f.forward(dev(x)[0], dthr, dord, dw).cpu().numpy()
     assert np.array_equal(got, ho.forward(kind, x, thr, ord_, w), equal_nan=True)
     assert f.ordinal_flags() == 0
+
+
+# evaluations per tree around whole slices (960 with three or five lanes per row, 1024 otherwise), leaves that a few or all
+# evaluations share, samples that begin inside a slice; pieces of one, two and four numbers, listed rows and others
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("M", [2, 3, 5, 10, 12, 20, 26, 32, 64])
+@pytest.mark.parametrize("B, inner, depth", [(959, (), 7), (960, (), 1), (961, (), 9), (1024, (), 2), (1025, (), 8), (1923, (), 4),
+                                             (7, (11, 25), 5)])
+def test_slices_of_the_sorted_backward(B, inner, depth, M, dtype):
+    T, C = -(-32768 // (B * int(np.prod(inner, dtype=int)))) + 1, 10
+    kind = "tree" if M % 2 == 0 else "fern"
+    x, thr, ord_, w = random_forest_inputs(500 + M, kind, B, C, inner, T, depth, (M,), quantise=True)
+    want = ho.forward(kind, x, thr, ord_, w)
+    g = np.random.default_rng(7).standard_normal(want.shape).astype(np.float32)
+    ref = ho.backward(kind, x, thr, ord_, w, g)
+    sizes = ho.backward_magnitudes(kind, x, thr, ord_, w, g)
+    # double precision on the same numbers: the oracle's sums in single precision are as good as the bar
+    dx, dthr, dord, dw, dg = [a if a.dtype == torch.int64 else a.to(dtype) for a in dev(x, thr, ord_, w, g)]
+    from hingetreefortorch_b200._ext import hingetree_cpp
+    gx, gthr, _, gw = getattr(hingetree_cpp, kind + "_backward")(dx, True, dthr, True, dord, False, dw, True, dg)
+    for got, r, s in zip((gx, gthr, gw), ref, sizes):
+        assert grad_close(got, r, s)
 
 
 @pytest.mark.parametrize("depth", [5, 8])
