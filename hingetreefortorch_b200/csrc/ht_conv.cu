@@ -10,6 +10,7 @@
 // deterministic and equal to the reference CPU loop bit for bit.
 #include "ht_common.cuh"
 #include "ht_conv_tiled.cuh"
+#include "ht_counting_sort.cuh"
 
 #include <algorithm>
 
@@ -36,18 +37,18 @@ struct ConvArgsOf : ConvShape {
 };
 using ConvArgs = ConvArgsOf<float>;
 
-// Offsets (in elements along z, y, x; dilation applied) of every window cell, 10 bits each.
-__device__ __forceinline__ void fill_cell_table(const ConvShape &a, uint32_t *table) {
-  for (int q = threadIdx.x; q < a.cells; q += blockDim.x) {
-    int rest = q;
-    uint32_t packed = 0;
-    for (int d = a.dims - 1; d >= 0; --d) {
-      const int qd = rest % a.kernel[d];
-      rest /= a.kernel[d];
-      packed |= (uint32_t)(qd * a.dil[d]) << (10 * (a.dims - 1 - d));
-    }
-    table[q] = packed;
+// Offsets (in elements along z, y, x; dilation applied) of a window cell, 10 bits each.
+__device__ __forceinline__ uint32_t packed_cell(const ConvShape &a, int cell) {
+  uint32_t packed = 0;
+  for (int d = a.dims - 1; d >= 0; --d) {
+    const int qd = cell % a.kernel[d];
+    cell /= a.kernel[d];
+    packed |= (uint32_t)(qd * a.dil[d]) << (10 * (a.dims - 1 - d));
   }
+  return packed;
+}
+__device__ __forceinline__ void fill_cell_table(const ConvShape &a, uint32_t *table) {
+  for (int q = threadIdx.x; q < a.cells; q += blockDim.x) table[q] = packed_cell(a, q);
 }
 
 // Image coordinates of the first window cell of output position p (may be negative: padding).
@@ -60,6 +61,22 @@ __device__ __forceinline__ void window_origin(const ConvShape &a, int64_t p, int
       origin[d] = od * a.stride[d] - a.pad[d];
     } else {
       origin[d] = 0;
+    }
+  }
+}
+
+// The same with quotients by multiplication (positions below 2^31).
+struct PositionDivisors {
+  Divisor size[3];
+};
+__device__ __forceinline__ void window_origin(const ConvShape &a, const PositionDivisors &by, uint32_t p, int (&origin)[3]) {
+#pragma unroll
+  for (int d = 2; d >= 0; --d) {
+    origin[d] = 0;
+    if (d < a.dims) {
+      const uint32_t rest = by.size[d].quotient(p);
+      origin[d] = (int)(p - rest * by.size[d].number) * a.stride[d] - a.pad[d];
+      p = rest;
     }
   }
 }
@@ -130,7 +147,59 @@ __global__ void __launch_bounds__(kBlock) conv_forward_kernel(ConvArgsOf<Real> a
   }
 }
 
+// The same sums for calls with too few outputs to fill the machine: a warp per input channel walks, eight at a time, and leaves
+// |margin| and the leaf's place; then a thread per output adds the eight in ascending order.  What bounds the kernel above there is
+// the chain of Ci walks of a thread (1458 outputs of 30 channels, depth 7: 92 us, 19 here).
+constexpr int kSharing = 8;       // channels under way
+constexpr int kSharedOutputs = 8;  // outputs that a thread adds up: M <= kSharing * kSharedOutputs
+template <int KIND, typename Real>
+__global__ void __launch_bounds__(32 * kSharing) conv_forward_shared_kernel(ConvArgsOf<Real> a, Real *__restrict__ out) {
+  __shared__ uint32_t table[kMaxCells];
+  __shared__ Real sizes[2][kSharing][32];
+  __shared__ uint32_t leaves[2][kSharing][32];
+  fill_cell_table(a, table);
+  __syncthreads();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t outputs = a.B * a.Co * a.out_count, mine = (int64_t)blockIdx.x * 32 + lane;
+  const int64_t e = min(mine, outputs - 1);  // (i, j, p), p fastest
+  const int64_t p = e % a.out_count;
+  const int64_t j = (e / a.out_count) % a.Co;
+  const int64_t i = e / (a.out_count * a.Co);
+  int origin[3];
+  window_origin(a, p, origin);
+  Real acc[kSharedOutputs] = {};
+  int buffer = 0;
+  for (int64_t c0 = 0; c0 < a.Ci; c0 += kSharing, buffer ^= 1) {
+    const int64_t c = c0 + warp;
+    if (c < a.Ci) {
+      const int64_t tree = j * a.Ci + c;
+      const WindowFeatureOf<Real> feat{a, a.x + (i * a.Ci + c) * a.in_count, origin, table};
+      const PathOf<Real> path = traverse<KIND>(feat, a.thr + tree * a.N, a.ord + tree * a.N, a.depth);
+      sizes[buffer][warp][lane] = abs_of(path.margin);
+      leaves[buffer][warp][lane] = (uint32_t)(tree * a.L) + path.key;  // Co * Ci * L < 2^32 (host)
+    }
+    __syncthreads();  // one per round: the next round writes the other buffer
+    const int here = (int)min((int64_t)kSharing, a.Ci - c0);
+#pragma unroll
+    for (int r = 0; r < kSharedOutputs; ++r) {
+      const int m = warp + r * kSharing;
+      if (m >= a.M) break;
+      Real weight[kSharing];
+#pragma unroll
+      for (int u = 0; u < kSharing; ++u) weight[u] = u < here ? __ldg(a.w + (int64_t)leaves[buffer][u][lane] * a.M + m) : (Real)0;
+#pragma unroll
+      for (int u = 0; u < kSharing; ++u)
+        if (u < here) acc[r] = add_rn(acc[r], mul_rn(weight[u], sizes[buffer][u][lane]));
+    }
+  }
+  if (mine >= outputs) return;
+#pragma unroll
+  for (int r = 0; r < kSharedOutputs; ++r)
+    if (warp + r * kSharing < a.M) out[e * a.M + warp + r * kSharing] = acc[r];
+}
+
 // One thread per (i, j, p) walking the input channels; the three gradients are scattered with atomics.
+// Trees of many leaves (launch_backward_sorted says which).
 template <int KIND, typename Real>
 __global__ void __launch_bounds__(kBlock) conv_backward_kernel(ConvArgsOf<Real> a, const Real *__restrict__ g, Real *gx,
                                                                Real *gthr, Real *gw) {
@@ -163,6 +232,172 @@ __global__ void __launch_bounds__(kBlock) conv_backward_kernel(ConvArgsOf<Real> 
     }
     if (gthr != nullptr) atomicAdd(gthr + tree * a.N + path.vertex, -acc);
   }
+}
+
+// CTA per (tree, slice of its evaluations): the slice's walks are sorted by leaf and by deciding vertex by counting in shared
+// memory, so that the terms of a bin lie together, and a warp hands in one sum per run of 32 of them.
+// What bounds the kernel above is where its reductions meet: the trees of a convolution see every position of every sample, so
+// that a handful of thresholds and leaves take all terms one after the other.  It also walks the input channels of a position in
+// one thread.  159744 positions of 135 ferns of depth 3 (3-D): 3923 us there, 532 here; 30375 of 24 trees of depth 3 242 and 24;
+// 9947 of 420 trees of depth 4 with 4 outputs 468 and 137.  It is bound by latency: walks through L1, then six barriers per slice.
+// Slices of a tree next to each other instead of trees of a slice: 728 us for the first, 532 here (its tree's sums meet).
+constexpr int kSortedBins = 2048;  // leaves + decisions, at most: depth 10
+template <typename Real>
+__host__ __device__ constexpr int sorted_terms() { return 16 / (int)sizeof(Real); }  // outputs of a leaf at a time
+
+// Where its arrays lie in shared memory: terms by bin [outputs at a time][slice], the tree's thresholds, bins, the tree's cells,
+// partial sums, and the bin of every term.
+struct ConvSortedPlaces {
+  uint32_t thresholds, bins, cells, partial, keys, bytes;
+};
+template <typename Real>
+__host__ __device__ inline ConvSortedPlaces conv_sorted_places(const ConvShape &a, uint32_t slice) {
+  const uint32_t N = (uint32_t)a.N, outputs = a.M < sorted_terms<Real>() ? (uint32_t)a.M : (uint32_t)sorted_terms<Real>();
+  ConvSortedPlaces at;
+  at.thresholds = outputs * slice * (uint32_t)sizeof(Real);
+  at.bins = (at.thresholds + N * (uint32_t)sizeof(Real) + 15u) & ~15u;
+  at.cells = at.bins + 16u * (((uint32_t)a.L + N + 4u) / 4u);
+  at.partial = at.cells + 4u * N;
+  at.keys = at.partial + 4u * (kBlock / 32);
+  at.bytes = at.keys + 2u * slice;
+  return at;
+}
+
+template <int KIND, typename Real, int PER>
+__global__ void __launch_bounds__(kBlock, sizeof(Real) == 4 ? 4 : 2) conv_backward_sorted_kernel(ConvArgsOf<Real> a, Divisor positions, PositionDivisors by,
+                                                                      uint32_t evals, uint32_t trees, int quad_sums, const Real *__restrict__ g, Real *gx, Real *gthr, Real *gw) {
+  constexpr int S = kBlock * PER, W = sorted_terms<Real>();
+  extern __shared__ __align__(16) unsigned char smem[];
+  const ConvSortedPlaces at = conv_sorted_places<Real>(a, S);
+  Real *terms = reinterpret_cast<Real *>(smem), *thresholds = reinterpret_cast<Real *>(smem + at.thresholds);
+  uint32_t *bins = reinterpret_cast<uint32_t *>(smem + at.bins);  // leaves, then vertices: counts, then first places
+  uint32_t *cells = reinterpret_cast<uint32_t *>(smem + at.cells), *partial = reinterpret_cast<uint32_t *>(smem + at.partial);
+  unsigned short *keys = reinterpret_cast<unsigned short *>(smem + at.keys);
+  const int L = (int)a.L, N = (int)a.N, quads = (L + N + 4) / 4;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const uint32_t tree = blockIdx.x % trees, first = blockIdx.x / trees * S;
+  const int n = (int)min((uint32_t)S, evals - first);
+  const int64_t j = tree / (uint32_t)a.Ci, c = tree - j * a.Ci;
+  for (int b = tid; b < quads; b += kBlock) reinterpret_cast<uint4 *>(bins)[b] = make_uint4(0u, 0u, 0u, 0u);
+  for (int v = tid; v < N; v += kBlock) {
+    thresholds[v] = __ldg(a.thr + (int64_t)tree * N + v);
+    cells[v] = packed_cell(a, __ldg(a.ord + (int64_t)tree * N + v));
+  }
+  __syncthreads();
+  // the walks, all of a thread's at once; threads without an evaluation walk the slice's first
+  int origin[PER][3];
+  uint32_t sample[PER], position[PER], key[PER], vertex[PER], v[PER];
+  Real margin[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    const int t = tid + u * kBlock;
+    const uint32_t q = first + (uint32_t)(t < n ? t : 0);
+    sample[u] = positions.quotient(q);
+    position[u] = q - sample[u] * positions.number;
+    window_origin(a, by, position[u], origin[u]);
+    key[u] = vertex[u] = v[u] = 0;
+    margin[u] = (Real)0;
+  }
+  for (int l = 0; l < a.depth; ++l) {
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      const uint32_t here = KIND == FERN ? (uint32_t)l : v[u];
+      const int idx = cell_index(a, origin[u], cells[here]);
+      const Real m = (idx < 0 ? (Real)0 : __ldg(a.x + ((int64_t)sample[u] * a.Ci + c) * a.in_count + idx)) - thresholds[here];
+      const uint32_t bit = m > (Real)0 ? 1u : 0u;
+      if (l == 0 || abs_of(m) < abs_of(margin[u])) {
+        margin[u] = m;
+        vertex[u] = here;
+      }
+      key[u] |= bit << l;
+      v[u] = 2 * v[u] + 1 + bit;
+    }
+  }
+  uint32_t by_leaf[PER], by_vertex[PER];
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    by_leaf[u] = by_vertex[u] = 0;
+    if (tid + u * kBlock < n) {
+      by_leaf[u] = atomicAdd(&bins[key[u]], 1u);
+      by_vertex[u] = atomicAdd(&bins[L + vertex[u]], 1u);
+    }
+  }
+  __syncthreads();
+  exclusive_sums<kBlock>(reinterpret_cast<uint4 *>(bins), quads, partial);
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    by_leaf[u] += bins[key[u]];
+    by_vertex[u] += bins[L + vertex[u]] - (uint32_t)n;
+    if (tid + u * kBlock < n) keys[by_leaf[u]] = (unsigned short)key[u];
+  }
+
+  // sums of runs: `to(bin, sums)` takes those of one
+  auto hand_in = [&](auto numbers, auto to) {
+    constexpr int count = decltype(numbers)::value;
+    for (int e0 = warp * 32; e0 < n; e0 += kBlock) {
+      const int e = e0 + lane;
+      Real sum[count];
+#pragma unroll
+      for (int k = 0; k < count; ++k) sum[k] = e < n && (k == 0 || k < a.M) ? terms[k * S + e] : (Real)0;
+      const uint32_t bin = e < n ? keys[e] : 0xffffu;
+      if (sums_of_runs(bin, sum, lane) && e < n) to(bin, sum);
+    }
+  };
+  const Real *w = a.w + (int64_t)tree * L * a.M;
+  Real through[PER];  // the gradient that arrives at the margin
+#pragma unroll
+  for (int u = 0; u < PER; ++u) through[u] = (Real)0;
+  for (int64_t m0 = 0; m0 < a.M; m0 += W) {
+    const int here = (int)min((int64_t)W, a.M - m0);
+#pragma unroll
+    for (int u = 0; u < PER; ++u) {
+      if (tid + u * kBlock >= n) continue;
+      const Real s = sign_of(margin[u]), am = abs_of(margin[u]);
+      const Real *gl = g + (((int64_t)sample[u] * a.Co + j) * a.out_count + position[u]) * a.M + m0, *wl = w + (int64_t)key[u] * a.M + m0;
+#pragma unroll
+      for (int k = 0; k < W; ++k) {
+        if (k >= here) break;
+        const Real gm = __ldg(gl + k);
+        through[u] = add_rn(through[u], mul_rn(mul_rn(s, __ldg(wl + k)), gm));
+        if (gw != nullptr) terms[k * S + by_leaf[u]] = mul_rn(am, gm);
+      }
+    }
+    if (gw == nullptr) continue;
+    __syncthreads();
+    Real *dst = gw + (int64_t)tree * L * a.M + m0;
+    if (here == 1) {
+      hand_in(std::integral_constant<int, 1>{}, [&](uint32_t bin, Real(&sum)[1]) { atomicAdd(dst + (int64_t)bin * a.M, sum[0]); });
+    } else {
+      hand_in(std::integral_constant<int, W>{}, [&](uint32_t bin, Real(&sum)[W]) {
+        Real *to = dst + (int64_t)bin * a.M;
+        if constexpr (W == 4) {
+          if (quad_sums) return red_add_quad(to, sum[0], sum[1], sum[2], sum[3]);
+        }
+#pragma unroll
+        for (int k = 0; k < W; ++k)
+          if (k < here) atomicAdd(to + k, sum[k]);
+      });
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    if (tid + u * kBlock >= n) continue;
+    if (gx != nullptr) {
+      const int idx = cell_index(a, origin[u], cells[vertex[u]]);
+      if (idx >= 0) atomicAdd(gx + ((int64_t)sample[u] * a.Ci + c) * a.in_count + idx, through[u]);  // a padding cell has no gradient
+    }
+  }
+  if (gthr == nullptr) return;
+  __syncthreads();  // every thread has read its place among the leaves, and the leaves' sums have been read
+#pragma unroll
+  for (int u = 0; u < PER; ++u) {
+    if (tid + u * kBlock >= n) continue;
+    terms[by_vertex[u]] = -through[u];
+    keys[by_vertex[u]] = (unsigned short)vertex[u];
+  }
+  __syncthreads();
+  hand_in(std::integral_constant<int, 1>{}, [&](uint32_t bin, Real(&sum)[1]) { atomicAdd(gthr + (int64_t)tree * N + bin, sum[0]); });
 }
 
 // ---- contract / expand: non-overlapping windows <-> image, any element size ----------------
@@ -490,6 +725,15 @@ int run_patches(bool contract, int dims, int elem_bytes, const void *in, void *o
   }
 }
 
+// Whether a call's outputs are too few for a thread each to fill the machine (and the leaves' places fit 32 bits).  Up to some 85 000
+// of them eight warps per channel are better, fewer where there are fewer channels than warps: 60000 outputs of 24 channels 62 us with
+// a thread each, 38 shared; 20776 of 7 21 and 8; 81000 of 52 198 and 127; but 144342 of 29 71 and 85, 69984 of 6 14.6 and 16.6, 25984
+// of 2 8.6 and 10.5.
+bool shares_channels(const ConvShape &a) {
+  return a.Ci > 2 && a.M <= kSharing * kSharedOutputs && a.Co * a.Ci * a.L <= 0xffffffffll &&
+         a.B * a.Co * a.out_count * kSharing <= 148 * 576 * std::min<int64_t>(a.Ci, kSharing);
+}
+
 // Forward / backward for either precision; the shared-memory tile kernels are single precision only.
 template <typename Real>
 int conv_forward(const ht_conv_problem *p, const Real *x, const Real *thr, const int64_t *ord, const Real *w, Real *out,
@@ -517,10 +761,40 @@ int conv_forward(const ht_conv_problem *p, const Real *x, const Real *thr, const
       }
     }
   }
-  if (p->kind == TREE)
-    conv_forward_kernel<TREE, Real><<<blocks_for(threads), kBlock, 0, s>>>(a, out);
-  else
-    conv_forward_kernel<FERN, Real><<<blocks_for(threads), kBlock, 0, s>>>(a, out);
+  if (shares_channels(a)) {
+    auto kernel = p->kind == TREE ? conv_forward_shared_kernel<TREE, Real> : conv_forward_shared_kernel<FERN, Real>;
+    kernel<<<(unsigned)((threads + 31) / 32), 32 * kSharing, 0, s>>>(a, out);
+  } else {
+    auto kernel = p->kind == TREE ? conv_forward_kernel<TREE, Real> : conv_forward_kernel<FERN, Real>;
+    kernel<<<blocks_for(threads), kBlock, 0, s>>>(a, out);
+  }
+  HT_CHECK_LAUNCH();
+  return HT_OK;
+}
+
+// HT_ERR_UNSUPPORTED: trees with too many bins, more evaluations than 31 bits count, and calls that conv_backward_kernel serves better:
+// enough outputs for a thread each, one output per leaf, and leaves enough for the reductions to spread (2486 trees of depth 7,
+// 3-D: 1264 us there, 1479 sorted; 3132 of depth 6 216 and 266; 2856 of depth 7 and 139944 outputs, the step, 450 and 473; but 2499 ferns of depth 3 479 and 407, and with few outputs 1254 trees
+// of depth 6 92 and 22).
+template <typename Real>
+int launch_backward_sorted(const ConvArgsOf<Real> &a, int kind, const Real *g, Real *gx, Real *gthr, Real *gw, cudaStream_t stream) {
+  const int64_t evals = a.B * a.out_count, trees = a.Co * a.Ci;
+  if (a.L + a.N > kSortedBins || evals >= ((int64_t)1 << 31) || trees >= ((int64_t)1 << 31)) return HT_ERR_UNSUPPORTED;
+  if (a.M == 1 && trees * a.L >= 131072 && evals * a.Co >= 148 * 768) return HT_ERR_UNSUPPORTED;
+  // Four evaluations per thread where the last slices are not too empty and there are CTAs enough: 6000 evaluations of 363 trees 83 us
+  // with one per thread, 72 with four; 28090 of 575 633 and 531; but 390 of 1254 22 and 30, 10658 of 9 6 and 11.
+  const int64_t slices = (evals + 4 * kBlock - 1) / (4 * kBlock);
+  const bool wide = slices * trees >= 4 * 148 && slices * 4 * kBlock * 3 <= evals * 4;
+  const int per = wide ? 4 : 1;
+  const int64_t grid = (evals + per * kBlock - 1) / (per * kBlock) * trees;
+  if (grid > 0x7fffffff) return HT_ERR_UNSUPPORTED;
+  const int quad_sums = sorted_terms<Real>() == 4 && a.M % 4 == 0 && (reinterpret_cast<uintptr_t>(gw) & 15u) == 0;
+  auto kernel = kind == TREE ? (wide ? conv_backward_sorted_kernel<TREE, Real, 4> : conv_backward_sorted_kernel<TREE, Real, 1>)
+                             : (wide ? conv_backward_sorted_kernel<FERN, Real, 4> : conv_backward_sorted_kernel<FERN, Real, 1>);
+  PositionDivisors by;
+  for (int d = 0; d < 3; ++d) by.size[d] = Divisor((uint32_t)a.osize[d]);
+  kernel<<<(unsigned)grid, kBlock, conv_sorted_places<Real>(a, (uint32_t)(per * kBlock)).bytes, stream>>>(a, Divisor((uint32_t)a.out_count), by, (uint32_t)evals,
+                                                                            (uint32_t)trees, quad_sums, g, gx, gthr, gw);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }
@@ -558,10 +832,10 @@ int conv_backward(const ht_conv_problem *p, const Real *x, const Real *thr, cons
       }
     }
   }
-  if (p->kind == TREE)
-    conv_backward_kernel<TREE, Real><<<blocks_for(threads), kBlock, 0, s>>>(a, g, gx, gthr, gw);
-  else
-    conv_backward_kernel<FERN, Real><<<blocks_for(threads), kBlock, 0, s>>>(a, g, gx, gthr, gw);
+  const int sorted = launch_backward_sorted<Real>(a, p->kind, g, gx, gthr, gw, s);
+  if (sorted != HT_ERR_UNSUPPORTED) return sorted;
+  auto kernel = p->kind == TREE ? conv_backward_kernel<TREE, Real> : conv_backward_kernel<FERN, Real>;
+  kernel<<<blocks_for(threads), kBlock, 0, s>>>(a, g, gx, gthr, gw);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }

@@ -4,6 +4,7 @@
 // together.
 // sorted_backward_kernel: the paths of one tree and a slice of the samples are sorted by leaf in shared memory, after which
 // the leaf-weight gradient of a leaf is a sum in registers.
+#include "ht_counting_sort.cuh"
 #include "ht_forest_multi.cuh"
 #include "ht_tile_common.cuh"
 
@@ -166,40 +167,6 @@ __host__ __device__ constexpr int sort_blocks(int numbers) {
 template <typename Real>
 __host__ __device__ constexpr int sort_ahead(int numbers) {
   return numbers * (int)sizeof(Real) > 16 ? 2 : 4;
-}
-
-// Turns counts[0 .. 4 * quads) into the sums of what is before each.  All threads of the block; partial: a number per warp.
-template <int THREADS>
-__device__ __forceinline__ void exclusive_sums(uint4 *counts, int quads, uint32_t *partial) {
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int per = (quads + THREADS - 1) / THREADS;  // 16 bytes each: one up to 1024 numbers
-  const int first = min(tid * per, quads), last = min(first + per, quads);
-  uint32_t mine = 0;
-  for (int b = first; b < last; ++b) {
-    const uint4 c = counts[b];
-    mine += c.x + c.y + c.z + c.w;
-  }
-  uint32_t sum = mine;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t below = __shfl_up_sync(0xffffffffu, sum, d);
-    if (lane >= d) sum += below;
-  }
-  if (lane == 31) partial[warp] = sum;
-  __syncthreads();
-  uint32_t base = sum - mine;
-#pragma unroll
-  for (int k = 0; k < THREADS / 32 - 1; ++k) base += k < warp ? partial[k] : 0u;
-  for (int b = first; b < last; ++b) {
-    uint4 c = counts[b], before;
-    before.x = base;
-    before.y = before.x + c.x;
-    before.z = before.y + c.y;
-    before.w = before.z + c.z;
-    base = before.w + c.w;
-    counts[b] = before;
-  }
-  __syncthreads();
 }
 
 // Evaluations per CTA: whole rounds for every group of lanes (three and five lanes per evaluation leave 80 and 48 groups).
@@ -576,21 +543,12 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
     }
     return;
   }
-  // warps sum runs of 32: a lane adds what is d lanes above while that is the same vertex
+  // warps sum runs of 32
   for (int e0 = warp * 32; e0 < n; e0 += kSortThreads) {
     const int e = e0 + lane;
-    Real sum = e < n ? by_vertex[e] : (Real)0;
+    Real sum[1] = {e < n ? by_vertex[e] : (Real)0};
     const uint32_t vertex = e < n ? vertices[e] : 0xffffu;
-    const uint32_t before = __shfl_up_sync(0xffffffffu, vertex, 1);
-    const bool leads = lane == 0 || before != vertex;
-    const uint32_t leaders = __ballot_sync(0xffffffffu, leads) & ~((2u << lane) - 1u);  // of the runs above this lane's
-    const int last = (leaders != 0u ? __ffs((int)leaders) - 1 : 32) - lane;             // lanes to the end of the run
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const Real other = __shfl_down_sync(0xffffffffu, sum, d);
-      if (d < last) sum += other;
-    }
-    if (e < n && leads) atomicAdd(a.gthr + j * a.N + vertex, -sum);
+    if (sums_of_runs(vertex, sum, lane) && e < n) atomicAdd(a.gthr + j * a.N + vertex, -sum[0]);
   }
 }
 
