@@ -200,6 +200,33 @@ struct Divisor {
   __device__ __forceinline__ uint32_t quotient_above_one(uint32_t n) const { return __umulhi(n, factor) >> (shift - 1); }
 };
 
+// (i, j, k) of evaluation e = (i * T + j) * K + k.  Two divisions of 64 bits are some 200 instructions, more than the walk of a tree of
+// ten levels; up to 2^31 evaluations the quotients are products.
+struct EvalDivisors {
+  Divisor T, K;
+  int narrow = 0;
+  EvalDivisors() = default;
+  EvalDivisors(int64_t evals, int64_t trees, int64_t positions) {
+    if (evals <= 0 || evals >= ((int64_t)1 << 31)) return;
+    T = Divisor((uint32_t)trees);
+    K = Divisor((uint32_t)positions);
+    narrow = 1;
+  }
+  __device__ __forceinline__ void split(int64_t e, int64_t trees, int64_t positions, int64_t &i, int64_t &j, int64_t &k) const {
+    if (narrow) {
+      const uint32_t ij = K.quotient((uint32_t)e), row = T.quotient(ij);
+      k = (uint32_t)e - ij * K.number;
+      j = ij - row * T.number;
+      i = row;
+    } else {
+      const int64_t ij = e / positions;
+      k = e - ij * positions;
+      i = ij / trees;
+      j = ij - i * trees;
+    }
+  }
+};
+
 // Memory to be zeroed before the kernels of a call add into it.
 struct ClearList {
   static constexpr int kMost = 5;

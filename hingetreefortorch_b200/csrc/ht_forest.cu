@@ -54,21 +54,13 @@ struct ForestArgsOf {
   const Real *w;
   int64_t B, C, K, T, N, L, M;
   int depth;
+  EvalDivisors by;
 };
 using ForestArgs = ForestArgsOf<float>;
 
 template <typename Real>
 __device__ __forceinline__ void split_index(const ForestArgsOf<Real> &a, int64_t e, int64_t &i, int64_t &j, int64_t &k) {
-  if (a.K == 1) {
-    k = 0;
-    i = e / a.T;
-    j = e - i * a.T;
-  } else {
-    const int64_t ij = e / a.K;
-    k = e - ij * a.K;
-    i = ij / a.T;
-    j = ij - i * a.T;
-  }
+  a.by.split(e, a.T, a.K, i, j, k);
 }
 
 enum { MODE_FORWARD = 0, MODE_LEAFMAP = 1, MODE_MARGINMAP = 2, MODE_REACH = 3 };
@@ -333,6 +325,7 @@ int prepare(const ht_forest_problem *p, const Real *x, const Real *thr, const in
   a.L = ((int64_t)1) << p->depth;
   out.stream = reinterpret_cast<cudaStream_t>(stream);
   out.evals = p->B * p->T * p->K;
+  a.by = EvalDivisors(out.evals, p->T, p->K);
   return HT_OK;
 }
 

@@ -78,6 +78,7 @@ struct MultiForwardArgs {
   void *where;
   int64_t evals, T, C, K, N, L;
   int M, depth, narrow;
+  EvalDivisors by;
   uint32_t divide_M;  // ceil(2^32 / M): quotients of numbers below 32 M (0: M is too large for it)
 };
 
@@ -92,16 +93,8 @@ __global__ void __launch_bounds__(kForwardThreads) multi_forward_kernel(const __
   Real am = (Real)0;
   uint32_t leaf = 0;
   if (e < a.evals) {
-    int64_t i, j, k = 0;
-    if (a.K == 1) {
-      i = e / a.T;
-      j = e - i * a.T;
-    } else {
-      const int64_t ij = e / a.K;
-      k = e - ij * a.K;
-      i = ij / a.T;
-      j = ij - i * a.T;
-    }
+    int64_t i, j, k;
+    a.by.split(e, a.T, a.K, i, j, k);
     const PlainFeatureOf<Real> feat{a.x + i * a.C * a.K + k, a.K};
     PathOf<Real> p;
     if constexpr (WIDE) {
@@ -636,6 +629,7 @@ int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, co
   a.depth = p->depth;
   a.narrow = where_bytes(p->depth) == 2;
   a.divide_M = p->M > kMaxDivisor ? 0 : (uint32_t)(((1ull << 32) + p->M - 1) / (uint64_t)p->M);
+  a.by = EvalDivisors(a.evals, a.T, a.K);
   a.margin = paths.margin;
   a.where = paths.where;
   const int width = vector_width(p->M, sizeof(Real), {w, out});
