@@ -495,6 +495,25 @@ static bool rows_are_better(const ht_forest_problem *p, bool keep) {
   return rows < (tiles < 0.0 ? thread_forward_cost(p, keep) : tiles);
 }
 
+// Whether resident tiles of samples are better than a thread per evaluation (inner positions; one walk is as good as the other where
+// the tiles do not take the sizes): where their estimate is the lower one.  Tiles read all features of a sample once, threads the ones
+// that a walk meets, whose lanes are on as many cache lines as the level has vertices; so tiles are for many trees on few features.
+// Both estimates are fits to 360 forwards of random sizes that were timed both ways in one session; time of the chosen kernels over
+// that of the better ones, all calls together 1.012, geometric mean 1.013 (always tiles 1.217 and 1.535, never 1.616 and 1.291, tiles
+// for one output per leaf alone 1.306 and 1.284).  2796 x 284 x 169, 8 trees of depth 4: tiles 520 us, threads 47; 228 x 47 x 576,
+// 466 trees of depth 5: 208 and 673.
+static bool inner_tiles_are_better(const ht_forest_problem *p, bool keep) {
+  const double tiles = inner_tiled_cost(p, keep);
+  if (tiles < 0.0) return false;
+  const double evals = 1e-6 * (double)p->B * (double)p->K * (double)p->T;
+  double lines = 0.0;  // cache lines that a warp's levels are on
+  for (int l = 0; l < p->depth; ++l) lines += p->kind == FERN ? 1.0 : std::min(24.0, (double)(1u << l));
+  const bool far = p->C * p->K * 4 > 2000000;  // the features of a row leave L1
+  const double threads = 5.3 + evals * (5.46 + (far ? 0.840 : 0.647) * p->depth + 0.0373 * lines + 0.253 * (double)p->M +
+                                        0.705 * (double)p->M / vector_width(p->M, sizeof(float), {}) + (keep && p->M > 1 ? 1.48 : 0.0));
+  return tiles < threads;
+}
+
 // What a backward keeps per evaluation: the records of the tile kernels (one output per leaf), or the paths (several) and,
 // in fixed-order mode, their lists.
 static size_t records_bytes(const ht_forest_problem *p) {
@@ -515,6 +534,7 @@ int ht_forest_forward_kernel(const ht_forest_problem *p) {
   if (rc != HT_OK) return rc;
   const bool keep = (p->flags & HT_SAVE_FOR_BACKWARD) != 0 && ht_forest_forward_saves(p);
   if (rows_are_better(p, keep)) return HT_FORWARD_ROWS;
+  if (p->K > 1 && !inner_tiles_are_better(p, keep)) return HT_FORWARD_THREADS;
   return forward_tiled_workspace_bytes(p) > 0 ? HT_FORWARD_TILES : HT_FORWARD_THREADS;
 }
 
@@ -543,7 +563,7 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
   const WideOrdinals wide = {ord, p->C};
   int32_t *packed = static_cast<int32_t *>(workspace);
   const bool by_rows = rows_are_better(p, eval_records != nullptr);
-  if (!by_rows) {
+  if (!by_rows && (p->K == 1 || inner_tiles_are_better(p, eval_records != nullptr))) {
     rc = forward_tiled(p, x, thr, packed, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream, &wide);
     if (rc != HT_ERR_UNSUPPORTED) return rc;
   }
@@ -649,7 +669,7 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
         const PathRecordsOf<float> paths = saved_paths(p, eval_records);
         int prc = HT_ERR_UNSUPPORTED;
         if (rows_are_better(p, true)) prc = rows_forward(p, x, thr, a.ord, w, none, paths.margin, paths.where, status_word, pr.stream);
-        if (prc == HT_ERR_UNSUPPORTED && p->M > 1)
+        if (prc == HT_ERR_UNSUPPORTED && p->M > 1 && (p->K == 1 || inner_tiles_are_better(p, true)))
           prc = forward_tiled(p, x, thr, static_cast<int32_t *>(workspace), w, none, ws + ordinals_bytes(p), eval_records, status_word,
                               pr.stream);
         if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, paths, pr.stream);

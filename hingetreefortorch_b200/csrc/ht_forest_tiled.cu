@@ -1,7 +1,7 @@
 // Shared-memory tile kernels for the forest forward.
 //
-// forest_forward_tiled_kernel: tabular input (K == 1), one or several outputs per leaf.
-// forest_forward_tiled_inner_kernel: inputs with inner positions (x [B, C, K...]), one output per leaf.
+// forest_forward_tiled_kernel: tabular input (K == 1), one or several outputs per leaf.  Inputs with inner positions:
+// ht_forest_tiled_inner.cu.
 //
 // Work decomposition (one CTA of 1024 threads per tile, sized for one CTA per SM):
 //   * a CTA owns S consecutive samples and walks ALL trees (or, when the batch alone gives too
@@ -37,6 +37,7 @@
 // |feature - threshold| bit for bit.
 #include "ht_eval_records.cuh"
 #include "ht_forest_multi.cuh"
+#include "ht_forest_tile_plan.cuh"
 #include "ht_forest_tiled.cuh"
 #include "ht_tile_common.cuh"
 #include "ht_tma.cuh"
@@ -50,16 +51,6 @@ using namespace tile;
 
 namespace {
 
-
-struct TilePlan {
-  bool weights;    // the records carry the leaf weights (one output per leaf)
-  int S;           // samples per tile
-  int G;           // trees per parameter group
-  int per_warp;    // trees a warp walks at once: G / slots
-  int ord_bytes;   // 1 or 2
-  RecordLayout rec;
-  size_t smem;
-};
 
 // Shared-memory layout of forest_forward_tiled_kernel, from a 1024-byte boundary: the results area (a
 // staging row per sample with one output per leaf — boxes the TMA engine can store —, or the warps'
@@ -97,45 +88,6 @@ bool make_plan(const ht_forest_problem *p, TilePlan &plan) {
   }
   return false;
 }
-
-// Inputs with inner positions (x [B, C, K], K > 1; one output per leaf): a sample is a (row, position)
-// pair and its features are K elements apart, so consecutive samples of a tile are consecutive
-// positions — contiguous in x and, for a fixed tree, in the output.  No staging of results is needed.
-bool make_inner_plan(const ht_forest_problem *p, TilePlan &plan) {
-  if (p->K <= 1 || p->M != 1) return false;
-  if (p->C > 65536 || p->depth > 12) return false;
-  if (p->B * p->K * p->T < 32 * 1024) return false;
-  plan.ord_bytes = p->C <= 256 ? 1 : 2;
-  plan.rec = record_layout(p->kind, p->depth, (uint32_t)plan.ord_bytes, true,
-                           paired_ordinals(p->kind, p->depth, (uint32_t)plan.ord_bytes));
-  plan.weights = true;
-  plan.per_warp = 4;
-  for (int S = 256; S >= 32; S >>= 1) {
-    plan.S = S;
-    plan.G = (kWarps / (S / 32)) * plan.per_warp;
-    plan.smem = (size_t)p->C * S * 4 + 2 * (size_t)plan.G * plan.rec.bytes + 64;
-    if (plan.smem <= kSmemBudget) return true;
-  }
-  return false;
-}
-
-struct TiledArgs {
-  CUtensorMap out_map;  // the output [B, T] in boxes of 32 rows x G trees (when tma_store is set)
-  const float *x;
-  const unsigned char *records;
-  const float *w;  // leaf weights in global memory, read when there are several outputs per leaf
-  float *out;
-  uint32_t *status_word;
-  int64_t B, T, K;
-  int C, S, G, per_warp, M;
-  int width;                 // several outputs per leaf: numbers per load and store
-  Divisor by_M, by_pieces;   // ... and what a place in a warp's outputs is divided by
-  int tma_store;  // results of full groups leave through the TMA engine (G is 16 or 32)
-  // a forward that saves its traversal for the backward (SAVE kernels): threshold - feature at the deciding
-  // vertex, and the packed vertex / leaf key, in the evaluation-record layout
-  float *save_margin;
-  void *save_where;
-};
 
 template <int KIND, int DEPTH, typename OrdT, bool WREC, bool SAVE = false>
 __global__ void __launch_bounds__(kThreads, 1) forest_forward_tiled_kernel(const __grid_constant__ TiledArgs a) {
@@ -488,130 +440,8 @@ __global__ void __launch_bounds__(kThreads, 1) forest_forward_tiled_kernel(const
   if (store_issuer) tma::wait_stores_read();  // shared memory stays valid until the last box has been read
 }
 
-template <int KIND, int DEPTH, typename OrdT>
-__global__ void __launch_bounds__(kThreads, 1) forest_forward_tiled_inner_kernel(const __grid_constant__ TiledArgs a) {
-  extern __shared__ __align__(1024) unsigned char smem[];
-  constexpr RecordLayout lay =
-      record_layout(KIND, DEPTH, (uint32_t)sizeof(OrdT), true, paired_ordinals(KIND, DEPTH, (uint32_t)sizeof(OrdT)));
-  const int S = a.S, G = a.G, C = a.C;
-  float *xs = reinterpret_cast<float *>(smem);
-  unsigned char *params = smem + (size_t)C * S * 4;
-  uint64_t *full = reinterpret_cast<uint64_t *>(params + 2 * (size_t)G * lay.bytes);
-  uint32_t *finished = reinterpret_cast<uint32_t *>(full + 2);
-
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-  const int groups_of_samples = S >> 5;
-  const int sample_group = warp % groups_of_samples;
-  const int slot = warp / groups_of_samples;
-  const int64_t samples = a.B * a.K;
-  const int64_t sample0 = (int64_t)blockIdx.x * S;
-  const int all_groups = (int)((a.T + G - 1) / G);
-  const int groups_per_cta = (all_groups + (int)gridDim.y - 1) / (int)gridDim.y;
-  const int group0 = (int)blockIdx.y * groups_per_cta;
-  const int num_groups = max(0, min(groups_per_cta, all_groups - group0));
-  const uint32_t params_addr = smem_addr(params);
-
-  auto issue = [&](int it) {
-    const int64_t first_tree = (int64_t)(group0 + it) * G;
-    const int64_t count = min((int64_t)G, a.T - first_tree);
-    const uint32_t bytes = (uint32_t)(count * lay.bytes);
-    uint64_t *bar = &full[it & 1];
-    mbar_expect_tx(bar, bytes);
-    bulk_load(params_addr + (uint32_t)(it & 1) * (uint32_t)G * lay.bytes, a.records + first_tree * lay.bytes, bytes, bar);
-  };
-  if (tid == 0) {
-    mbar_init(&full[0], 1);
-    mbar_init(&full[1], 1);
-    finished[0] = 0;
-    finished[1] = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (num_groups > 0) issue(0);
-    if (num_groups > 1) issue(1);
-  }
-
-  // features of the tile's samples, feature-major; consecutive samples are consecutive positions.
-  // A thread stages the features c0, c0 + step, ... of one sample, or of 4 consecutive positions
-  // at a time when the rows allow 16-byte loads (S divides the thread count; a tile starts on a
-  // multiple of S, so 4 positions never straddle a row when 4 divides K)
-  if ((a.K & 3) == 0) {
-    const int quads = S >> 2, t = (tid % quads) * 4, c_step = kThreads / quads;
-    const int64_t sample = sample0 + t;
-    const bool inside = sample < samples;  // then sample + 3 < samples as well
-    const int64_t row = inside ? sample / a.K : 0, k = inside ? sample - row * a.K : 0;
-    const float *src = a.x + row * C * a.K + k;
-    for (int c = tid / quads; c < C; c += c_step) {
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (inside) v = __ldg(reinterpret_cast<const float4 *>(src + (int64_t)c * a.K));
-      *reinterpret_cast<float4 *>(xs + c * S + t) = v;
-    }
-  } else {
-    const int t = tid % S, c_step = kThreads / S;
-    const int64_t sample = sample0 + t;
-    const bool inside = sample < samples;
-    const int64_t row = inside ? sample / a.K : 0, k = inside ? sample - row * a.K : 0;
-    const float *src = a.x + row * C * a.K + k;
-    for (int c = tid / S; c < C; c += c_step) xs[c * S + t] = inside ? __ldg(src + (int64_t)c * a.K) : 0.0f;
-  }
-  __syncthreads();
-
-  const int64_t my_sample = sample0 + sample_group * 32 + lane;
-  const bool valid = my_sample < samples;
-  const int64_t my_row = valid ? my_sample / a.K : 0, my_k = valid ? my_sample - my_row * a.K : 0;
-  float *my_out = a.out + my_row * a.T * a.K + my_k;  // tree j of this sample: + j * K
-  const uint32_t xl_addr = smem_addr(xs + sample_group * 32 + lane);
-  const uint32_t x_stride = (uint32_t)S * 4u;
-  const int t_first = slot * 4;
-  bool poisoned = false;
-
-  for (int it = 0; it < num_groups; ++it) {
-    const int group = group0 + it;
-    if (!poisoned && !mbar_wait(&full[it & 1], (uint32_t)((it >> 1) & 1))) {
-      poisoned = true;
-      if (a.status_word != nullptr) atomicOr(a.status_word, HT_FLAG_PIPELINE_TIMEOUT);
-    }
-    const int in_group = (int)min((int64_t)G, a.T - (int64_t)group * G);
-    const uint32_t base_addr = params_addr + (uint32_t)(it & 1) * (uint32_t)G * lay.bytes;
-    float result[4] = {0.f, 0.f, 0.f, 0.f};
-    if (t_first < in_group && !poisoned) {
-      uint32_t rec[4], unused[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) rec[u] = base_addr + (uint32_t)min(t_first + u, in_group - 1) * lay.bytes;
-      walk<KIND, DEPTH, OrdT, 4, true>(rec, xl_addr, x_stride, result, unused);
-    }
-    __syncwarp();
-    if (lane == 0) {
-      __threadfence_block();
-      const uint32_t before = atomicAdd(&finished[it & 1], 1u);
-      if (before == kWarps - 1) {
-        atomicExch(&finished[it & 1], 0u);
-        __threadfence_block();
-        if (it + 2 < num_groups) issue(it + 2);
-      }
-    }
-    if (valid) {
-      float *dst = my_out + ((int64_t)group * G + t_first) * a.K;
-#pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (t_first + u < in_group) dst[(int64_t)u * a.K] = result[u];
-    }
-  }
-}
-
-template <typename Kernel>
-int launch_one(Kernel kernel, const TilePlan &plan, const TiledArgs &a, dim3 grid, cudaStream_t stream) {
-  HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
-  kernel<<<grid, kThreads, plan.smem, stream>>>(a);
-  HT_CHECK_LAUNCH();
-  return HT_OK;
-}
-
 template <int KIND, int DEPTH>
 int launch_depth(const TilePlan &plan, const TiledArgs &a, dim3 grid, cudaStream_t stream) {
-  if (a.K > 1) {
-    if (plan.ord_bytes == 1) return launch_one(forest_forward_tiled_inner_kernel<KIND, DEPTH, uint8_t>, plan, a, grid, stream);
-    return launch_one(forest_forward_tiled_inner_kernel<KIND, DEPTH, uint16_t>, plan, a, grid, stream);
-  }
   const bool wrec = plan.weights;
   if (a.save_margin != nullptr) {
     if (plan.ord_bytes == 1)
@@ -694,15 +524,16 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
     return HT_ERR_UNSUPPORTED;
   const int64_t N = threshold_count(p->kind, p->depth);
   const int64_t L = ((int64_t)1) << p->depth;
-  const int64_t elements = p->T * (N + L);
+  const int outputs = plan.weights ? (int)p->M : 1;  // of a leaf, in the records
+  const int64_t elements = p->T * (N + L * outputs);
   const unsigned pack_grid = (unsigned)((elements + 255) / 256);
   unsigned char *rec = static_cast<unsigned char *>(records);
   PackOnTheWay pack;
   if (wide != nullptr) pack = PackOnTheWay{wide->at, wide->channels, ord, status_word};
   if (plan.ord_bytes == 1)
-    repack_records_kernel<uint8_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec, RecordMap(), pack);
+    repack_records_kernel<uint8_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec, RecordMap(), pack, outputs);
   else
-    repack_records_kernel<uint16_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec, RecordMap(), pack);
+    repack_records_kernel<uint16_t><<<pack_grid, 256, 0, stream>>>(thr, ord, w, rec, p->kind, p->depth, p->T, plan.rec, RecordMap(), pack, outputs);
   HT_CHECK_LAUNCH();
 
   TiledArgs a = {};
@@ -712,7 +543,8 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
   a.M = (int)p->M;
   a.width = vector_width(p->M, sizeof(float), {w, out});
   a.by_M = Divisor((uint32_t)p->M);
-  a.by_pieces = Divisor((uint32_t)(plan.per_warp * p->M / a.width));
+  a.by_K = Divisor((uint32_t)p->K);
+  a.by_pieces = Divisor((uint32_t)std::max<int64_t>(1, plan.per_warp * p->M / a.width));
   a.out = out;
   a.status_word = status_word;
   a.B = p->B;
@@ -722,6 +554,7 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
   a.S = plan.S;
   a.G = plan.G;
   a.per_warp = plan.per_warp;
+  a.record_bytes = plan.rec.bytes;
   a.save_margin = nullptr;
   a.save_where = nullptr;
   if (eval_records != nullptr && p->M > 1) {
@@ -745,6 +578,7 @@ int forward_tiled(const ht_forest_problem *p, const float *x, const float *thr, 
   if (tiles > 0x7fffffff) return HT_ERR_UNSUPPORTED;
   const int64_t groups = (p->T + plan.G - 1) / plan.G;
   const dim3 grid((unsigned)tiles, (unsigned)choose_splits(tiles, groups));
+  if (p->K > 1) return launch_inner(p->kind, p->depth, plan, a, grid, stream);
   return p->kind == TREE ? launch_kind<TREE>(p->depth, plan, a, grid, stream)
                          : launch_kind<FERN>(p->depth, plan, a, grid, stream);
 }

@@ -10,6 +10,8 @@ size_t forward_tiled_workspace_bytes(const ht_forest_problem *p);
 
 // Estimated microseconds of the tile kernel on tabular data; negative: not taken.
 double forward_tiled_cost(const ht_forest_problem *p);
+// ... and on inputs with inner positions; `keep`: the paths of several outputs per leaf are left, too.
+double inner_tiled_cost(const ht_forest_problem *p, bool keep);
 
 // Runs the forward with the tile kernel when the shape qualifies; returns HT_ERR_UNSUPPORTED
 // (and launches nothing) when it does not, so that the caller can use the any-shape kernel.

@@ -101,9 +101,9 @@ template <typename OrdT>
 __global__ void repack_records_kernel(const float *__restrict__ thr, const int32_t *__restrict__ ord,
                                       const float *__restrict__ w, unsigned char *__restrict__ records, int kind,
                                       int depth, int64_t T, RecordLayout lay, RecordMap map = RecordMap(),
-                                      PackOnTheWay pack = PackOnTheWay()) {
+                                      PackOnTheWay pack = PackOnTheWay(), int outputs = 1) {
   const int64_t N = threshold_count(kind, depth);
-  const int64_t L = ((int64_t)1) << depth;
+  const int64_t L = (((int64_t)1) << depth) * outputs;  // weights: `outputs` of a leaf side by side
   const int64_t per_tree = N + L;
   const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (e >= T * per_tree) return;
@@ -147,8 +147,8 @@ __global__ void repack_records_kernel(const float *__restrict__ thr, const int32
     }
     if (kind == TREE && r == 0) rec[13] = 0;
   } else if (lay.bytes > lay.w) {  // records that carry the leaf weights
-    const int64_t h = r - N;
-    reinterpret_cast<float *>(rec + lay.w)[h] = w[j * L + (int64_t)bit_reverse((uint32_t)h, depth)];
+    const uint32_t h = (uint32_t)(r - N), leaf = outputs == 1 ? h : h / (uint32_t)outputs;
+    reinterpret_cast<float *>(rec + lay.w)[h] = w[j * L + (int64_t)bit_reverse(leaf, depth) * outputs + (h - leaf * (uint32_t)outputs)];
   }
 }
 

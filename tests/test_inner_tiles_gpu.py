@@ -1,0 +1,74 @@
+"""Forwards of inputs with inner positions through resident tiles of samples: every form of the weights and of the outputs, rows that
+end inside a warp and inside a tile, last groups of trees that are short."""
+import ctypes
+
+import numpy as np
+import pytest
+import torch
+
+import hingetreefortorch_b200._cabi as _cabi
+from conftest import grad_close
+from oracle import hinge_oracle as ho
+from test_forest_gpu import dev, random_forest_inputs
+
+THREADS, TILES = 0, 1
+
+# B, C, inner, T, depth, M
+SHAPES = [
+    (40, 8, (33,), 401, 5, 2),      # rows of a warp and one position more
+    (200, 8, (7,), 403, 4, 3),      # several rows per warp; scalar staging
+    (2, 8, (20, 30), 517, 1, 4),
+    (3, 9, (516,), 530, 9, 5),      # dealt out one by one
+    (3, 9, (516,), 530, 7, 6),      # ... in twos
+    (3, 9, (516,), 530, 3, 8),      # ... in fours
+    (6, 300, (700,), 300, 6, 2),    # two-byte feature indices
+    (9, 20, (900,), 130, 9, 3),     # wide paths
+    (11, 16, (900,), 130, 10, 2),   # weights that leave no room for two trees at a time stay in global memory
+    (9, 12, (1000,), 60, 12, 7),
+    (5, 24, (1001,), 200, 8, 1),    # one output: weights in the records
+    (9, 200, (1000,), 200, 10, 1),  # ... in global memory
+    (60, 5, (85,), 70, 3, 1),
+]
+
+
+def taken(kind, x, w, keep=False):
+    p = _cabi.forest_problem(kind, x, w)
+    p.flags |= 4 if keep else 0  # HT_SAVE_FOR_BACKWARD
+    return _cabi.library().ht_forest_forward_kernel(ctypes.byref(p))
+
+
+def inputs(kind, shape):
+    B, C, inner, T, depth, M = shape
+    return random_forest_inputs(700 + SHAPES.index(shape), kind, B, C, inner, T, depth, (M,), quantise=True)
+
+
+@pytest.mark.parametrize("shape, want", [((2796, 284, (169,), 8, 4, 1), THREADS), ((228, 47, (576,), 466, 5, 1), TILES),
+                                         ((26, 1561, (3249,), 25, 4, 2), THREADS), ((135, 152, (2500,), 527, 3, 3), TILES)])
+def test_choice_between_tiles_and_threads(shape, want):
+    B, C, inner, T, depth, M = shape
+    assert taken("tree", torch.empty((B, C) + inner, device="meta"), torch.empty(T, 2 ** depth, M, device="meta")) == want
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["tree", "fern"])
+@pytest.mark.parametrize("shape", SHAPES, ids=[str(s) for s in SHAPES])
+def test_tiles_match_oracle(kind, shape):
+    x, thr, ord_, w = inputs(kind, shape)
+    want = ho.forward(kind, x, thr, ord_, w)
+    dx, dthr, dord, dw = dev(x, thr, ord_, w)
+    if kind == "tree":
+        assert taken(kind, dx, dw) == TILES
+    f = _cabi.Forest(kind, dx, dw)
+    assert np.array_equal(f.forward(dx, dthr, dord, dw).cpu().numpy(), want)
+    g = np.random.default_rng(5).standard_normal(want.shape).astype(np.float32)
+    ref, sizes = ho.backward(kind, x, thr, ord_, w, g), ho.backward_magnitudes(kind, x, thr, ord_, w, g)
+    dg, = dev(g)
+    assert np.array_equal(f.forward(dx, dthr, dord, dw, save=True).cpu().numpy(), want)
+    for got, r, s in zip(f.backward(dx, dthr, dord, dw, dg, saved=True), ref, sizes):
+        assert grad_close(got, r, s)
+    for got, r, s in zip(f.backward(dx, dthr, dord, dw, dg), ref, sizes):  # walked again
+        assert grad_close(got, r, s)
+    x.reshape(-1)[:3] = [np.inf, -np.inf, np.nan]
+    got = f.forward(dev(x)[0], dthr, dord, dw).cpu().numpy()
+    assert np.array_equal(got, ho.forward(kind, x, thr, ord_, w), equal_nan=True)
+    assert f.ordinal_flags() == 0
