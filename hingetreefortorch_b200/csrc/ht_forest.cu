@@ -498,10 +498,10 @@ static bool rows_are_better(const ht_forest_problem *p, bool keep) {
 // Whether resident tiles of samples are better than a thread per evaluation (inner positions; one walk is as good as the other where
 // the tiles do not take the sizes): where their estimate is the lower one.  Tiles read all features of a sample once, threads the ones
 // that a walk meets, whose lanes are on as many cache lines as the level has vertices; so tiles are for many trees on few features.
-// Both estimates are fits to 360 forwards of random sizes that were timed both ways in one session; time of the chosen kernels over
-// that of the better ones, all calls together 1.012, geometric mean 1.013 (always tiles 1.217 and 1.535, never 1.616 and 1.291, tiles
-// for one output per leaf alone 1.306 and 1.284).  2796 x 284 x 169, 8 trees of depth 4: tiles 520 us, threads 47; 228 x 47 x 576,
-// 466 trees of depth 5: 208 and 673.
+// Both estimates are fits to forwards of random sizes that were timed both ways in one session (profiles/inner_forward_choice.csv, 400
+// of them); time of the chosen kernels over that of the better ones, all calls together 1.010, geometric mean 1.011 (always tiles 1.189
+// in all, never 1.536, tiles for one output per leaf alone 1.266).  2796 x 284 x 169, 8 trees of depth 4: tiles 520 us, threads 47;
+// 228 x 47 x 576, 466 trees of depth 5: 208 and 673.
 static bool inner_tiles_are_better(const ht_forest_problem *p, bool keep) {
   const double tiles = inner_tiled_cost(p, keep);
   if (tiles < 0.0) return false;

@@ -72,3 +72,22 @@ def test_tiles_match_oracle(kind, shape):
     got = f.forward(dev(x)[0], dthr, dord, dw).cpu().numpy()
     assert np.array_equal(got, ho.forward(kind, x, thr, ord_, w), equal_nan=True)
     assert f.ordinal_flags() == 0
+
+
+def test_choice_against_the_times_of_both_kernels():
+    """profiles/inner_forward_choice.csv: forwards of random sizes, timed both ways."""
+    import csv
+    import math
+    import os
+    chosen = better = 0.0
+    logs = []
+    with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "profiles", "inner_forward_choice.csv")) as table:
+        for row in csv.DictReader(table):
+            B, C, K, T, depth, M = (int(row[c]) for c in ("B", "C", "K", "T", "depth", "M"))
+            p = _cabi.ForestProblem(_cabi.HT_KIND[row["kind"]], depth, B, C, K, T, M, 4 if row["keeps_paths"] == "1" else 0, 0)
+            takes = _cabi.library().ht_forest_forward_kernel(ctypes.byref(p))
+            tiles, threads = float(row["tiles_us"]), float(row["threads_us"])
+            chosen += tiles if takes == TILES else threads
+            better += min(tiles, threads)
+            logs.append(math.log((tiles if takes == TILES else threads) / min(tiles, threads)))
+    assert chosen <= 1.02 * better and math.exp(sum(logs) / len(logs)) <= 1.03
