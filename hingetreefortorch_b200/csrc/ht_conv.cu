@@ -239,7 +239,8 @@ __global__ void __launch_bounds__(kBlock) conv_backward_kernel(ConvArgsOf<Real> 
 // What bounds the kernel above is where its reductions meet: the trees of a convolution see every position of every sample, so
 // that a handful of thresholds and leaves take all terms one after the other.  It also walks the input channels of a position in
 // one thread.  159744 positions of 135 ferns of depth 3 (3-D): 3923 us there, 532 here; 30375 of 24 trees of depth 3 242 and 24;
-// 9947 of 420 trees of depth 4 with 4 outputs 468 and 137.  It is bound by latency: walks through L1, then six barriers per slice.
+// 9947 of 420 trees of depth 4 with 4 outputs 468 and 137.  Issue slots bound it (78 % used): 772 instructions per 32
+// evaluations at depth 4 with 4 outputs.
 // Slices of a tree next to each other instead of trees of a slice: 728 us for the first, 532 here (its tree's sums meet).
 constexpr int kSortedBins = 2048;  // leaves + decisions, at most: depth 10
 template <typename Real>
