@@ -148,6 +148,9 @@ inline int check_forest_problem(const ht_forest_problem *p) {
   return HT_OK;
 }
 
+// The workspace that a single-precision call is refused without; ht_forest_workspace_bytes() adds what makes it faster (ht_forest.cu).
+size_t least_forest_workspace_bytes(const ht_forest_problem *p);
+
 // The int64 feature indices of a call, read in place: out-of-range ones count as 0.
 struct WideOrdinals {
   const int64_t *__restrict__ at;

@@ -280,7 +280,8 @@ __global__ void __launch_bounds__(32) forest_backward_params_ordered_kernel(Fore
     for (int64_t t = lane; t < LM; t += 32) gw[j * LM + t] = w_bins[t];
 }
 
-// The workspace starts with the compact int32 ordinals; the tile kernel's records follow.
+// The workspace starts with the compact int32 ordinals; the tile kernel's records follow, then what a backward keeps, then the tile
+// records that a call can do without.
 inline size_t ordinals_bytes(const ht_forest_problem *p) {
   return align_up((size_t)(p->T * threshold_count(p->kind, p->depth)) * sizeof(int32_t), 256);
 }
@@ -307,7 +308,7 @@ int prepare(const ht_forest_problem *p, const Real *x, const Real *thr, const in
       (need_w && w == nullptr && p->T * p->M > 0))
     return HT_ERR_INVALID_ARGUMENT;
   // the double precision entry points run the any-shape kernels only: compact ordinals are all they keep
-  const size_t need = sizeof(Real) == 4 ? ht_forest_workspace_bytes(p) : ordinals_bytes(p) + 256;
+  const size_t need = sizeof(Real) == 4 ? least_forest_workspace_bytes(p) : ordinals_bytes(p) + 256;
   if (workspace == nullptr || workspace_bytes < need || (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0)
     return HT_ERR_WORKSPACE;
   ForestArgsOf<Real> &a = out.args;
@@ -524,6 +525,16 @@ static size_t records_bytes(const ht_forest_problem *p) {
 // What still serves the fixed order without the lists.
 static size_t records_without_lists(const ht_forest_problem *p) { return p->M == 1 ? backward_records_bytes(p) : 0; }
 
+// Where a forward finds room for the tile kernel's records (null: nowhere); `kept`: bytes that the call keeps for a backward.
+static void *tile_records_at(const ht_forest_problem *p, void *workspace, size_t workspace_bytes, size_t kept, bool keep) {
+  unsigned char *ws = static_cast<unsigned char *>(workspace);
+  if (p->K > 1 && !inner_tiles_are_better(p, keep)) return nullptr;
+  const size_t spare = inner_spare_records_bytes(p);
+  if (spare == 0) return ws + ordinals_bytes(p);
+  const size_t at = align_up(ordinals_bytes(p) + kept, 256);  // those records are there instead of others
+  return workspace_bytes >= at + spare ? ws + at : nullptr;
+}
+
 int ht_forest_forward_saves(const ht_forest_problem *p) {
   if (check_forest_problem(p) != HT_OK) return 0;
   return p->M == 1 ? forward_saves(p) : records_bytes(p) > 0;
@@ -534,14 +545,16 @@ int ht_forest_forward_kernel(const ht_forest_problem *p) {
   if (rc != HT_OK) return rc;
   const bool keep = (p->flags & HT_SAVE_FOR_BACKWARD) != 0 && ht_forest_forward_saves(p);
   if (rows_are_better(p, keep)) return HT_FORWARD_ROWS;
-  if (p->K > 1 && !inner_tiles_are_better(p, keep)) return HT_FORWARD_THREADS;
+  if (p->K > 1) return inner_tiles_are_better(p, keep) ? HT_FORWARD_TILES : HT_FORWARD_THREADS;
   return forward_tiled_workspace_bytes(p) > 0 ? HT_FORWARD_TILES : HT_FORWARD_THREADS;
 }
 
 size_t ht_forest_workspace_bytes(const ht_forest_problem *p) {
   if (check_forest_problem(p) != HT_OK) return 0;
-  const size_t base = ordinals_bytes(p) + forward_tiled_workspace_bytes(p) + 256;
-  return (p->flags & HT_WORKSPACE_FOR_BACKWARD) != 0 ? base + records_bytes(p) : base;
+  const size_t least = least_forest_workspace_bytes(p);
+  // with and without kept paths, so that the mode of a call does not matter
+  return p->K > 1 && (inner_tiles_are_better(p, false) || inner_tiles_are_better(p, true)) ? align_up(least, 256) + inner_spare_records_bytes(p)
+                                                                                            : least;
 }
 
 int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const float *thr, const int64_t *ord,
@@ -555,16 +568,21 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
   // HT_SAVE_FOR_BACKWARD: the traversal goes to the evaluation-record area of the workspace, when it is there
   unsigned char *ws = static_cast<unsigned char *>(workspace);
   void *eval_records = nullptr;
+  size_t kept = 0;
   if ((p->flags & HT_SAVE_FOR_BACKWARD) != 0 && ht_forest_forward_saves(p)) {
     const size_t records_at = ordinals_bytes(p) + forward_tiled_workspace_bytes(p);
-    const size_t kept = p->M == 1 ? records_without_lists(p) : records_bytes(p);
-    if (workspace_bytes >= records_at + kept) eval_records = ws + records_at;
+    const size_t bytes = p->M == 1 ? records_without_lists(p) : records_bytes(p);
+    if (workspace_bytes >= records_at + bytes) {
+      eval_records = ws + records_at;
+      kept = bytes;
+    }
   }
   const WideOrdinals wide = {ord, p->C};
   int32_t *packed = static_cast<int32_t *>(workspace);
   const bool by_rows = rows_are_better(p, eval_records != nullptr);
-  if (!by_rows && (p->K == 1 || inner_tiles_are_better(p, eval_records != nullptr))) {
-    rc = forward_tiled(p, x, thr, packed, w, out, ws + ordinals_bytes(p), eval_records, status_word, pr.stream, &wide);
+  void *tile_records = by_rows ? nullptr : tile_records_at(p, ws, workspace_bytes, kept, eval_records != nullptr);
+  if (tile_records != nullptr) {
+    rc = forward_tiled(p, x, thr, packed, w, out, tile_records, eval_records, status_word, pr.stream, &wide);
     if (rc != HT_ERR_UNSUPPORTED) return rc;
   }
   if (eval_records == nullptr && !by_rows && small_enough_for_wide(pr)) {
@@ -669,9 +687,9 @@ int ht_forest_backward_f32(const ht_forest_problem *p, const float *x, const flo
         const PathRecordsOf<float> paths = saved_paths(p, eval_records);
         int prc = HT_ERR_UNSUPPORTED;
         if (rows_are_better(p, true)) prc = rows_forward(p, x, thr, a.ord, w, none, paths.margin, paths.where, status_word, pr.stream);
-        if (prc == HT_ERR_UNSUPPORTED && p->M > 1 && (p->K == 1 || inner_tiles_are_better(p, true)))
-          prc = forward_tiled(p, x, thr, static_cast<int32_t *>(workspace), w, none, ws + ordinals_bytes(p), eval_records, status_word,
-                              pr.stream);
+        void *tile_records = p->M > 1 ? tile_records_at(p, workspace, workspace_bytes, eval_bytes, true) : nullptr;
+        if (prc == HT_ERR_UNSUPPORTED && tile_records != nullptr)
+          prc = forward_tiled(p, x, thr, static_cast<int32_t *>(workspace), w, none, tile_records, eval_records, status_word, pr.stream);
         if (prc == HT_ERR_UNSUPPORTED) prc = multi_forward(p, x, thr, a.ord, w, none, paths, pr.stream);
         if (prc != HT_OK) return prc;
       }
@@ -767,3 +785,12 @@ int ht_forest_backward_f64(const ht_forest_problem *p, const double *x, const do
 }
 
 }  // extern "C"
+
+namespace ht {
+
+size_t least_forest_workspace_bytes(const ht_forest_problem *p) {
+  const size_t base = ordinals_bytes(p) + forward_tiled_workspace_bytes(p) + 256;
+  return (p->flags & HT_WORKSPACE_FOR_BACKWARD) != 0 ? base + records_bytes(p) : base;
+}
+
+}  // namespace ht

@@ -54,7 +54,7 @@ int ht_forest_forward_static_f32(const ht_forest_problem *p, const float *x, con
   // the forward needs no backward records: size the request without them, whatever the caller's flags say
   ht_forest_problem forward_only = *p;
   forward_only.flags &= ~HT_WORKSPACE_FOR_BACKWARD;
-  if (ht_forest_workspace_bytes(&forward_only) > kStaticScratchBytes) return HT_ERR_WORKSPACE;
+  if (ht::least_forest_workspace_bytes(&forward_only) > kStaticScratchBytes) return HT_ERR_WORKSPACE;
   void *scratch = nullptr;
   const int src = resolve_scratch(&scratch);
   if (src != HT_OK) return src;

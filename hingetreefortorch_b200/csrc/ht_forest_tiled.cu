@@ -485,11 +485,21 @@ int launch_kind(int depth, const TilePlan &plan, const TiledArgs &a, dim3 grid, 
 
 size_t forward_tiled_workspace_bytes(const ht_forest_problem *p) {
   TilePlan plan;
-  if (!(p->K > 1 ? make_inner_plan(p, plan) : make_plan(p, plan))) return 0;
+  if (p->K > 1) {
+    if (p->M != 1 || !make_inner_plan(p, plan) || !plan.weights) return 0;
+  } else if (!make_plan(p, plan)) {
+    return 0;
+  }
   // one output per leaf: the backward's records carry the leaf weights whatever the forward's do
   const size_t with_weights =
       p->M == 1 ? record_layout(p->kind, p->depth, (uint32_t)plan.ord_bytes, true, plan.rec.paired).bytes : 0;
   return align_up((size_t)p->T * std::max<size_t>(plan.rec.bytes, with_weights), 256);
+}
+
+size_t inner_spare_records_bytes(const ht_forest_problem *p) {
+  TilePlan plan;
+  if (p->K <= 1 || forward_tiled_workspace_bytes(p) > 0 || !make_inner_plan(p, plan)) return 0;
+  return align_up((size_t)p->T * plan.rec.bytes, 256);
 }
 
 // Rounds of CTAs, each staging its tile and walking its share of the tree groups; one, two or four trees per warp at once

@@ -6,7 +6,11 @@
 namespace ht {
 
 // Bytes of per-tree records the tile kernel needs in the workspace (0 when the shape does not qualify).
+// Without them the calls of such a shape are refused.
 size_t forward_tiled_workspace_bytes(const ht_forest_problem *p);
+// ... of inputs with inner positions that are served without tiles, too: several outputs per leaf, or one whose weights stay in
+// global memory.  They lie behind everything else in the workspace, and a call that has no room for them takes another kernel.
+size_t inner_spare_records_bytes(const ht_forest_problem *p);
 
 // Estimated microseconds of the tile kernel on tabular data; negative: not taken.
 double forward_tiled_cost(const ht_forest_problem *p);
@@ -16,7 +20,7 @@ double inner_tiled_cost(const ht_forest_problem *p, bool keep);
 // Runs the forward with the tile kernel when the shape qualifies; returns HT_ERR_UNSUPPORTED
 // (and launches nothing) when it does not, so that the caller can use the any-shape kernel.
 // `ord` are the compact (validated, clamped) int32 ordinals; `records` is 256-byte aligned
-// scratch of forward_tiled_workspace_bytes() bytes.
+// scratch of forward_tiled_workspace_bytes() bytes, or of inner_spare_records_bytes().
 // With `eval_records` (backward_records_bytes() bytes) and a problem for which forward_saves() holds, the forward
 // also leaves its traversal there: the signed margin and the deciding vertex / leaf of every evaluation, from which
 // backward_saved() computes the gradients without walking the trees again.  Several outputs per leaf: `eval_records` is

@@ -17,7 +17,6 @@
 //   * without it (default mode only): fire-and-forget global reductions (red.global.add.f32) from
 //     the traversal kernel itself.
 // There is no block-wide barrier after the feature tile has been staged.
-#include "ht_forest_tile_plan.cuh"
 #include "ht_forest_tiled.cuh"
 #include "ht_eval_records.cuh"
 #include "ht_tile_common.cuh"
@@ -1108,11 +1107,9 @@ int backward_tiled(const ht_forest_problem *p, const float *x, const float *thr,
                    uint32_t *status_word, cudaStream_t stream) {
   BwdPlan plan;
   if (!make_bwd_plan(p, plan, eval_records != nullptr)) return HT_ERR_UNSUPPORTED;
-  if (forward_tiled_workspace_bytes(p) == 0) return HT_ERR_UNSUPPORTED;  // the workspace holds no records otherwise
-  // Inner positions: with so many features that four trees' weights per warp do not fit beside a tile of the forward, scatters are
-  // better (601 x 914 x 64, 35 ferns of depth 7: 239 us, with tiles and reductions 442).
-  TilePlan inner;
-  if (p->K > 1 && !(make_inner_plan(p, inner) && inner.weights)) return HT_ERR_UNSUPPORTED;
+  // The workspace holds no records otherwise.  Inner positions: with so many features that four trees' weights per warp do not fit
+  // beside a tile of the forward, scatters are better (601 x 914 x 64, 35 ferns of depth 7: 239 us, with tiles and reductions 442).
+  if (forward_tiled_workspace_bytes(p) == 0) return HT_ERR_UNSUPPORTED;
   if (((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(g) | reinterpret_cast<uintptr_t>(gx)) & 15u) != 0)
     return HT_ERR_UNSUPPORTED;
   if (eval_records == nullptr && (p->flags & HT_DETERMINISTIC) != 0) return HT_ERR_UNSUPPORTED;

@@ -83,7 +83,8 @@ int ht_selftest_bounded_wait(uint32_t *status_word, ht_stream_t stream);
  * 6 (8), each up to 32 GiB and none where those paths do not take the problem; with HT_DETERMINISTIC 16 bytes more (one
  * output per leaf: up to 2^26 evaluations), and no bound.  The results do not depend on it: whenever the workspace passed
  * is smaller, the backward uses its other paths (in fixed-order mode with one output per leaf a workspace of the default
- * mode's size still serves the record path).  The workspace must be 256-byte aligned device memory. */
+ * mode's size still serves the record path).  Nor does it on the tile records that this counts for inputs with inner positions and
+ * several outputs per leaf: a forward without room for them takes another kernel.  The workspace must be 256-byte aligned device memory. */
 size_t ht_forest_workspace_bytes(const ht_forest_problem *p);
 
 /* Saving the forward's traversal for the backward.  The reference's backward walks every tree again, three
@@ -119,8 +120,8 @@ int ht_forest_forward_f32(const ht_forest_problem *p, const float *x, const floa
  * lives in a fixed array inside the library image (ht_forest_static_scratch_bytes() bytes,
  * currently 16 MiB, resident on every device that loads the library until the process exits).
  *   - Nothing is allocated or freed, here or in anything this calls.
- *   - A problem whose ht_forest_workspace_bytes() exceeds the array is refused with
- *     HT_ERR_WORKSPACE; use ht_forest_forward_f32 with your own workspace for those.
+ *   - A problem whose ht_forest_workspace_bytes() exceeds the array (without the tile records that a
+ *     forward can do without, see there) is refused with HT_ERR_WORKSPACE; use ht_forest_forward_f32 with your own workspace for those.
  *   - The first call on a device looks up the array's device address (once per device, with
  *     that device current); make that first call outside any stream capture.  The address is
  *     kept for the life of the device's primary context: after cudaDeviceReset() this entry

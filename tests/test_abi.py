@@ -51,6 +51,36 @@ def test_workspace_query_and_argument_screening():
     assert rc == -1
 
 
+def test_image_shaped_forwards_run_without_room_for_tile_records():
+    """The packed ordinals are enough where no tile kernel is needed, and room for what a backward keeps where that is asked for.  (The
+    workspace's size is looked at before the missing output; nothing here is read.)"""
+    lib = _cabi.library()
+    host = (ctypes.c_char * 256)()
+    for kind, B, C, K, T, depth, M in [(0, 8, 16, 64, 4096, 8, 2), (0, 135, 152, 2500, 527, 3, 3), (1, 228, 47, 576, 466, 5, 2),
+                                       (0, 9, 200, 1000, 200, 10, 1)]:
+        for flags in (0, 2):  # HT_WORKSPACE_FOR_BACKWARD
+            p = _cabi.ForestProblem(kind, depth, B, C, K, T, M, flags, 0)
+            ordinals = (T * (depth if kind else 2 ** depth - 1) * 4 + 255) // 256 * 256 + 256
+            backward = 0
+            if flags and M > 1:
+                backward = lib.ht_forest_workspace_bytes(ctypes.byref(p))
+                p.flags = 0
+                backward -= lib.ht_forest_workspace_bytes(ctypes.byref(p))
+                p.flags = flags
+                assert backward >= T * B * K * 6
+            elif flags:
+                continue
+
+            def call(workspace_bytes):
+                at = ctypes.c_void_p((ctypes.addressof(host) + 255) // 256 * 256)
+                some = ctypes.c_void_p(ctypes.addressof(host))
+                return lib.ht_forest_forward_f32(ctypes.byref(p), some, some, some, some, None, at, ctypes.c_size_t(workspace_bytes), None, None)
+
+            assert call(ordinals + backward) == -1  # the missing output
+            assert call(ordinals - 257) == -4
+            assert lib.ht_forest_workspace_bytes(ctypes.byref(p)) >= ordinals + backward
+
+
 def test_convolution_plans_at_hand_are_those_of_the_question():
     """Sizes asked for in turn, and each in a thread of its own, which has no earlier plan at hand: the same answers."""
     lib = _cabi.library()

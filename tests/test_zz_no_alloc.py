@@ -75,3 +75,17 @@ def test_problem_larger_than_the_static_scratch_is_refused():
                                           ctypes.c_void_p(x.data_ptr()), None, None)
     assert rc == -4
     assert b"workspace" in lib.ht_status_string(rc)
+
+
+def test_image_shaped_forward_whose_tile_records_do_not_fit_the_static_scratch():
+    """4096 trees of depth 8 with two and three outputs per leaf: 4 MB of ordinals, 18 and 22 MB with the tile kernel's records."""
+    from hingetreefortorch_b200 import _cabi
+    for B, M in ((8, 2), (8, 3), (400, 2)):
+        x, thr, ord_, w = random_forest_inputs(200 + M, "tree", B, 16, (64,), 4096, 8, (M,))
+        dx, dthr, dord, dw = dev(x, thr, ord_, w)
+        forest = _cabi.Forest("tree", dx, dw, backward_workspace=False)
+        got = forest.forward_static(dx, dthr, dord, dw)
+        assert torch.equal(got, forest.forward(dx, dthr, dord, dw))
+        if B < 100:
+            assert np.array_equal(got.cpu().numpy(), ho.forward("tree", x, thr, ord_, w))
+        assert forest.ordinal_flags() == 0
