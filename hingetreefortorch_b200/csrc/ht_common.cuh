@@ -204,7 +204,7 @@ struct Divisor {
 };
 
 // (i, j, k) of evaluation e = (i * T + j) * K + k.  Two divisions of 64 bits are some 200 instructions, more than the walk of a tree of
-// ten levels; up to 2^31 evaluations the quotients are products.
+// ten levels; up to 2^31 evaluations the quotients are products, and beyond that tabular data take one division.
 struct EvalDivisors {
   Divisor T, K;
   int narrow = 0;
@@ -222,7 +222,7 @@ struct EvalDivisors {
       j = ij - row * T.number;
       i = row;
     } else {
-      const int64_t ij = e / positions;
+      const int64_t ij = positions == 1 ? e : e / positions;
       k = e - ij * positions;
       i = ij / trees;
       j = ij - i * trees;
