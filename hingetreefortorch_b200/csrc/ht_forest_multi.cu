@@ -35,11 +35,10 @@ __device__ __forceinline__ void red_add_if(float *p, const float (&v)[V], bool n
                  : "memory");
 }
 // base + index without the second instruction that a 64-bit sum of two registers takes
-template <typename Real>
-__device__ __forceinline__ const Real *element(const Real *base, uint32_t index) {
+__device__ __forceinline__ const float *element(const float *base, uint32_t index) {
   uint64_t at;
-  asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(at) : "r"(index), "n"((int)sizeof(Real)), "l"(base));
-  return reinterpret_cast<const Real *>(at);
+  asm("mad.wide.u32 %0, %1, 4, %2;" : "=l"(at) : "r"(index), "l"(base));
+  return reinterpret_cast<const float *>(at);
 }
 // r = p[0 .. V) where `now` is set, without a branch
 template <int V>
@@ -54,17 +53,6 @@ __device__ __forceinline__ void load_if(Vec<float, V> &r, const float *p, bool n
                  : "l"(p), "r"((int)now));
   else
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p ld.global.nc.f32 %0, [%1];\n\t}" : "+f"(r.v[0]) : "l"(p), "r"((int)now));
-}
-template <int V>
-__device__ __forceinline__ void load_if(Vec<double, V> &r, const double *p, bool now) {
-  if (now) r = load_vec<double, V>(p);
-}
-template <int V>
-__device__ __forceinline__ void red_add_if(double *p, const double (&v)[V], bool now) {
-  if (now) {
-#pragma unroll
-    for (int k = 0; k < V; ++k) atomicAdd(p + k, v[k]);
-  }
 }
 
 template <typename Real>
@@ -138,13 +126,12 @@ __global__ void __launch_bounds__(kForwardThreads) multi_forward_kernel(const __
 
 // ---- backward, default mode ------------------------------------------------------------------------------------------
 
-template <typename Real>
 struct SortedArgs {
-  const Real *margin;
+  const float *margin;
   const void *where;
   const int32_t *ord;
-  const Real *w, *g;
-  Real *gx, *gthr, *gw;
+  const float *w, *g;
+  float *gx, *gthr, *gw;
   int64_t T, C, N, L;
   Divisor K;           // positions per sample
   uint32_t P;          // evaluations per tree
@@ -152,15 +139,9 @@ struct SortedArgs {
 };
 
 // CTAs per SM that the registers are shared out for
-template <typename Real>
-__host__ __device__ constexpr int sort_blocks(int numbers) {
-  return numbers * (int)sizeof(Real) > 8 ? 3 : 4;
-}
+__host__ __device__ constexpr int sort_blocks(int numbers) { return numbers > 2 ? 3 : 4; }
 // g rows (and rows of weights) in flight per group of lanes, as far as registers go
-template <typename Real>
-__host__ __device__ constexpr int sort_ahead(int numbers) {
-  return numbers * (int)sizeof(Real) > 16 ? 2 : 4;
-}
+__host__ __device__ constexpr int sort_ahead(int numbers) { return numbers > 4 ? 2 : 4; }
 
 // Evaluations per CTA: whole rounds for every group of lanes (three and five lanes per evaluation leave 80 and 48 groups).
 __host__ __device__ constexpr uint32_t sort_slice(int lanes) { return lanes == 3 || lanes == 5 ? 960u : 1024u; }
@@ -178,17 +159,16 @@ __host__ __device__ constexpr bool sort_rows_listed(int lanes) { return lanes >=
 
 // Where the arrays of sorted_backward_kernel lie in its shared memory; the counts, whose number varies, come last.
 struct SortedPlaces {
-  uint32_t sizes, dots, partial, bins;
+  uint32_t dots, partial, bins;
 };
-__host__ __device__ constexpr SortedPlaces sorted_places(uint32_t real_bytes, int lanes) {
+__host__ __device__ constexpr SortedPlaces sorted_places(int lanes) {
   SortedPlaces at = {};
   const uint32_t slice = sort_slice(lanes), entries = slice + (uint32_t)(32 / lanes * (kSortThreads / 32));
-  const uint32_t columns = kMaxSortDepth * kSortThreads * real_bytes;  // of the ferns' thresholds, in the list's place after the walk
-  at.sizes = entries * (sort_rows_listed(lanes) ? 16u : 8u);
-  at.dots = at.sizes + (real_bytes == 4 ? 0u : (entries * real_bytes + 15u) & ~15u);
-  at.dots = at.dots < slice * (real_bytes + 4u) ? slice * (real_bytes + 4u) : at.dots;  // terms and vertices, after the walk as well
+  const uint32_t columns = kMaxSortDepth * kSortThreads * 4u;  // of the ferns' thresholds, in the list's place after the walk
+  at.dots = entries * (sort_rows_listed(lanes) ? 16u : 8u);
+  at.dots = at.dots < slice * 8u ? slice * 8u : at.dots;  // terms and vertices, after the walk as well
   at.dots = at.dots < columns ? columns : at.dots;
-  at.partial = at.dots + (((kNobody + 1u) * (uint32_t)sort_dots(lanes) * real_bytes + 15u) & ~15u);
+  at.partial = at.dots + (((kNobody + 1u) * (uint32_t)sort_dots(lanes) * 4u + 15u) & ~15u);
   at.bins = at.partial + ((4u * (kSortThreads / 32) + 15u) & ~15u);
   return at;
 }
@@ -197,14 +177,14 @@ __host__ __device__ inline int sorted_bin_quads(int L, int N, bool fern) { retur
 // Sums of dot[0 .. LEFT) over groups of 2 D lanes, D a power of two: lanes hand each other the halves of the list that they drop,
 // as long as there is more than one number, so that sum u ends in the lanes whose upper bits (of the lane in its group) say u.
 // Those bits are appended to `mine`; the lane is left with dot[0 .. LEFT / 2 D), at least one.
-template <int D, int LEFT, typename Real, int A>
-__device__ __forceinline__ void sums_over_lanes(Real (&dot)[A], int q, int &mine) {
+template <int D, int LEFT, int A>
+__device__ __forceinline__ void sums_over_lanes(float (&dot)[A], int q, int &mine) {
   if constexpr (D >= 1) {
     if constexpr (LEFT > 1) {
       const bool upper = (q & D) != 0;
 #pragma unroll
       for (int u = 0; u < LEFT / 2; ++u) {
-        const Real away = upper ? dot[u] : dot[u + LEFT / 2], kept = upper ? dot[u + LEFT / 2] : dot[u];
+        const float away = upper ? dot[u] : dot[u + LEFT / 2], kept = upper ? dot[u + LEFT / 2] : dot[u];
         dot[u] = kept + __shfl_xor_sync(0xffffffffu, away, D);
       }
       mine = mine * 2 + (upper ? 1 : 0);
@@ -237,23 +217,22 @@ __device__ __forceinline__ void sums_over_lanes(Real (&dot)[A], int q, int &mine
 // Slices of 2048 and 4096 evaluations: ferns 98 and 137 us against 83 in the earlier form (registers).  Asking for the rows
 // ahead of the sort (prefetches into L2): 65 -> 73 us.  Two rows in flight instead of four, in exchange for five or six CTAs per
 // SM: ferns 57 and 73 us, 64 outputs 71 and 61.
-template <typename Real, int V, int LANES, int R>
-__global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted_backward_kernel(const __grid_constant__ SortedArgs<Real> a) {
+template <int V, int LANES, int R>
+__global__ void __launch_bounds__(kSortThreads, sort_blocks(R * V)) sorted_backward_kernel(const __grid_constant__ SortedArgs a) {
   extern __shared__ __align__(16) unsigned char smem[];
-  constexpr int kAhead = sort_ahead<Real>(R * V), kGroupsPerWarp = 32 / LANES, kGroups = kGroupsPerWarp * (kSortThreads / 32);
+  constexpr int kAhead = sort_ahead(R * V), kGroupsPerWarp = 32 / LANES, kGroups = kGroupsPerWarp * (kSortThreads / 32);
   constexpr uint32_t S = sort_slice(LANES);
   constexpr int PER = (int)((S + kSortThreads - 1) / kSortThreads);
   constexpr int kParts = sort_dots(LANES);
   static_assert(S % (kGroups * kAhead) == 0, "whole rounds");
-  constexpr SortedPlaces at = sorted_places((uint32_t)sizeof(Real), LANES);
+  constexpr SortedPlaces at = sorted_places(LANES);
   constexpr bool kListed = sort_rows_listed(LANES);
   using Entry = typename std::conditional<kListed, uint4, uint2>::type;
-  Entry *list = reinterpret_cast<Entry *>(smem);              // by leaf: {tag, |margin| (float)}, and where listed {g row, weight row}
-  [[maybe_unused]] Real *sizes = reinterpret_cast<Real *>(smem + at.sizes);  // by leaf: |margin| (double)
-  Real *dots = reinterpret_cast<Real *>(smem + at.dots);      // by place in the slice: D, or its parts
+  Entry *list = reinterpret_cast<Entry *>(smem);              // by leaf: {tag, |margin|}, and where listed {g row, weight row}
+  float *dots = reinterpret_cast<float *>(smem + at.dots);      // by place in the slice: D, or its parts
   uint32_t *partial = reinterpret_cast<uint32_t *>(smem + at.partial);
   uint32_t *bins = reinterpret_cast<uint32_t *>(smem + at.bins);  // leaves, then vertices: counts, then first places
-  Real *by_vertex = reinterpret_cast<Real *>(smem);               // after the walk: signed D by vertex, or the ferns' columns
+  float *by_vertex = reinterpret_cast<float *>(smem);               // after the walk: signed D by vertex, or the ferns' columns
   uint32_t *vertices = reinterpret_cast<uint32_t *>(by_vertex + S);  // ... and the vertices
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -270,7 +249,7 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
 
   // every thread's evaluations tid, tid + 256, ... are loaded at once and stay in registers; `whole`: a full slice, all of them there
   uint32_t where[PER], keep[PER];
-  Real margin[PER];
+  float margin[PER];
   const int quads = sorted_bin_quads(L, N, a.fern != 0);
   const int share = ((n + kGroups - 1) / kGroups + kAhead - 1) / kAhead * kAhead;
   auto here = [&](int u, bool whole) {
@@ -285,9 +264,9 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
     const uint32_t sample = p0 + (uint32_t)tid, blocks = (uint32_t)a.T * kRecordBlock;
     const int64_t from = (int64_t)(sample / kRecordBlock) * blocks + j * kRecordBlock + sample % kRecordBlock;
     static_assert(kSortThreads == kRecordBlock, "a thread's evaluations are one record block apart");
-    const Real *margins = a.margin + from;
+    const float *margins = a.margin + from;
 #pragma unroll
-    for (int u = 0; u < PER; ++u) margin[u] = here(u, whole) ? -__ldg(margins + (int64_t)u * blocks) : (Real)0;
+    for (int u = 0; u < PER; ++u) margin[u] = here(u, whole) ? -__ldg(margins + (int64_t)u * blocks) : 0.0f;
     if (a.narrow) {
       const unsigned short *wheres = static_cast<const unsigned short *>(a.where) + from;
 #pragma unroll
@@ -305,7 +284,7 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
 #pragma unroll
     for (int u = 0; u < PER; ++u) {
       const uint32_t leaf = where[u] >> 16, vertex = where[u] & 0xffffu;
-      keep[u] = vertex | (margin[u] > (Real)0 ? kPositive : 0u) | (margin[u] < (Real)0 ? kNegative : 0u);
+      keep[u] = vertex | (margin[u] > 0.0f ? kPositive : 0u) | (margin[u] < 0.0f ? kNegative : 0u);
       if (here(u, whole)) {
         if (N > 0) keep[u] |= atomicAdd(&bins[L - 1 + vertex], 1u) << 13;
         where[u] = leaf << 12 | atomicAdd(&bins[leaf], 1u);
@@ -321,18 +300,15 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
       if (here(u, whole)) {
         const int t = tid + u * kSortThreads;
         const uint32_t leaf = where[u] >> 12, rank = where[u] & 0xfffu, next = bins[leaf + 1];
-        const uint32_t to = bins[leaf] + rank, slot = slot_of(to);
+        const uint32_t to = bins[leaf] + rank;
         Entry entry = {};
         entry.x = (uint32_t)t | leaf << 12 | kHere | (rank == 0 ? kFirst : 0u) | (to + 1 == next ? kLast : 0u);
         if constexpr (kListed) {
           entry.z = g_row(from_first + (uint32_t)t);
           entry.w = leaf * M;
         }
-        if constexpr (sizeof(Real) == 4)
-          entry.y = __float_as_uint(fabsf((float)margin[u]));
-        else
-          sizes[slot] = abs_of(margin[u]);
-        list[slot] = entry;
+        entry.y = __float_as_uint(fabsf(margin[u]));
+        list[slot_of(to)] = entry;
         if (N > 0) keep[u] += (bins[L - 1 + (keep[u] & 0x1fffu)] - (uint32_t)n) << 13;
       }
     }
@@ -342,7 +318,6 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
         nobody.x = kNobody;
         if constexpr (kListed) nobody.z = g_row(from_first);
         list[slot_of(to)] = nobody;
-        if constexpr (sizeof(Real) != 4) sizes[slot_of(to)] = (Real)0;
       }
     }
   };
@@ -358,7 +333,6 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
     const int group_in_warp = min(lane / LANES, kGroupsPerWarp - 1), q = lane - group_in_warp * LANES;
     const int part = warp * kGroupsPerWarp + group_in_warp;
     const Entry *my_list = list + part * (share + 1);
-    [[maybe_unused]] const Real *my_sizes = sizes + part * (share + 1);
     bool on[R];
     uint32_t piece[R];
 #pragma unroll
@@ -366,30 +340,27 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
       on[r] = q < LANES && (q + r * LANES) * V < a.M;
       piece[r] = on[r] ? (uint32_t)((q + r * LANES) * V) : 0u;
     }
-    const Real *g_first = a.g + ((int64_t)i0 * a.T + j) * K * M;
-    const Real *w_first = a.w + j * L * M;
-    const Real *gw_first = a.gw + j * L * M;
+    const float *g_first = a.g + ((int64_t)i0 * a.T + j) * K * M;
+    const float *w_first = a.w + j * L * M;
+    const float *gw_first = a.gw + j * L * M;
     const bool want_w = a.gw != nullptr;
-    Real sums[R][V], weight[R][V];
+    float sums[R][V], weight[R][V];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int v = 0; v < V; ++v) sums[r][v] = weight[r][v] = (Real)0;
+      for (int v = 0; v < V; ++v) sums[r][v] = weight[r][v] = 0.0f;
     auto hand_in = [&](uint32_t leaf_row, bool now) {
 #pragma unroll
-      for (int r = 0; r < R; ++r) red_add_if<V>(const_cast<Real *>(element(gw_first, leaf_row + piece[r])), sums[r], now && on[r]);
+      for (int r = 0; r < R; ++r) red_add_if<V>(const_cast<float *>(element(gw_first, leaf_row + piece[r])), sums[r], now && on[r]);
     };
     // a ring of kAhead evaluations: their list entries, g rows, and the weights of the leaves that they enter
-    Vec<Real, V> rows[kAhead][R], entered[kAhead][R] = {};
+    Vec<float, V> rows[kAhead][R], entered[kAhead][R] = {};
     uint32_t tag[kAhead], leaf_row[kAhead];
-    Real size[kAhead];
+    float size[kAhead];
     auto fetch = [&](int u, int t, bool enters) {
       const Entry entry = my_list[t];
       tag[u] = entry.x | (enters ? kFirst : 0u);
-      if constexpr (sizeof(Real) == 4)
-        size[u] = __uint_as_float(entry.y);
-      else
-        size[u] = my_sizes[t];
+      size[u] = __uint_as_float(entry.y);
       uint32_t row;
       if constexpr (kListed) {
         row = entry.z;
@@ -400,33 +371,33 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
       }
 #pragma unroll
       for (int r = 0; r < R; ++r) {
-        rows[u][r] = load_vec<Real, V>(element(g_first, row + piece[r]));
+        rows[u][r] = load_vec<float, V>(element(g_first, row + piece[r]));
         load_if<V>(entered[u][r], element(w_first, leaf_row[u] + piece[r]), (tag[u] & kFirst) != 0);
       }
     };
     auto round = [&](int t0, auto more) {
       uint32_t place[kAhead];
-      Real dot[kAhead];
+      float dot[kAhead];
 #pragma unroll
       for (int u = 0; u < kAhead; ++u) {
         place[u] = tag[u];
-        dot[u] = (Real)0;
+        dot[u] = 0.0f;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-          Real mine = (Real)0;
+          float mine = 0.0f;
 #pragma unroll
           for (int v = 0; v < V; ++v) {
             weight[r][v] = (tag[u] & kFirst) ? entered[u][r].v[v] : weight[r][v];
             sums[r][v] += size[u] * rows[u][r].v[v];
             mine += weight[r][v] * rows[u][r].v[v];
           }
-          dot[u] += kParts > 1 || on[r] ? mine : (Real)0;
+          dot[u] += kParts > 1 || on[r] ? mine : 0.0f;
         }
         hand_in(leaf_row[u], want_w && (tag[u] & kLast) != 0);
 #pragma unroll
         for (int r = 0; r < R; ++r)
 #pragma unroll
-          for (int v = 0; v < V; ++v) sums[r][v] = (tag[u] & kLast) ? (Real)0 : sums[r][v];
+          for (int v = 0; v < V; ++v) sums[r][v] = (tag[u] & kLast) ? 0.0f : sums[r][v];
         if constexpr (decltype(more)::value) fetch(u, t0 + u + kAhead, false);
       }
       if constexpr (kParts > 1) {
@@ -469,8 +440,8 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
           for (int r = 0; r < R; ++r)
 #pragma unroll
             for (int v = 0; v < V; ++v) {
-              const Real other = __shfl_down_sync(0xffffffffu, sums[r][v], d * LANES);
-              sums[r][v] += join ? other : (Real)0;
+              const float other = __shfl_down_sync(0xffffffffu, sums[r][v], d * LANES);
+              sums[r][v] += join ? other : 0.0f;
             }
         }
         const uint32_t before = __shfl_up_sync(0xffffffffu, current, LANES);
@@ -484,7 +455,7 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
 
   // thread per evaluation again
   if (a.fern && a.gthr != nullptr)
-    for (int l = 0; l < (int)a.N; ++l) by_vertex[l * kSortThreads + tid] = (Real)0;
+    for (int l = 0; l < (int)a.N; ++l) by_vertex[l * kSortThreads + tid] = 0.0f;
   auto finish = [&](auto whole_slice) {
     constexpr bool whole = decltype(whole_slice)::value;
     const int32_t *features = a.ord + j * a.N - 1;
@@ -492,12 +463,12 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
     for (int u = 0; u < PER; ++u) {
       if (here(u, whole)) {
         const int t = tid + u * kSortThreads;
-        Real d = dots[t * kParts];
+        float d = dots[t * kParts];
 #pragma unroll
         for (int part = 1; part < kParts; ++part) d += dots[t * kParts + part];
         const uint32_t vertex = keep[u] & 0x1fffu;
-        Real term = (keep[u] & kPositive) ? d : -d;  // sign(margin) * D
-        if ((keep[u] & (kPositive | kNegative)) == 0) term = (Real)0 * d;
+        float term = (keep[u] & kPositive) ? d : -d;  // sign(margin) * D
+        if ((keep[u] & (kPositive | kNegative)) == 0) term = 0.0f * d;
         if (a.gx != nullptr) {
           const uint32_t f = (uint32_t)__ldg(features + vertex);
           if (K == 1) {
@@ -527,7 +498,7 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
   __syncthreads();
   if (a.fern) {
     for (int l = warp; l < (int)a.N; l += kSortThreads / 32) {
-      Real sum = (Real)0;
+      float sum = 0.0f;
 #pragma unroll
       for (int e = 0; e < kSortThreads; e += 32) sum += by_vertex[l * kSortThreads + e + lane];
 #pragma unroll
@@ -539,32 +510,32 @@ __global__ void __launch_bounds__(kSortThreads, sort_blocks<Real>(R * V)) sorted
   // warps sum runs of 32
   for (int e0 = warp * 32; e0 < n; e0 += kSortThreads) {
     const int e = e0 + lane;
-    Real sum[1] = {e < n ? by_vertex[e] : (Real)0};
+    float sum[1] = {e < n ? by_vertex[e] : 0.0f};
     const uint32_t vertex = e < n ? vertices[e] : 0xffffu;
     if (sums_of_runs(vertex, sum, lane) && e < n) atomicAdd(a.gthr + j * a.N + vertex, -sum[0]);
   }
 }
 
-template <typename Real, int V, int LANES, int R>
-int launch_sorted(const SortedArgs<Real> &a, cudaStream_t stream) {
+template <int V, int LANES, int R>
+int launch_sorted(const SortedArgs &a, cudaStream_t stream) {
   constexpr uint32_t slice = sort_slice(LANES);
   const int64_t grid = (int64_t)((a.P + slice - 1) / slice) * a.T;
   if (grid > 0x7fffffff) return HT_ERR_UNSUPPORTED;
-  auto kernel = sorted_backward_kernel<Real, V, LANES, R>;
-  const size_t smem = sorted_places((uint32_t)sizeof(Real), LANES).bins + 16 * (size_t)sorted_bin_quads((int)a.L, (int)a.N, a.fern != 0);
+  auto kernel = sorted_backward_kernel<V, LANES, R>;
+  const size_t smem = sorted_places(LANES).bins + 16 * (size_t)sorted_bin_quads((int)a.L, (int)a.N, a.fern != 0);
   if (smem > 48 * 1024) HT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kernel<<<(unsigned)grid, kSortThreads, smem, stream>>>(a);
   HT_CHECK_LAUNCH();
   return HT_OK;
 }
 
-template <typename Real, int V>
-int launch_sorted_width(const SortedArgs<Real> &a, cudaStream_t stream) {
+template <int V>
+int launch_sorted_width(const SortedArgs &a, cudaStream_t stream) {
   // one load per lane and row up to half a warp per row (64 outputs: 68 us, with two loads and 8 lanes 78)
   const int pieces = (a.M + V - 1) / V;
   const bool one = pieces <= 16;
 #define HT_SORTED(LANES, R) \
-  if (pieces <= LANES * R && one == (R == 1)) return launch_sorted<Real, V, LANES, R>(a, stream);
+  if (pieces <= LANES * R && one == (R == 1)) return launch_sorted<V, LANES, R>(a, stream);
   HT_SORTED(1, 1)
   HT_SORTED(2, 1)
   HT_SORTED(3, 1)
@@ -641,12 +612,11 @@ int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, co
   return p->kind == TREE ? launch_forward<TREE, false>(a, width, stream) : launch_forward<FERN, false>(a, width, stream);
 }
 
-template <typename Real>
-int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w, const Real *g, Real *gx, Real *gthr,
-                   Real *gw, void *area, cudaStream_t stream) {
-  if (!multi_takes(p, sizeof(Real)) || (p->flags & HT_DETERMINISTIC) != 0) return HT_ERR_UNSUPPORTED;
-  const PathRecordsOf<Real> paths = multi_paths<Real>(p, area);
-  SortedArgs<Real> a = {};
+int backward_multi(const ht_forest_problem *p, const int32_t *ord, const float *w, const float *g, float *gx, float *gthr,
+                   float *gw, void *area, cudaStream_t stream) {
+  if (!multi_takes(p, sizeof(float)) || (p->flags & HT_DETERMINISTIC) != 0) return HT_ERR_UNSUPPORTED;
+  const PathRecordsOf<float> paths = multi_paths<float>(p, area);
+  SortedArgs a = {};
   a.margin = paths.margin;
   a.where = paths.where;
   a.ord = ord;
@@ -666,20 +636,15 @@ int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w
   a.fern = p->kind == FERN;
   a.narrow = where_bytes(p->depth) == 2;
   if ((int64_t)1024 * p->T * p->M + (int64_t)p->T * p->K * p->M > 0x7fffffff) return HT_ERR_UNSUPPORTED;  // g row offsets
-  const int width = vector_width(p->M, sizeof(Real), {w, g, gw});
-  if (width == 1) return launch_sorted_width<Real, 1>(a, stream);
-  if (width == 2) return launch_sorted_width<Real, 2>(a, stream);
-  if constexpr (sizeof(Real) == 4) return launch_sorted_width<Real, 4>(a, stream);
-  return HT_ERR_UNSUPPORTED;
+  const int width = vector_width(p->M, sizeof(float), {w, g, gw});
+  if (width == 1) return launch_sorted_width<1>(a, stream);
+  if (width == 2) return launch_sorted_width<2>(a, stream);
+  return launch_sorted_width<4>(a, stream);
 }
 
 template int multi_forward<float>(const ht_forest_problem *, const float *, const float *, const int32_t *, const float *,
                                   float *, PathRecordsOf<float>, cudaStream_t, const WideOrdinals *, uint32_t *);
 template int multi_forward<double>(const ht_forest_problem *, const double *, const double *, const int32_t *, const double *,
                                    double *, PathRecordsOf<double>, cudaStream_t, const WideOrdinals *, uint32_t *);
-template int backward_multi<float>(const ht_forest_problem *, const int32_t *, const float *, const float *, float *, float *,
-                                   float *, void *, cudaStream_t);
-template int backward_multi<double>(const ht_forest_problem *, const int32_t *, const double *, const double *, double *,
-                                    double *, double *, void *, cudaStream_t);
 
 }  // namespace ht

@@ -36,10 +36,10 @@ template <typename Real>
 int multi_forward(const ht_forest_problem *p, const Real *x, const Real *thr, const int32_t *ord, const Real *w, Real *out,
                   PathRecordsOf<Real> paths, cudaStream_t stream, const WideOrdinals *wide = nullptr, uint32_t *status_word = nullptr);
 
-// Gradients from the paths in `area`.  The gradients that are asked for (the others are null) must have been cleared.
-template <typename Real>
-int backward_multi(const ht_forest_problem *p, const int32_t *ord, const Real *w, const Real *g, Real *gx, Real *gthr,
-                   Real *gw, void *area, cudaStream_t stream);
+// Gradients from the paths in `area`, single precision (double precision scatters: ht_forest_backward_f64).  The gradients that are
+// asked for (the others are null) must have been cleared.
+int backward_multi(const ht_forest_problem *p, const int32_t *ord, const float *w, const float *g, float *gx, float *gthr,
+                   float *gw, void *area, cudaStream_t stream);
 
 // Fixed-order mode (ht_forest_ordered.cu), any number of outputs per leaf: bytes of the lists that the paths are sorted
 // into (0: not for this problem), and the threshold and leaf-weight gradients from the paths.
