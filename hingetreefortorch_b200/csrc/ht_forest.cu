@@ -515,15 +515,18 @@ static bool inner_tiles_are_better(const ht_forest_problem *p, bool keep) {
   return tiles < threads;
 }
 
-// What a backward keeps per evaluation: the records of the tile kernels (one output per leaf), or the paths (several) and,
-// in fixed-order mode, their lists.
-static size_t records_bytes(const ht_forest_problem *p) {
-  if (ordered_from_paths(p)) return saved_bytes(p) + ordered_list_bytes(p, sizeof(float));
-  return p->M > 1 ? multi_area_bytes(p, sizeof(float)) : backward_records_bytes(p);
+// The records of the tile kernels (one output per leaf), where backward_tiled() takes the problem: it refuses what the workspace has
+// no tree records for.
+static size_t records_without_lists(const ht_forest_problem *p) {
+  return p->M == 1 && forward_tiled_workspace_bytes(p) > 0 ? backward_records_bytes(p) : 0;
 }
 
-// What still serves the fixed order without the lists.
-static size_t records_without_lists(const ht_forest_problem *p) { return p->M == 1 ? backward_records_bytes(p) : 0; }
+// What a backward keeps per evaluation: those records, which serve the fixed order as well, or the paths (several outputs per leaf);
+// in fixed-order mode the lists, too.
+static size_t records_bytes(const ht_forest_problem *p) {
+  if (ordered_from_paths(p)) return saved_bytes(p) + ordered_list_bytes(p, sizeof(float));
+  return p->M > 1 ? multi_area_bytes(p, sizeof(float)) : records_without_lists(p);
+}
 
 // Where a forward finds room for the tile kernel's records (null: nowhere); `kept`: bytes that the call keeps for a backward.
 static void *tile_records_at(const ht_forest_problem *p, void *workspace, size_t workspace_bytes, size_t kept, bool keep) {

@@ -81,6 +81,22 @@ def test_image_shaped_forwards_run_without_room_for_tile_records():
             assert lib.ht_forest_workspace_bytes(ctypes.byref(p)) >= ordinals + backward
 
 
+def test_backward_workspace_counts_records_only_where_they_are_used():
+    """One output per leaf on more features than the tile kernels take: the gradients are scattered, in either mode of the workspace."""
+    lib = _cabi.library()
+
+    def size(flags, kind, B, C, K, T, depth):
+        return lib.ht_forest_workspace_bytes(ctypes.byref(_cabi.ForestProblem(kind, depth, B, C, K, T, 1, flags, 0)))
+
+    for shape in [(1, 601, 914, 64, 35, 7), (0, 64, 1000, 4096, 256, 8), (0, 40000, 1800, 1, 64, 6)]:
+        evaluations = shape[1] * shape[3] * shape[4]
+        assert size(2, *shape) == size(0, *shape)  # HT_WORKSPACE_FOR_BACKWARD
+        if evaluations <= 1 << 26:
+            assert size(3, *shape) >= size(0, *shape) + 22 * evaluations  # fixed order: paths and lists
+    for shape in [(1, 601, 91, 64, 35, 7), (0, 40000, 180, 1, 64, 6)]:
+        assert size(2, *shape) >= size(0, *shape) + 10 * shape[1] * shape[3] * shape[4]
+
+
 def test_convolution_plans_at_hand_are_those_of_the_question():
     """Sizes asked for in turn, and each in a thread of its own, which has no earlier plan at hand: the same answers."""
     lib = _cabi.library()
