@@ -499,20 +499,20 @@ static bool rows_are_better(const ht_forest_problem *p, bool keep) {
 // Whether resident tiles of samples are better than a thread per evaluation (inner positions; one walk is as good as the other where
 // the tiles do not take the sizes): where their estimate is the lower one.  Tiles read all features of a sample once, threads the ones
 // that a walk meets, whose lanes are on as many cache lines as the level has vertices; so tiles are for many trees on few features.
-// Both estimates are fits to forwards of random sizes that were timed both ways in one session (profiles/inner_forward_choice.csv, 400
-// of them); time of the chosen kernels over that of the better ones, all calls together 1.010, geometric mean 1.011 (always tiles 1.189
-// in all, never 1.536, tiles for one output per leaf alone 1.266).  2796 x 284 x 169, 8 trees of depth 4: tiles 520 us, threads 47;
-// 228 x 47 x 576, 466 trees of depth 5: 208 and 673.
+// Both estimates are fits to 788 of the 1050 forwards of random sizes in profiles/inner_forward_choice.csv, each timed both ways in one
+// session with the module's own parameters.  Time of the chosen kernels over that of the better ones, all calls together, on the 262
+// others: 1.006 (always tiles 1.225, never 1.568), none over 1.13; on those of the fit 1.003.  2796 x 284 x 169, 8 trees of
+// depth 4: tiles 520 us, threads 47; 228 x 47 x 576, 466 trees of depth 5: 208 and 673.
 static bool inner_tiles_are_better(const ht_forest_problem *p, bool keep) {
   const double tiles = inner_tiled_cost(p, keep);
   if (tiles < 0.0) return false;
   const double evals = 1e-6 * (double)p->B * (double)p->K * (double)p->T;
   double lines = 0.0;  // cache lines that a warp's levels are on
   for (int l = 0; l < p->depth; ++l) lines += p->kind == FERN ? 1.0 : std::min(24.0, (double)(1u << l));
-  const bool far = p->C * p->K * 4 > 2000000;  // the features of a row leave L1
-  const double threads = 5.3 + evals * (5.46 + (far ? 0.840 : 0.647) * p->depth + 0.0373 * lines + 0.253 * (double)p->M +
-                                        0.705 * (double)p->M / vector_width(p->M, sizeof(float), {}) + (keep && p->M > 1 ? 1.48 : 0.0));
-  return tiles < threads;
+  const bool wide = p->C * p->K * 4 > 2000000;  // rows of x beyond which a level was dearer in the table
+  const double threads = 4.64 + evals * (4.97 + (wide ? 0.888 : 0.678) * p->depth + 0.0391 * lines + 0.238 * (double)p->M +
+                                         0.710 * (double)p->M / vector_width(p->M, sizeof(float), {}) + (keep && p->M > 1 ? 1.58 : 0.0));
+  return tiles < threads + 1.0;  // as near as that, tiles: the total is the same to 0.05 %
 }
 
 // The records of the tile kernels (one output per leaf), where backward_tiled() takes the problem: it refuses what the workspace has

@@ -40,19 +40,23 @@ bool make_inner_plan(const ht_forest_problem *p, TilePlan &plan) {
 
 }  // namespace tile
 
-// Rounds of CTAs, each staging its tile and walking its share of the tree groups, like forward_tiled_cost(); the outputs of a group
-// cost what their form does.
+// Rounds of CTAs, each staging its tile and walking its share of the tree groups, like forward_tiled_cost().  A group costs the walks
+// of a warp's trees and, for several outputs per leaf, what their form does: dealing out (five and more) pays for the 32 / K rows that a
+// warp's samples are on.  Tiles read all of x and write all outputs, in bursts that the walks hide in part: 0.15 and 0.06 us per MB, and
+// as much again for x where it does not stay in L2.  Scalar loads (K no multiple of four) stage a tile in 0.29 us per 1000 numbers.
 double inner_tiled_cost(const ht_forest_problem *p, bool keep) {
   tile::TilePlan plan;
   if (!tile::make_inner_plan(p, plan)) return -1.0;
   const int64_t tiles = (p->B * p->K + plan.S - 1) / plan.S, groups = (p->T + plan.G - 1) / plan.G;
   const int splits = tile::choose_splits(tiles, groups);
   const double waves = (double)((tiles * splits + 147) / 148), per_cta = (double)((groups + splits - 1) / splits);
-  const double level = plan.per_warp == 1 ? 0.0241 : plan.per_warp == 2 ? 0.0832 : 0.150;
+  const double walk = plan.per_warp == 4 ? 0.553 + 0.161 * p->depth : plan.per_warp == 2 ? 0.675 + 0.0986 * p->depth : 0.952 + 0.0326 * p->depth;
   const double evals = 1e-3 * plan.G * plan.S, pieces = evals * (double)p->M / vector_width(p->M, sizeof(float), {});
-  const double output = pieces * ((p->M > 4 ? 0.182 : p->M > 1 ? 0.0225 : 0.0) + (plan.weights ? 0.0 : 0.107)) +
-                        evals * (0.0110 * (double)p->M + (keep && p->M > 1 ? 0.217 : 0.0));
-  return 0.3 + waves * (1.87 + 0.226e-3 * plan.S * (double)p->C + per_cta * (0.968 + level * p->depth + output));
+  const double output = pieces * ((p->M > 4 ? 0.136 + 0.0166 * 32.0 / (double)p->K : p->M > 1 ? 0.0260 : 0.0) + (plan.weights ? 0.0 : 0.0855)) +
+                        (keep && p->M > 1 ? 0.223 * evals : 0.0);
+  const double staging = (double)p->C * (0.0899e-3 + ((p->K & 3) != 0 ? 0.292e-3 * plan.S : 0.0));
+  const double read = 4e-6 * (double)p->B * (double)p->C * (double)p->K, written = 4e-6 * (double)p->B * (double)p->K * (double)p->T * (double)p->M;
+  return 3.60 + waves * (2.42 + staging + per_cta * (walk + output)) + 0.154 * read + 0.158 * std::max(0.0, read - 100.0) + 0.0645 * written;
 }
 
 namespace tile {

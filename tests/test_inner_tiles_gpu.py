@@ -91,3 +91,22 @@ def test_choice_against_the_times_of_both_kernels():
             better += min(tiles, threads)
             logs.append(math.log((tiles if takes == TILES else threads) / min(tiles, threads)))
     assert chosen <= 1.02 * better and math.exp(sum(logs) / len(logs)) <= 1.03
+
+
+def test_choice_on_forwards_that_the_estimates_were_not_fitted_to():
+    """The rows of profiles/inner_forward_choice.csv that were kept out of the fit."""
+    import csv
+    import os
+    chosen = better = 0.0
+    with open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "profiles", "inner_forward_choice.csv")) as table:
+        for row in csv.DictReader(table):
+            if row["held_out"] == "0":
+                continue
+            B, C, K, T, depth, M = (int(row[c]) for c in ("B", "C", "K", "T", "depth", "M"))
+            p = _cabi.ForestProblem(_cabi.HT_KIND[row["kind"]], depth, B, C, K, T, M, 4 if row["keeps_paths"] == "1" else 0, 0)
+            takes = _cabi.library().ht_forest_forward_kernel(ctypes.byref(p))
+            times = {TILES: float(row["tiles_us"]), THREADS: float(row["threads_us"])}
+            chosen += times[takes]
+            better += min(times.values())
+            assert times[takes] <= 1.15 * min(times.values()) or min(times.values()) < 100.0, row
+    assert better > 0.0 and chosen <= 1.01 * better
