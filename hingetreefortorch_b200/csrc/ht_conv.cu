@@ -13,6 +13,7 @@
 #include "ht_counting_sort.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace ht {
 
@@ -199,7 +200,7 @@ __global__ void __launch_bounds__(32 * kSharing) conv_forward_shared_kernel(Conv
 }
 
 // One thread per (i, j, p) walking the input channels; the three gradients are scattered with atomics.
-// Trees of many leaves (launch_backward_sorted says which).
+// sorting_is_better() says when.
 template <int KIND, typename Real>
 __global__ void __launch_bounds__(kBlock) conv_backward_kernel(ConvArgsOf<Real> a, const Real *__restrict__ g, Real *gx,
                                                                Real *gthr, Real *gw) {
@@ -727,7 +728,7 @@ int run_patches(bool contract, int dims, int elem_bytes, const void *in, void *o
 }
 
 // Whether a call's outputs are too few for a thread each to fill the machine (and the leaves' places fit 32 bits).  Up to some 85 000
-// of them eight warps per channel are better, fewer where there are fewer channels than warps: 60000 outputs of 24 channels 62 us with
+// of them a warp per channel, eight under way, is better, fewer outputs where there are fewer channels than warps: 60000 outputs of 24 channels 62 us with
 // a thread each, 38 shared; 20776 of 7 21 and 8; 81000 of 52 198 and 127; but 144342 of 29 71 and 85, 69984 of 6 14.6 and 16.6, 25984
 // of 2 8.6 and 10.5.
 bool shares_channels(const ConvShape &a) {
@@ -773,25 +774,61 @@ int conv_forward(const ht_conv_problem *p, const Real *x, const Real *thr, const
   return HT_OK;
 }
 
-// HT_ERR_UNSUPPORTED: trees with too many bins, more evaluations than 31 bits count, and calls that conv_backward_kernel serves better:
-// enough outputs for a thread each, one output per leaf, and leaves enough for the reductions to spread (2486 trees of depth 7,
-// 3-D: 1264 us there, 1479 sorted; 3132 of depth 6 216 and 266; 2856 of depth 7 and 139944 outputs, the step, 450 and 473; but 2499 ferns of depth 3 479 and 407, and with few outputs 1254 trees
-// of depth 6 92 and 22).
+// Evaluations per thread of the sorted backward: four where the last slices are not too empty and there are CTAs enough.  6000
+// evaluations of 363 trees 83 us with one per thread, 72 with four; 28090 of 575 633 and 531; but 390 of 1254 22 and 30, 10658 of 9 6 and 11.
+int evaluations_per_thread(const ConvShape &a) {
+  const int64_t evals = a.B * a.out_count, slices = (evals + 4 * kBlock - 1) / (4 * kBlock);
+  return slices * a.Co * a.Ci >= 4 * 148 && slices * 4 * kBlock * 3 <= evals * 4 ? 4 : 1;
+}
+
+// Whether a backward sorts (conv_backward_sorted_kernel) rather than scatters (conv_backward_kernel): where its estimate is the lower
+// one, in microseconds.  Sorting pays for its evaluations and for its CTAs, which clear and sum their bins.  A scatter is bound by its
+// reductions, by those that meet in one threshold (a vertex that decides often) or one leaf, which are the fewer the more trees are
+// under way (some 300 000 threads on consecutive positions, at different channels), or, with few outputs, by the chain of Ci walks
+// of a thread; no two of them hide one another entirely, hence the norm of order 3/2.  Fits to 780 of the 1040 backwards of random
+// sizes in profiles/conv_backward_choice.csv, timed both ways in one session; on the 260 others, all calls together, the chosen kernels
+// take 1.013 (single precision; always sorted 1.013, always scattered 3.27) and 1.016 (double; 1.058, 2.83) of the better ones'
+// time, on those of the fit 1.006 (1.021, 3.15) and 1.003 (1.076, 2.25).  [35, 30, 7, 7, 7], 75 x 30 trees of depth 3, 2 x 2 x 2, padding 1:
+// sorted 982 us, scattered 695; in double precision [28, 11, 1466], 54 x 11 of depth 5: 790 and 494.
+struct ConvBackwardRates {
+  double sort, eval, level, output, piece, cta, cta_piece, cta_bin;
+  double scatter, walk, line, reduction, tree_vertex, fern_vertex, leaf, chain_level, chain_output;
+};
+constexpr ConvBackwardRates kSingleRates = {7.38, 12.8, 1.40, 0.805, 6.69, 6.79e-4, 1.77e-4, 3.82e-6, 6.64, 0.0, 0.166, 11.6, 14600, 13500, 3710, 0.436, 0.121};
+constexpr ConvBackwardRates kDoubleRates = {7.56, 17.4, 1.12, 3.10, 2.91, 17.4e-4, 20.6e-4, 6.68e-6, 6.89, 0.449, 0.183, 11.3, 10600, 10500, 2130, 0.432, 0.266};
+
+template <typename Real>
+bool sorting_is_better(const ConvShape &a, int kind) {
+  const int64_t evals = a.B * a.out_count, trees = a.Co * a.Ci;
+  if (a.L + a.N > kSortedBins || evals >= ((int64_t)1 << 31) || trees >= ((int64_t)1 << 31)) return false;
+  const int64_t slice = evaluations_per_thread(a) * kBlock, ctas = (evals + slice - 1) / slice * trees;
+  if (ctas > 0x7fffffff) return false;
+  const ConvBackwardRates &r = sizeof(Real) == 4 ? kSingleRates : kDoubleRates;
+  const double E = 1e-6 * (double)evals * (double)trees, M = (double)a.M, levels = (double)a.depth;
+  const double pieces = (double)((a.M + sorted_terms<Real>() - 1) / sorted_terms<Real>());
+  const double sorted = r.sort + E * (r.eval + r.level * levels + r.output * M + r.piece * pieces) +
+                        (double)ctas * (r.cta + r.cta_piece * pieces + r.cta_bin * (double)(a.L + a.N));
+  double lines = 0.0;  // cache lines that a warp's levels are on
+  for (int l = 0; l < a.depth; ++l) lines += kind == FERN ? 1.0 : std::min(24.0, (double)(1u << l));
+  const double under_way = std::pow(std::min((double)a.Co, std::max(1.0, 148 * 2048.0 / (double)a.out_count)), 0.8) * std::pow((double)a.Ci, 0.6);
+  const double work = E * (r.walk + r.line * lines + r.reduction * M);
+  const double vertices = E / under_way * (kind == FERN ? r.fern_vertex / levels : r.tree_vertex / (levels * std::sqrt(levels)));
+  const double leaves = E * M / under_way * r.leaf / std::sqrt((double)a.L);
+  const double chain = (double)a.Ci * (r.chain_level * levels + r.chain_output * M);
+  const double sum = work * std::sqrt(work) + vertices * std::sqrt(vertices) + leaves * std::sqrt(leaves) + chain * std::sqrt(chain);
+  return sorted <= r.scatter + std::cbrt(sum * sum);
+}
+
+// HT_ERR_UNSUPPORTED: sizes that sorting is not for, or not the better way for.
 template <typename Real>
 int launch_backward_sorted(const ConvArgsOf<Real> &a, int kind, const Real *g, Real *gx, Real *gthr, Real *gw, cudaStream_t stream) {
+  if (!sorting_is_better<Real>(a, kind)) return HT_ERR_UNSUPPORTED;
   const int64_t evals = a.B * a.out_count, trees = a.Co * a.Ci;
-  if (a.L + a.N > kSortedBins || evals >= ((int64_t)1 << 31) || trees >= ((int64_t)1 << 31)) return HT_ERR_UNSUPPORTED;
-  if (a.M == 1 && trees * a.L >= 131072 && evals * a.Co >= 148 * 768) return HT_ERR_UNSUPPORTED;
-  // Four evaluations per thread where the last slices are not too empty and there are CTAs enough: 6000 evaluations of 363 trees 83 us
-  // with one per thread, 72 with four; 28090 of 575 633 and 531; but 390 of 1254 22 and 30, 10658 of 9 6 and 11.
-  const int64_t slices = (evals + 4 * kBlock - 1) / (4 * kBlock);
-  const bool wide = slices * trees >= 4 * 148 && slices * 4 * kBlock * 3 <= evals * 4;
-  const int per = wide ? 4 : 1;
+  const int per = evaluations_per_thread(a);
   const int64_t grid = (evals + per * kBlock - 1) / (per * kBlock) * trees;
-  if (grid > 0x7fffffff) return HT_ERR_UNSUPPORTED;
   const int quad_sums = sorted_terms<Real>() == 4 && a.M % 4 == 0 && (reinterpret_cast<uintptr_t>(gw) & 15u) == 0;
-  auto kernel = kind == TREE ? (wide ? conv_backward_sorted_kernel<TREE, Real, 4> : conv_backward_sorted_kernel<TREE, Real, 1>)
-                             : (wide ? conv_backward_sorted_kernel<FERN, Real, 4> : conv_backward_sorted_kernel<FERN, Real, 1>);
+  auto kernel = kind == TREE ? (per == 4 ? conv_backward_sorted_kernel<TREE, Real, 4> : conv_backward_sorted_kernel<TREE, Real, 1>)
+                             : (per == 4 ? conv_backward_sorted_kernel<FERN, Real, 4> : conv_backward_sorted_kernel<FERN, Real, 1>);
   PositionDivisors by;
   for (int d = 0; d < 3; ++d) by.size[d] = Divisor((uint32_t)a.osize[d]);
   kernel<<<(unsigned)grid, kBlock, conv_sorted_places<Real>(a, (uint32_t)(per * kBlock)).bytes, stream>>>(a, Divisor((uint32_t)a.out_count), by, (uint32_t)evals,
@@ -855,6 +892,17 @@ int ht_conv_output_size(const ht_conv_problem *p, int64_t *osize) {
   if (osize == nullptr) return HT_ERR_INVALID_ARGUMENT;
   for (int d = 0; d < p->dims; ++d) osize[d] = a.osize[d];
   return HT_OK;
+}
+
+int ht_conv_backward_kernel(const ht_conv_problem *p, int real_bytes) {
+  ConvArgs a;
+  const int rc = check_conv(p, a);
+  if (rc != HT_OK) return rc;
+  if (real_bytes != 4 && real_bytes != 8) return HT_ERR_INVALID_ARGUMENT;
+  ConvTileProblem t;
+  if (real_bytes == 4 && tile_problem(p, a, t) && conv_backward_tiled_workspace_bytes(t) != 0) return HT_CONV_BACKWARD_TILES;
+  const bool sorts = real_bytes == 4 ? sorting_is_better<float>(a, p->kind) : sorting_is_better<double>(a, p->kind);
+  return sorts ? HT_CONV_BACKWARD_SORTED : HT_CONV_BACKWARD_SCATTERED;
 }
 
 size_t ht_conv_workspace_bytes(const ht_conv_problem *p) {

@@ -287,6 +287,10 @@ size_t ht_conv_workspace_bytes(const ht_conv_problem *p);
 /* For a single precision backward that walks once for all gradients: room for 2 bytes per evaluation beyond
  * ht_conv_workspace_bytes(p) (at most 8 GiB; the batch then goes in parts).  With less the kernels walk for themselves. */
 size_t ht_conv_backward_workspace_bytes(const ht_conv_problem *p);
+/* Which kernels a backward takes (real_bytes 4: ht_conv_backward_f32 with a workspace of ht_conv_workspace_bytes(p); 8: ht_conv_backward_f64):
+ * tiles, or one of two for any shape: gradients sorted by leaf and vertex before they meet memory, or scattered. */
+enum { HT_CONV_BACKWARD_SCATTERED = 0, HT_CONV_BACKWARD_SORTED = 1, HT_CONV_BACKWARD_TILES = 2 };
+int ht_conv_backward_kernel(const ht_conv_problem *p, int real_bytes);
 int ht_conv_forward_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
                         float *out, void *workspace, size_t workspace_bytes, uint32_t *status_word, ht_stream_t stream);
 int ht_conv_backward_f32(const ht_conv_problem *p, const float *x, const float *thr, const int64_t *ord, const float *w,
