@@ -110,3 +110,37 @@ def test_choice_on_forwards_that_the_estimates_were_not_fitted_to():
             better += min(times.values())
             assert times[takes] <= 1.15 * min(times.values()) or min(times.values()) < 100.0, row
     assert better > 0.0 and chosen <= 1.01 * better
+
+
+# sizes at which tiles are taken for trees and for ferns, with and without kept paths
+FORMS = [
+    (96, 9, (33,), 131, 5, 2),
+    (96, 9, (5, 6), 131, 2, 3),
+    (6, 9, (500,), 131, 1, 4),
+    (16, 9, (516,), 131, 9, 5),     # dealt out one by one
+    (6, 9, (515,), 131, 7, 6),      # ... in twos
+    (6, 9, (516,), 131, 3, 8),      # ... in fours
+    (256, 9, (45,), 131, 6, 10),    # rows that end inside a warp
+    (6, 9, (515,), 131, 10, 2),     # weights in global memory
+    (24, 9, (515,), 131, 12, 7),
+]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("kind", ["tree", "fern"])
+@pytest.mark.parametrize("shape", FORMS, ids=[str(s) for s in FORMS])
+def test_every_form_of_the_tiles(kind, shape):
+    B, C, inner, T, depth, M = shape
+    x, thr, ord_, w = random_forest_inputs(800 + FORMS.index(shape), kind, B, C, inner, T, depth, (M,), quantise=True)
+    dx, dthr, dord, dw = dev(x, thr, ord_, w)
+    assert taken(kind, dx, dw) == TILES and taken(kind, dx, dw, keep=True) == TILES
+    f = _cabi.Forest(kind, dx, dw)
+    want = ho.forward(kind, x, thr, ord_, w)
+    assert np.array_equal(f.forward(dx, dthr, dord, dw).cpu().numpy(), want)
+    assert np.array_equal(f.forward(dx, dthr, dord, dw, save=True).cpu().numpy(), want)
+    g = np.random.default_rng(5).standard_normal(want.shape).astype(np.float32)
+    dg, = dev(g)
+    for got, r, s in zip(f.backward(dx, dthr, dord, dw, dg, saved=True), ho.backward(kind, x, thr, ord_, w, g),
+                         ho.backward_magnitudes(kind, x, thr, ord_, w, g)):
+        assert grad_close(got, r, s)
+    assert f.ordinal_flags() == 0
