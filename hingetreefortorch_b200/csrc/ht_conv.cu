@@ -789,7 +789,7 @@ int evaluations_per_thread(const ConvShape &a) {
 // sizes in profiles/conv_backward_choice.csv, timed both ways in one session; on the 260 others, all calls together, the chosen kernels
 // take 1.013 (single precision; always sorted 1.013, always scattered 3.27) and 1.016 (double; 1.058, 2.83) of the better ones'
 // time, on those of the fit 1.006 (1.021, 3.15) and 1.003 (1.076, 2.25).  [35, 30, 7, 7, 7], 75 x 30 trees of depth 3, 2 x 2 x 2, padding 1:
-// sorted 982 us, scattered 695; in double precision [28, 11, 1466], 54 x 11 of depth 5: 790 and 494.
+// sorted 982 us, scattered 695; in double precision [24, 20, 1900], 72 x 20 of depth 5: 1983 and 1247.
 struct ConvBackwardRates {
   double sort, eval, level, output, piece, cta, cta_piece, cta_bin;
   double scatter, walk, line, reduction, tree_vertex, fern_vertex, leaf, chain_level, chain_output;

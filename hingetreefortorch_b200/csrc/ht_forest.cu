@@ -501,8 +501,8 @@ static bool rows_are_better(const ht_forest_problem *p, bool keep) {
 // that a walk meets, whose lanes are on as many cache lines as the level has vertices; so tiles are for many trees on few features.
 // Both estimates are fits to 788 of the 1050 forwards of random sizes in profiles/inner_forward_choice.csv, each timed both ways in one
 // session with the module's own parameters.  Time of the chosen kernels over that of the better ones, all calls together, on the 262
-// others: 1.006 (always tiles 1.225, never 1.568), none over 1.13; on those of the fit 1.003.  2796 x 284 x 169, 8 trees of
-// depth 4: tiles 520 us, threads 47; 228 x 47 x 576, 466 trees of depth 5: 208 and 673.
+// others: 1.006 (always tiles 1.225, never 1.568), none over 1.13; on those of the fit 1.003.  78 x 1394 x 1225, 411 trees of
+// depth 5, 2 outputs: tiles 766 us, threads 557; 228 x 47 x 576, 466 of depth 5, one output: 191 and 651.
 static bool inner_tiles_are_better(const ht_forest_problem *p, bool keep) {
   const double tiles = inner_tiled_cost(p, keep);
   if (tiles < 0.0) return false;
