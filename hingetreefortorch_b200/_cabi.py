@@ -28,7 +28,7 @@ SYMBOLS = [
     "ht_forest_static_scratch_bytes", "ht_forest_forward_static_f32",
     "ht_forest_fusion_workspace_bytes", "ht_forest_fusion_forward_f32", "ht_forest_fusion_backward_f32",
     "ht_forest_linear_workspace_bytes", "ht_forest_linear_forward_f32", "ht_forest_linear_backward_f32",
-    "ht_conv_output_size", "ht_conv_workspace_bytes", "ht_conv_backward_workspace_bytes", "ht_conv_forward_f32", "ht_conv_backward_f32",
+    "ht_conv_output_size", "ht_conv_workspace_bytes", "ht_conv_backward_kernel", "ht_conv_backward_workspace_bytes", "ht_conv_forward_f32", "ht_conv_backward_f32",
     "ht_conv_saved_bytes", "ht_conv_forward_saving_f32", "ht_conv_backward_saved_f32",
     "ht_contract", "ht_expand",
     "ht_trie_forward_f32", "ht_trie_backward_f32", "ht_forest_touched_f32", "ht_linear_tf32_stats_f32",
